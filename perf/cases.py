@@ -52,8 +52,8 @@ def listed():
         # circles and polygons in containers, stepped through pinned host memory by eight handles
         dict(name="balls_1024_io", kind="io", scene="balls", worlds=1024, bodies=128, sweeps=8, settle=90, handles=8),
         # one large world in a container: the order-preserving solve, then the coloured sweep
-        dict(name="pile_32771", kind="rollout", scene="pile", worlds=1, bodies=32771, sweeps=4, settle=80, steps=2),
-        dict(name="pile_65539_coloured", kind="rollout", scene="pile", worlds=1, bodies=65539, sweeps=4, settle=80,
+        dict(name="pile_32771", kind="rollout", scene="pile", worlds=1, bodies=32771, sweeps=4, settle=140, steps=2),
+        dict(name="pile_65539_coloured", kind="rollout", scene="pile", worlds=1, bodies=65539, sweeps=4, settle=140,
              steps=2, coloured=True),
         # contact queries only: the 65,536-polygon workload between moving frames, and a plugin's small world
         dict(name="field_65536", kind="collide", bodies=65536),
@@ -96,7 +96,7 @@ def draw(rng):
     elif scene == "balls":
         c.update(worlds=_log(rng, 2, 700), bodies=rng.randint(20, 160), settle=80, steps=rng.randint(1, 3))
     else:
-        c.update(worlds=1, bodies=_log(rng, 4200, 32771), sweeps=4, settle=60, steps=rng.randint(1, 2),
+        c.update(worlds=1, bodies=_log(rng, 4200, 32771), sweeps=4, settle=120, steps=rng.randint(1, 2),
                  coloured=rng.random() < 0.3)
     if kind == "io":
         c.update(handles=rng.choice([2, 4, 8]), worlds=max(c["worlds"], 16), steps=1, packed=False)
@@ -108,28 +108,34 @@ def draw(rng):
 
 
 def _pile(seed, n, sweeps):
-    """One container of n bodies, half again as high as it is wide: polygons of
-    3 to 8 vertices on a close grid, so that most touch within a few frames."""
+    """One container of n bodies, four times as wide as high, close enough that
+    most touch once the settling steps have run: boxes of nearly the grid's
+    pitch and, two in five, polygons of 3 to 8 vertices."""
     rng = np.random.default_rng(seed)
-    nb = n - 3
-    xy, nvs, area, inertia = scenes.polygons_arrays(rng, nb, 0.6, 1.0)
-    pitch = 1.9
-    cols = max(4, int(math.sqrt(nb / 1.5)))
-    width = cols * pitch + 1.0
+    nb, pitch = n - 3, 1.5
+    xy, nvs, area, inertia = scenes.polygons_arrays(rng, nb, 0.48 * pitch, 0.52 * pitch)
+    side, box = rng.uniform(0.93, 0.99, nb) * pitch, np.arange(nb) % 5 < 3
+    hulls = np.split(xy, np.cumsum(nvs)[:-1])
+    for k in np.flatnonzero(box):
+        hulls[k] = scenes.rectangle_vertices(side[k], side[k])
+    nvs = np.where(box, 4, nvs)
+    area, inertia = np.where(box, side ** 2, area), np.where(box, side ** 4 / 6.0, inertia)
+    cols = max(4, int(math.sqrt(4.0 * nb)))
+    width = cols * pitch + 0.5
     high = (nb // cols + 2) * pitch + 40.0
-    rects = [scenes.rectangle_vertices(width + 4.0, 2.0), scenes.rectangle_vertices(2.0, high),
+    walls = [scenes.rectangle_vertices(width + 4.0, 2.0), scenes.rectangle_vertices(2.0, high),
              scenes.rectangle_vertices(2.0, high)]
     f = {k: np.zeros(n) for k in _lib.BODY_FIELDS}
     k = np.arange(nb)
-    f["pos_x"][3:] = (k % cols - (cols - 1) / 2.0) * pitch + rng.uniform(-0.05, 0.05, nb)
-    f["pos_y"][3:] = (k // cols + 0.55) * pitch
-    f["rot"][3:] = rng.uniform(0.0, 2.0 * np.pi, nb)
+    f["pos_x"][3:] = (k % cols - (cols - 1) / 2.0) * pitch
+    f["pos_y"][3:] = (k // cols + 0.51) * pitch
+    f["rot"][3:] = np.where(box, rng.uniform(-0.02, 0.02, nb), rng.uniform(0.0, 2.0 * np.pi, nb))
     f["inv_mass_lin"][3:], f["inv_mass_rot"][3:] = 1.0 / area, 1.0 / inertia
     f["mu"][:] = scenes.DEFAULT_MU
     f["pos_y"][0] = -1.0
     f["pos_x"][1:3] = -(width / 2.0 + 1.0), width / 2.0 + 1.0
     f["pos_y"][1:3] = high / 2.0 - 2.0
-    return scenes.assemble([n], f, np.concatenate(rects + [xy]), np.concatenate([[4, 4, 4], nvs]), dt=1.0 / 120.0,
+    return scenes.assemble([n], f, np.concatenate(walls + hulls), np.concatenate([[4, 4, 4], nvs]), dt=1.0 / 120.0,
                            baumgarte=scenes.DEFAULT_BAUMGARTE, slop=scenes.DEFAULT_SLOP, accel=(0.0, -9.8),
                            iterations=sweeps, steps=1)
 
@@ -285,6 +291,8 @@ def prepare(case, seed):
         b.set_judge(np.full(n, 2.0), np.full(n, 1.0))
         cfg = _config(s, learned=True, residual=True)
         return dict(kind=kind, batch=b, net=net, cfg=cfg, start=b.get_bodies(), steps=case["steps"])
+    if case["scene"] == "pile":  # settles at twice the time step
+        plain.dt *= 2.0
     b.step(plain, case["settle"])
     return dict(kind=kind, batch=b, cfg=_config(s, coloured=bool(case.get("coloured"))), start=b.get_bodies(),
                 steps=case["steps"])
