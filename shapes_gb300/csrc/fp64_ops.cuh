@@ -12,59 +12,77 @@
 
 namespace shapes {
 
+/* The two words of a binary64.  Sign and magnitude are taken from them with
+ * 32-bit operations: the compiler turns `bits ^ sign` and `bits & ~sign` on the
+ * whole double back into a negation and an absolute value, which are FP64 pipe
+ * instructions unless another FP64 instruction takes them as a modifier
+ * (measured: 31 FP64 instructions an update instead of 20). */
+__device__ __forceinline__ uint32_t hi_word(double x) { return (uint32_t)__double2hiint(x); }
+__device__ __forceinline__ uint32_t lo_word(double x) { return (uint32_t)__double2loint(x); }
+__device__ __forceinline__ double from_words(uint32_t hi, uint32_t lo) { return __hiloint2double((int)hi, (int)lo); }
+
+/* -x */
+__device__ __forceinline__ double flip_sign(double x) { return from_words(hi_word(x) ^ 0x80000000u, lo_word(x)); }
+
+/* |x| as bits, and x as an integer of the same order (-0 and +0 both 0). */
+__device__ __forceinline__ uint64_t mag_bits(double x) {
+  return (uint64_t)(hi_word(x) & 0x7fffffffu) << 32 | lo_word(x);
+}
+__device__ __forceinline__ int64_t signed_key(double x) {
+  const int32_t neg = (int32_t)hi_word(x) >> 31;
+  const int64_t wide = (int64_t)neg;
+  return ((int64_t)mag_bits(x) ^ wide) - wide;
+}
+
 /* Order-preserving key of a binary64: for non-NaN a, b,
  * a < b  <=>  okey(a) < okey(b), and a == b <=> okey(a) == okey(b)
  * (-0 and +0 map to the same key). */
-__device__ __forceinline__ uint64_t okey(double d) {
-  uint64_t u = (uint64_t)__double_as_longlong(d);
-  if (u == 0x8000000000000000ull) u = 0;
-  return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
-}
+__device__ __forceinline__ uint64_t okey(double d) { return (uint64_t)signed_key(d) ^ 0x8000000000000000ull; }
 
-__device__ __forceinline__ bool nan_bits(double x) {
-  return ((uint64_t)__double_as_longlong(x) & 0x7fffffffffffffffull) > 0x7ff0000000000000ull;
-}
+__device__ __forceinline__ bool nan_bits(double x) { return mag_bits(x) > 0x7ff0000000000000ull; }
 
-/* a <= b and a < b as IEEE comparisons (false when either is NaN). */
-__device__ __forceinline__ bool f_le(double a, double b) {
-  return !nan_bits(a) && !nan_bits(b) && okey(a) <= okey(b);
+/* a <= b and a < b as IEEE comparisons (false when either is NaN), without
+ * branches: lanes of a warp that clamp differently stay together. */
+__device__ __forceinline__ bool no_nan(double a, double b) {
+  return (mag_bits(a) <= 0x7ff0000000000000ull) & (mag_bits(b) <= 0x7ff0000000000000ull);
 }
-__device__ __forceinline__ bool f_lt(double a, double b) {
-  return !nan_bits(a) && !nan_bits(b) && okey(a) < okey(b);
+__device__ __forceinline__ bool f_le(double a, double b) { return no_nan(a, b) & (signed_key(a) <= signed_key(b)); }
+__device__ __forceinline__ bool f_lt(double a, double b) { return no_nan(a, b) & (signed_key(a) < signed_key(b)); }
+
+/* x clamped to [-limit, limit] as SolutionProcessors.hs:44-53 spells it:
+ * limit where limit < x, else -limit where x < -limit, else x (NaN compares
+ * false). */
+__device__ __forceinline__ double clamp_abs(double x, double limit) {
+  const int64_t kx = signed_key(x), kl = signed_key(limit);
+  const bool ok = no_nan(x, limit);
+  const double low = ok & (kx < -kl) ? flip_sign(limit) : x;
+  return ok & (kl < kx) ? limit : low;
 }
 
 /* Finite (not infinite, not NaN). */
-__device__ __forceinline__ bool finite_bits(double x) {
-  return ((uint64_t)__double_as_longlong(x) & 0x7ff0000000000000ull) != 0x7ff0000000000000ull;
-}
+__device__ __forceinline__ bool finite_bits(double x) { return (hi_word(x) & 0x7ff00000u) != 0x7ff00000u; }
+
+__device__ __forceinline__ bool is_zero(double x) { return ((hi_word(x) << 1) | lo_word(x)) == 0; }
 
 /* 0.0 * x for finite x: a zero with x's sign. */
-__device__ __forceinline__ double signed_zero(double x) {
-  return __longlong_as_double(__double_as_longlong(x) & (long long)0x8000000000000000ull);
-}
+__device__ __forceinline__ double signed_zero(double x) { return from_words(hi_word(x) & 0x80000000u, 0); }
 
 /* x + z for finite x and a signed zero z: x unless x is a zero, and the sum
  * of two zeros is -0 only when both are -0 (round to nearest). */
 __device__ __forceinline__ double add_zero(double x, double z) {
-  const uint64_t ux = (uint64_t)__double_as_longlong(x);
-  if (ux & 0x7fffffffffffffffull) return x;
-  return __longlong_as_double((long long)(ux & (uint64_t)__double_as_longlong(z)));
+  return is_zero(x) ? from_words(hi_word(x) & hi_word(z), 0) : x;
 }
 
 /* x + 0.0: only -0 changes (to +0); NaN stays NaN. */
-__device__ __forceinline__ double plus_zero(double x) {
-  return __double_as_longlong(x) == (long long)0x8000000000000000ull ? 0.0 : x;
-}
+__device__ __forceinline__ double plus_zero(double x) { return is_zero(x) ? 0.0 : x; }
 
-__device__ __forceinline__ int exp_field(double x) {
-  return (int)(((uint64_t)__double_as_longlong(x) >> 52) & 0x7ff);
-}
+__device__ __forceinline__ int exp_field(double x) { return (int)((hi_word(x) >> 20) & 0x7ffu); }
 
 /* |x| < 2^500: finite and far from overflow. */
-__device__ __forceinline__ bool small_mag(double x) { return exp_field(x) < 1523; }
+__device__ __forceinline__ bool small_mag(double x) { return (hi_word(x) & 0x7fffffffu) < (1523u << 20); }
 
 /* |x| < 2. */
-__device__ __forceinline__ bool below_two(double x) { return exp_field(x) < 1024; }
+__device__ __forceinline__ bool below_two(double x) { return (hi_word(x) & 0x7fffffffu) < (1024u << 20); }
 
 /* 2^-500 <= |b| < 2^500: denominators whose reciprocal is used by div_rn. */
 __device__ __forceinline__ bool recip_ok(double b) {
@@ -80,20 +98,27 @@ __device__ __forceinline__ bool recip_ok(double b) {
  * RN(q + r y) is the correctly rounded quotient.  q0 = RN(a y) is within one
  * ulp of a/b.  The fast path is taken when a is a normal number with
  * 2^-400 <= |a| < 2^400, so nothing overflows or underflows (|q| stays
- * within 2^+-900 and |r| above 2^-460); zeros, NaN, infinities and extreme
- * magnitudes use the hardware division, and so does any b outside
- * recip_ok (signalled by y == 0).  Three dependent FP64 instructions
- * replace the division's longer sequence.  Explicit __fma_rn: the fused
+ * within 2^+-900 and |r| above 2^-460); a zero's quotient is a y, a zero of
+ * the right sign; NaN, infinities and extreme magnitudes use the hardware
+ * division, and so does any b outside recip_ok (signalled by y == 0), in a
+ * function of its own so that none of its instructions are issued ahead of the
+ * branch.  Three dependent FP64 instructions replace the division's longer
+ * sequence.  Explicit __fma_rn: the fused
  * operations here are part of this algorithm, not contractions of the
  * reference's expressions. */
+static __device__ __noinline__ double div_hw(double a, double b) { return a / b; }
+
 __device__ __forceinline__ double div_rn(double a, double b, double y) {
   const int ea = exp_field(a);
-  if (ea >= 623 && ea < 1423 && __double_as_longlong(y) != 0) {
+  const bool zero = is_zero(a);
+  if ((zero | ((ea >= 623) & (ea < 1423))) & !is_zero(y)) {
     const double q0 = __dmul_rn(a, y);
     const double r = __fma_rn(-q0, b, a);
-    return __fma_rn(r, y, q0);
+    const double q = __fma_rn(r, y, q0);
+    /* a zero's quotient is q0, a zero of the quotient's sign (q adds +0 to it) */
+    return zero ? q0 : q;
   }
-  return a / b;
+  return div_hw(a, b);
 }
 
 /* a * b in binary64, round to nearest even, computed on the integer pipe.
