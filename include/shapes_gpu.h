@@ -249,29 +249,28 @@ int shapes_batch_get_stats(shapes_batch* b, shapes_stats* out);
  * No counterpart in the reference. */
 int shapes_batch_get_world_metrics(shapes_batch* b, double* residual, double* max_depth);
 
-/* Solver packing.  Worlds are sorted by size and packed into groups, one warp
+/* Solver packing.  Worlds are sorted by size and packed into groups, one CTA
  * per group; target_bodies_per_group > 0 closes a group once it holds that many
- * bodies (0 = automatic: about one warp of updates per dependency level);
- * threads = warps per CTA x 32, at most 256 (0 = 32).  Results do not depend
- * on the packing. */
+ * bodies (0 = automatic: four groups per SM, at most 512 bodies each).  threads
+ * (a multiple of 32, at most 256; 0 = 32) is kept and reported; the warps of a
+ * group are shapes_batch_set_group_warps'.  Results do not depend on the
+ * packing. */
 int shapes_batch_set_launch(shapes_batch* b, int32_t target_bodies_per_group, int32_t threads);
-/* Same, with a fixed number of worlds per warp group (1..32), as chosen by
+/* Same, with a fixed number of worlds per group (1..32), as chosen by
  * shapes_batch_autotune. */
 int shapes_batch_set_launch_groups(shapes_batch* b, int32_t worlds_per_group, int32_t threads);
 
-/* Cooperative groups: 2, 4 or 8 warps share each group (one group per CTA;
- * the level's updates are spread over all of them, __syncthreads between
- * levels); 1 (default) = one warp per group, `threads` / 32 groups per CTA.
- * Results do not depend on it. */
+/* Solver warps of each group: 1, 2, 4 or 8 (one more warp of the group finds
+ * the dependency levels).  Until this is called the library chooses (and
+ * shapes_batch_get_launch reports 1): 8 when every group has an SM to itself,
+ * else 4.  Results do not depend on it. */
 int shapes_batch_set_group_warps(shapes_batch* b, int32_t warps);
-/* Cooperative groups compute the dependency levels of the updates in
- * parallel (default 1): one walk over each world's contacts records every
- * update's predecessors, then the passes are levelled chunk by chunk to a
- * fixed point; 0 walks over every update in order, one thread per world.
- * Both give every update the same level. */
+/* Kept for callers that choose between two ways of finding the dependency
+ * levels (default 1): there is one way now, the levels are found while they
+ * are solved, and the value is only reported back. */
 int shapes_batch_set_parallel_levels(shapes_batch* b, int32_t enabled);
 int shapes_batch_get_parallel_levels(shapes_batch* b, int32_t* enabled);
-/* Cooperative groups: launch the heaviest groups first, one per SM, then the
+/* Launch the heaviest groups first, one per SM, then the
  * others lightest first (default 0: heaviest first throughout), so a heavy
  * group shares its SM with light ones.  Results do not depend on it. */
 int shapes_batch_set_spread_heavy(shapes_batch* b, int32_t enabled);
@@ -294,8 +293,7 @@ int shapes_batch_get_world_levels(shapes_batch* b, int32_t* levels);
 
 /* Autotuner for the solver packing: from the current state, times
  * `steps_per_trial` steps for each candidate (worlds per group x warps per
- * CTA, and worlds per group x warps per cooperative group x parallel or
- * walked dependency levels, each in size and in level order) after one untimed
+ * group, each in size and in level order) after one untimed
  * step, restores the state exactly after every trial, and keeps the fastest (read it back with
  * shapes_batch_get_launch).  The world state and cache are left exactly as they were; results
  * never depend on the packing.  Tune on a state that has contacts (e.g. after
@@ -363,7 +361,8 @@ int shapes_batch_set_wait_limit(shapes_batch* b, int64_t polls);
 int shapes_batch_set_profiling(shapes_batch* b, int32_t enabled);
 int shapes_batch_get_profile(shapes_batch* b, double* ms, int64_t* launches);
 /* While profiling: per solver group of the last step, 8 int64 each
- * (clock at start, after the dependency scan, after the level sort, at end;
+ * (clock at start, when the updates' lists are built, when the last dependency
+ * level is found, at end;
  * dependency levels; updates; bodies; worlds).  *n_groups receives the group
  * count; `out` may be NULL to query it. */
 int shapes_batch_get_group_clocks(shapes_batch* b, int64_t* out, int32_t* n_groups);

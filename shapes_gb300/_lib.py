@@ -399,11 +399,11 @@ class Batch:
         return out
 
     def set_parallel_levels(self, enabled: bool) -> None:
-        """Cooperative groups: dependency levels in parallel (default) or by a walk over the updates."""
+        """Kept and reported only: the levels are found while they are solved."""
         check(lib().shapes_batch_set_parallel_levels(self._h, int(bool(enabled))), "shapes_batch_set_parallel_levels")
 
     def set_spread_heavy(self, enabled: bool) -> None:
-        """Cooperative groups: heaviest groups first, one per SM, then lightest first."""
+        """Heaviest groups first, one per SM, then lightest first."""
         check(lib().shapes_batch_set_spread_heavy(self._h, int(bool(enabled))), "shapes_batch_set_spread_heavy")
 
     def spread_heavy(self) -> bool:
@@ -412,7 +412,7 @@ class Batch:
         return bool(v.value)
 
     def set_group_warps(self, warps: int) -> None:
-        """Warps cooperating on each solver group (1, 2, 4 or 8)."""
+        """Solver warps of each group (1, 2, 4 or 8; chosen by the library until called)."""
         check(lib().shapes_batch_set_group_warps(self._h, warps), "shapes_batch_set_group_warps")
 
     def set_stream(self, cuda_stream: int | None) -> None:
@@ -436,7 +436,7 @@ class Batch:
             self.set_group_warps(group_warps)
 
     def group_clocks(self) -> np.ndarray:
-        """Per solver group of the last profiled step: [start, after scan, after sort, end,
+        """Per solver group of the last profiled step: [start, lists built, last level found, end,
         levels, updates, bodies, worlds] (clock64 units)."""
         g = ctypes.c_int32()
         check(lib().shapes_batch_get_group_clocks(self._h, None, ctypes.byref(g)), "shapes_batch_get_group_clocks")

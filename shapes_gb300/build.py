@@ -24,7 +24,7 @@ NVCC_FLAGS = [ARCH, "-O3", "-lineinfo", "-std=c++17", "-fmad=false", "--expt-rel
               "-Xcompiler", "-fPIC,-ffp-contract=off,-O2,-pthread", "-shared", "-lpthread"]
 
 SOURCES = [CSRC / "shapes_gpu.cu", CSRC / "mlp.cu"]
-HEADERS = [CSRC / "step_kernels.cuh", CSRC / "large_world.cuh", CSRC / "lw_order.cuh", CSRC / "learned.cuh",
+HEADERS = [CSRC / "step_kernels.cuh", CSRC / "frontier.cuh", CSRC / "large_world.cuh", CSRC / "lw_order.cuh", CSRC / "learned.cuh",
            CSRC / "fp64_ops.cuh", CSRC / "shapes_sincos.h", CSRC / "shapes_sincos_tables.h", CSRC / "mlp.h",
            CSRC / "tc05.cuh", HERE.parent / "include" / "shapes_gpu.h"]
 

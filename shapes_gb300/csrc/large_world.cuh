@@ -181,51 +181,23 @@ __global__ void k_lw_gravity(Dev d, LW w, double ax, double ay, double dt) {
   }
 }
 
-/* One update of a contact from its constants cp, the velocities v of its two
- * bodies (updated in place), the inverse masses m and its accumulated
- * Lagrangians lam2 (Solvers/Contact.hs:74-157; warm = the warm-start pass's
- * application of the cached impulses). */
-__device__ __forceinline__ void lw_contact_math(const double2* cp, double v[6], const double m[6], double2* lam2,
-                                                bool warm) {
-  double j_n[6], j_f[6];
-  const double2 a0 = cp[0], a1 = cp[1], a2 = cp[2], a3 = cp[3], a4 = cp[4], a5 = cp[5];
-  j_n[0] = a0.x; j_n[1] = a0.y; j_n[2] = a1.x; j_n[3] = a1.y; j_n[4] = a2.x; j_n[5] = a2.y;
-  j_f[0] = a3.x; j_f[1] = a3.y; j_f[2] = a4.x; j_f[3] = a4.y; j_f[4] = a5.x; j_f[5] = a5.y;
+/* One update of a contact from its record, the velocities v of its two bodies
+ * (updated in place) and its accumulated Lagrangians lam2
+ * (Solvers/Contact.hs:74-157; warm = the warm-start pass's application of the
+ * cached impulses). */
+__device__ __forceinline__ void lw_contact_math(const Con* con, double v[6], double2* lam2, bool warm) {
+  const double2* cp = reinterpret_cast<const double2*>(con);
+  const double2 n0 = cp[0], n1 = cp[1], f0 = cp[2], f1 = cp[3], ma = cp[7], mb = cp[8];
+  const double rn[4] = {n0.x, n0.y, n1.x, n1.y}, rf[4] = {f0.x, f0.y, f1.x, f1.y}, im[4] = {ma.x, ma.y, mb.x, mb.y};
   const double2 cached = __ldcg(lam2);
-  double ln_apply, lf_apply;
-  if (warm) {
-    ln_apply = cached.x;
-    lf_apply = cached.y;
-  } else {
-    const double2 b6 = cp[6], b9 = cp[9], b10 = cp[10], b11 = cp[11], b12 = cp[12];
-    const double cn = cached.x, cf = cached.y;
-    const uint64_t ebits = (uint64_t)__double_as_longlong(b11.y) & 0x7fffffffffffffffull;
-    const bool fastflag = __double_as_longlong(cp[13].x) != 0;
-    double bias;
-    if (ebits == 0 && fastflag && small_mag(v[0]) && small_mag(v[1]) && small_mag(v[2]) && small_mag(v[3]) &&
-        small_mag(v[4]) && small_mag(v[5])) {
-      bias = b6.y;
-    } else {
-      const double2 b7 = cp[7], b8 = cp[8];
-      const double nwa = -v[2];
-      const double cvx = ((-v[0] + (-(nwa * b7.y))) + v[3]) + (-(v[5] * b8.y));
-      const double cvy = ((-v[1] + nwa * b7.x) + v[4]) + v[5] * b8.x;
-      const double tb = b11.y * (cvx * b9.x + cvy * b9.y);
-      bias = b6.x + (f_le(0.0, tb) ? 0.0 : tb);
-    }
-    const double ln_new = div_rn(-(dot6(j_n, v) + bias), b10.x, b12.x);
-    const double lf_new = div_rn(-plus_zero(dot6(j_f, v)), b10.y, b12.y);
-    const double neg_cn = -cn;
-    ln_apply = f_le(ln_new, neg_cn) ? neg_cn : ln_new;
-    const double ln_cache = cn + ln_apply;
-    const double thr = ln_cache * b11.x;
-    const double acc = cf + lf_new;
-    const double acc2 = f_lt(thr, acc) ? thr : (f_lt(acc, -thr) ? -thr : acc);
-    lf_apply = acc2 - cf;
-    __stcg(lam2, make_double2(ln_cache, acc2));
+  double ln = cached.x, lf = cached.y;
+  if (!warm) {
+    double2 now;
+    contact_impulses(con, rn, rf, v, cached, &ln, &lf, &now);
+    __stcg(lam2, now);
   }
-  apply_impulse(j_n, ln_apply, v, m);
-  apply_impulse(j_f, lf_apply, v, m);
+  row_apply(rn, ln, v, im);
+  row_apply(rf, lf, v, im);
 }
 
 /* The update of contact c (global index), with the generic velocity store. */
@@ -236,10 +208,7 @@ __device__ __forceinline__ void lw_solve_item(const Dev& d, uint32_t item, const
   double v[6];
   vs.load(ga, 0, v[0], v[1], v[2]);
   vs.load(gb, 0, v[3], v[4], v[5]);
-  const double ima = __ldg(d.iml + ga), ira = __ldg(d.imr + ga), imb = __ldg(d.iml + gb), irb = __ldg(d.imr + gb);
-  const double m[6] = {ima, ima, ira, imb, imb, irb};
-  lw_contact_math(reinterpret_cast<const double2*>(d.con + c), v, m, reinterpret_cast<double2*>(d.lam) + c,
-                  (item & kWarmBit) != 0);
+  lw_contact_math(d.con + c, v, reinterpret_cast<double2*>(d.lam) + c, (item & kWarmBit) != 0);
   const uint8_t info = d.c_hit[c];
   if (info & kInfoDynA) vs.store(ga, 0, v[0], v[1], v[2]);
   if (info & kInfoDynB) vs.store(gb, 0, v[3], v[4], v[5]);
@@ -330,7 +299,7 @@ __global__ void __launch_bounds__(kOrderedThreads) k_lw_ordered(Dev d, LW w, int
   bool has = false, exhausted = total == 0, dyn_i = false;
   int stage = 0, pass = 0, k = 0, k1 = 0, m = 0, gi = 0, want_i = 0;
   int4 cur = make_int4(0, -1, 0, 0); /* side entry of contact k's second body */
-  double vi[3] = {0.0, 0.0, 0.0}, ima = 0.0, ira = 0.0;
+  double vi[3] = {0.0, 0.0, 0.0};
   long long polls = 0;
   int empty = 0;
   for (;;) {
@@ -363,8 +332,6 @@ __global__ void __launch_bounds__(kOrderedThreads) k_lw_ordered(Dev d, LW w, int
             gi = e0.x;
             dyn_i = e0.y >= 0;
             want_i = lw_want(e0, pass);
-            ima = __ldg(d.iml + gi);
-            ira = __ldg(d.imr + gi);
             cur = w.side[(k << 1) | 1];
           }
         }
@@ -391,10 +358,7 @@ __global__ void __launch_bounds__(kOrderedThreads) k_lw_ordered(Dev d, LW w, int
       const int4 nxt = kn < k1 ? w.side[(kn << 1) | 1] : cur;
       const int c = w.c0 + k, gb = cur.x;
       double v[6] = {vi[0], vi[1], vi[2], __ldcg(d.vx + gb), __ldcg(d.vy + gb), __ldcg(d.w + gb)};
-      const double imb = __ldg(d.iml + gb), irb = __ldg(d.imr + gb);
-      const double mm[6] = {ima, ima, ira, imb, imb, irb};
-      lw_contact_math(reinterpret_cast<const double2*>(d.con + c), v, mm, reinterpret_cast<double2*>(d.lam) + c,
-                      pass == 0);
+      lw_contact_math(d.con + c, v, reinterpret_cast<double2*>(d.lam) + c, pass == 0);
       if (dyn_i) {
         vi[0] = v[0];
         vi[1] = v[1];

@@ -45,13 +45,8 @@ __global__ void k_learned_features(Dev d, int external, double ax, double ay, do
     }
     const double g[6] = {acc_a ? ax * dt : 0.0, acc_a ? ay * dt : 0.0, 0.0,
                          acc_b ? ax * dt : 0.0, acc_b ? ay * dt : 0.0, 0.0};
-    double jn[6], jf[6];
-    for (int k = 0; k < 6; ++k) {
-      jn[k] = cc.jn[k];
-      jf[k] = cc.jf[k];
-    }
-    const double vn = dot6(jn, v), vf = dot6(jf, v), gn = dot6(jn, g);
-    const double mcn = cc.mcn, mcf = cc.mcf;
+    const double vn = row_dot(cc.row[0], v), vf = row_dot(cc.row[1], v), gn = row_dot(cc.row[0], g);
+    const double mcn = cc.mc[0], mcf = cc.mc[1];
     const bool okn = mcn > 0.0, okf = mcf > 0.0;
     int pair_n = 1;
     if (c > 0 && d.c_ga[c - 1] == ga && d.c_gb[c - 1] == gb) ++pair_n;
@@ -66,13 +61,13 @@ __global__ void k_learned_features(Dev d, int external, double ax, double ay, do
     f[mlp::kFL0f] = okf ? (float)(-vf / mcf) : 0.f;
     f[mlp::kFMu] = (float)cc.mu;
     f[mlp::kFDepth] = (float)d.c_val[5 * (size_t)c + 4];
-    f[mlp::kFNx] = (float)cc.rnx;
-    f[mlp::kFNy] = (float)cc.rny;
+    f[mlp::kFNx] = (float)cc.rn[0];
+    f[mlp::kFNy] = (float)cc.rn[1];
     f[mlp::kFGrav] = okn ? (float)(-gn / mcn) : 0.f;
     f[mlp::kFPairN] = (float)pair_n;
     f[mlp::kFStatic] = ((info & kInfoDynA) && (info & kInfoDynB)) ? 0.f : 1.f;
-    f[mlp::kFArmA] = (float)jn[2];
-    f[mlp::kFArmB] = (float)jn[5];
+    f[mlp::kFArmA] = (float)cc.row[0][2];
+    f[mlp::kFArmB] = (float)cc.row[0][3];
     float4* out = reinterpret_cast<float4*>(d.mfeat + (size_t)row * mlp::kIn);
     for (int k = 0; k < 4; ++k) out[k] = make_float4(f[4 * k], f[4 * k + 1], f[4 * k + 2], f[4 * k + 3]);
   }

@@ -27,6 +27,7 @@
 
 #include "../../include/shapes_gpu.h"
 #include "step_kernels.cuh"
+#include "frontier.cuh"
 #include "large_world.cuh"
 #include "learned.cuh"
 #include "mlp.h"
@@ -236,21 +237,15 @@ struct shapes_batch {
   double* c_val = nullptr;
   Con* con = nullptr;
   /* scheduler */
-  int32_t* last = nullptr;
-  int32_t* last_hit = nullptr; /* [N] scheduler scratch: last cache-hit contact of a body */
-  int4* c_pred = nullptr;      /* [contact_cap] previous contacts of each side (any / hit) */
-  int32_t* c_lvl = nullptr;    /* [2 * contact_cap] dependency levels of two consecutive passes */
-  uint32_t* items = nullptr;
-  int32_t* ilevel = nullptr;
-  uint32_t* isorted = nullptr;
-  int32_t* ihist = nullptr;
+  int4* sched_info = nullptr; /* lists of solver groups too large for shared memory (frontier.cuh) */
+  int32_t* sched_list = nullptr;
+  int32_t* sched_arr = nullptr;
+  int32_t* sched_body = nullptr;
+  uint32_t* sched_cur = nullptr;
   int4* gdesc = nullptr;
-  int4* idesc = nullptr;
-  int32_t* ghist = nullptr;
   long long* phase_clock = nullptr; /* [8 * G], allocated while profiling */
   int32_t phase_clock_groups = 0;
   int32_t* world_levels = nullptr;
-  int32_t* group_depth = nullptr;
   int32_t* group_world_off = nullptr;
   int32_t* group_worlds = nullptr;
   std::vector<int32_t> h_group_world_off;
@@ -284,9 +279,12 @@ struct shapes_batch {
   int32_t worlds_per_group_override = 0;
   int32_t target_group_bodies = 0;
   int32_t solve_threads = 32;
-  int32_t group_warps = 1; /* > 1: that many warps cooperate on each group (k_group_solve) */
-  bool parallel_levels = true; /* cooperative groups: dependency levels by chunked fixed point */
-  bool spread_heavy = false;   /* cooperative groups: heaviest groups first, one per SM, then lightest first */
+  int32_t group_warps = 1;       /* solver warps of each group, when the caller chose them */
+  bool group_warps_auto = true;  /* until then launch_groups chooses */
+  int32_t group_max_bodies = 0;  /* bodies of the largest group */
+  int32_t handles_in_flight = 1; /* handles whose steps share the GPU with this one's (shapes_batches_*) */
+  bool parallel_levels = true; /* kept for the caller, see shapes_batch_set_parallel_levels */
+  bool spread_heavy = false;   /* heaviest groups first, one per SM, then lightest first */
   int num_sms() {
     if (sm_count <= 0) {
       int dev = 0;
@@ -544,20 +542,14 @@ struct shapes_batch {
     d.old_cwo = cwo[1 - write_buf];
     d.world_pair_off = world_pair_off;
     d.world_contact_off = cwo[write_buf];
-    d.last = last;
-    d.last_hit = last_hit;
-    d.c_pred = c_pred;
-    d.c_lvl = c_lvl;
-    d.items = items;
-    d.ilevel = ilevel;
-    d.isorted = isorted;
-    d.ihist = ihist;
+    d.sched_info = sched_info;
+    d.sched_list = sched_list;
+    d.sched_arr = sched_arr;
+    d.sched_body = sched_body;
+    d.sched_cur = sched_cur;
     d.gdesc = gdesc;
-    d.idesc = idesc;
     d.phase_clock = profiling ? phase_clock : nullptr;
-    d.ghist = ghist;
     d.world_levels = world_levels;
-    d.group_depth = group_depth;
     d.group_world_off = group_world_off;
     d.group_worlds = group_worlds;
     d.counters = counters;
@@ -600,11 +592,9 @@ struct shapes_batch {
     np_perm = nullptr;
     for (int k = 0; k < 2; ++k) { dfree(c_key[k]); dfree(lam[k]); }
     dfree(c_ga); dfree(c_gb); dfree(c_slot); dfree(c_flip); dfree(c_hit); dfree(c_val); dfree(con);
-    dfree(c_pred); dfree(c_lvl);
-    c_pred = nullptr;
-    c_lvl = nullptr;
-    dfree(items); dfree(ilevel); dfree(isorted); dfree(ihist); dfree(gdesc); dfree(ghist); dfree(idesc);
-    idesc = nullptr;
+    dfree(sched_info); dfree(sched_list); dfree(sched_arr); dfree(gdesc);
+    sched_info = nullptr;
+    sched_list = sched_arr = nullptr;
     dfree(tile_sums);
     dfree(snap_key); dfree(snap_lam);
     free_row_buffers();
@@ -623,10 +613,7 @@ struct shapes_batch {
     c_flip = c_hit = nullptr;
     c_val = nullptr;
     con = nullptr;
-    items = isorted = nullptr;
-    ilevel = ihist = nullptr;
     gdesc = nullptr;
-    ghist = nullptr;
     tile_sums = nullptr;
     snap_key = nullptr;
     snap_lam = nullptr;
@@ -669,15 +656,10 @@ struct shapes_batch {
     c_hit = dalloc<uint8_t>(contact_cap, "cudaMalloc contacts");
     c_val = dalloc<double>(5 * (size_t)contact_cap, "cudaMalloc contacts");
     con = dalloc<Con>(contact_cap, "cudaMalloc constraints");
-    c_pred = dalloc<int4>(contact_cap, "cudaMalloc constraints");
-    c_lvl = dalloc<int32_t>(2 * (size_t)contact_cap, "cudaMalloc constraints");
-    items = dalloc<uint32_t>(1, "cudaMalloc items");
-    ilevel = dalloc<int32_t>(item_cap, "cudaMalloc items");
-    isorted = dalloc<uint32_t>(1, "cudaMalloc items");
-    ihist = dalloc<int32_t>(1, "cudaMalloc items");
+    sched_info = dalloc<int4>(contact_cap, "cudaMalloc constraints");
+    sched_list = dalloc<int32_t>(2 * (size_t)contact_cap, "cudaMalloc constraints");
+    sched_arr = dalloc<int32_t>(contact_cap, "cudaMalloc constraints");
     gdesc = dalloc<int4>(item_cap + W + 1, "cudaMalloc items");
-    ghist = dalloc<int32_t>(item_cap + W + 1, "cudaMalloc items");
-    idesc = dalloc<int4>(item_cap, "cudaMalloc items");
     tile_cap = scan_tiles_needed();
     tile_sums = dalloc<int32_t>(tile_cap, "cudaMalloc scan");
     if (!large_worlds.empty()) {
@@ -714,22 +696,17 @@ struct shapes_batch {
     if ((int64_t)(iterations + 1) * contact_cap <= item_cap) return;
     ck(cudaStreamSynchronize(stream), "sync");
     invalidate_graphs();
-    dfree(items); dfree(ilevel); dfree(isorted); dfree(ihist); dfree(gdesc); dfree(ghist); dfree(idesc);
+    dfree(gdesc);
     item_cap = (int64_t)(iterations + 1) * contact_cap;
-    items = dalloc<uint32_t>(item_cap, "cudaMalloc items");
-    ilevel = dalloc<int32_t>(item_cap, "cudaMalloc items");
-    isorted = dalloc<uint32_t>(1, "cudaMalloc items");
-    ihist = dalloc<int32_t>(1, "cudaMalloc items");
     gdesc = dalloc<int4>(item_cap + W + 1, "cudaMalloc items");
-    ghist = dalloc<int32_t>(item_cap + W + 1, "cudaMalloc items");
-    idesc = dalloc<int4>(item_cap, "cudaMalloc items");
   }
 
   /* Solver groups: worlds sorted by body count (largest first, so the longest
-   * dependency chains start first) and packed `per_group` at a time, so that a
-   * level of a group offers about one warp of updates (a world yields about
-   * iterations+1 updates per level).  target_group_bodies > 0 overrides the
-   * count with "worlds until this many bodies". */
+   * dependency chains start first) and packed by the caller's choice of
+   * worlds or bodies per group, else so that four groups fall to each SM but
+   * a group closes at kAutoGroupBodies bodies: small batches get one world a
+   * group, spread over the GPU, large ones groups whose levels fill warps. */
+  static constexpr int kAutoGroupBodies = 512;
   void make_groups(int iterations) {
     if (stream) ck(cudaStreamSynchronize(stream), "sync"); /* no kernel may still read the old groups */
     invalidate_graphs();
@@ -744,16 +721,21 @@ struct shapes_batch {
       std::stable_sort(order.begin(), order.end(), [&](int a, int b) {
         return (h_world_body_off[a + 1] - h_world_body_off[a]) > (h_world_body_off[b + 1] - h_world_body_off[b]);
       });
-    int per_group = std::max(1, std::min(shapes::kMaxGroupWorlds, 32 / (iterations + 1)));
-    if (worlds_per_group_override > 0) per_group = std::min(shapes::kMaxGroupWorlds, worlds_per_group_override);
+    const bool by_worlds = worlds_per_group_override > 0;
+    const int per_group = by_worlds ? std::min(shapes::kMaxGroupWorlds, worlds_per_group_override) : 0;
+    int32_t target = by_worlds ? 0 : target_group_bodies;
+    if (!by_worlds && target <= 0) {
+      int64_t total = 0;
+      for (int w : order) total += h_world_body_off[w + 1] - h_world_body_off[w];
+      target = (int32_t)std::max<int64_t>(1, std::min<int64_t>(kAutoGroupBodies, total / (4 * num_sms())));
+    }
     h_group_world_off.assign(1, 0);
     int32_t max_bodies = 0, bodies = 0, in_group = 0;
     for (int k = 0; k < n_small; ++k) {
       const int w = order[k];
       bodies += h_world_body_off[w + 1] - h_world_body_off[w];
       ++in_group;
-      const bool close = target_group_bodies > 0 ? (bodies >= target_group_bodies || in_group == shapes::kMaxGroupWorlds)
-                                                 : in_group == per_group;
+      const bool close = target > 0 ? (bodies >= target || in_group == shapes::kMaxGroupWorlds) : in_group == per_group;
       if (close || k == n_small - 1) {
         h_group_world_off.push_back(k + 1);
         max_bodies = std::max(max_bodies, bodies);
@@ -764,14 +746,10 @@ struct shapes_batch {
     h_group_worlds = order;
     dfree(group_world_off);
     dfree(group_worlds);
-    dfree(group_depth);
     const size_t G = h_group_world_off.size() - 1;
-    /* shared slice per warp (int32 units): last levels (1 per body) during the
-     * scan, then velocities (3 doubles = 6 per body) during the solve */
-    smem_last_cap = std::min<int32_t>(6 * max_bodies, 10240);
+    group_max_bodies = max_bodies;
     group_world_off = dalloc<int32_t>(G + 1, "cudaMalloc groups");
     group_worlds = dalloc<int32_t>(std::max(n_small, 1), "cudaMalloc groups");
-    group_depth = dalloc<int32_t>(std::max<size_t>(G, 1), "cudaMalloc groups");
     ck(cudaMemcpy(group_world_off, h_group_world_off.data(), sizeof(int32_t) * (G + 1), cudaMemcpyHostToDevice),
        "upload groups");
     if (n_small > 0)
@@ -839,6 +817,36 @@ struct shapes_batch {
     w.seq_list = lw_seq_list;
     w.ctl = lw_ctl + 8 * k;
     return w;
+  }
+
+  /* The group solve (frontier.cuh) of every group.  Each CTA's shared memory
+   * holds the largest group at two and a half contacts a body (five where it
+   * has the SM to itself), up to a third of an SM's where groups share one (a
+   * group that does not fit keeps its lists and velocities in global memory).
+   * Groups that have an SM to themselves take eight warps, of which four
+   * prepare a narrow level while four solve one; groups that share one take
+   * four. */
+  template <int P>
+  void launch_frontier(const Dev& d, const shapes_config& cfg, int smem, int split_limit) {
+    const int G = num_groups();
+    ck(cudaFuncSetAttribute(shapes::k_frontier<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFrontierSmem),
+       "cudaFuncSetAttribute");
+    shapes::k_frontier<P><<<G, 32 * (P + 1), smem, stream>>>(d, cfg.iterations, cfg.warm_start, cfg.external,
+                                                             cfg.accel_x, cfg.accel_y, cfg.dt, G, smem,
+                                                             spread_heavy ? num_sms() : 0, split_limit);
+  }
+  static constexpr int kFrontierSmem = 220 * 1024;
+  void launch_groups(const Dev& d, const shapes_config& cfg) {
+    const int per_sm = (int)(((int64_t)num_groups() * handles_in_flight + num_sms() - 1) / num_sms());
+    const int P = !group_warps_auto ? group_warps : (per_sm <= 1 ? 8 : 4);
+    const int64_t contacts = (per_sm <= 1 ? 10LL : 5LL) * group_max_bodies / 2;
+    const size_t want = shapes::frontier_bytes(group_max_bodies, contacts, true);
+    const int smem = (int)std::min<size_t>(want, kFrontierSmem / std::min(per_sm, 3));
+    const int split_limit = per_sm <= 1 ? 16 : 4;
+    if (P == 1) launch_frontier<1>(d, cfg, smem, split_limit);
+    else if (P == 2) launch_frontier<2>(d, cfg, smem, split_limit);
+    else if (P == 4) launch_frontier<4>(d, cfg, smem, split_limit);
+    else launch_frontier<8>(d, cfg, smem, split_limit);
   }
 
   /* Solve one large world: ranks of every contact on its bodies, then the
@@ -1003,7 +1011,6 @@ struct shapes_batch {
     setup_incremental();
     setup_sap();
   }
-  int32_t smem_last_cap = 0; /* bodies whose last level fits the solver's shared memory */
 
   void scan(const int32_t* in, int n_cap, const unsigned long long* n_dev, int32_t* out) {
     stage(6, 3, [&]() { scan_raw(in, n_cap, n_dev, out); });
@@ -1041,6 +1048,7 @@ struct shapes_batch {
      * levels add up over the call */
     ck(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * 2, stream), "memset");
     ck(cudaMemsetAsync(counters + shapes::kCntGroupAlloc, 0, sizeof(unsigned long long), stream), "memset");
+    ck(cudaMemsetAsync(counters + shapes::kCntListAlloc, 0, sizeof(unsigned long long), stream), "memset");
     const bool inc = any_grid && d.nbr != nullptr;
     const bool sap = any_sap && !inc;
     if (!sap) d.world_sap = nullptr;
@@ -1117,7 +1125,7 @@ struct shapes_batch {
     stage(6, 1, [&]() { shapes::k_world_contact_offsets<<<grid_for(W + 1, 128), 128, 0, stream>>>(d); });
     stage(2, 2, [&]() {
       shapes::k_contact_slots<<<grid_for(2LL * pair_cap, 256), 256, 0, stream>>>(d);
-      shapes::k_build<<<grid_for(contact_cap, 128), 128, 0, stream>>>(d, cfg.dt, cfg.baumgarte, cfg.slop,
+      shapes::k_build<<<grid_for(contact_cap, 128), 128, 0, stream>>>(d, cfg.baumgarte / cfg.dt, cfg.slop,
                                                                       cfg.warm_start, solve ? 1 : 0);
     });
     if (!solve) return;
@@ -1136,37 +1144,8 @@ struct shapes_batch {
         }
       });
     }
-    const int G = num_groups(); /* groups for cfg.iterations were built by run() before this view */
-    const int wpc = solve_threads / 32;
-    /* each warp's slice of last levels: 40 KB of dynamic shared memory in all (static use is ~1 KB) */
-    const int per_warp = std::min<int>(smem_last_cap, (40 * 1024 / (int)sizeof(int32_t)) / wpc) & ~1;
-    if (G > 0 && group_warps > 1) {
-      /* one group per CTA of group_warps warps, the group's slice up to 40 KB */
-      const int ints = std::min<int>(smem_last_cap, 40 * 1024 / (int)sizeof(int32_t)) & ~1;
-      const size_t bytes = (size_t)ints * sizeof(int32_t);
-      stage(4, 1, [&]() {
-#define SHAPES_GROUP_SOLVE(PW, PL)                                                                              \
-  shapes::k_group_solve<PW, PL><<<G, 32 * PW, bytes, stream>>>(d, cfg.iterations, cfg.warm_start, cfg.external, \
-                                                               cfg.accel_x, cfg.accel_y, cfg.dt, G, ints,  \
-                                                               spread_heavy ? num_sms() : 0)
-        if (parallel_levels) {
-          if (group_warps == 2) SHAPES_GROUP_SOLVE(2, true);
-          else if (group_warps == 4) SHAPES_GROUP_SOLVE(4, true);
-          else SHAPES_GROUP_SOLVE(8, true);
-        } else {
-          if (group_warps == 2) SHAPES_GROUP_SOLVE(2, false);
-          else if (group_warps == 4) SHAPES_GROUP_SOLVE(4, false);
-          else SHAPES_GROUP_SOLVE(8, false);
-        }
-#undef SHAPES_GROUP_SOLVE
-      });
-    } else if (G > 0) {
-      stage(4, 1, [&]() {
-        shapes::k_schedule_solve<<<(G + wpc - 1) / wpc, solve_threads, (size_t)wpc * per_warp * sizeof(int32_t),
-                                   stream>>>(d, cfg.iterations, cfg.warm_start, cfg.external, cfg.accel_x,
-                                             cfg.accel_y, cfg.dt, G, per_warp);
-      });
-    }
+    /* groups for cfg.iterations were built by run() before this view */
+    if (num_groups() > 0) stage(4, 1, [&]() { launch_groups(d, cfg); });
     for (size_t k = 0; k < large_worlds.size(); ++k) solve_large_world(d, k, cfg);
     if ((cfg.flags & SHAPES_FLAG_RESIDUAL) || (learn && judge_set))
       stage(4, 1 + 2 * (int)large_worlds.size(), [&]() { world_metric_kernels(d, true); });
@@ -1258,7 +1237,11 @@ struct shapes_batch {
    * back is an asynchronous copy and the wait happens where the caller waits */
   unsigned long long* run_counters = nullptr;
 
-  void prepare(const shapes_config& cfg, bool solve) {
+  void prepare(const shapes_config& cfg, bool solve, int handles = 1) {
+    if (handles != handles_in_flight) { /* the launch shape of the group solve follows it */
+      handles_in_flight = handles;
+      invalidate_graphs();
+    }
     ensure_items(solve ? cfg.iterations : 0);
     /* (re)build the solver groups before any device view of this call is
      * taken: make_groups reallocates the group arrays */
@@ -1305,6 +1288,10 @@ struct shapes_batch {
     const unsigned long long* agg = run_counters;
     if (agg[shapes::kCntMlpErr]) {
       g_last_error = "learned warm start: a bounded tensor-core wait gave up";
+      return SHAPES_E_TIMEOUT;
+    }
+    if (agg[shapes::kCntSolveErr]) {
+      g_last_error = "group solver: a bounded wait gave up";
       return SHAPES_E_TIMEOUT;
     }
     if (!agg[shapes::kCntOverflow] && solve && !large_worlds.empty()) {
@@ -1399,7 +1386,7 @@ struct shapes_batch {
     }
     dfree(wx); dfree(wy); dfree(nx); dfree(ny); dfree(box); dfree(boxk); dfree(flags); dfree(body_changed);
     dfree(plo); dfree(phi);
-    dfree(row_cnt); dfree(row_off); dfree(world_pair_off); dfree(last); dfree(last_hit); dfree(world_levels);
+    dfree(row_cnt); dfree(row_off); dfree(world_pair_off); dfree(sched_body); dfree(sched_cur); dfree(world_levels);
     for (int k = 0; k < 6; ++k) dfree(snap_body[k]);
     dfree(active);
     active = nullptr;
@@ -1436,8 +1423,8 @@ struct shapes_batch {
     world_pair_off = dalloc<int32_t>(n_worlds + 1, "cudaMalloc");
     if (!cwo[0])
       for (int k = 0; k < 2; ++k) cwo[k] = dalloc<int32_t>(n_worlds + 1, "cudaMalloc");
-    last = dalloc<int32_t>(N, "cudaMalloc");
-    last_hit = dalloc<int32_t>(N, "cudaMalloc");
+    sched_body = dalloc<int32_t>(4 * (size_t)N, "cudaMalloc");
+    sched_cur = dalloc<uint32_t>(N, "cudaMalloc");
     world_levels = dalloc<int32_t>(n_worlds, "cudaMalloc");
     ck(cudaMemset(world_levels, 0, sizeof(int32_t) * n_worlds), "memset");
     if (!counters) counters = dalloc<unsigned long long>(shapes::kCntSlots, "cudaMalloc");
@@ -1555,7 +1542,7 @@ struct shapes_batch {
     dfree(radius);
     dfree(metric_part);
     for (int k = 0; k < 2; ++k) dfree(cwo[k]);
-    dfree(last); dfree(last_hit); dfree(world_levels); dfree(group_depth); dfree(group_world_off); dfree(group_worlds);
+    dfree(sched_body); dfree(sched_cur); dfree(world_levels); dfree(group_world_off); dfree(group_worlds);
     dfree(phase_clock);
     dfree(counters);
     dfree(np_cls);
@@ -1755,7 +1742,7 @@ int shapes_batches_step(shapes_batch* const* bs, int32_t n, const shapes_config*
      * each finished */
     for (int32_t k = 0; k < n; ++k) {
       ck(cudaSetDevice(bs[k]->device), "cudaSetDevice");
-      bs[k]->prepare(*cfg, true);
+      bs[k]->prepare(*cfg, true, n);
       bs[k]->run_retries = 0;
       bs[k]->enqueue_begin(true);
     }
@@ -1791,7 +1778,7 @@ int shapes_batches_step_io(shapes_batch* const* bs, int32_t n, const shapes_conf
     for (int32_t k = 0; k < n; ++k) {
       shapes_batch* b = bs[k];
       ck(cudaSetDevice(b->device), "cudaSetDevice");
-      b->prepare(*cfg, true);
+      b->prepare(*cfg, true, n);
       b->run_retries = 0;
       b->enqueue_begin(true); /* zeroes the counters and keeps the state a refusal returns to */
       b->io_upload(&in[k]);
@@ -1836,7 +1823,7 @@ int shapes_batches_run_io(shapes_batch* const* bs, int32_t n, const shapes_confi
       const bool is_mapped = mapped_host10(bp, mapped); /* resolved once for the whole run */
       double* const* mp = is_mapped ? mapped : nullptr;
       for (int32_t s = 0; s < nsteps; ++s) {
-        b->prepare(*cfg, true);
+        b->prepare(*cfg, true, n);
         b->run_retries = 0;
         b->enqueue_begin(true);
         b->io_upload(&state[k], mp);
@@ -2331,26 +2318,22 @@ int shapes_batch_autotune(shapes_batch* b, const shapes_config* cfg, int32_t ste
       if (lv[a] != lv[c]) return lv[a] > lv[c];
       return (b->h_world_body_off[a + 1] - b->h_world_body_off[a]) > (b->h_world_body_off[c + 1] - b->h_world_body_off[c]);
     });
-    /* (worlds per group, threads per CTA, warps per group, level order,
-     * parallel levels, heavy groups spread, target bodies per group: when
-     * non-zero, groups close at that many bodies instead of at a world
-     * count, so the largest worlds of a ragged batch get groups of their own) */
-    std::vector<std::array<int, 7>> cands;
-    auto add = [&](int wpg, int thr, int gw, int lo, int par, int spread = 0, int target = 0) {
-      const std::array<int, 7> c{wpg, thr, gw, lo, par, spread, target};
+    /* (worlds per group, warps per group, level order, heavy groups spread,
+     * target bodies per group: when non-zero, groups close at that many bodies
+     * instead of at a world count, so the largest worlds of a ragged batch get
+     * groups of their own) */
+    std::vector<std::array<int, 5>> cands;
+    auto add = [&](int wpg, int gw, int lo, int spread = 0, int target = 0) {
+      const std::array<int, 5> c{wpg, gw, lo, spread, target};
       if (wpg >= 1 && wpg <= shapes::kMaxGroupWorlds && std::find(cands.begin(), cands.end(), c) == cands.end())
         cands.push_back(c);
     };
-    for (int lo : {0, 1}) {
-      for (int wpg : {1, base / 2, base, base + 1, 2 * base})
-        for (int thr : {32, 64, 128}) add(std::min(wpg, W), thr, 1, lo, 0);
+    for (int lo : {0, 1})
       for (int wpg : {1, 2, base, base + 1, 2 * base, 3 * base, 4 * base})
-        for (int gw : {2, 4, 8})
-          for (int par : {0, 1}) {
-            add(std::min(wpg, W), 32 * gw, gw, lo, par);
-            if (par) add(std::min(wpg, W), 32 * gw, gw, lo, par, 1);
-          }
-    }
+        for (int gw : {1, 2, 4, 8}) {
+          add(std::min(wpg, W), gw, lo);
+          if (gw > 1) add(std::min(wpg, W), gw, lo, 1);
+        }
     int32_t min_n = INT32_MAX, max_n = 0;
     for (int w = 0; w < W; ++w) {
       const int32_t n = b->h_world_body_off[w + 1] - b->h_world_body_off[w];
@@ -2360,26 +2343,28 @@ int shapes_batch_autotune(shapes_batch* b, const shapes_config* cfg, int32_t ste
     }
     if (max_n > 2 * min_n) /* ragged batches: packings by body count */
       for (int target : {256, 512, 1024, 2048})
-        for (int gw : {2, 4, 8})
-          for (int par : {0, 1}) add(1, 32 * gw, gw, 0, par, 1, target);
+        for (int gw : {2, 4, 8}) add(1, gw, 0, 1, target);
     cudaEvent_t e0, e1;
     ck(cudaEventCreate(&e0), "event");
     ck(cudaEventCreate(&e1), "event");
     float best = 1e30f;
-    const bool par0 = b->parallel_levels, spread0 = b->spread_heavy;
-    std::array<int, 7> best_c{wpg0, thr0, gw0, -1, par0 ? 1 : 0, spread0 ? 1 : 0, tgt0};
+    const bool auto0 = b->group_warps_auto, spread0 = b->spread_heavy;
+    std::array<int, 5> best_c{wpg0, gw0, -1, spread0 ? 1 : 0, tgt0};
+    auto apply = [&](const std::array<int, 5>& c) {
+      b->worlds_per_group_override = c[4] ? 0 : c[0];
+      b->target_group_bodies = c[4];
+      b->solve_threads = 32 * c[1];
+      b->group_warps = c[1];
+      b->group_warps_auto = false;
+      b->spread_heavy = c[3] != 0;
+      if (c[2]) b->world_order = by_levels; else b->world_order.clear();
+    };
     int rc = rc0;
     if (rc0 != SHAPES_OK) cands.clear();
     for (const auto& c : cands) {
       restore_state();
-      b->worlds_per_group_override = c[6] ? 0 : c[0];
-      b->target_group_bodies = c[6];
-      b->solve_threads = c[1];
-      b->group_warps = c[2];
-      b->parallel_levels = c[4] != 0;
-      b->spread_heavy = c[5] != 0;
+      apply(c);
       b->invalidate_graphs();
-      if (c[3]) b->world_order = by_levels; else b->world_order.clear();
       b->make_groups(cfg->iterations);
       rc = b->run(*cfg, 1, true); /* untimed: captures this packing's step graphs */
       if (rc != SHAPES_OK) break;
@@ -2398,20 +2383,14 @@ int shapes_batch_autotune(shapes_batch* b, const shapes_config* cfg, int32_t ste
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     restore_state();
-    if (rc == SHAPES_OK && best_c[3] >= 0) {
-      b->worlds_per_group_override = best_c[6] ? 0 : best_c[0];
-      b->target_group_bodies = best_c[6];
-      b->solve_threads = best_c[1];
-      b->group_warps = best_c[2];
-      b->parallel_levels = best_c[4] != 0;
-      b->spread_heavy = best_c[5] != 0;
-      if (best_c[3]) b->world_order = by_levels; else b->world_order.clear();
+    if (rc == SHAPES_OK && best_c[2] >= 0) {
+      apply(best_c);
     } else {
       b->worlds_per_group_override = wpg0;
       b->target_group_bodies = tgt0;
       b->solve_threads = thr0;
       b->group_warps = gw0;
-      b->parallel_levels = par0;
+      b->group_warps_auto = auto0;
       b->spread_heavy = spread0;
       b->world_order = order0;
     }
@@ -2980,6 +2959,7 @@ int shapes_batch_set_group_warps(shapes_batch* b, int32_t warps) {
   return guarded([&]() -> int {
     ck(cudaStreamSynchronize(b->stream), "sync");
     b->group_warps = warps;
+    b->group_warps_auto = false;
     b->invalidate_graphs();
     return SHAPES_OK;
   });
@@ -3384,7 +3364,7 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   shapes::k_narrowphase<<<grid_for(kNaMaxPairs, 128), 128, 0, st>>>(d);
   scan(d.slot_cnt, kNaMaxPairs, d.counters + shapes::kCntPairs, d.slot_off);
   shapes::k_world_contact_offsets<<<1, 32, 0, st>>>(d);
-  shapes::k_build<<<grid_for(2LL * kNaMaxPairs, 128), 128, 0, st>>>(d, 1.0, 0.0, 0.0, 0, 0);
+  shapes::k_build<<<grid_for(2LL * kNaMaxPairs, 128), 128, 0, st>>>(d, 0.0, 0.0, 0, 0);
   e = cudaMemcpyAsync(cnt, d.counters, sizeof(cnt), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = cudaGetLastError();

@@ -35,17 +35,26 @@ constexpr uint8_t kInfoDynB = 4;
  * effective-mass denominators (effMassM2, Constraint.hs:173-179), pairMu
  * (Friction.hs:46-48) and min bounciness (Restitution.hs:51). */
 struct __align__(16) Con {
-  double jn[6];
-  double jf[6];
-  double bn, bn0; /* baumgarte term, and bn + 0.0 */
-  double rax, ray, rbx, rby, rnx, rny;
-  double mcn, mcf; /* effective-mass denominators */
-  double mu;
+  /* normal and friction row, {x, y, angular of a, angular of b}: the Jacobian
+   * row is (-x, -y, angular of a, x, y, angular of b), because the normal and the
+   * tangent enter the two bodies with opposite signs and a Flip only swaps the
+   * halves */
+  double row[2][4];
+  double mc[2];       /* effective-mass denominators */
+  double rc[2];       /* RN(1 / mc) for div_rn, or 0 when out of its range */
+  double mu, bn0;     /* bn0 = bn + 0.0 */
+  double im[4];       /* inverse masses: linear and rotational of a, then of b */
+  int32_t no_bounce;  /* 1 when e is a zero, both radii are below 2^500 and the normal below 2: the bounce term is +0
+                         for velocities below 2^500 */
+  int32_t pad;
+  double bn;          /* baumgarte term */
+  /* a solver needs the 160 bytes above, two 128-byte lines wherever the record starts */
   double e;
-  double rcn, rcf; /* RN(1/mcn), RN(1/mcf) for div_rn, or 0 when out of its range */
-  double fast;     /* 1 when both radii are below 2^500 and the normal below 2 (exact zero-bounce path) */
-  double pad;
+  double ra[4];       /* contact point from a's and from b's position */
+  double rn[2];
 };
+static_assert(sizeof(Con) == 224, "records start on 32-byte sectors");
+constexpr int kConHot = 160;
 
 /* Device view of a batch; passed by value to every kernel. */
 struct Dev {
@@ -143,20 +152,14 @@ struct Dev {
   const int32_t* old_cwo;  /* [W+1] previous cache world offsets */
   int32_t* world_pair_off;    /* [W+1] */
   int32_t* world_contact_off; /* [W+1] */
-  int32_t* last;              /* [N] scheduler scratch */
-  int32_t* last_hit;          /* [N] scheduler scratch: last cache-hit contact of each body */
-  int4* c_pred;               /* [contact_cap] per contact: previous contact touching side a, side b; previous hit contact of a, b (-1: none) */
-  int32_t* c_lvl;             /* [2 * contact_cap] levels of the current and the previous pass */
-  uint32_t* items;            /* [item_cap] */
-  int32_t* ilevel;            /* [item_cap] */
-  uint32_t* isorted;          /* [item_cap] */
-  int32_t* ihist;             /* [item_cap] (unused by the warp-group solver) */
-  int4* gdesc;                /* [item_cap + W + 1] per-group updates sorted by level: {id, a, b, info | world << 8} */
-  int4* idesc;                /* [item_cap] the same descriptors in sequential order, per world region */
+  int4* sched_info;           /* [contact_cap] lists of groups too large for shared memory (frontier.cuh) */
+  int32_t* sched_list;        /* [2 * contact_cap] */
+  int32_t* sched_arr;         /* [contact_cap] */
+  int32_t* sched_body;        /* [4 * N] */
+  uint32_t* sched_cur;        /* [N] */
+  int4* gdesc;                /* [item_cap + W + 1] per-group updates, level by level: {contact and warm bit, slots, flags} */
   long long* phase_clock;     /* [G * 8] per-group phase clocks when profiling, else null */
-  int32_t* ghist;             /* [item_cap + W + 1] per-group level ends */
   int32_t* world_levels;      /* [W] dependency levels of each small world's last solve */
-  int32_t* group_depth;       /* [G] */
   const int32_t* group_world_off; /* [G+1] offsets into group_worlds */
   const int32_t* group_worlds;    /* [W] world ids, grouped */
   unsigned long long* counters;   /* [kCntSlots] see kCnt* */
@@ -188,6 +191,8 @@ enum {
   kCntPredicted = 8,  /* contacts started from the network (summed over the call) */
   kCntReverted = 9,   /* worlds the judge switched back to the plain start */
   kCntMlpErr = 10,    /* set when a tensor-core wait of the network gave up */
+  kCntListAlloc = 11, /* bump allocator of the lists kept in global memory (reset every step) */
+  kCntSolveErr = 12,  /* set when a wait between a solver group's warps gave up */
   kCntSlots = 16,
 };
 
@@ -1820,10 +1825,6 @@ __global__ void k_narrowphase_lanes(Dev d) {
 /* A8-A9 constraint build + warm-start lookup                                 */
 /* ------------------------------------------------------------------------ */
 
-__device__ __forceinline__ double cross2(double ax, double ay, double bx, double by) {
-  return ax * by - ay * bx;
-}
-
 /* world_contact_off[w] = slot_off[world_pair_off[w]]; totals + overflow. */
 __global__ void k_world_contact_offsets(Dev d) {
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w <= d.n_worlds; w += gridDim.x * blockDim.x) {
@@ -1859,7 +1860,7 @@ __global__ void k_contact_slots(Dev d) {
   }
 }
 
-__global__ void k_build(Dev d, double dt, double beta, double slop, int warm_start, int build_solver) {
+__global__ void k_build(Dev d, double beta_dt, double slop, int warm_start, int build_solver) {
   const int P = min((int)d.counters[kCntPairs], d.pair_cap);
   const int C = (int)d.counters[kCntContacts];
   if (C > d.contact_cap) return;
@@ -1893,58 +1894,50 @@ __global__ void k_build(Dev d, double dt, double beta, double slop, int warm_sta
     cv[4] = depth;
     if (!build_solver) continue;
     /* constraintGen: positions of (a, b) = (i, j); a Flip contact is built
-     * with the bodies swapped, then its Jacobian halves are swapped back. */
-    const double xi = d.px[ga], yi = d.py[ga], xj = d.px[gb], yj = d.py[gb];
-    const double xa = flip ? xj : xi, ya = flip ? yj : yi;
-    const double xb = flip ? xi : xj, yb = flip ? yi : yj;
-    double jn[6], jf[6];
-    jn[0] = -nx;
-    jn[1] = -ny;
-    jn[2] = cross2(xa - px, ya - py, nx, ny);
-    jn[3] = nx;
-    jn[4] = ny;
-    jn[5] = cross2(px - xb, py - yb, nx, ny);
-    const double tbx = ny, tby = -nx;
-    const double tax = -tbx, tay = -tby;
-    jf[0] = tax;
-    jf[1] = tay;
-    jf[2] = cross2(px - xa, py - ya, tax, tay);
-    jf[3] = tbx;
-    jf[4] = tby;
-    jf[5] = cross2(px - xb, py - yb, tbx, tby);
+     * with the bodies swapped, then its Jacobian halves are swapped back.  The
+     * differences and products that the two rows, the restitution radii and the
+     * effective masses share up to sign are computed once: (-p) * q is -(p * q)
+     * and p - q is -(q - p) exactly, and the rows' linear parts are each other's
+     * swapped, so (x m) x and (y m) y serve both folds. */
     Con cc;
-    for (int k = 0; k < 3; ++k) {
-      cc.jn[k] = flip ? jn[k + 3] : jn[k];
-      cc.jn[k + 3] = flip ? jn[k] : jn[k + 3];
-      cc.jf[k] = flip ? jf[k + 3] : jf[k];
-      cc.jf[k + 3] = flip ? jf[k] : jf[k + 3];
-    }
-    cc.bn = depth > slop ? (beta / dt) * (slop - depth) : 0.0;
-    cc.bn0 = cc.bn + 0.0;
-    cc.rax = px - xi;
-    cc.ray = py - yi;
-    cc.rbx = px - xj;
-    cc.rby = py - yj;
-    cc.rnx = flip ? -nx : nx;
-    cc.rny = flip ? -ny : ny;
+    cc.ra[0] = px - d.px[ga];
+    cc.ra[1] = py - d.py[ga];
+    cc.ra[2] = px - d.px[gb];
+    cc.ra[3] = py - d.py[gb];
+    const double dxa = flip ? cc.ra[2] : cc.ra[0], dya = flip ? cc.ra[3] : cc.ra[1];
+    const double dxb = flip ? cc.ra[0] : cc.ra[2], dyb = flip ? cc.ra[1] : cc.ra[3];
+    const double na = dya * nx - dxa * ny, nb = dxb * ny - dyb * nx;       /* cross2 of the arms and the normal */
+    const double fa_ = dxa * nx + dya * ny, fb_ = -(dxb * nx) - dyb * ny; /* and the tangent (ny, -nx) */
+    cc.row[0][0] = flip ? flip_sign(nx) : nx;
+    cc.row[0][1] = flip ? flip_sign(ny) : ny;
+    cc.row[0][2] = flip ? nb : na;
+    cc.row[0][3] = flip ? na : nb;
+    cc.row[1][0] = cc.row[0][1];
+    cc.row[1][1] = flip_sign(cc.row[0][0]);
+    cc.row[1][2] = flip ? fb_ : fa_;
+    cc.row[1][3] = flip ? fa_ : fb_;
+    cc.bn = f_lt(slop, depth) ? beta_dt * (slop - depth) : 0.0;
+    cc.bn0 = plus_zero(cc.bn);
+    cc.rn[0] = flip ? flip_sign(nx) : nx;
+    cc.rn[1] = flip ? flip_sign(ny) : ny;
     const double ima = d.iml[ga], ira = d.imr[ga], imb = d.iml[gb], irb = d.imr[gb];
-    const double m[6] = {ima, ima, ira, imb, imb, irb};
-    double mcn = (cc.jn[0] * m[0]) * cc.jn[0];
-    double mcf = (cc.jf[0] * m[0]) * cc.jf[0];
-    for (int k = 1; k < 6; ++k) {
-      mcn = mcn + (cc.jn[k] * m[k]) * cc.jn[k];
-      mcf = mcf + (cc.jf[k] * m[k]) * cc.jf[k];
-    }
-    cc.mcn = mcn;
-    cc.mcf = mcf;
-    cc.rcn = recip_ok(mcn) ? 1.0 / mcn : 0.0;
-    cc.rcf = recip_ok(mcf) ? 1.0 / mcf : 0.0;
+    const double xa2 = (nx * ima) * nx, ya2 = (ny * ima) * ny, xb2 = (nx * imb) * nx, yb2 = (ny * imb) * ny;
+    const double lin_a = xa2 + ya2;
+    cc.mc[0] = ((lin_a + (cc.row[0][2] * ira) * cc.row[0][2]) + xb2) + yb2;
+    cc.mc[0] = cc.mc[0] + (cc.row[0][3] * irb) * cc.row[0][3];
+    cc.mc[1] = ((lin_a + (cc.row[1][2] * ira) * cc.row[1][2]) + yb2) + xb2;
+    cc.mc[1] = cc.mc[1] + (cc.row[1][3] * irb) * cc.row[1][3];
+    for (int k = 0; k < 2; ++k) cc.rc[k] = recip_ok(cc.mc[k]) ? 1.0 / cc.mc[k] : 0.0;
+    cc.im[0] = ima;
+    cc.im[1] = ira;
+    cc.im[2] = imb;
+    cc.im[3] = irb;
     cc.mu = (d.mu[ga] + d.mu[gb]) / 2.0;
     const double ea = d.bounce[ga], eb = d.bounce[gb];
-    cc.e = ea <= eb ? ea : eb;
-    cc.fast = (small_mag(cc.rax) && small_mag(cc.ray) && small_mag(cc.rbx) && small_mag(cc.rby) &&
-               below_two(cc.rnx) && below_two(cc.rny)) ? 1.0 : 0.0;
-    cc.pad = 0.0;
+    cc.e = f_le(ea, eb) ? ea : eb;
+    cc.no_bounce = (small_mag(cc.ra[0]) & small_mag(cc.ra[1]) & small_mag(cc.ra[2]) & small_mag(cc.ra[3]) &
+                    below_two(nx) & below_two(ny) & (mag_bits(cc.e) == 0)) ? 1 : 0;
+    cc.pad = 0;
     d.con[c] = cc;
     /* warm-start lookup */
     double l0 = 0.0, l1 = 0.0;
@@ -1975,7 +1968,7 @@ __global__ void k_build(Dev d, double dt, double beta, double slop, int warm_sta
 }
 
 /* ------------------------------------------------------------------------ */
-/* A9-A10 dependency-level schedule                                           */
+/* A9-A10 one update                                                          */
 /* ------------------------------------------------------------------------ */
 
 /* Block-wide exclusive scan of in-place int array a[0..n), returns total. */
@@ -2011,847 +2004,62 @@ __device__ int block_exclusive_scan(int32_t* a, int n, int32_t* smem /* >= 32 */
   return carry;
 }
 
-/* applyLagrangian2 (Constraint.hs:197-204): v += (J * lambda) * invMass.
- * Every contact Jacobian built by k_build has J[0] = -J[3] and J[1] = -J[4]
- * (the normal and the tangent enter the two bodies with opposite signs, and
- * a Flip only swaps the halves), and (-x) * l is exactly -(x * l) in IEEE
- * arithmetic, so those two products are computed once. */
-__device__ __forceinline__ void apply_impulse(const double j[6], double l, double v[6],
-                                              const double m[6]) {
-  const double p3 = j[3] * l, p4 = j[4] * l;
-  v[0] = v[0] + (-p3) * m[0];
-  v[1] = v[1] + (-p4) * m[1];
-  v[2] = v[2] + (j[2] * l) * m[2];
-  v[3] = v[3] + p3 * m[3];
-  v[4] = v[4] + p4 * m[4];
-  v[5] = v[5] + (j[5] * l) * m[5];
+/* J . v as a left fold (Shapes/Linear/Template.hs:108-110) of a stored row. */
+__device__ __forceinline__ double row_dot(const double r[4], const double v[6]) {
+  double s = (-r[0]) * v[0];
+  s = s + (-r[1]) * v[1];
+  s = s + r[2] * v[2];
+  s = s + r[0] * v[3];
+  s = s + r[1] * v[4];
+  return s + r[3] * v[5];
 }
 
-/* J . v as a left fold (Shapes/Linear/Template.hs:108-110). */
-__device__ __forceinline__ double dot6(const double j[6], const double v[6]) {
-  double s = j[0] * v[0];
-#pragma unroll
-  for (int k = 1; k < 6; ++k) s = s + j[k] * v[k];
-  return s;
+/* applyLagrangian2 (Constraint.hs:197-204): v += (J * lambda) * invMass; the
+ * two bodies' linear products differ only in sign and are computed once. */
+__device__ __forceinline__ void row_apply(const double r[4], double l, double v[6], const double im[4]) {
+  const double px = r[0] * l, py = r[1] * l;
+  v[0] = v[0] + (-px) * im[0];
+  v[1] = v[1] + (-py) * im[0];
+  v[2] = v[2] + (r[2] * l) * im[1];
+  v[3] = v[3] + px * im[2];
+  v[4] = v[4] + py * im[2];
+  v[5] = v[5] + (r[3] * l) * im[3];
 }
 
-/* Where a solver group keeps its bodies' velocities during the solve: in the
- * warp's shared-memory slice (slot = global body index + delta of its world)
- * when the group fits, else in global memory. */
-struct VelStore {
-  double* s;   /* shared: 3 doubles per slot */
-  const Dev* d;
-  __device__ __forceinline__ void load(int g, int delta, double& x, double& y, double& w) const {
-    if (s) {
-      const double* p = s + 3 * (g + delta);
-      x = p[0]; y = p[1]; w = p[2];
-    } else {
-      x = d->vx[g]; y = d->vy[g]; w = d->w[g];
-    }
-  }
-  __device__ __forceinline__ void store(int g, int delta, double x, double y, double w) const {
-    if (s) {
-      double* p = s + 3 * (g + delta);
-      p[0] = x; p[1] = y; p[2] = w;
-    } else {
-      d->vx[g] = x; d->vy[g] = y; d->w[g] = w;
-    }
-  }
-};
-
-/* Pulls a constraint record's cache lines into L1 ahead of its level. */
-__device__ __forceinline__ void prefetch_con(const Con* c) {
-  const char* p = reinterpret_cast<const char*>(c);
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(p + 128));
-  asm volatile("prefetch.global.L1 [%0];" ::"l"(p + sizeof(Con) - 8));
+/* The restitution term (bounceB, Restitution.hs:34-51): min 0 (e * (closing
+ * velocity . n)), closing velocity ((-va + (-wa) z x ra) + vb) + wb z x rb. */
+__device__ __forceinline__ double bounce_term(const Con* con, const double v[6]) {
+  const double nwa = -v[2];
+  const double cvx = ((-v[0] + (-(nwa * con->ra[1]))) + v[3]) + (-(v[5] * con->ra[3]));
+  const double cvy = ((-v[1] + nwa * con->ra[0]) + v[4]) + v[5] * con->ra[2];
+  const double tb = con->e * (cvx * con->rn[0] + cvy * con->rn[1]);
+  return f_le(0.0, tb) ? 0.0 : tb;
 }
 
-/* One update.  Warm: applySln of the cached Lagrangians
- * (Solvers/Contact.hs:105-113).  Otherwise improveContactSln
- * (Solvers/Contact.hs:124-143): both new Lagrangians from the same velocities
- * (contactLagrangian, Constraints/Contact.hs:86-95; bounceB,
- * Restitution.hs:34-51; lagrangian2, Constraint.hs:164-169), then positive /
- * clampAbs (SolutionProcessors.hs:33-53) and applySln (non-penetration first).
- * bounceB is min 0 (e * (v_closing . n)); when e = 0 and every velocity and
- * radius is below 2^500 the product is a signed zero and the result is +0, so
- * b + bounceB equals the precomputed b + 0.0 bit for bit. */
-__device__ __forceinline__ void solve_item(const Dev& d, uint32_t item, int ga, int gb, uint8_t info,
-                                           const VelStore& vs, int delta) {
-  const int c = (int)(item & ~kWarmBit);
-  const double2* cp = reinterpret_cast<const double2*>(d.con + c);
-  double j_n[6], j_f[6];
-  {
-    const double2 a0 = cp[0], a1 = cp[1], a2 = cp[2], a3 = cp[3], a4 = cp[4], a5 = cp[5];
-    j_n[0] = a0.x; j_n[1] = a0.y; j_n[2] = a1.x; j_n[3] = a1.y; j_n[4] = a2.x; j_n[5] = a2.y;
-    j_f[0] = a3.x; j_f[1] = a3.y; j_f[2] = a4.x; j_f[3] = a4.y; j_f[4] = a5.x; j_f[5] = a5.y;
-  }
-  double v[6];
-  vs.load(ga, delta, v[0], v[1], v[2]);
-  vs.load(gb, delta, v[3], v[4], v[5]);
-  const double ima = __ldg(d.iml + ga), ira = __ldg(d.imr + ga), imb = __ldg(d.iml + gb), irb = __ldg(d.imr + gb);
-  const double m[6] = {ima, ima, ira, imb, imb, irb};
-  double ln_apply, lf_apply;
-  double2* lam2 = reinterpret_cast<double2*>(d.lam) + c;
-  const double2 cached = *lam2;
-  if (item & kWarmBit) {
-    ln_apply = cached.x;
-    lf_apply = cached.y;
-  } else {
-    const double2 b6 = cp[6];   /* bn, bn0 */
-    const double2 b9 = cp[9];   /* rnx, rny */
-    const double2 b10 = cp[10]; /* mcn, mcf */
-    const double2 b11 = cp[11]; /* mu, e */
-    const double2 b12 = cp[12]; /* RN(1/mcn), RN(1/mcf) */
-    const double cn = cached.x, cf = cached.y;
-    const uint64_t ebits = (uint64_t)__double_as_longlong(b11.y) & 0x7fffffffffffffffull;
-    const bool fastflag = __double_as_longlong(cp[13].x) != 0;
-    double bias;
-    if (ebits == 0 && fastflag && small_mag(v[0]) && small_mag(v[1]) && small_mag(v[2]) &&
-        small_mag(v[3]) && small_mag(v[4]) && small_mag(v[5])) {
-      bias = b6.y;
-    } else {
-      const double2 b7 = cp[7]; /* rax, ray */
-      const double2 b8 = cp[8]; /* rbx, rby */
-      /* closing velocity ((-va + (-wa) z× ra) + vb) + wb z× rb */
-      const double nwa = -v[2];
-      const double cvx = ((-v[0] + (-(nwa * b7.y))) + v[3]) + (-(v[5] * b8.y));
-      const double cvy = ((-v[1] + nwa * b7.x) + v[4]) + v[5] * b8.x;
-      const double tb = b11.y * (cvx * b9.x + cvy * b9.y);
-      const double bounce = f_le(0.0, tb) ? 0.0 : tb;
-      bias = b6.x + bounce;
-    }
-    const double ln_new = div_rn(-(dot6(j_n, v) + bias), b10.x, b12.x);
-    const double lf_new = div_rn(-plus_zero(dot6(j_f, v)), b10.y, b12.y);
-    const double neg_cn = -cn;
-    ln_apply = f_le(ln_new, neg_cn) ? neg_cn : ln_new;
-    const double ln_cache = cn + ln_apply;
-    const double thr = ln_cache * b11.x;
-    const double acc = cf + lf_new;
-    const double acc2 = f_lt(thr, acc) ? thr : (f_lt(acc, -thr) ? -thr : acc);
-    lf_apply = acc2 - cf;
-    *lam2 = make_double2(ln_cache, acc2);
-  }
-  apply_impulse(j_n, ln_apply, v, m);
-  apply_impulse(j_f, lf_apply, v, m);
-  if (info & kInfoDynA) vs.store(ga, delta, v[0], v[1], v[2]);
-  if (info & kInfoDynB) vs.store(gb, delta, v[3], v[4], v[5]);
+/* Every velocity component below 2^500 in magnitude. */
+__device__ __forceinline__ bool small_velocities(const double v[6]) {
+  return small_mag(v[0]) & small_mag(v[1]) & small_mag(v[2]) & small_mag(v[3]) & small_mag(v[4]) & small_mag(v[5]);
 }
 
-/* The reference applies warm starts then `iterations` sweeps strictly in
- * contact order (Solvers/Contact.hs:74-157).  Each update reads and writes only
- * its two bodies' velocities and its own Lagrangians, so running update u after
- * every earlier update that shares a non-static body with it reproduces the
- * sequential result bit for bit; static bodies are never written in the step.
- * level(u) = 1 + max(level of the last earlier update on each of its dynamic
- * bodies), and updates of one level touch disjoint bodies.  The levels pipeline
- * the sweeps: sweep s+1 starts on a body as soon as sweep s is done with it, so
- * a world offers about iterations+1 independent updates per level.
- *
- * Each warp owns one solver group: up to 32 worlds of similar size (the host
- * sorts worlds by size and packs them so that a level fills about one warp).
- * A warp never waits for another warp:
- *   1. applyExternal (World.hs:156-158, constantAccel External.hs:23-28) on the
- *      group's bodies;
- *   2. lane l scans world l's updates in sequential order, keeping each body's
- *      last level in the warp's slice of shared memory when it fits;
- *   3. the warp counting-sorts each world's updates by level in place;
- *   4. the warp runs the levels in order, lanes taking the level's updates of
- *      all its worlds, with __syncwarp between levels.
- * Steps 2-3 are latency-bound integer work that overlaps the FP64-bound step 4
- * of the other warps on the SM. */
-constexpr int kMaxGroupWorlds = 32;
-
-constexpr int kScanBlock = 8;
-
-__global__ void k_schedule_solve(Dev d, int iterations, int warm_start, int external, double ax, double ay,
-                                 double dt, int n_groups, int smem_last_per_warp) {
-  extern __shared__ __align__(16) int32_t s_dyn[];
-  __shared__ int32_t s_delta[8][kMaxGroupWorlds];
-  if (d.counters[kCntOverflow]) return; /* buffers incomplete: the host retries */
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int grp = blockIdx.x * (blockDim.x >> 5) + wib;
-  if (grp >= n_groups) return;
-  const int o0 = d.group_world_off[grp], o1 = d.group_world_off[grp + 1];
-  const int nw = o1 - o0;
-  const int stride = iterations + 1;
-  int32_t* s_last = s_dyn + wib * smem_last_per_warp;
-  if (d.phase_clock && lane == 0) d.phase_clock[8 * grp + 0] = clock64();
-  /* 1. gravity, 2a. reset last levels (lane-parallel over each world) */
-  int group_bodies = 0;
-  for (int k = 0; k < nw; ++k) {
-    const int wld = d.group_worlds[o0 + k];
-    group_bodies += d.world_body_off[wld + 1] - d.world_body_off[wld];
-  }
-  const bool smem_last = group_bodies <= smem_last_per_warp;
-  {
-    int base = 0;
-    for (int k = 0; k < nw; ++k) {
-      const int wld = d.group_worlds[o0 + k];
-      const int b0 = d.world_body_off[wld], b1 = d.world_body_off[wld + 1];
-      for (int g = b0 + lane; g < b1; g += 32) {
-        if (external && !(0.0 == d.iml[g]) && !(d.flags[g] & kFlagInactive)) {
-          d.vx[g] = d.vx[g] + ax * dt;
-          d.vy[g] = d.vy[g] + ay * dt;
-        }
-        if (smem_last) s_last[base + g - b0] = 0;
-        else d.last[g] = 0;
-      }
-      base += b1 - b0;
-    }
-  }
-  __syncwarp();
-  /* 2b. lane l scans world l */
-  int my_depth = 0, my_items = 0, my_hits = 0;
-  size_t my_region = 0;
-  int c0 = 0, c1 = 0;
-  int32_t* last = d.last;
-  if (lane < nw) {
-    const int wld = d.group_worlds[o0 + lane];
-    int base = 0;
-    for (int k = 0; k < lane; ++k) {
-      const int w2 = d.group_worlds[o0 + k];
-      base += d.world_body_off[w2 + 1] - d.world_body_off[w2];
-    }
-    const int b0 = d.world_body_off[wld];
-    last = smem_last ? s_last + base - b0 : d.last;
-    c0 = d.world_contact_off[wld];
-    c1 = d.world_contact_off[wld + 1];
-    my_region = (size_t)stride * c0;
-  }
-  /* Sequential scan of this lane's world, pass by pass.  The only
-   * loop-carried dependency is through last[]; contacts are read in blocks of
-   * kScanBlock and the next block is loaded while the current one is
-   * processed, so the global-load latency hides behind kScanBlock updates of
-   * shared-memory work (loads past the world's end are clamped to its last
-   * contact and never used). */
-  if (lane < nw && c0 < c1) {
-    for (int pass = warm_start ? 0 : 1; pass <= iterations; ++pass) {
-      uint8_t inf[kScanBlock];
-      int ia[kScanBlock], ib[kScanBlock];
-#pragma unroll
-      for (int k = 0; k < kScanBlock; ++k) {
-        const int cc = min(c0 + k, c1 - 1);
-        inf[k] = d.c_hit[cc];
-        ia[k] = d.c_ga[cc];
-        ib[k] = d.c_gb[cc];
-      }
-      for (int cb = c0; cb < c1; cb += kScanBlock) {
-        uint8_t inf2[kScanBlock];
-        int ia2[kScanBlock], ib2[kScanBlock];
-#pragma unroll
-        for (int k = 0; k < kScanBlock; ++k) {
-          const int cc = min(cb + kScanBlock + k, c1 - 1);
-          inf2[k] = d.c_hit[cc];
-          ia2[k] = d.c_ga[cc];
-          ib2[k] = d.c_gb[cc];
-        }
-#pragma unroll
-        for (int k = 0; k < kScanBlock; ++k) {
-          const int cur_c = cb + k;
-          const uint8_t info = inf[k];
-          if (cur_c < c1 && !(pass == 0 && !(info & kInfoHit))) {
-            const int ga = ia[k], gb = ib[k];
-            const bool da = info & kInfoDynA, db = info & kInfoDynB;
-            const int la = da ? last[ga] : 0, lb = db ? last[gb] : 0;
-            const int lvl = (la > lb ? la : lb) + 1;
-            if (da) last[ga] = lvl;
-            if (db) last[gb] = lvl;
-            d.idesc[my_region + my_items] =
-                make_int4((int)((uint32_t)cur_c | (pass == 0 ? kWarmBit : 0u)), ga, gb, (int)info | (lane << 8));
-            d.ilevel[my_region + my_items] = lvl;
-            ++my_items;
-            my_depth = lvl > my_depth ? lvl : my_depth;
-            my_hits += pass == 0;
-          }
-          inf[k] = inf2[k];
-          ia[k] = ia2[k];
-          ib[k] = ib2[k];
-        }
-      }
-    }
-  }
-  if (lane < nw) d.world_levels[d.group_worlds[o0 + lane]] = my_depth;
-  if (d.phase_clock && lane == 0) d.phase_clock[8 * grp + 1] = clock64();
-  /* 3. the group's updates counting-sorted by level into a region of gdesc /
-   *    ghist taken from a bump allocator, as packed descriptors, so that a
-   *    level is one contiguous run */
-  int max_depth = my_depth, tot_items = my_items, tot_hits = my_hits;
-  for (int o = 16; o > 0; o >>= 1) {
-    max_depth = max(max_depth, __shfl_xor_sync(0xffffffffu, max_depth, o));
-    tot_items += __shfl_xor_sync(0xffffffffu, tot_items, o);
-    tot_hits += __shfl_xor_sync(0xffffffffu, tot_hits, o);
-  }
-  int gbase = 0;
-  if (lane == 0) {
-    atomicAdd(&d.counters[kCntLevels], (unsigned long long)max_depth);
-    atomicAdd(&d.counters[kCntHits], (unsigned long long)tot_hits);
-    atomicAdd(&d.counters[kCntItems], (unsigned long long)tot_items);
-    gbase = (int)atomicAdd(&d.counters[kCntGroupAlloc], (unsigned long long)(tot_items + 1));
-  }
-  gbase = __shfl_sync(0xffffffffu, gbase, 0);
-  int32_t* gh = d.ghist + gbase;
-  int4* gdesc = d.gdesc + gbase;
-  /* the histogram lives in the warp's shared slice when the depth fits (the
-   * last levels are dead by now), else in gh */
-  int32_t* hist = max_depth <= smem_last_per_warp ? s_last : gh;
-  for (int t = lane; t < max_depth; t += 32) hist[t] = 0;
-  __syncwarp();
-  for (int k = 0; k < nw; ++k) {
-    const int n_items = __shfl_sync(0xffffffffu, my_items, k);
-    const size_t region = (size_t)__shfl_sync(0xffffffffu, (unsigned long long)my_region, k);
-#pragma unroll 8
-    for (int t = lane; t < n_items; t += 32) atomicAdd(&hist[d.ilevel[region + t] - 1], 1);
-  }
-  __syncwarp();
-  {
-    int carry = 0;
-    for (int t0 = 0; t0 < max_depth; t0 += 32) {
-      const int t = t0 + lane;
-      const int x = t < max_depth ? hist[t] : 0;
-      int incl = x;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      if (t < max_depth) hist[t] = carry + incl - x;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-  }
-  __syncwarp();
-  for (int k = 0; k < nw; ++k) {
-    const int n_items = __shfl_sync(0xffffffffu, my_items, k);
-    const size_t region = (size_t)__shfl_sync(0xffffffffu, (unsigned long long)my_region, k);
-#pragma unroll 8
-    for (int t = lane; t < n_items; t += 32) {
-      const int4 u = d.idesc[region + t];
-      gdesc[atomicAdd(&hist[d.ilevel[region + t] - 1], 1)] = u;
-    }
-  }
-  __syncwarp();
-  if (hist != gh)
-    for (int t = lane; t < max_depth; t += 32) gh[t] = hist[t];
-  __syncwarp();
-  if (d.phase_clock && lane == 0) d.phase_clock[8 * grp + 2] = clock64();
-  /* 4. levels.  gh[L] is now the end of level L (0-based) in gdesc.  The
-   *    group's velocities move to the warp's shared slice when they fit (3
-   *    doubles per body), so the only dependent access per level is a
-   *    shared-memory load.  A two-deep software pipeline keeps everything else
-   *    off that path: while level L runs, the descriptors of level L+1 are in
-   *    registers with their constraint lines being pulled into L1, and the
-   *    descriptors and end offset of level L+2 are loading. */
-  const bool smem_vel = 6 * group_bodies <= smem_last_per_warp;
-  int32_t* dl = s_delta[wib];
-  if (lane < nw) {
-    const int wld = d.group_worlds[o0 + lane];
-    int base = 0;
-    for (int k = 0; k < lane; ++k) {
-      const int w2 = d.group_worlds[o0 + k];
-      base += d.world_body_off[w2 + 1] - d.world_body_off[w2];
-    }
-    dl[lane] = base - d.world_body_off[wld];
-  }
-  __syncwarp();
-  VelStore vs;
-  vs.d = &d;
-  vs.s = smem_vel ? reinterpret_cast<double*>(s_last) : nullptr;
-  if (smem_vel) {
-    for (int k = 0; k < nw; ++k) {
-      const int wld = d.group_worlds[o0 + k];
-      const int b0 = d.world_body_off[wld], b1 = d.world_body_off[wld + 1];
-      for (int g = b0 + lane; g < b1; g += 32) {
-        double* p = vs.s + 3 * (g + dl[k]);
-        p[0] = d.vx[g];
-        p[1] = d.vy[g];
-        p[2] = d.w[g];
-      }
-    }
-  }
-  __syncwarp();
-  const int4 none = make_int4(0, 0, 0, 0);
-  /* e_prev = start of level L, e_cur = end of level L, e_next = end of L+1 */
-  int e_prev = 0;
-  int e_cur = max_depth > 0 ? gh[0] : 0;
-  int e_next = max_depth > 1 ? gh[1] : e_cur;
-  int4 cur = lane < e_cur ? gdesc[lane] : none;
-  int4 nxt = e_cur + lane < e_next ? gdesc[e_cur + lane] : none;
-  if (lane < e_cur) prefetch_con(d.con + (cur.x & ~kWarmBit));
-  for (int L = 0; L < max_depth; ++L) {
-    /* issue level L+2's loads; they are consumed one iteration later */
-    const int e_next2 = L + 2 < max_depth ? gh[L + 2] : e_next;
-    const int4 nxt2 = e_next + lane < tot_items ? gdesc[e_next + lane] : none;
-    if (e_cur + lane < e_next) prefetch_con(d.con + (nxt.x & ~kWarmBit));
-    const int count = e_cur - e_prev;
-    if (lane < count)
-      solve_item(d, (uint32_t)cur.x, cur.y, cur.z, (uint8_t)(cur.w & 0xff), vs, dl[cur.w >> 8]);
-    for (int t = lane + 32; t < count; t += 32) { /* levels wider than a warp */
-      const int4 u = gdesc[e_prev + t];
-      solve_item(d, (uint32_t)u.x, u.y, u.z, (uint8_t)(u.w & 0xff), vs, dl[u.w >> 8]);
-    }
-    __syncwarp();
-    cur = nxt;
-    nxt = nxt2;
-    e_prev = e_cur;
-    e_cur = e_next;
-    e_next = e_next2;
-  }
-  if (smem_vel) {
-    for (int k = 0; k < nw; ++k) {
-      const int wld = d.group_worlds[o0 + k];
-      const int b0 = d.world_body_off[wld], b1 = d.world_body_off[wld + 1];
-      for (int g = b0 + lane; g < b1; g += 32) {
-        const double* p = vs.s + 3 * (g + dl[k]);
-        d.vx[g] = p[0];
-        d.vy[g] = p[1];
-        d.w[g] = p[2];
-      }
-    }
-  }
-  if (d.phase_clock && lane == 0) {
-    d.phase_clock[8 * grp + 3] = clock64();
-    d.phase_clock[8 * grp + 4] = max_depth;
-    d.phase_clock[8 * grp + 5] = tot_items;
-    d.phase_clock[8 * grp + 6] = group_bodies;
-    d.phase_clock[8 * grp + 7] = nw;
-  }
-}
-
-/* The same schedule and solve with P warps per group (one group per CTA of
- * 32 P threads).  A group's worlds are scanned by P warps at once (world k by
- * lane k / P of warp k % P), the counting sort and the level loop use all
- * 32 P threads, and __syncthreads separates the levels.  Updates of one level
- * touch disjoint dynamic bodies, so splitting a level over more threads
- * changes nothing in the results; it lets the host pack more worlds into a
- * group (fuller FP64 instructions: one warp instruction serves 32 updates)
- * without lengthening each warp's share of a level. */
-template <int P, bool PAR>
-__global__ void __launch_bounds__(32 * P) k_group_solve(Dev d, int iterations, int warm_start, int external,
-                                                        double ax, double ay, double dt, int n_groups,
-                                                        int smem_ints, int heavy_first) {
-  constexpr int NT = 32 * P;
-  extern __shared__ __align__(16) int32_t s_dyn[];
-  __shared__ int32_t s_delta[kMaxGroupWorlds];
-  __shared__ int32_t s_coff[kMaxGroupWorlds + 1]; /* PAR: prefix of the worlds' contact counts */
-  __shared__ int32_t s_c0[kMaxGroupWorlds];       /* PAR: first contact of each world */
-  __shared__ int32_t s_wdepth[kMaxGroupWorlds];   /* PAR: levels of each world */
-  __shared__ int32_t s_nitems[kMaxGroupWorlds];
-  __shared__ unsigned long long s_region[kMaxGroupWorlds];
-  __shared__ int32_t s_red[3][P];
-  __shared__ int32_t s_gbase;
-  if (d.counters[kCntOverflow]) return; /* buffers incomplete: the host retries */
-  const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
-  /* Groups come sorted heaviest first.  With heavy_first = h > 0 the first h
-   * CTAs (one wave over the SMs) take the h heaviest groups and the rest take
-   * the others lightest first, so that a heavy group starts beside light ones
-   * instead of beside the next heaviest. */
-  const int hf = min(heavy_first, n_groups);
-  const int grp = (int)blockIdx.x < hf ? (int)blockIdx.x : n_groups - 1 - ((int)blockIdx.x - hf);
-  if (grp >= n_groups) return;
-  const int o0 = d.group_world_off[grp], o1 = d.group_world_off[grp + 1];
-  const int nw = o1 - o0;
-  const int stride = iterations + 1;
-  int32_t* s_last = s_dyn;
-  if (d.phase_clock && tid == 0) d.phase_clock[8 * grp + 0] = clock64();
-  /* 1. gravity, 2a. reset last levels */
-  int group_bodies = 0;
-  for (int k = 0; k < nw; ++k) {
-    const int wld = d.group_worlds[o0 + k];
-    group_bodies += d.world_body_off[wld + 1] - d.world_body_off[wld];
-  }
-  /* PAR keeps two per-body entries (last contact, last cache-hit contact) */
-  const bool smem_last = (PAR ? 2 : 1) * group_bodies <= smem_ints;
-  {
-    int base = 0;
-    for (int k = 0; k < nw; ++k) {
-      const int wld = d.group_worlds[o0 + k];
-      const int b0 = d.world_body_off[wld], b1 = d.world_body_off[wld + 1];
-      for (int g = b0 + tid; g < b1; g += NT) {
-        if (external && !(0.0 == d.iml[g]) && !(d.flags[g] & kFlagInactive)) {
-          d.vx[g] = d.vx[g] + ax * dt;
-          d.vy[g] = d.vy[g] + ay * dt;
-        }
-        if (PAR) {
-          if (smem_last) {
-            s_last[base + g - b0] = -1;
-            s_last[group_bodies + base + g - b0] = -1;
-          } else {
-            d.last[g] = -1;
-            d.last_hit[g] = -1;
-          }
-        } else {
-          if (smem_last) s_last[base + g - b0] = 0;
-          else d.last[g] = 0;
-        }
-      }
-      if (tid == 0) s_delta[k] = base - b0;
-      base += b1 - b0;
-    }
-  }
-  __syncthreads();
-  if constexpr (PAR) {
-    if (tid == 0) {
-      int acc = 0;
-      for (int k = 0; k < nw; ++k) {
-        const int wld = d.group_worlds[o0 + k];
-        s_coff[k] = acc;
-        s_c0[k] = d.world_contact_off[wld];
-        s_wdepth[k] = 0;
-        acc += d.world_contact_off[wld + 1] - d.world_contact_off[wld];
-      }
-      s_coff[nw] = acc;
-    }
-    __syncthreads();
-  }
-  int my_depth = 0, my_items = 0, my_hits = 0;
-  if constexpr (!PAR) {
-  /* 2b. world k is scanned by lane k / P of warp k % P */
-  const int my_k = lane * P + wib;
-  size_t my_region = 0;
-  int c0 = 0, c1 = 0;
-  int32_t* last = d.last;
-  if (my_k < nw) {
-    const int wld = d.group_worlds[o0 + my_k];
-    last = smem_last ? s_last + s_delta[my_k] : d.last;
-    c0 = d.world_contact_off[wld];
-    c1 = d.world_contact_off[wld + 1];
-    my_region = (size_t)stride * c0;
-  }
-  if (my_k < nw && c0 < c1) {
-    for (int pass = warm_start ? 0 : 1; pass <= iterations; ++pass) {
-      uint8_t inf[kScanBlock];
-      int ia[kScanBlock], ib[kScanBlock];
-#pragma unroll
-      for (int k = 0; k < kScanBlock; ++k) {
-        const int cc = min(c0 + k, c1 - 1);
-        inf[k] = d.c_hit[cc];
-        ia[k] = d.c_ga[cc];
-        ib[k] = d.c_gb[cc];
-      }
-      for (int cb = c0; cb < c1; cb += kScanBlock) {
-        uint8_t inf2[kScanBlock];
-        int ia2[kScanBlock], ib2[kScanBlock];
-#pragma unroll
-        for (int k = 0; k < kScanBlock; ++k) {
-          const int cc = min(cb + kScanBlock + k, c1 - 1);
-          inf2[k] = d.c_hit[cc];
-          ia2[k] = d.c_ga[cc];
-          ib2[k] = d.c_gb[cc];
-        }
-#pragma unroll
-        for (int k = 0; k < kScanBlock; ++k) {
-          const int cur_c = cb + k;
-          const uint8_t info = inf[k];
-          if (cur_c < c1 && !(pass == 0 && !(info & kInfoHit))) {
-            const int ga = ia[k], gb = ib[k];
-            const bool da = info & kInfoDynA, db = info & kInfoDynB;
-            const int la = da ? last[ga] : 0, lb = db ? last[gb] : 0;
-            const int lvl = (la > lb ? la : lb) + 1;
-            if (da) last[ga] = lvl;
-            if (db) last[gb] = lvl;
-            d.idesc[my_region + my_items] =
-                make_int4((int)((uint32_t)cur_c | (pass == 0 ? kWarmBit : 0u)), ga, gb, (int)info | (my_k << 8));
-            d.ilevel[my_region + my_items] = lvl;
-            ++my_items;
-            my_depth = lvl > my_depth ? lvl : my_depth;
-            my_hits += pass == 0;
-          }
-          inf[k] = inf2[k];
-          ia[k] = ia2[k];
-          ib[k] = ib2[k];
-        }
-      }
-    }
-  }
-  if (my_k < nw) {
-    s_nitems[my_k] = my_items;
-    s_region[my_k] = (unsigned long long)my_region;
-    d.world_levels[d.group_worlds[o0 + my_k]] = my_depth;
-  }
-  } else {
-    /* 2b. Dependency levels without a walk over every update.  Phase A: the
-     * lane of world k walks the world's contacts once and records, for each
-     * dynamic side, the previous contact of the world on that body and the
-     * previous cache-hit contact (c_pred); the per-body arrays end holding
-     * each body's last contact and last hit contact. */
-    int32_t* lastc = smem_last ? s_last : d.last;
-    int32_t* lasth = smem_last ? s_last + group_bodies : d.last_hit;
-    const int my_k = lane * P + wib;
-    if (my_k < nw) {
-      const int dl = smem_last ? s_delta[my_k] : 0;
-      const int c0 = s_c0[my_k], c1 = c0 + (s_coff[my_k + 1] - s_coff[my_k]);
-      if (c0 < c1) {
-        uint8_t inf[kScanBlock];
-        int ia[kScanBlock], ib[kScanBlock];
-#pragma unroll
-        for (int k = 0; k < kScanBlock; ++k) {
-          const int cc = min(c0 + k, c1 - 1);
-          inf[k] = d.c_hit[cc];
-          ia[k] = d.c_ga[cc];
-          ib[k] = d.c_gb[cc];
-        }
-        for (int cb = c0; cb < c1; cb += kScanBlock) {
-          uint8_t inf2[kScanBlock];
-          int ia2[kScanBlock], ib2[kScanBlock];
-#pragma unroll
-          for (int k = 0; k < kScanBlock; ++k) {
-            const int cc = min(cb + kScanBlock + k, c1 - 1);
-            inf2[k] = d.c_hit[cc];
-            ia2[k] = d.c_ga[cc];
-            ib2[k] = d.c_gb[cc];
-          }
-#pragma unroll
-          for (int k = 0; k < kScanBlock; ++k) {
-            const int c = cb + k;
-            if (c < c1) {
-              const uint8_t info = inf[k];
-              const bool hit = info & kInfoHit;
-              int4 pr = make_int4(-1, -1, -1, -1);
-              if (info & kInfoDynA) {
-                const int sa = ia[k] + dl;
-                pr.x = lastc[sa];
-                pr.z = lasth[sa];
-                lastc[sa] = c;
-                if (hit) lasth[sa] = c;
-              }
-              if (info & kInfoDynB) {
-                const int sb = ib[k] + dl;
-                pr.y = lastc[sb];
-                pr.w = lasth[sb];
-                lastc[sb] = c;
-                if (hit) lasth[sb] = c;
-              }
-              d.c_pred[c] = pr;
-            }
-            inf[k] = inf2[k];
-            ia[k] = ia2[k];
-            ib[k] = ib2[k];
-          }
-        }
-      }
-    }
-    __syncthreads();
-    /* Phase B: the passes in order over the group's contacts in chunks of the
-     * CTA's threads.  An update's level is one more than its predecessors'
-     * on each dynamic body: the previous contact of the same pass touching
-     * it, else the body's last contact of the previous pass (only cache hits
-     * are updates of the warm-start pass).  Within a chunk the levels are
-     * raised to a fixed point (they only grow and stay at or below the final
-     * values), which gives every update the level a walk over the updates in
-     * order gives it.  Update (pass p, contact c) of world k takes slot
-     * (p - p0) n_k + (c - c0_k) of the world's region; a slot without an
-     * update (the warm-start pass of a contact without a cache hit) keeps
-     * level 0. */
-    const int NC = s_coff[nw];
-    const int p0 = warm_start ? 0 : 1;
-    for (int p = p0; p <= iterations; ++p) {
-      int32_t* Lc = d.c_lvl + (size_t)(p & 1) * d.contact_cap;
-      const int32_t* Lp = d.c_lvl + (size_t)((p + 1) & 1) * d.contact_cap;
-      for (int s0 = 0; s0 < NC; s0 += NT) {
-        const int gc = s0 + tid;
-        int k = 0, c = -1, ga = 0, gb = 0;
-        uint8_t info = 0;
-        int4 pr = make_int4(-1, -1, -1, -1);
-        if (gc < NC) {
-          while (k + 1 < nw && s_coff[k + 1] <= gc) ++k;
-          c = s_c0[k] + (gc - s_coff[k]);
-          info = d.c_hit[c];
-          ga = d.c_ga[c];
-          gb = d.c_gb[c];
-          pr = d.c_pred[c];
-        }
-        const bool live = c >= 0 && !(p == 0 && !(info & kInfoHit));
-        const int dl = smem_last ? s_delta[k] : 0;
-        int a_same = -1, b_same = -1, base = 0;
-        if (live && (info & kInfoDynA)) {
-          a_same = p == 0 ? pr.z : pr.x;
-          if (a_same < 0 && p > p0) {
-            const int q = p - 1 == 0 ? lasth[ga + dl] : lastc[ga + dl];
-            if (q >= 0) base = max(base, Lp[q]);
-          }
-        }
-        if (live && (info & kInfoDynB)) {
-          b_same = p == 0 ? pr.w : pr.y;
-          if (b_same < 0 && p > p0) {
-            const int q = p - 1 == 0 ? lasth[gb + dl] : lastc[gb + dl];
-            if (q >= 0) base = max(base, Lp[q]);
-          }
-        }
-        if (live) Lc[c] = 0;
-        __syncthreads();
-        int L = 0;
-        for (;;) {
-          int v = base;
-          if (a_same >= 0) v = max(v, Lc[a_same]);
-          if (b_same >= 0) v = max(v, Lc[b_same]);
-          const int nl = live ? v + 1 : 0;
-          const bool changed = nl != L;
-          L = nl;
-          __syncthreads(); /* every read of this round before any write */
-          if (changed) Lc[c] = L;
-          if (!__syncthreads_or(changed)) break;
-        }
-        if (c >= 0) {
-          const size_t slot = (size_t)stride * s_c0[k] + (size_t)(p - p0) * (s_coff[k + 1] - s_coff[k]) +
-                              (size_t)(gc - s_coff[k]);
-          if (live) {
-            d.idesc[slot] = make_int4((int)((uint32_t)c | (p == 0 ? kWarmBit : 0u)), ga, gb, (int)info | (k << 8));
-            ++my_items;
-            my_depth = L > my_depth ? L : my_depth;
-            my_hits += p == 0;
-            atomicMax(&s_wdepth[k], L);
-          }
-          d.ilevel[slot] = L; /* 0: no update in this slot */
-        }
-      }
-      __syncthreads();
-    }
-    if (tid < nw) {
-      const int n_k = s_coff[tid + 1] - s_coff[tid];
-      s_nitems[tid] = (iterations + 1 - p0) * n_k;
-      s_region[tid] = (unsigned long long)stride * (unsigned long long)s_c0[tid];
-      d.world_levels[d.group_worlds[o0 + tid]] = s_wdepth[tid];
-    }
-    __syncthreads();
-  }
-  if (d.phase_clock && tid == 0) d.phase_clock[8 * grp + 1] = clock64();
-  /* 3. counting sort by level into a region of gdesc / ghist */
-  int max_depth = my_depth, tot_items = my_items, tot_hits = my_hits;
-  for (int o = 16; o > 0; o >>= 1) {
-    max_depth = max(max_depth, __shfl_xor_sync(0xffffffffu, max_depth, o));
-    tot_items += __shfl_xor_sync(0xffffffffu, tot_items, o);
-    tot_hits += __shfl_xor_sync(0xffffffffu, tot_hits, o);
-  }
-  if (lane == 0) {
-    s_red[0][wib] = max_depth;
-    s_red[1][wib] = tot_items;
-    s_red[2][wib] = tot_hits;
-  }
-  __syncthreads();
-  max_depth = 0;
-  tot_items = 0;
-  tot_hits = 0;
-#pragma unroll
-  for (int w = 0; w < P; ++w) {
-    max_depth = max(max_depth, s_red[0][w]);
-    tot_items += s_red[1][w];
-    tot_hits += s_red[2][w];
-  }
-  if (tid == 0) {
-    atomicAdd(&d.counters[kCntLevels], (unsigned long long)max_depth);
-    atomicAdd(&d.counters[kCntHits], (unsigned long long)tot_hits);
-    atomicAdd(&d.counters[kCntItems], (unsigned long long)tot_items);
-    s_gbase = (int)atomicAdd(&d.counters[kCntGroupAlloc], (unsigned long long)(tot_items + 1));
-  }
-  __syncthreads();
-  const int gbase = s_gbase;
-  int32_t* gh = d.ghist + gbase;
-  int4* gdesc = d.gdesc + gbase;
-  int32_t* hist = max_depth <= smem_ints ? s_last : gh; /* the last levels are dead by now */
-  for (int t = tid; t < max_depth; t += NT) hist[t] = 0;
-  __syncthreads();
-  for (int k = 0; k < nw; ++k) {
-    const int n_items = s_nitems[k];
-    const size_t region = (size_t)s_region[k];
-#pragma unroll 4
-    for (int t = tid; t < n_items; t += NT) {
-      const int lvl = d.ilevel[region + t];
-      if (!PAR || lvl > 0) atomicAdd(&hist[lvl - 1], 1);
-    }
-  }
-  __syncthreads();
-  if (wib == 0) { /* exclusive scan of the level counts by warp 0 */
-    int carry = 0;
-    for (int t0 = 0; t0 < max_depth; t0 += 32) {
-      const int t = t0 + lane;
-      const int x = t < max_depth ? hist[t] : 0;
-      int incl = x;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += y;
-      }
-      if (t < max_depth) hist[t] = carry + incl - x;
-      carry += __shfl_sync(0xffffffffu, incl, 31);
-    }
-  }
-  __syncthreads();
-  for (int k = 0; k < nw; ++k) {
-    const int n_items = s_nitems[k];
-    const size_t region = (size_t)s_region[k];
-#pragma unroll 4
-    for (int t = tid; t < n_items; t += NT) {
-      const int lvl = d.ilevel[region + t];
-      if (PAR && lvl <= 0) continue;
-      const int4 u = d.idesc[region + t];
-      gdesc[atomicAdd(&hist[lvl - 1], 1)] = u;
-    }
-  }
-  __syncthreads();
-  if (hist != gh)
-    for (int t = tid; t < max_depth; t += NT) gh[t] = hist[t];
-  __syncthreads();
-  if (d.phase_clock && tid == 0) d.phase_clock[8 * grp + 2] = clock64();
-  /* 4. levels, velocities in shared memory when they fit */
-  const bool smem_vel = 6 * group_bodies <= smem_ints;
-  VelStore vs;
-  vs.d = &d;
-  vs.s = smem_vel ? reinterpret_cast<double*>(s_last) : nullptr;
-  if (smem_vel) {
-    for (int k = 0; k < nw; ++k) {
-      const int wld = d.group_worlds[o0 + k];
-      const int b0 = d.world_body_off[wld], b1 = d.world_body_off[wld + 1];
-      for (int g = b0 + tid; g < b1; g += NT) {
-        double* p = vs.s + 3 * (g + s_delta[k]);
-        p[0] = d.vx[g];
-        p[1] = d.vy[g];
-        p[2] = d.w[g];
-      }
-    }
-  }
-  __syncthreads();
-  const int4 none = make_int4(0, 0, 0, 0);
-  int e_prev = 0;
-  int e_cur = max_depth > 0 ? gh[0] : 0;
-  int e_next = max_depth > 1 ? gh[1] : e_cur;
-  int4 cur = tid < e_cur ? gdesc[tid] : none;
-  int4 nxt = e_cur + tid < e_next ? gdesc[e_cur + tid] : none;
-  if (tid < e_cur) prefetch_con(d.con + (cur.x & ~kWarmBit));
-  for (int L = 0; L < max_depth; ++L) {
-    const int e_next2 = L + 2 < max_depth ? gh[L + 2] : e_next;
-    const int4 nxt2 = e_next + tid < tot_items ? gdesc[e_next + tid] : none;
-    if (e_cur + tid < e_next) prefetch_con(d.con + (nxt.x & ~kWarmBit));
-    const int count = e_cur - e_prev;
-    if (tid < count)
-      solve_item(d, (uint32_t)cur.x, cur.y, cur.z, (uint8_t)(cur.w & 0xff), vs, s_delta[cur.w >> 8]);
-    for (int t = tid + NT; t < count; t += NT) { /* levels wider than the CTA */
-      const int4 u = gdesc[e_prev + t];
-      solve_item(d, (uint32_t)u.x, u.y, u.z, (uint8_t)(u.w & 0xff), vs, s_delta[u.w >> 8]);
-    }
-    __syncthreads();
-    cur = nxt;
-    nxt = nxt2;
-    e_prev = e_cur;
-    e_cur = e_next;
-    e_next = e_next2;
-  }
-  if (smem_vel) {
-    for (int k = 0; k < nw; ++k) {
-      const int wld = d.group_worlds[o0 + k];
-      const int b0 = d.world_body_off[wld], b1 = d.world_body_off[wld + 1];
-      for (int g = b0 + tid; g < b1; g += NT) {
-        const double* p = vs.s + 3 * (g + s_delta[k]);
-        d.vx[g] = p[0];
-        d.vy[g] = p[1];
-        d.w[g] = p[2];
-      }
-    }
-  }
-  if (d.phase_clock && tid == 0) {
-    d.phase_clock[8 * grp + 3] = clock64();
-    d.phase_clock[8 * grp + 4] = max_depth;
-    d.phase_clock[8 * grp + 5] = tot_items;
-    d.phase_clock[8 * grp + 6] = group_bodies;
-    d.phase_clock[8 * grp + 7] = nw;
-  }
+/* improveContactSln (Solvers/Contact.hs:124-143) up to the clamps, on one
+ * lane: the impulses to apply and the new accumulated Lagrangians.  Both new
+ * Lagrangians come from the same velocities (contactLagrangian,
+ * Constraints/Contact.hs:86-95; lagrangian2, Constraint.hs:164-169), then
+ * positive / clampAbs (SolutionProcessors.hs:33-53).  Where no_bounce holds and
+ * the velocities are below 2^500 the bounce product is a signed zero and its
+ * minimum with 0 is +0, so b + bounceB is the stored b + 0.0 bit for bit. */
+__device__ __forceinline__ void contact_impulses(const Con* con, const double rn[4], const double rf[4],
+                                                 const double v[6], double2 cached, double* ln, double* lf,
+                                                 double2* now) {
+  double bias = con->bn0;
+  if (!(con->no_bounce && small_velocities(v))) bias = con->bn + bounce_term(con, v);
+  const double ln_new = div_rn(flip_sign(row_dot(rn, v) + bias), con->mc[0], con->rc[0]);
+  const double lf_new = div_rn(flip_sign(plus_zero(row_dot(rf, v))), con->mc[1], con->rc[1]);
+  const double neg_cn = flip_sign(cached.x);
+  *ln = f_le(ln_new, neg_cn) ? neg_cn : ln_new;
+  now->x = cached.x + *ln;
+  now->y = clamp_abs(cached.y + lf_new, now->x * con->mu);
+  *lf = now->y - cached.y;
 }
 
 /* Per-world solver residual after the last sweep: one more improveContactSln
@@ -2861,27 +2069,12 @@ __global__ void __launch_bounds__(32 * P) k_group_solve(Dev d, int iterations, i
  * contact: */
 __device__ __forceinline__ double residual_term(const Dev& d, int c) {
   const int ga = d.c_ga[c], gb = d.c_gb[c];
-  const double2* cp = reinterpret_cast<const double2*>(d.con + c);
-  double j_n[6], j_f[6];
-  const double2 a0 = cp[0], a1 = cp[1], a2 = cp[2], a3 = cp[3], a4 = cp[4], a5 = cp[5];
-  j_n[0] = a0.x; j_n[1] = a0.y; j_n[2] = a1.x; j_n[3] = a1.y; j_n[4] = a2.x; j_n[5] = a2.y;
-  j_f[0] = a3.x; j_f[1] = a3.y; j_f[2] = a4.x; j_f[3] = a4.y; j_f[4] = a5.x; j_f[5] = a5.y;
+  const Con* con = d.con + c;
   const double v[6] = {d.vx[ga], d.vy[ga], d.w[ga], d.vx[gb], d.vy[gb], d.w[gb]};
-  const double2 b6 = cp[6], b7 = cp[7], b8 = cp[8], b9 = cp[9], b10 = cp[10], b11 = cp[11], b12 = cp[12];
-  const double2 cached = reinterpret_cast<const double2*>(d.lam)[c];
-  const double nwa = -v[2];
-  const double cvx = ((-v[0] + (-(nwa * b7.y))) + v[3]) + (-(v[5] * b8.y));
-  const double cvy = ((-v[1] + nwa * b7.x) + v[4]) + v[5] * b8.x;
-  const double tb = b11.y * (cvx * b9.x + cvy * b9.y);
-  const double bias = b6.x + (f_le(0.0, tb) ? 0.0 : tb);
-  const double ln_new = div_rn(-(dot6(j_n, v) + bias), b10.x, b12.x);
-  const double lf_new = div_rn(-plus_zero(dot6(j_f, v)), b10.y, b12.y);
-  const double ln_apply = f_le(ln_new, -cached.x) ? -cached.x : ln_new;
-  const double thr = (cached.x + ln_apply) * b11.x;
-  const double acc = cached.y + lf_new;
-  const double acc2 = f_lt(thr, acc) ? thr : (f_lt(acc, -thr) ? -thr : acc);
-  const double lf_apply = acc2 - cached.y;
-  return ln_apply * ln_apply + lf_apply * lf_apply;
+  double ln, lf;
+  double2 now;
+  contact_impulses(con, con->row[0], con->row[1], v, reinterpret_cast<const double2*>(d.lam)[c], &ln, &lf, &now);
+  return ln * ln + lf * lf;
 }
 
 /* One warp per world (fixed summation order); worlds of `split_from` bodies
