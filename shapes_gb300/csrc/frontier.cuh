@@ -389,18 +389,16 @@ __device__ __forceinline__ void prefetch_l1(const char* p) { asm volatile("prefe
 
 /* An update is spread over two or eight lanes.  Of the lanes' rows, the even
  * lanes carry the normal row and the odd lanes the friction row: its fold, its
- * quotient and its accumulated Lagrangian.  Warm: applySln of the cached
- * Lagrangians (Solvers/Contact.hs:105-113).  Otherwise improveContactSln
+ * quotient and its accumulated Lagrangian `cached`.  Warm: applySln of the
+ * cached Lagrangians (Solvers/Contact.hs:105-113).  Otherwise improveContactSln
  * (Solvers/Contact.hs:124-143), see contact_impulses; adding +0.0 to the
- * friction fold is the reference's `+ 0`.  update_impulse finishes it from the
- * row's fold: the impulses (non-penetration, friction) to apply. */
-template <bool SM>
-__device__ __forceinline__ double2 update_impulse(const int4 u, double dot, double bias, double mc, double rc,
-                                                  double mu, bool live, bool writer, const BodyStore<SM>& bs) {
+ * friction fold is the reference's `+ 0`.  update_impulse finishes an update
+ * from the row's fold: the impulses (non-penetration, friction) to apply, and
+ * the row's new accumulated Lagrangian. */
+__device__ __forceinline__ double2 update_impulse(bool warm, double dot, double bias, double mc, double rc, double mu,
+                                                  double cached, double* now) {
   const unsigned kAll = 0xffffffffu;
-  const bool fric = threadIdx.x & 1, warm = ((uint32_t)u.x & kWarmBit) != 0;
-  double* lam = bs.lagrangians(u) + fric;
-  const double cached = *lam;
+  const bool fric = threadIdx.x & 1;
   const double fresh = div_rn(flip_sign(dot + bias), mc, rc);
   const double neg = flip_sign(cached);
   /* even lanes: the normal impulse, clamped so that the total stays non-negative */
@@ -409,7 +407,7 @@ __device__ __forceinline__ double2 update_impulse(const int4 u, double dot, doub
   const double thr = __shfl_sync(kAll, total * mu, threadIdx.x & 30);
   const double held = clamp_abs(total, thr); /* odd lanes: the friction total */
   const double slide = held - cached;
-  if (writer & live & !warm) *lam = fric ? held : total;
+  *now = fric ? held : total;
   const double mine = warm ? cached : (fric ? slide : amount);
   const double other = __shfl_xor_sync(kAll, mine, 1);
   return fric ? make_double2(other, mine) : make_double2(mine, other);
@@ -467,7 +465,11 @@ __device__ __forceinline__ void solve_pair(const Dev& d, const int4 u, const Lan
   bs.load(u.z, v[3], v[4], v[5]);
   double bias = fric ? 0.0 : k.bn0;
   if (!(k.no_bounce && small_velocities(v)) && !fric) bias = con_of(d, u)->bn + bounce_term(con_of(d, u), v);
-  const double2 l = update_impulse(u, row_dot(k.c, v), bias, k.mc, k.rc, k.mu, live, true, bs);
+  const bool warm = ((uint32_t)u.x & kWarmBit) != 0;
+  double* lam = bs.lagrangians(u) + fric;
+  double now;
+  const double2 l = update_impulse(warm, row_dot(k.c, v), bias, k.mc, k.rc, k.mu, *lam, &now);
+  if (live & !warm) *lam = now;
   /* this lane's body: its row and the other row on it */
   const double sx = fric ? k.c[0] : flip_sign(k.c[0]), sy = fric ? k.c[1] : flip_sign(k.c[1]);
   const double sa = fric ? k.c[3] : k.c[2];
@@ -484,52 +486,74 @@ __device__ __forceinline__ void solve_pair(const Dev& d, const int4 u, const Lan
   if (live && (u.w & (fric ? kInfoDynB : kInfoDynA))) bs.store(fric ? u.z : u.y, x, y, w);
 }
 
-__device__ __forceinline__ void load_split(const Dev& d, const int4 u, LaneConstants& x) {
-  const int j = threadIdx.x & 7, comp = j < 6 ? j : j - 2, side = comp >= 3, k = comp - 3 * side;
-  const int at = k < 2 ? k : 2 + side;
-  const Con* con = con_of(d, u);
+/* Lane j of eight: velocity component, and side and component of the body it
+ * belongs to.  Lanes 6 and 7 repeat 4 and 5 and store nothing. */
+struct SplitLane {
+  int j, side, k, fric;
+  __device__ __forceinline__ SplitLane() {
+    j = threadIdx.x & 7;
+    const int comp = j < 6 ? j : j - 2;
+    side = comp >= 3;
+    k = comp - 3 * side;
+    fric = j & 1;
+  }
+};
+
+__device__ __forceinline__ void load_split(const Con* con, LaneConstants& x) {
+  const SplitLane t;
+  const int at = t.k < 2 ? t.k : 2 + t.side;
   x.c[0] = con->row[0][at];
   x.c[1] = con->row[1][at];
-  x.c[2] = con->im[2 * side + (k == 2)];
-  load_common(con, j & 1, x);
+  x.c[2] = con->im[2 * t.side + (t.k == 2)];
+  load_common(con, t.fric, x);
 }
 
 /* Eight lanes to an update, four updates a warp (all 32 lanes call it, live or
- * not).  Lane j < 6 holds velocity component j of the two bodies (lanes 6 and
- * 7 repeat 4 and 5 and store nothing).  The lanes' products change places so
- * that every even lane has the normal row's six and every odd lane the friction
+ * not): from this lane's velocity component v0 and its row's Lagrangian, the
+ * new component and Lagrangian.  The lanes' products change places so that
+ * every even lane has the normal row's six and every odd lane the friction
  * row's.  20 FP64 instructions. */
-template <bool SM>
-__device__ __forceinline__ void solve_split(const Dev& d, const int4 u, const LaneConstants& x, bool live,
-                                            const BodyStore<SM>& bs) {
+__device__ __forceinline__ double split_update(const Con* con, const LaneConstants& x, bool warm, double v0,
+                                               double cached, double* now) {
   const unsigned kAll = 0xffffffffu;
-  const int j = threadIdx.x & 7, comp = j < 6 ? j : j - 2, side = comp >= 3, k = comp - 3 * side, fric = j & 1;
-  const int s = side ? u.z : u.y;
-  const double v0 = bs.component(s, k);
-  const double jn = comp < 2 ? flip_sign(x.c[0]) : x.c[0], jf = comp < 2 ? flip_sign(x.c[1]) : x.c[1], m = x.c[2];
+  const SplitLane t;
+  const bool flip = t.side == 0 && t.k < 2;
+  const double jn = flip ? flip_sign(x.c[0]) : x.c[0], jf = flip ? flip_sign(x.c[1]) : x.c[1], m = x.c[2];
   const unsigned slow = __ballot_sync(kAll, !((x.no_bounce != 0) & small_mag(v0)));
-  double bias = fric ? 0.0 : x.bn0;
+  double bias = t.fric ? 0.0 : x.bn0;
   if (slow) { /* some update of the warp has a restitution term */
     double v[6];
 #pragma unroll
     for (int q = 0; q < 6; ++q) v[q] = __shfl_sync(kAll, v0, q, 8);
-    if (!fric && ((slow >> (threadIdx.x & 24)) & 0xffu)) bias = con_of(d, u)->bn + bounce_term(con_of(d, u), v);
+    if (!t.fric && ((slow >> (threadIdx.x & 24)) & 0xffu)) bias = con->bn + bounce_term(con, v);
   }
   const double pn = jn * v0, pf = jf * v0;
   /* pairs of lanes trade: an even lane 2 i ends with the normal row's products 2 i and 2 i + 1, its neighbour with the
    * friction row's */
-  const double got = __shfl_xor_sync(kAll, fric ? pn : pf, 1);
-  const double lo = fric ? got : pn, hi = fric ? pf : got;
-  double dot = __shfl_sync(kAll, lo, fric, 8);
-  dot = dot + __shfl_sync(kAll, hi, fric, 8);
-  dot = dot + __shfl_sync(kAll, lo, 2 + fric, 8);
-  dot = dot + __shfl_sync(kAll, hi, 2 + fric, 8);
-  dot = dot + __shfl_sync(kAll, lo, 4 + fric, 8);
-  dot = dot + __shfl_sync(kAll, hi, 4 + fric, 8);
-  const double2 l = update_impulse(u, dot, bias, x.mc, x.rc, x.mu, live, j < 2, bs);
-  double v1 = v0 + (jn * l.x) * m;
-  v1 = v1 + (jf * l.y) * m;
-  if (live && j < 6 && (u.w & (side ? kInfoDynB : kInfoDynA))) bs.set_component(s, k, v1);
+  const double got = __shfl_xor_sync(kAll, t.fric ? pn : pf, 1);
+  const double lo = t.fric ? got : pn, hi = t.fric ? pf : got;
+  double dot = __shfl_sync(kAll, lo, t.fric, 8);
+  dot = dot + __shfl_sync(kAll, hi, t.fric, 8);
+  dot = dot + __shfl_sync(kAll, lo, 2 + t.fric, 8);
+  dot = dot + __shfl_sync(kAll, hi, 2 + t.fric, 8);
+  dot = dot + __shfl_sync(kAll, lo, 4 + t.fric, 8);
+  dot = dot + __shfl_sync(kAll, hi, 4 + t.fric, 8);
+  const double2 l = update_impulse(warm, dot, bias, x.mc, x.rc, x.mu, cached, now);
+  const double v1 = v0 + (jn * l.x) * m;
+  return v1 + (jf * l.y) * m;
+}
+
+template <bool SM>
+__device__ __forceinline__ void solve_split(const Dev& d, const int4 u, const LaneConstants& x, bool live,
+                                            const BodyStore<SM>& bs) {
+  const SplitLane t;
+  const int s = t.side ? u.z : u.y;
+  const bool warm = ((uint32_t)u.x & kWarmBit) != 0;
+  double* lam = bs.lagrangians(u) + t.fric;
+  double now;
+  const double v1 = split_update(con_of(d, u), x, warm, bs.component(s, t.k), *lam, &now);
+  if (live & !warm & (t.j < 2)) *lam = now;
+  if (live && t.j < 6 && (u.w & (t.side ? kInfoDynB : kInfoDynA))) bs.set_component(s, t.k, v1);
 }
 
 /* How a level of `count` updates is dealt: `pairs` chunks of sixteen updates,
@@ -571,7 +595,7 @@ __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, c
   };
   auto load = [&](const Deal& deal, int t, const int4 u, LaneConstants& k) {
     if (t < deal.pairs) load_pair(d, u, k);
-    else load_split(d, u, k);
+    else load_split(con_of(d, u), k);
   };
   int begin = 0;
   bool ahead = false, live = false;

@@ -14,19 +14,21 @@
  *   sweep p (1-based): r = h_a + (p - 1) n_a + r_a(k).
  * Contacts are in descending (i, j) order with i > j the first body, so a
  * pass is a sequence of rows, one per first body i; within a pass no update
- * after i's row touches i.  A row is one unit of work ("ticket"): one lane
- * waits once for i's earlier updates, keeps i's velocity in registers through
- * the row and waits per contact only for the second body's.  Tickets are
- * handed out in the order p S + r (pass p, row r, S the pass skew: row r of
- * pass p + 1 waits on nothing of pass p at a row >= r + S), which puts every
- * wait on an earlier ticket and lets the tickets in flight cover several
- * passes' wavefronts; the earliest unfinished ticket can always run.  Lanes
- * never block: a warp polls each lane's next dependency once and all lanes
- * whose dependency is met run their update together.  Waits are bounded: past
- * the limit the kernel raises an error flag (SHAPES_E_TIMEOUT) that stays set
- * for the rest of the run, and stops.  Velocities and Lagrangians are read
- * and written at L2 (no stale L1 lines across SMs); a release precedes each
- * counter increment and each met count is read with acquire semantics.
+ * after i's row touches i.  A row is one unit of work ("ticket"): eight lanes
+ * wait for i's earlier updates, keep i's velocity in registers through the
+ * row and wait per contact only for the second body's.  Tickets are handed out
+ * in the order p S + r (pass p, row r, S the pass skew: row r of pass p + 1
+ * waits on nothing of pass p at a row >= r + S), which puts every wait on an
+ * earlier ticket and lets the tickets in flight cover several passes'
+ * wavefronts; the earliest unfinished ticket can always run.  Lanes never
+ * block: a warp polls each row's next dependency once and the rows whose
+ * dependency is met run their updates together (split_update, eight lanes
+ * each).
+ * A velocity component travels with its body's completion count in one 16-byte
+ * word, a Lagrangian with its pass, so that one load at L2 both finds whether
+ * the update may run and brings its operand: no fences, no separate counters.
+ * Waits are bounded: past the limit the kernel raises an error flag
+ * (SHAPES_E_TIMEOUT) that stays set for the rest of the run, and stops.
  * Static bodies take no part in the ordering (they are never written).
  * Results are bit-identical to the sequential sweep.
  *
@@ -38,8 +40,8 @@
  * residual and penetration.
  */
 #pragma once
+#include "frontier.cuh"
 #include "lw_order.cuh"
-#include "step_kernels.cuh"
 
 namespace shapes {
 
@@ -55,7 +57,8 @@ struct LW {
   int32_t* hrank;           /* [2 nc] hr_s(k) */
   int32_t* bh;              /* [nb] hits per body */
   int32_t* bn;              /* [nb] contacts per body */
-  int32_t* done;            /* [nb] completed updates per body */
+  ulonglong2* vel;          /* [3 nb] ordered path: {velocity component, updates of the body completed} */
+  ulonglong2* lag;          /* [2 nc] ordered path: {Lagrangian, pass that wrote it} */
   int32_t* hitflag;         /* [nc] */
   int32_t* hitoff;          /* [nc + 1] scanned */
   int32_t* color;           /* [nc] */
@@ -72,14 +75,20 @@ struct LW {
   int4* side;               /* [2 nc] per contact side: see k_lw_side */
 };
 
-__device__ __forceinline__ int32_t ld_acquire_gpu(const int32_t* p) {
-  int32_t v;
-  asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+/* 16-byte words read and written whole, at L2 (other SMs write them). */
+__device__ __forceinline__ ulonglong2 ld_word(const ulonglong2* p) {
+  ulonglong2 v;
+  asm volatile("{\n\t.reg .b128 q;\n\tld.relaxed.gpu.global.b128 q, [%2];\n\tmov.b128 {%0, %1}, q;\n\t}"
+               : "=l"(v.x), "=l"(v.y)
+               : "l"(p)
+               : "memory");
   return v;
 }
 
-__device__ __forceinline__ void red_release_gpu_add(int32_t* p, int32_t v) {
-  asm volatile("red.release.gpu.global.add.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+__device__ __forceinline__ void st_word(ulonglong2* p, double x, uint64_t tag) {
+  asm volatile("{\n\t.reg .b128 q;\n\tmov.b128 q, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], q;\n\t}" ::"l"(p),
+               "l"(__double_as_longlong(x)), "l"(tag)
+               : "memory");
 }
 
 constexpr int kMaxColors = 64;
@@ -160,7 +169,6 @@ __global__ void k_lw_rank(Dev d, LW w) {
     }
     w.bh[b] = hits;
     w.bn[b] = r1 - r0;
-    w.done[b] = 0;
   }
 }
 
@@ -266,22 +274,60 @@ __global__ void k_lw_side(Dev d, LW w) {
 
 __device__ __forceinline__ int lw_want(int4 e, int pass) { return pass == 0 ? e.y : e.z + pass * e.w; }
 
+/* The ordered path's words: velocities after gravity with no update completed,
+ * Lagrangians of pass 0. */
+__global__ void k_lw_begin(Dev d, LW w, int external, double ax, double ay, double dt) {
+  lw_range(w);
+  const int stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int b = t0; b < w.nb; b += stride) {
+    const int g = w.b0 + b;
+    double vx = d.vx[g], vy = d.vy[g];
+    if (external && !(0.0 == d.iml[g]) && !(d.flags[g] & kFlagInactive)) {
+      vx = vx + ax * dt;
+      vy = vy + ay * dt;
+    }
+    w.vel[3 * (size_t)b] = make_ulonglong2((uint64_t)__double_as_longlong(vx), 0);
+    w.vel[3 * (size_t)b + 1] = make_ulonglong2((uint64_t)__double_as_longlong(vy), 0);
+    w.vel[3 * (size_t)b + 2] = make_ulonglong2((uint64_t)__double_as_longlong(d.w[g]), 0);
+  }
+  for (int q = t0; q < 2 * w.nc; q += stride)
+    w.lag[q] = make_ulonglong2((uint64_t)__double_as_longlong(d.lam[2 * (size_t)w.c0 + q]), 0);
+}
+
+__global__ void k_lw_end(Dev d, LW w) {
+  if (d.counters[kCntOverflow]) return;
+  lw_range(w);
+  const int stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int b = t0; b < w.nb; b += stride) {
+    const int g = w.b0 + b;
+    d.vx[g] = __longlong_as_double((long long)w.vel[3 * (size_t)b].x);
+    d.vy[g] = __longlong_as_double((long long)w.vel[3 * (size_t)b + 1].x);
+    d.w[g] = __longlong_as_double((long long)w.vel[3 * (size_t)b + 2].x);
+  }
+  for (int q = t0; q < 2 * w.nc; q += stride)
+    d.lam[2 * (size_t)w.c0 + q] = __longlong_as_double((long long)w.lag[q].x);
+}
+
 /* The ordered solve of one large world.  Rows are tickets in the skewed order
- * (lw_ticket); a lane holds one row: it waits for the row's first body i,
- * then runs the row's contacts in order with i's velocity in registers,
- * waiting before each for the second body's earlier updates, and finally
- * stores i's velocity and releases i's counter by the row's update count.
- * No lane blocks: each pass of a warp's loop polls every lane's next
- * dependency once, then all lanes whose dependency is met run their update
- * together (the FP64 pipe charges a warp instruction in full however few
- * lanes it carries, so lanes that spin and then solve alone pay for every
- * update separately).  A lane whose row is finished takes the next ticket on
+ * (lw_ticket); eight lanes hold one row: lanes 0-2 wait for the row's first
+ * body i and keep its velocity, lanes 3-5 wait for each contact's second body
+ * and hand its velocity on after the update, lanes 0 and 1 do so with the
+ * contact's Lagrangians; at the end of the row lanes 0-2 hand i on, its count
+ * raised by the row's updates.  No lane blocks: each pass of a warp's loop
+ * polls what every row still waits for once, then the rows that have all of it
+ * run their update together.  A row that is finished takes the next ticket on
  * the following pass (one atomic per warp).  The earliest unfinished ticket
  * finds its dependencies met on its warp's next poll, so the solve always
- * progresses; a lane that polls one dependency poll_limit times (default
- * kPollLimit, shapes_batch_set_wait_limit) raises the
- * timeout flag and every warp returns. */
-constexpr int kOrderedThreads = 128;
+ * progresses; a row that polls one dependency poll_limit times (default
+ * kPollLimit, shapes_batch_set_wait_limit) raises the timeout flag and every
+ * warp returns.
+ * What bounds it: the chain of dependent updates, each a hand-over through L2
+ * and 20 FP64 instructions of 64 cycles, and how far the rows in flight reach
+ * along the ticket order.  A settled pile of 32,771 bodies (1518 levels, 562 k
+ * updates a step): 7.13 ms with a row on one lane, counters beside the
+ * velocities and fences between them; 3.07 ms so.  Rows in flight (rows an SM:
+ * time): 4: 8.1 ms, 16: 3.83, 32: 3.32, 64: 3.07, 64 in one block: 3.29. */
+constexpr int kOrderedThreads = 256;
 constexpr long long kPollLimit = 1ll << 22; /* polls of one dependency before giving up */
 constexpr int kOrderedBlocksPerSM = 2;
 
@@ -291,107 +337,108 @@ __global__ void __launch_bounds__(kOrderedThreads) k_lw_ordered(Dev d, LW w, int
   lw_range(w);
   const unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
+  const unsigned row_mask = 0xffu << (lane & 24), leaders_below = 0x01010101u & ((1u << (lane & 24)) - 1u);
+  const SplitLane t;
   const int n_rows = w.rowoff[w.nc];
   const int passes = warm_start ? iterations + 1 : iterations;
   const long long total = (long long)passes * n_rows;
   const int skew = max(1, min((int)w.ctl[3], n_rows));
-  bool has = false, exhausted = total == 0, dyn_i = false;
-  int stage = 0, pass = 0, k = 0, k1 = 0, m = 0, gi = 0, want_i = 0;
-  int4 cur = make_int4(0, -1, 0, 0); /* side entry of contact k's second body */
-  double vi[3] = {0.0, 0.0, 0.0};
+  /* the same in the eight lanes of a row */
+  bool has = false, exhausted = total == 0;
+  int pass = 0, k = 0, k1 = 0;
   long long polls = 0;
+  /* this lane's */
+  int m = 0;              /* updates of the row (lanes of i) */
+  int4 side = make_int4(0, -1, 0, 0);
+  bool have_v = false, have_l = false;
+  double v = 0.0, cached = 0.0;
+  LaneConstants x;
+  const Con* con = d.con;
   int empty = 0;
+  auto take_contact = [&]() { /* contact k of the row becomes current: what this lane waits for, and its constants */
+    if (t.side) {
+      side = w.side[(k << 1) | 1];
+      have_v = false;
+    }
+    have_l = false;
+    con = d.con + w.c0 + k;
+    load_split(con, x);
+  };
   for (;;) {
-    if (!exhausted) { /* lanes without a row take the next tickets, in order */
-      const unsigned need = __ballot_sync(kAll, !has);
+    if (!exhausted) { /* rows that are free take the next tickets, in order */
+      const unsigned need = __ballot_sync(kAll, !has) & 0x01010101u;
       if (need) {
-        const int leader = __ffs(need) - 1;
         unsigned long long base = 0;
-        if (lane == leader) base = atomicAdd(&w.ctl[0], (unsigned long long)__popc(need));
-        base = __shfl_sync(kAll, base, leader);
-        const long long t = (long long)base + __popc(need & below);
-        if (!has && t < total) {
+        if (lane == 0) base = atomicAdd(&w.ctl[0], (unsigned long long)__popc(need));
+        base = __shfl_sync(kAll, base, 0);
+        const long long ticket = (long long)base + __popc(need & leaders_below);
+        if (!has && ticket < total) {
           int pi, r;
-          lw_ticket(t, passes, skew, n_rows, pi, r);
+          lw_ticket(ticket, passes, skew, n_rows, pi, r);
           pass = pi + (warm_start ? 0 : 1);
-          const int k0 = w.row_start[r];
+          k = w.row_start[r];
           k1 = r + 1 < n_rows ? w.row_start[r + 1] : w.nc;
-          k = k0;
-          m = k1 - k0;
+          m = k1 - k;
           if (pass == 0) { /* the warm-start pass updates the cache hits only */
             while (k < k1 && !w.hitflag[k]) ++k;
             m = 0;
-            for (int x = k; x < k1; ++x) m += w.hitflag[x];
+            for (int q = k; q < k1; ++q) m += w.hitflag[q];
           }
           if (m > 0) {
             has = true;
-            stage = 0;
             polls = 0;
-            const int4 e0 = w.side[k << 1];
-            gi = e0.x;
-            dyn_i = e0.y >= 0;
-            want_i = lw_want(e0, pass);
-            cur = w.side[(k << 1) | 1];
+            have_v = false;
+            if (!t.side) side = w.side[k << 1];
+            take_contact();
           }
         }
         if ((long long)base + __popc(need) >= total) exhausted = true;
       }
     }
     if (exhausted && !__any_sync(kAll, has)) break;
-    /* poll each lane's next dependency once */
-    bool ready = false;
-    if (has && stage == 0 && (!dyn_i || ld_acquire_gpu(w.done + (gi - w.b0)) == want_i)) {
-      vi[0] = __ldcg(d.vx + gi);
-      vi[1] = __ldcg(d.vy + gi);
-      vi[2] = __ldcg(d.w + gi);
-      stage = 1;
-      polls = 0;
+    /* poll what this lane still waits for, once */
+    if (has && !have_v) {
+      const ulonglong2 q = ld_word(w.vel + 3 * (size_t)(side.x - w.b0) + t.k);
+      have_v = side.y < 0 || q.y == (uint64_t)lw_want(side, pass);
+      if (have_v) v = __longlong_as_double((long long)q.x);
     }
-    const bool dyn_j = cur.y >= 0;
-    if (has && stage == 1) ready = !dyn_j || ld_acquire_gpu(w.done + (cur.x - w.b0)) == lw_want(cur, pass);
-    /* the ready lanes' updates, together */
-    if (ready) {
-      int kn = k + 1; /* the next contact's side entry, fetched beside the update */
-      if (pass == 0)
-        while (kn < k1 && !w.hitflag[kn]) ++kn;
-      const int4 nxt = kn < k1 ? w.side[(kn << 1) | 1] : cur;
-      const int c = w.c0 + k, gb = cur.x;
-      double v[6] = {vi[0], vi[1], vi[2], __ldcg(d.vx + gb), __ldcg(d.vy + gb), __ldcg(d.w + gb)};
-      lw_contact_math(d.con + c, v, reinterpret_cast<double2*>(d.lam) + c, pass == 0);
-      if (dyn_i) {
-        vi[0] = v[0];
-        vi[1] = v[1];
-        vi[2] = v[2];
-      }
-      if (dyn_j) {
-        __stcg(d.vx + gb, v[3]);
-        __stcg(d.vy + gb, v[4]);
-        __stcg(d.w + gb, v[5]);
-        red_release_gpu_add(w.done + (gb - w.b0), 1);
-      }
-      k = kn;
-      cur = nxt;
-      polls = 0;
-      if (k >= k1) {
-        if (dyn_i) {
-          __stcg(d.vx + gi, vi[0]);
-          __stcg(d.vy + gi, vi[1]);
-          __stcg(d.w + gi, vi[2]);
-          red_release_gpu_add(w.done + (gi - w.b0), m); /* release: the row's writes of i before the counter */
+    if (has && !have_l) {
+      const ulonglong2 q = ld_word(w.lag + 2 * (size_t)k + t.fric);
+      have_l = q.y == (uint64_t)(pass > 0 ? pass - 1 : 0);
+      if (have_l) cached = __longlong_as_double((long long)q.x);
+    }
+    const unsigned have = __ballot_sync(kAll, has & have_v & have_l);
+    const bool ready = (have & row_mask) == row_mask;
+    if (__any_sync(kAll, ready)) {
+      double now;
+      const double v1 = split_update(con, x, pass == 0, ready ? v : 0.0, ready ? cached : 0.0, &now);
+      if (ready) {
+        const bool dynamic = side.y >= 0;
+        if (dynamic) v = v1;
+        if (t.j < 2 && pass > 0) st_word(w.lag + 2 * (size_t)k + t.fric, now, (uint64_t)pass);
+        if (t.side && t.j < 6 && dynamic)
+          st_word(w.vel + 3 * (size_t)(side.x - w.b0) + t.k, v, (uint64_t)lw_want(side, pass) + 1);
+        ++k;
+        if (pass == 0)
+          while (k < k1 && !w.hitflag[k]) ++k;
+        polls = 0;
+        if (k < k1) {
+          take_contact();
+        } else {
+          if (!t.side && dynamic)
+            st_word(w.vel + 3 * (size_t)(side.x - w.b0) + t.k, v, (uint64_t)lw_want(side, pass) + (uint64_t)m);
+          has = false;
         }
-        has = false;
       }
-    } else if (has && ++polls > poll_limit) {
-      atomicExch(&w.ctl[1], 1ull);
-    }
-    if (!__any_sync(kAll, ready)) {
-      const unsigned long long flag = *reinterpret_cast<volatile unsigned long long*>(&w.ctl[1]);
-      if (__shfl_sync(kAll, flag, 0)) break; /* an update timed out */
-      if (++empty > 16) __nanosleep(64);
-    } else {
       empty = 0;
+    } else {
+      if ((++empty & 15) == 0) {
+        const unsigned long long flag = *reinterpret_cast<volatile unsigned long long*>(&w.ctl[1]);
+        if (__shfl_sync(kAll, flag, 0)) break; /* an update timed out */
+      }
+      if (empty > 64) __nanosleep(64);
     }
+    if (has && !ready && ++polls > poll_limit) atomicExch(&w.ctl[1], 1ull);
   }
 }
 

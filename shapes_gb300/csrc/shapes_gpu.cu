@@ -27,7 +27,6 @@
 
 #include "../../include/shapes_gpu.h"
 #include "step_kernels.cuh"
-#include "frontier.cuh"
 #include "large_world.cuh"
 #include "learned.cuh"
 #include "mlp.h"
@@ -259,7 +258,8 @@ struct shapes_batch {
   int32_t* lw_bstart = nullptr;
   int32_t* lw_bh = nullptr;
   int32_t* lw_bn = nullptr;
-  int32_t* lw_done = nullptr;
+  ulonglong2* lw_vel = nullptr; /* ordered path: velocities and Lagrangians with their counts */
+  ulonglong2* lw_lag = nullptr;
   int32_t* lw_refs = nullptr;
   int32_t* lw_rank = nullptr;
   int32_t* lw_hrank = nullptr;
@@ -599,7 +599,8 @@ struct shapes_batch {
     dfree(snap_key); dfree(snap_lam);
     free_row_buffers();
     dfree(lw_refs); dfree(lw_rank); dfree(lw_hrank); dfree(lw_hitflag); dfree(lw_hitoff);
-    dfree(lw_rowflag); dfree(lw_rowoff); dfree(lw_row_start); dfree(lw_side);
+    dfree(lw_rowflag); dfree(lw_rowoff); dfree(lw_row_start); dfree(lw_side); dfree(lw_lag);
+    lw_lag = nullptr;
     lw_rowflag = lw_rowoff = lw_row_start = nullptr;
     lw_side = nullptr;
     dfree(lw_color); dfree(lw_color_list); dfree(lw_seqflag); dfree(lw_seqoff); dfree(lw_seq_list);
@@ -672,6 +673,7 @@ struct shapes_batch {
       lw_rowoff = dalloc<int32_t>((size_t)contact_cap + 1, "cudaMalloc large world");
       lw_row_start = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
       lw_side = dalloc<int4>(2 * (size_t)contact_cap, "cudaMalloc large world");
+      lw_lag = dalloc<ulonglong2>(2 * (size_t)contact_cap, "cudaMalloc large world");
       lw_color = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
       lw_color_list = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
       lw_seqflag = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
@@ -766,8 +768,9 @@ struct shapes_batch {
   /* Worlds with at least large_world_bodies bodies are solved by the
    * large-world paths; their per-body scratch is sized for the largest. */
   void setup_large_worlds() {
-    dfree(lw_bcnt); dfree(lw_bstart); dfree(lw_bh); dfree(lw_bn); dfree(lw_done); dfree(lw_color_cnt); dfree(lw_ctl);
-    lw_bcnt = lw_bstart = lw_bh = lw_bn = lw_done = lw_color_cnt = nullptr;
+    dfree(lw_bcnt); dfree(lw_bstart); dfree(lw_bh); dfree(lw_bn); dfree(lw_vel); dfree(lw_color_cnt); dfree(lw_ctl);
+    lw_bcnt = lw_bstart = lw_bh = lw_bn = lw_color_cnt = nullptr;
+    lw_vel = nullptr;
     lw_ctl = nullptr;
     large_worlds.clear();
     lw_nb_max = 0;
@@ -783,7 +786,7 @@ struct shapes_batch {
     lw_bstart = dalloc<int32_t>((size_t)lw_nb_max + 1, "cudaMalloc large world");
     lw_bh = dalloc<int32_t>(lw_nb_max, "cudaMalloc large world");
     lw_bn = dalloc<int32_t>(lw_nb_max, "cudaMalloc large world");
-    lw_done = dalloc<int32_t>(lw_nb_max, "cudaMalloc large world");
+    lw_vel = dalloc<ulonglong2>(3 * (size_t)lw_nb_max, "cudaMalloc large world");
     lw_color_cnt = dalloc<int32_t>(shapes::kMaxColors + 1, "cudaMalloc large world");
     lw_ctl = dalloc<unsigned long long>(8 * large_worlds.size(), "cudaMalloc large world");
     ck(cudaMemset(lw_ctl, 0, sizeof(unsigned long long) * 8 * large_worlds.size()), "memset");
@@ -802,7 +805,8 @@ struct shapes_batch {
     w.hrank = lw_hrank;
     w.bh = lw_bh;
     w.bn = lw_bn;
-    w.done = lw_done;
+    w.vel = lw_vel;
+    w.lag = lw_lag;
     w.hitflag = lw_hitflag;
     w.hitoff = lw_hitoff;
     w.rowflag = lw_rowflag;
@@ -893,14 +897,17 @@ struct shapes_batch {
     });
     const int passes = cfg.iterations + (cfg.warm_start ? 1 : 0);
     const int colour_launches = 1 + 128 + 1 + 3 + 1 + 3 + 1 + passes * (shapes::kSeqColor + 1);
-    stage(4, (ordered ? 1 : colour_launches) + (cfg.external ? 1 : 0), [&]() {
-      if (cfg.external)
-        shapes::k_lw_gravity<<<grid_for(w.nb, 256), 256, 0, stream>>>(d, w, cfg.accel_x, cfg.accel_y, cfg.dt);
+    stage(4, ordered ? 3 : colour_launches + (cfg.external ? 1 : 0), [&]() {
       if (ordered) {
+        shapes::k_lw_begin<<<grid_for(2LL * cap, 256), 256, 0, stream>>>(d, w, cfg.external, cfg.accel_x, cfg.accel_y,
+                                                                         cfg.dt);
         shapes::k_lw_ordered<<<kSMs * shapes::kOrderedBlocksPerSM, shapes::kOrderedThreads, 0, stream>>>(
             d, w, cfg.iterations, cfg.warm_start, lw_poll_limit);
+        shapes::k_lw_end<<<grid_for(2LL * cap, 256), 256, 0, stream>>>(d, w);
         return;
       }
+      if (cfg.external)
+        shapes::k_lw_gravity<<<grid_for(w.nb, 256), 256, 0, stream>>>(d, w, cfg.accel_x, cfg.accel_y, cfg.dt);
       shapes::k_lw_color_init<<<grid_for(cap, 256), 256, 0, stream>>>(w);
       /* Jones-Plassmann rounds until every contact has a colour (rounds after
        * that return at once; whatever is left after the last goes to the
@@ -1548,7 +1555,7 @@ struct shapes_batch {
     dfree(np_cls);
     dfree(export_keys);
     dfree(export_vals);
-    dfree(lw_bcnt); dfree(lw_bstart); dfree(lw_bh); dfree(lw_bn); dfree(lw_done); dfree(lw_color_cnt); dfree(lw_ctl);
+    dfree(lw_bcnt); dfree(lw_bstart); dfree(lw_bh); dfree(lw_bn); dfree(lw_vel); dfree(lw_color_cnt); dfree(lw_ctl);
     dfree(world_residual);
     dfree(world_depth);
     dfree(learned_mask); dfree(judge_res); dfree(judge_depth);
