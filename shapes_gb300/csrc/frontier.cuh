@@ -373,6 +373,8 @@ struct BodyStore {
       d->vx[s] = x; d->vy[s] = y; d->w[s] = w;
     }
   }
+  __device__ __forceinline__ double lagrangian(const int4 u, int fric) const { return lagrangians(u)[fric]; }
+  __device__ __forceinline__ void set_lagrangian(const int4 u, int fric, double x) const { lagrangians(u)[fric] = x; }
   __device__ __forceinline__ double component(int s, int k) const {
     if (SM) return vel[3 * s + k];
     return k == 0 ? d->vx[s] : (k == 1 ? d->vy[s] : d->w[s]);
@@ -456,9 +458,9 @@ __device__ __forceinline__ void load_pair(const Dev& d, const int4 u, LaneConsta
  * all six velocity components, then moves one body (the even lane a, the odd
  * lane b).  36 FP64 instructions for sixteen updates; one lane to an update
  * took 65 for 32, the same pipe time for twice the latency. */
-template <bool SM>
+template <class Store>
 __device__ __forceinline__ void solve_pair(const Dev& d, const int4 u, const LaneConstants& k, bool live,
-                                           const BodyStore<SM>& bs) {
+                                           const Store& bs) {
   const int fric = threadIdx.x & 1;
   double v[6];
   bs.load(u.y, v[0], v[1], v[2]);
@@ -466,10 +468,9 @@ __device__ __forceinline__ void solve_pair(const Dev& d, const int4 u, const Lan
   double bias = fric ? 0.0 : k.bn0;
   if (!(k.no_bounce && small_velocities(v)) && !fric) bias = con_of(d, u)->bn + bounce_term(con_of(d, u), v);
   const bool warm = ((uint32_t)u.x & kWarmBit) != 0;
-  double* lam = bs.lagrangians(u) + fric;
   double now;
-  const double2 l = update_impulse(warm, row_dot(k.c, v), bias, k.mc, k.rc, k.mu, *lam, &now);
-  if (live & !warm) *lam = now;
+  const double2 l = update_impulse(warm, row_dot(k.c, v), bias, k.mc, k.rc, k.mu, bs.lagrangian(u, fric), &now);
+  if (live & !warm) bs.set_lagrangian(u, fric, now);
   /* this lane's body: its row and the other row on it */
   const double sx = fric ? k.c[0] : flip_sign(k.c[0]), sy = fric ? k.c[1] : flip_sign(k.c[1]);
   const double sa = fric ? k.c[3] : k.c[2];
@@ -549,10 +550,9 @@ __device__ __forceinline__ void solve_split(const Dev& d, const int4 u, const La
   const SplitLane t;
   const int s = t.side ? u.z : u.y;
   const bool warm = ((uint32_t)u.x & kWarmBit) != 0;
-  double* lam = bs.lagrangians(u) + t.fric;
   double now;
-  const double v1 = split_update(con_of(d, u), x, warm, bs.component(s, t.k), *lam, &now);
-  if (live & !warm & (t.j < 2)) *lam = now;
+  const double v1 = split_update(con_of(d, u), x, warm, bs.component(s, t.k), bs.lagrangian(u, t.fric), &now);
+  if (live & !warm & (t.j < 2)) bs.set_lagrangian(u, t.fric, now);
   if (live && t.j < 6 && (u.w & (t.side ? kInfoDynB : kInfoDynA))) bs.set_component(s, t.k, v1);
 }
 

@@ -264,17 +264,12 @@ struct shapes_batch {
   int32_t* lw_rank = nullptr;
   int32_t* lw_hrank = nullptr;
   int32_t* lw_hitflag = nullptr;
-  int32_t* lw_hitoff = nullptr;
   int32_t* lw_rowflag = nullptr; /* ordered path by rows: row starts (flag, scanned, list) */
   int32_t* lw_rowoff = nullptr;
   int32_t* lw_row_start = nullptr;
   int4* lw_side = nullptr;
   int32_t* lw_color = nullptr;
   int32_t* lw_color_cnt = nullptr;
-  int32_t* lw_color_list = nullptr;
-  int32_t* lw_seqflag = nullptr;
-  int32_t* lw_seqoff = nullptr;
-  int32_t* lw_seq_list = nullptr;
   unsigned long long* lw_ctl = nullptr; /* 8 per large world */
   int32_t worlds_per_group_override = 0;
   int32_t target_group_bodies = 0;
@@ -598,14 +593,13 @@ struct shapes_batch {
     dfree(tile_sums);
     dfree(snap_key); dfree(snap_lam);
     free_row_buffers();
-    dfree(lw_refs); dfree(lw_rank); dfree(lw_hrank); dfree(lw_hitflag); dfree(lw_hitoff);
+    dfree(lw_refs); dfree(lw_rank); dfree(lw_hrank); dfree(lw_hitflag);
     dfree(lw_rowflag); dfree(lw_rowoff); dfree(lw_row_start); dfree(lw_side); dfree(lw_lag);
     lw_lag = nullptr;
     lw_rowflag = lw_rowoff = lw_row_start = nullptr;
     lw_side = nullptr;
-    dfree(lw_color); dfree(lw_color_list); dfree(lw_seqflag); dfree(lw_seqoff); dfree(lw_seq_list);
-    lw_refs = lw_rank = lw_hrank = lw_hitflag = lw_hitoff = lw_color = lw_color_list = nullptr;
-    lw_seqflag = lw_seqoff = lw_seq_list = nullptr;
+    dfree(lw_color);
+    lw_refs = lw_rank = lw_hrank = lw_hitflag = lw_color = nullptr;
     pair_a = pair_b = slot_cnt = slot_off = slot_feat = nullptr;
     slot_val = nullptr;
     c_key[0] = c_key[1] = nullptr;
@@ -668,17 +662,12 @@ struct shapes_batch {
       lw_rank = dalloc<int32_t>(2 * (size_t)contact_cap, "cudaMalloc large world");
       lw_hrank = dalloc<int32_t>(2 * (size_t)contact_cap, "cudaMalloc large world");
       lw_hitflag = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
-      lw_hitoff = dalloc<int32_t>((size_t)contact_cap + 1, "cudaMalloc large world");
       lw_rowflag = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
       lw_rowoff = dalloc<int32_t>((size_t)contact_cap + 1, "cudaMalloc large world");
       lw_row_start = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
       lw_side = dalloc<int4>(2 * (size_t)contact_cap, "cudaMalloc large world");
       lw_lag = dalloc<ulonglong2>(2 * (size_t)contact_cap, "cudaMalloc large world");
       lw_color = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
-      lw_color_list = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
-      lw_seqflag = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
-      lw_seqoff = dalloc<int32_t>((size_t)contact_cap + 1, "cudaMalloc large world");
-      lw_seq_list = dalloc<int32_t>(contact_cap, "cudaMalloc large world");
     }
     snap_cap = contact_cap;
     snap_key = dalloc<uint64_t>(snap_cap, "cudaMalloc snapshot");
@@ -808,17 +797,12 @@ struct shapes_batch {
     w.vel = lw_vel;
     w.lag = lw_lag;
     w.hitflag = lw_hitflag;
-    w.hitoff = lw_hitoff;
     w.rowflag = lw_rowflag;
     w.rowoff = lw_rowoff;
     w.row_start = lw_row_start;
     w.side = lw_side;
     w.color = lw_color;
     w.color_cnt = lw_color_cnt;
-    w.color_list = lw_color_list;
-    w.seqflag = lw_seqflag;
-    w.seqoff = lw_seqoff;
-    w.seq_list = lw_seq_list;
     w.ctl = lw_ctl + 8 * k;
     return w;
   }
@@ -878,26 +862,18 @@ struct shapes_batch {
     shapes::LW w = lw_view(k);
     const int cap = contact_cap;
     const bool ordered = !(cfg.flags & SHAPES_FLAG_COLOURED);
-    stage(3, ordered ? 18 : 11, [&]() {
+    stage(3, ordered ? 11 : 7, [&]() {
       shapes::k_lw_setup<<<grid_for(w.nb + 1, 256), 256, 0, stream>>>(d, w);
-      shapes::k_lw_count<<<grid_for(cap, 256), 256, 0, stream>>>(d, w);
+      shapes::k_lw_count<<<grid_for(cap, 256), 256, 0, stream>>>(d, w, cfg.iterations);
       scan_raw(w.bcnt, w.nb, nullptr, w.bstart);
       shapes::k_lw_scatter<<<grid_for(cap, 256), 256, 0, stream>>>(d, w);
       shapes::k_lw_rank<<<grid_for(w.nb, 128), 128, 0, stream>>>(d, w);
-      scan_raw(w.hitflag, cap, w.ctl + 4, w.hitoff);
-      shapes::k_lw_item_counts<<<1, 1, 0, stream>>>(w, counters + shapes::kCntHits, counters + shapes::kCntItems,
-                                                    cfg.iterations);
-      if (ordered) { /* the sequence's rows (runs of contacts with one first body), pass skew, side entries */
-        shapes::k_lw_rowflag<<<grid_for(cap, 256), 256, 0, stream>>>(d, w);
+      if (ordered) { /* the sequence's rows, pass skew, side entries */
         scan_raw(w.rowflag, cap, w.ctl + 4, w.rowoff);
-        shapes::k_lw_row_list<<<grid_for(cap, 256), 256, 0, stream>>>(w);
-        shapes::k_lw_skew<<<grid_for(cap, 256), 256, 0, stream>>>(d, w);
-        shapes::k_lw_side<<<grid_for(2 * cap, 256), 256, 0, stream>>>(d, w);
+        shapes::k_lw_rows<<<grid_for(cap, 256), 256, 0, stream>>>(d, w);
       }
     });
-    const int passes = cfg.iterations + (cfg.warm_start ? 1 : 0);
-    const int colour_launches = 1 + 128 + 1 + 3 + 1 + 3 + 1 + passes * (shapes::kSeqColor + 1);
-    stage(4, ordered ? 3 : colour_launches + (cfg.external ? 1 : 0), [&]() {
+    stage(4, ordered ? 3 : 1, [&]() {
       if (ordered) {
         shapes::k_lw_begin<<<grid_for(2LL * cap, 256), 256, 0, stream>>>(d, w, cfg.external, cfg.accel_x, cfg.accel_y,
                                                                          cfg.dt);
@@ -906,23 +882,18 @@ struct shapes_batch {
         shapes::k_lw_end<<<grid_for(2LL * cap, 256), 256, 0, stream>>>(d, w);
         return;
       }
-      if (cfg.external)
-        shapes::k_lw_gravity<<<grid_for(w.nb, 256), 256, 0, stream>>>(d, w, cfg.accel_x, cfg.accel_y, cfg.dt);
-      shapes::k_lw_color_init<<<grid_for(cap, 256), 256, 0, stream>>>(w);
-      /* Jones-Plassmann rounds until every contact has a colour (rounds after
-       * that return at once; whatever is left after the last goes to the
-       * sequential colour) */
-      for (int r = 0; r < 128; ++r) shapes::k_lw_color_round<<<grid_for(cap, 256), 256, 0, stream>>>(d, w, r);
-      shapes::k_lw_color_count<<<grid_for(cap, 256), 256, 0, stream>>>(w);
-      scan_raw(w.color_cnt, shapes::kMaxColors, nullptr, w.color_cnt);
-      shapes::k_lw_color_scatter<<<grid_for(cap, 256), 256, 0, stream>>>(w);
-      scan_raw(w.seqflag, cap, w.ctl + 4, w.seqoff);
-      shapes::k_lw_seq_list<<<grid_for(cap, 256), 256, 0, stream>>>(w);
-      for (int pass = cfg.warm_start ? 0 : 1; pass <= cfg.iterations; ++pass) {
-        for (int col = 0; col < shapes::kSeqColor; ++col)
-          shapes::k_lw_color_pass<<<grid_for(cap / 8 + 1, 128), 128, 0, stream>>>(d, w, col, pass == 0);
-        shapes::k_lw_color_seq<<<1, 32, 0, stream>>>(d, w, pass == 0);
-      }
+      cudaLaunchConfig_t lc{};
+      lc.gridDim = dim3(num_sms() * shapes::kColourBlocksPerSM);
+      lc.blockDim = dim3(shapes::kColourThreads);
+      lc.stream = stream;
+      cudaLaunchAttribute at[1];
+      at[0].id = cudaLaunchAttributeCooperative;
+      at[0].val.cooperative = 1;
+      lc.attrs = at;
+      lc.numAttrs = 1;
+      ck(cudaLaunchKernelEx(&lc, shapes::k_lw_coloured, d, w, cfg.iterations, cfg.warm_start, cfg.external, cfg.accel_x,
+                            cfg.accel_y, cfg.dt),
+         "k_lw_coloured");
     });
   }
 
