@@ -381,7 +381,7 @@ void shapes_batch_destroy(shapes_batch* b);
  * library routine.
  *   Limits: n_bodies <= SHAPES_NOALLOC_MAX_BODIES, n_verts <=
  *   SHAPES_NOALLOC_MAX_VERTS, broadphase pairs <= SHAPES_NOALLOC_MAX_PAIRS;
- *   beyond them it returns SHAPES_E_CAPACITY.  The array (about 10 MB) is
+ *   beyond them it returns SHAPES_E_CAPACITY.  The array (about 11 MB) is
  *   held by every GPU that loads the library until the process exits.
  *   The call cannot be captured into a CUDA graph: it synchronizes
  *   `cuda_stream` and reads counters on the host between kernels.  The first

@@ -59,6 +59,18 @@ __device__ __forceinline__ double clamp_abs(double x, double limit) {
   return ok & (kl < kx) ? limit : low;
 }
 
+/* x in binary32, rounded toward zero (relative error below 2^-23) on the
+ * integer pipe; magnitudes below 2^-126 become zero, those from 2^128 on, and
+ * NaN, become infinity or NaN. */
+__device__ __forceinline__ float to_float(double x) {
+  const uint32_t hi = hi_word(x), e = (hi >> 20) & 0x7ffu, sign = hi & 0x80000000u;
+  const uint32_t mant = (hi & 0xfffffu) << 3 | lo_word(x) >> 29;
+  uint32_t u = (e - 896u) << 23 | mant;
+  if (e < 897u) u = 0;
+  if (e >= 1151u) u = 0x7f800000u | (nan_bits(x) ? 1u : 0u);
+  return __uint_as_float(sign | u);
+}
+
 /* Finite (not infinite, not NaN). */
 __device__ __forceinline__ bool finite_bits(double x) { return (hi_word(x) & 0x7ff00000u) != 0x7ff00000u; }
 

@@ -96,8 +96,8 @@ struct shapes_batch {
   double* wy = nullptr;
   double* nx = nullptr;
   double* ny = nullptr;
-  double* plo = nullptr; /* [V] self extents of each edge (SAT) */
-  double* phi = nullptr;
+  float4* vf = nullptr; /* [V] posed vertices and normals in binary32 (narrowphase filter) */
+  float2* ef = nullptr; /* [V] self extents of each edge in binary32 */
   double* box = nullptr;
   uint64_t* boxk = nullptr;
   uint8_t* flags = nullptr;
@@ -483,8 +483,8 @@ struct shapes_batch {
     d.wy = wy;
     d.nx = nx;
     d.ny = ny;
-    d.plo = plo;
-    d.phi = phi;
+    d.vf = vf;
+    d.ef = ef;
     d.box = box;
     d.boxk = boxk;
     d.flags = flags;
@@ -1085,7 +1085,11 @@ struct shapes_batch {
       if (any_grid) shapes::k_grid_sort_rows<<<grid_for(N, 128), 128, 0, stream>>>(d);
     });
     stage(6, 1, [&]() { shapes::k_world_pair_offsets<<<grid_for(W + 1, 128), 128, 0, stream>>>(d); });
-    stage(1, 4, [&]() {
+    stage(1, np_lanes > 1 ? 4 : 1, [&]() {
+      if (np_lanes <= 1) {
+        shapes::k_narrowphase<<<grid_for(pair_cap, shapes::kNpThreads), shapes::kNpThreads, 0, stream>>>(d);
+        return;
+      }
       ck(cudaMemsetAsync(np_cls, 0, sizeof(int32_t) * shapes::kNpClasses, stream), "memset");
       shapes::k_np_count<<<grid_for(pair_cap, 256), 256, 0, stream>>>(d);
       shapes::k_np_offsets<<<1, 32, 0, stream>>>(d);
@@ -1095,8 +1099,7 @@ struct shapes_batch {
         case 4: shapes::k_narrowphase_lanes<4><<<grid_for(4LL * pair_cap, 128), 128, 0, stream>>>(d); break;
         case 8: shapes::k_narrowphase_lanes<8><<<grid_for(8LL * pair_cap, 128), 128, 0, stream>>>(d); break;
         case 16: shapes::k_narrowphase_lanes<16><<<grid_for(16LL * pair_cap, 128), 128, 0, stream>>>(d); break;
-        case 32: shapes::k_narrowphase_lanes<32><<<grid_for(32LL * pair_cap, 128), 128, 0, stream>>>(d); break;
-        default: shapes::k_narrowphase<<<grid_for(pair_cap, 128), 128, 0, stream>>>(d);
+        default: shapes::k_narrowphase_lanes<32><<<grid_for(32LL * pair_cap, 128), 128, 0, stream>>>(d); break;
       }
     });
     scan(slot_cnt, pair_cap, counters + shapes::kCntPairs, slot_off);
@@ -1363,7 +1366,7 @@ struct shapes_batch {
       dfree(body_stage[k]);
     }
     dfree(wx); dfree(wy); dfree(nx); dfree(ny); dfree(box); dfree(boxk); dfree(flags); dfree(body_changed);
-    dfree(plo); dfree(phi);
+    dfree(vf); dfree(ef);
     dfree(row_cnt); dfree(row_off); dfree(world_pair_off); dfree(sched_body); dfree(sched_cur); dfree(world_levels);
     for (int k = 0; k < 6; ++k) dfree(snap_body[k]);
     dfree(active);
@@ -1390,8 +1393,8 @@ struct shapes_batch {
     wy = dalloc<double>(V, "cudaMalloc");
     nx = dalloc<double>(V, "cudaMalloc");
     ny = dalloc<double>(V, "cudaMalloc");
-    plo = dalloc<double>(V, "cudaMalloc");
-    phi = dalloc<double>(V, "cudaMalloc");
+    vf = dalloc<float4>(V, "cudaMalloc");
+    ef = dalloc<float2>(V, "cudaMalloc");
     box = dalloc<double>(4 * (size_t)N, "cudaMalloc");
     boxk = dalloc<uint64_t>(4 * (size_t)N, "cudaMalloc");
     flags = dalloc<uint8_t>(N, "cudaMalloc");
@@ -1510,7 +1513,7 @@ struct shapes_batch {
       dfree(body_stage[k]);
     }
     dfree(wx); dfree(wy); dfree(nx); dfree(ny); dfree(box); dfree(boxk); dfree(flags); dfree(body_changed);
-    dfree(plo); dfree(phi);
+    dfree(vf); dfree(ef);
     dfree(row_cnt); dfree(row_off); dfree(world_pair_off);
     dfree(grid_T); dfree(grid_base); dfree(grid_inv_s); dfree(grid_lim); dfree(bucket_cnt); dfree(bucket_off);
     dfree(grid_ids); dfree(cell_x); dfree(cell_y); dfree(row_mode); dfree(large_cnt); dfree(large_ids);
@@ -3067,7 +3070,7 @@ constexpr int kNaTiles = (kNaMaxPairs + 1 + shapes::kScanTile - 1) / shapes::kSc
 
 /* Byte offsets of the scratch arrays, each 256-byte aligned. */
 struct NaPlan {
-  size_t world_body_off, body_world, lx, ly, emin, emax, wx, wy, nx, ny, box, boxk, flags, row_mode, row_cnt,
+  size_t world_body_off, body_world, lx, ly, emin, emax, wx, wy, nx, ny, vf, ef, box, boxk, flags, row_mode, row_cnt,
       row_off, pair_a, pair_b, slot_cnt, slot_off, slot_feat, slot_val, world_pair_off, cwo, c_key, c_ga, c_gb,
       c_flip, c_hit, c_val, tile_sums, counters, total;
 };
@@ -3091,6 +3094,8 @@ constexpr NaPlan na_plan() {
   p.wy = na_take(o, kNaMaxVerts * sizeof(double));
   p.nx = na_take(o, kNaMaxVerts * sizeof(double));
   p.ny = na_take(o, kNaMaxVerts * sizeof(double));
+  p.vf = na_take(o, kNaMaxVerts * sizeof(float4));
+  p.ef = na_take(o, kNaMaxVerts * sizeof(float2));
   p.box = na_take(o, 4 * kNaMaxBodies * sizeof(double));
   p.boxk = na_take(o, 4 * kNaMaxBodies * sizeof(uint64_t));
   p.flags = na_take(o, kNaMaxBodies);
@@ -3276,6 +3281,8 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   d.wy = reinterpret_cast<double*>(base + kNaPlan.wy);
   d.nx = reinterpret_cast<double*>(base + kNaPlan.nx);
   d.ny = reinterpret_cast<double*>(base + kNaPlan.ny);
+  d.vf = reinterpret_cast<float4*>(base + kNaPlan.vf);
+  d.ef = reinterpret_cast<float2*>(base + kNaPlan.ef);
   d.box = reinterpret_cast<double*>(base + kNaPlan.box);
   d.boxk = reinterpret_cast<uint64_t*>(base + kNaPlan.boxk);
   d.flags = base + kNaPlan.flags;
@@ -3339,7 +3346,7 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   scan(d.row_cnt, n_bodies, nullptr, d.row_off);
   shapes::k_broadphase<false><<<grid_for((long long)n_bodies * 32, 256), 256, 0, st>>>(d);
   shapes::k_world_pair_offsets<<<1, 32, 0, st>>>(d);
-  shapes::k_narrowphase<<<grid_for(kNaMaxPairs, 128), 128, 0, st>>>(d);
+  shapes::k_narrowphase<<<grid_for(kNaMaxPairs, shapes::kNpThreads), shapes::kNpThreads, 0, st>>>(d);
   scan(d.slot_cnt, kNaMaxPairs, d.counters + shapes::kCntPairs, d.slot_off);
   shapes::k_world_contact_offsets<<<1, 32, 0, st>>>(d);
   shapes::k_build<<<grid_for(2LL * kNaMaxPairs, 128), 128, 0, st>>>(d, 0.0, 0.0, 0, 0);
