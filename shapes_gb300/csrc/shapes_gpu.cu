@@ -71,6 +71,14 @@ inline int grid_for(long long n, int threads) {
   return (int)blocks;
 }
 
+/* Small batches spread over more blocks of fewer bodies. */
+inline void launch_pose(cudaStream_t stream, int n, const Dev& d, double dt, int advance,
+                        const uint8_t* only = nullptr) {
+  const int per_block = n >= 2 * kSMs * shapes::kPoseThreads ? shapes::kPoseThreads : 32;
+  shapes::k_integrate_pose<<<grid_for(n, per_block), shapes::kPoseThreads, 0, stream>>>(d, dt, advance, per_block,
+                                                                                        only);
+}
+
 }  // namespace
 
 struct shapes_batch {
@@ -146,7 +154,6 @@ struct shapes_batch {
   int32_t* slot_feat = nullptr;
   double* slot_val = nullptr;
   int32_t* np_perm = nullptr;
-  int32_t* pose_order = nullptr; /* [N] bodies grouped by vertex count within chunks of 1024 */
   int32_t* ext_chunk = nullptr;      /* extent reduction: chunk body ranges, per-world chunk offsets, partials */
   int32_t* ext_chunk_off = nullptr;
   double* ext_part_sum = nullptr;
@@ -446,7 +453,6 @@ struct shapes_batch {
     d.world_body_off = world_body_off;
     d.body_world = body_world;
     d.vert_off = vert_off;
-    d.pose_order = pose_order;
     d.ext_chunk = ext_chunk;
     d.ext_chunk_off = ext_chunk_off;
     d.ext_part_sum = ext_part_sum;
@@ -1003,7 +1009,7 @@ struct shapes_batch {
 
   void pose(int advance, double dt) {
     Dev d = view(0);
-    shapes::k_integrate_pose<<<grid_for(N, 128), 128, 0, stream>>>(d, dt, advance);
+    launch_pose(stream, N, d, dt, advance);
   }
 
   /* Broadphase + narrowphase into buffer `wb`; with `solve`, also constraint
@@ -1137,7 +1143,7 @@ struct shapes_batch {
         shapes::k_collect<<<grid_for(contact_cap, 256), 256, 0, stream>>>(d, ds_feat, ds_tgt, ds_count, ds_cap);
         shapes::k_collect_advance<<<1, 1, 0, stream>>>(miss_n, ds_count, ds_cap);
       });
-    stage(5, 1, [&]() { shapes::k_integrate_pose<<<grid_for(N, 128), 128, 0, stream>>>(d, cfg.dt, 1); });
+    stage(5, 1, [&]() { launch_pose(stream, N, d, cfg.dt, 1); });
   }
 
   /* The state a refused or regrown step returns to: the pose-and-velocity
@@ -1194,7 +1200,7 @@ struct shapes_batch {
     shapes::k_commit_bodies<<<grid_for(N, 256), 256, 0, stream>>>(p, N, body_changed,
                                                                   counters + shapes::kCntBadInput);
     Dev d = view(0);
-    shapes::k_integrate_pose<<<grid_for(N, 128), 128, 0, stream>>>(d, 0.0, 0, body_changed);
+    launch_pose(stream, N, d, 0.0, 0, body_changed);
     ck(cudaGetLastError(), "launch");
   }
   /* The first `fields` body arrays (10: all; kStepFields: velocities and pose,
@@ -1359,7 +1365,6 @@ struct shapes_batch {
     free_step_buffers();
     dfree(world_body_off); dfree(body_world); dfree(vert_off); dfree(lx); dfree(ly); dfree(emin); dfree(emax);
     dfree(radius);
-    dfree(pose_order);
     radius = nullptr;
     for (int k = 0; k < 10; ++k) {
       dfree(body[k]);
@@ -1418,28 +1423,6 @@ struct shapes_batch {
        "upload");
     ck(cudaMemcpy(body_world, h_body_world.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice), "upload");
     ck(cudaMemcpy(vert_off, vert_offsets, sizeof(int32_t) * (N + 1), cudaMemcpyHostToDevice), "upload");
-    {
-      /* pose order: stable counting sort by vertex count within each chunk of
-       * 1024 bodies (a warp of the pose kernel then runs one loop length;
-       * chunks keep the gathers local) */
-      std::vector<int32_t> order(N);
-      constexpr int32_t kChunk = 1024;
-      for (int32_t c0 = 0; c0 < N; c0 += kChunk) {
-        const int32_t c1 = std::min<int32_t>(N, c0 + kChunk);
-        int32_t cnt[shapes::kMaxVerts + 2] = {0};
-        for (int32_t b = c0; b < c1; ++b) ++cnt[std::min<int32_t>(vert_offsets[b + 1] - vert_offsets[b], shapes::kMaxVerts + 1)];
-        int32_t pos[shapes::kMaxVerts + 2];
-        int32_t acc = c0;
-        for (int k = 0; k < shapes::kMaxVerts + 2; ++k) {
-          pos[k] = acc;
-          acc += cnt[k];
-        }
-        for (int32_t b = c0; b < c1; ++b)
-          order[pos[std::min<int32_t>(vert_offsets[b + 1] - vert_offsets[b], shapes::kMaxVerts + 1)]++] = b;
-      }
-      pose_order = dalloc<int32_t>(std::max<int32_t>(N, 1), "cudaMalloc");
-      if (N) ck(cudaMemcpy(pose_order, order.data(), sizeof(int32_t) * N, cudaMemcpyHostToDevice), "upload");
-    }
     /* a circle's one local point (radius, 0) becomes radius[b] and the local
      * centre (0, 0) (circleWithRadius, Contact/Circle.hs:24-25) */
     h_radius.assign(N, 0.0);
@@ -1507,7 +1490,6 @@ struct shapes_batch {
     free_step_buffers();
     dfree(world_body_off); dfree(body_world); dfree(vert_off); dfree(lx); dfree(ly);
     dfree(emin); dfree(emax);
-    dfree(pose_order);
     for (int k = 0; k < 10; ++k) {
       dfree(body[k]);
       dfree(body_stage[k]);
@@ -1999,7 +1981,7 @@ int shapes_batch_set_bodies(shapes_batch* b, const shapes_bodies* in) {
     shapes::k_commit_bodies<<<grid_for(b->N, 256), 256, 0, b->stream>>>(p, b->N, b->body_changed);
     {
       Dev d = b->view(0);
-      shapes::k_integrate_pose<<<grid_for(b->N, 128), 128, 0, b->stream>>>(d, 0.0, 0, b->body_changed);
+      launch_pose(b->stream, b->N, d, 0.0, 0, b->body_changed);
     }
     ck(cudaGetLastError(), "launch");
     ck(cudaStreamSynchronize(b->stream), "upload");
@@ -3341,7 +3323,7 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
     return SHAPES_E_NONCONVEX;
   }
   shapes::k_init_extents<<<grid_for(n_verts, 128), 128, 0, st>>>(d);
-  shapes::k_integrate_pose<<<grid_for(n_bodies, 128), 128, 0, st>>>(d, 0.0, 0);
+  launch_pose(st, n_bodies, d, 0.0, 0);
   shapes::k_broadphase<true><<<grid_for((long long)n_bodies * 32, 256), 256, 0, st>>>(d);
   scan(d.row_cnt, n_bodies, nullptr, d.row_off);
   shapes::k_broadphase<false><<<grid_for((long long)n_bodies * 32, 256), 256, 0, st>>>(d);

@@ -134,8 +134,6 @@ struct Dev {
   int32_t* sap_cursor;      /* [n_bodies] per row (mirrored index): the next free slot of the row */
   uint64_t* sap_range;      /* [2 * n_worlds] min and max order key of the small bodies' lower x */
   int32_t* sap_end;         /* [n_worlds] end of the world's run in sap_ids */
-  const int32_t* pose_order; /* [n_bodies] pose-kernel order: within chunks of 1024 bodies, grouped by vertex
-                                count, so that a warp's vertex loops have one length (null: index order) */
   int32_t* np_cls;     /* [2 * kNpClasses + 1] class counts, then offsets and cursors */
   double* slot_val;    /* [2*pair_cap*5] nx ny px py depth */
   uint64_t* c_key;     /* [contact_cap] packed world-local key */
@@ -387,140 +385,167 @@ __global__ void k_init_extents(Dev d) {
   }
 }
 
+/* A body's box, its ordered keys and its flags. */
+__device__ __forceinline__ void write_box(const Dev& d, int g, double x0, double x1, double y0, double y1, uint8_t f) {
+  d.box[4 * g + 0] = x0;
+  d.box[4 * g + 1] = x1;
+  d.box[4 * g + 2] = y0;
+  d.box[4 * g + 3] = y1;
+  d.boxk[4 * g + 0] = okey(x0);
+  d.boxk[4 * g + 1] = okey(x1);
+  d.boxk[4 * g + 2] = okey(y0);
+  d.boxk[4 * g + 3] = okey(y1);
+  if (is_zero(d.iml[g]) && is_zero(d.imr[g])) f |= kFlagStatic;
+  if (nan_bits(x0) || nan_bits(x1) || nan_bits(y0) || nan_bits(y1)) f |= kFlagBoxNaN;
+  d.flags[g] = f;
+}
+
 /* advanceObj (Constraint.hs:225-229) when `advance`, then moveShape
  * (World.hs:132-133): rotation matrix from shapes_sincos, the 3x3 product of
  * toTransform (Transform.hs:34-38, 73-77; MatrixTemplate.hs:47-67), afmul
  * (Linear.hs:217-220) per vertex, unitEdgeNormal (ConvexHull.hs:218-226) per
  * edge, then hullToAabb (Aabb.hs:81-84, 106-110) and its ordered keys.
- * One thread per body, bodies taken in pose_order: the FP64 pipe charges a
- * warp instruction in full whatever its active lanes, so a warp whose hulls
- * have 3..8 vertices would run 8 iterations for all of them; grouped by vertex
- * count, its loops have one length.  Each body still writes only its own
- * outputs, so the order changes no result. */
-__global__ void k_integrate_pose(Dev d, double dt, int advance, const uint8_t* only = nullptr) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < d.n_bodies; t += gridDim.x * blockDim.x) {
-    const int g = d.pose_order ? d.pose_order[t] : t;
-    if (only && !only[g]) continue; /* re-pose: this body's pose inputs did not change */
-    if (d.active && !d.active[g]) { /* empty slot: left as it was, out of the broadphase */
-      d.flags[g] = kFlagInactive;
-      continue;
-    }
-    double px = d.px[g], py = d.py[g], th = d.th[g];
-    if (advance) {
-      const double vx = d.vx[g], vy = d.vy[g], w = d.w[g];
-      px = (vx * dt) + px;
-      py = (vy * dt) + py;
-      th = (dt * w) + th;
-      d.px[g] = px;
-      d.py[g] = py;
-      d.th[g] = th;
-    }
-    double s, c;
-    shapes_sincos(th, &s, &c);
-    const double ms = -s;
-    /* rows of translate(px,py) times columns of rotate(c,s), summed in the
-     * reference's order (joinTransforms, Transform.hs:73-77) */
-    double m00, m01, m02, m10, m11, m12;
-    if (finite_bits(c) && finite_bits(s) && finite_bits(px) && finite_bits(py)) {
-      /* every product by 1.0 or 0.0 is exact, so the sums reduce to
-       * signed-zero rules on the integer pipe */
-      const double zc = signed_zero(c), zs = signed_zero(s), zms = signed_zero(ms);
-      const double zpx = signed_zero(px), zpy = signed_zero(py);
-      m00 = add_zero(add_zero(c, zs), zpx);
-      m01 = add_zero(add_zero(ms, zc), zpx);
-      m02 = plus_zero(px);
-      m10 = add_zero(add_zero(s, zc), zpy);
-      m11 = add_zero(add_zero(c, zms), zpy);
-      m12 = plus_zero(py);
-    } else {
-      m00 = (1.0 * c + 0.0 * s) + px * 0.0;
-      m01 = (1.0 * ms + 0.0 * c) + px * 0.0;
-      m02 = (1.0 * 0.0 + 0.0 * 0.0) + px * 1.0;
-      m10 = (0.0 * c + 1.0 * s) + py * 0.0;
-      m11 = (0.0 * ms + 1.0 * c) + py * 0.0;
-      m12 = (0.0 * 0.0 + 1.0 * 0.0) + py * 1.0;
-    }
-    /* m02 * 1.0 == m02 and m12 * 1.0 == m12 unless NaN (then both are NaN) */
-    const bool t_nan = nan_bits(m02) || nan_bits(m12);
-    const int b0 = d.vert_off[g], nv = d.vert_off[g + 1] - b0;
-    const double rad = d.radius ? d.radius[g] : 0.0;
-    if (rad > 0.0) {
-      /* setCircleTransform (Circle.hs:60-64): the transformed local origin;
-       * circleToAabb (Aabb.hs:86-89): centre -+ radius */
-      const double lx = d.lx[b0], ly = d.ly[b0];
-      const double x = t_nan ? (m00 * lx + m01 * ly) + m02 * 1.0 : (mul_rn_int(m00, lx) + m01 * ly) + m02;
-      const double y = t_nan ? (m10 * lx + m11 * ly) + m12 * 1.0 : (mul_rn_int(m10, lx) + m11 * ly) + m12;
-      d.wx[b0] = x;
-      d.wy[b0] = y;
-      d.nx[b0] = 0.0;
-      d.ny[b0] = 0.0;
-      const double cb0 = x - rad, cb1 = x + rad, cb2 = y - rad, cb3 = y + rad;
-      d.box[4 * g + 0] = cb0;
-      d.box[4 * g + 1] = cb1;
-      d.box[4 * g + 2] = cb2;
-      d.box[4 * g + 3] = cb3;
-      d.boxk[4 * g + 0] = okey(cb0);
-      d.boxk[4 * g + 1] = okey(cb1);
-      d.boxk[4 * g + 2] = okey(cb2);
-      d.boxk[4 * g + 3] = okey(cb3);
-      uint8_t f = kFlagCircle;
-      if (d.iml[g] == 0.0 && d.imr[g] == 0.0) f |= kFlagStatic;
-      if (nan_bits(cb0) || nan_bits(cb1) || nan_bits(cb2) || nan_bits(cb3)) f |= kFlagBoxNaN;
-      d.flags[g] = f;
-      continue;
-    }
-    double x0 = 0, y0 = 0, xp = 0, yp = 0;
-    double bx0 = 0, bx1 = 0, by0 = 0, by1 = 0;
-    for (int k = 0; k < nv; ++k) {
-      const double lx = d.lx[b0 + k], ly = d.ly[b0 + k];
-      /* one product per coordinate on the integer pipe (exact), as in SAT */
-      const double x = t_nan ? (m00 * lx + m01 * ly) + m02 * 1.0 : (mul_rn_int(m00, lx) + m01 * ly) + m02;
-      const double y = t_nan ? (m10 * lx + m11 * ly) + m12 * 1.0 : (mul_rn_int(m10, lx) + m11 * ly) + m12;
-      d.wx[b0 + k] = x;
-      d.wy[b0 + k] = y;
-      if (k == 0) {
-        x0 = x; y0 = y;
-        bx0 = x; bx1 = x; by0 = y; by1 = y;
+ * A block takes per_block bodies (a warp's worth in small batches, so that
+ * their vertices are one round of its threads) in turns: a thread per body for the angle
+ * and the matrix, a thread per vertex for the points, a thread per edge for the
+ * normals (a square root and two divisions, two thirds of a hull's FP64 work),
+ * a thread per body for the box.  The FP64 pipe charges a warp instruction in
+ * full whatever its active lanes, and here every warp but a block's last is
+ * full however many vertices the hulls have; with a thread per body the vertex
+ * loop was also one long chain.  1024 x 256 mixed worlds: 0.181 ms a step as a
+ * thread per body (bodies ordered by vertex count). */
+constexpr int kPoseThreads = 128;
+__global__ void __launch_bounds__(kPoseThreads) k_integrate_pose(Dev d, double dt, int advance, int per_block,
+                                                                 const uint8_t* only = nullptr) {
+  __shared__ double mat[6][kPoseThreads];   /* the matrix's two rows */
+  __shared__ int32_t vstart[kPoseThreads + 1];
+  __shared__ uint8_t kind[kPoseThreads];    /* a hull to pose: 1, with a NaN translation: 2; else 0 */
+  const int tid = threadIdx.x;
+  for (int base = blockIdx.x * per_block; base < d.n_bodies; base += gridDim.x * per_block) {
+    const int nb = min(per_block, d.n_bodies - base), g = base + tid;
+    if (tid < nb) {
+      vstart[tid] = d.vert_off[g];
+      if (tid == nb - 1) vstart[nb] = d.vert_off[g + 1];
+      kind[tid] = 0;
+      if (only && !only[g]) { /* re-pose: this body's pose inputs did not change */
+      } else if (d.active && !d.active[g]) { /* empty slot: left as it was, out of the broadphase */
+        d.flags[g] = kFlagInactive;
       } else {
-        const double ddx = x - xp, ddy = y - yp;
-        const double ex = ddy, ey = -ddx;
-        const double len = sqrt(ex * ex + ey * ey);
-        d.nx[b0 + k - 1] = ex / len;
-        d.ny[b0 + k - 1] = ey / len;
+        double px = d.px[g], py = d.py[g], th = d.th[g];
+        if (advance) {
+          const double vx = d.vx[g], vy = d.vy[g], w = d.w[g];
+          px = (vx * dt) + px;
+          py = (vy * dt) + py;
+          th = (dt * w) + th;
+          d.px[g] = px;
+          d.py[g] = py;
+          d.th[g] = th;
+        }
+        double s, c;
+        shapes_sincos(th, &s, &c);
+        const double ms = flip_sign(s);
+        /* rows of translate(px,py) times columns of rotate(c,s), summed in the
+         * reference's order (joinTransforms, Transform.hs:73-77) */
+        double m00, m01, m02, m10, m11, m12;
+        if (finite_bits(c) && finite_bits(s) && finite_bits(px) && finite_bits(py)) {
+          /* every product by 1.0 or 0.0 is exact, so the sums reduce to
+           * signed-zero rules on the integer pipe */
+          const double zc = signed_zero(c), zs = signed_zero(s), zms = signed_zero(ms);
+          const double zpx = signed_zero(px), zpy = signed_zero(py);
+          m00 = add_zero(add_zero(c, zs), zpx);
+          m01 = add_zero(add_zero(ms, zc), zpx);
+          m02 = plus_zero(px);
+          m10 = add_zero(add_zero(s, zc), zpy);
+          m11 = add_zero(add_zero(c, zms), zpy);
+          m12 = plus_zero(py);
+        } else {
+          m00 = (1.0 * c + 0.0 * s) + px * 0.0;
+          m01 = (1.0 * ms + 0.0 * c) + px * 0.0;
+          m02 = (1.0 * 0.0 + 0.0 * 0.0) + px * 1.0;
+          m10 = (0.0 * c + 1.0 * s) + py * 0.0;
+          m11 = (0.0 * ms + 1.0 * c) + py * 0.0;
+          m12 = (0.0 * 0.0 + 1.0 * 0.0) + py * 1.0;
+        }
+        /* m02 * 1.0 == m02 and m12 * 1.0 == m12 unless NaN (then both are NaN) */
+        const bool t_nan = nan_bits(m02) || nan_bits(m12);
+        const double rad = d.radius ? d.radius[g] : 0.0;
+        if (rad > 0.0) {
+          /* setCircleTransform (Circle.hs:60-64): the transformed local origin;
+           * circleToAabb (Aabb.hs:86-89): centre -+ radius */
+          const int b0 = vstart[tid];
+          const double lx = d.lx[b0], ly = d.ly[b0];
+          const double x = t_nan ? (m00 * lx + m01 * ly) + m02 * 1.0 : (mul_rn_int(m00, lx) + m01 * ly) + m02;
+          const double y = t_nan ? (m10 * lx + m11 * ly) + m12 * 1.0 : (mul_rn_int(m10, lx) + m11 * ly) + m12;
+          d.wx[b0] = x;
+          d.wy[b0] = y;
+          d.nx[b0] = 0.0;
+          d.ny[b0] = 0.0;
+          write_box(d, g, x - rad, x + rad, y - rad, y + rad, kFlagCircle);
+        } else {
+          kind[tid] = t_nan ? 2 : 1;
+          mat[0][tid] = m00;
+          mat[1][tid] = m01;
+          mat[2][tid] = m02;
+          mat[3][tid] = m10;
+          mat[4][tid] = m11;
+          mat[5][tid] = m12;
+        }
+      }
+    }
+    __syncthreads();
+    const int v0 = vstart[0], v1 = vstart[nb];
+    auto owner = [&](int v) { /* the body of vertex v */
+      int lo = 0, hi = nb;
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (vstart[mid] <= v) lo = mid;
+        else hi = mid;
+      }
+      return lo;
+    };
+    for (int v = v0 + tid; v < v1; v += kPoseThreads) {
+      const int k = owner(v);
+      if (!kind[k]) continue;
+      const double lx = d.lx[v], ly = d.ly[v], m02 = mat[2][k], m12 = mat[5][k];
+      const bool t_nan = kind[k] == 2;
+      /* one product per coordinate on the integer pipe (exact), as in SAT */
+      const double m00 = mat[0][k], m01 = mat[1][k], m10 = mat[3][k], m11 = mat[4][k];
+      d.wx[v] = t_nan ? (m00 * lx + m01 * ly) + m02 * 1.0 : (mul_rn_int(m00, lx) + m01 * ly) + m02;
+      d.wy[v] = t_nan ? (m10 * lx + m11 * ly) + m12 * 1.0 : (mul_rn_int(m10, lx) + m11 * ly) + m12;
+    }
+    __syncthreads();
+    for (int v = v0 + tid; v < v1; v += kPoseThreads) {
+      const int k = owner(v);
+      if (!kind[k]) continue;
+      const int n1 = v + 1 < vstart[k + 1] ? v + 1 : vstart[k];
+      const double x = d.wx[v], y = d.wy[v];
+      const double ddx = d.wx[n1] - x, ex = d.wy[n1] - y, ey = flip_sign(ddx);
+      const double len = sqrt(ex * ex + ey * ey);
+      const double nx = ex / len, ny = ey / len;
+      d.nx[v] = nx;
+      d.ny[v] = ny;
+      d.vf[v] = make_float4(to_float(x), to_float(y), to_float(nx), to_float(ny));
+    }
+    __syncthreads();
+    for (int v = v0 + tid; v < v1; v += kPoseThreads) { /* extentAlongSelf (ConvexHull.hs:107-118) */
+      const int k = owner(v);
+      if (!kind[k]) continue;
+      const float4 n = d.vf[v], lo = d.vf[vstart[k] + d.emin[v]], hi = d.vf[vstart[k] + d.emax[v]];
+      d.ef[v] = make_float2(__fmaf_rn(lo.x, n.z, lo.y * n.w), __fmaf_rn(hi.x, n.z, hi.y * n.w));
+    }
+    if (tid < nb && kind[tid]) {
+      const int b0 = vstart[tid], b1 = vstart[tid + 1];
+      double bx0 = d.wx[b0], bx1 = bx0, by0 = d.wy[b0], by1 = by0;
+      for (int v = b0 + 1; v < b1; ++v) {
+        const double x = d.wx[v], y = d.wy[v];
         bx0 = f_lt(bx0, x) ? bx0 : x;
         bx1 = f_lt(x, bx1) ? bx1 : x;
         by0 = f_lt(by0, y) ? by0 : y;
         by1 = f_lt(y, by1) ? by1 : y;
       }
-      xp = x;
-      yp = y;
+      write_box(d, g, bx0, bx1, by0, by1, 0);
     }
-    {
-      const double ddx = x0 - xp, ddy = y0 - yp;
-      const double ex = ddy, ey = -ddx;
-      const double len = sqrt(ex * ex + ey * ey);
-      d.nx[b0 + nv - 1] = ex / len;
-      d.ny[b0 + nv - 1] = ey / len;
-    }
-    for (int k = 0; k < nv; ++k)
-      d.vf[b0 + k] = make_float4(to_float(d.wx[b0 + k]), to_float(d.wy[b0 + k]), to_float(d.nx[b0 + k]),
-                                 to_float(d.ny[b0 + k]));
-    for (int e = 0; e < nv; ++e) { /* extentAlongSelf (ConvexHull.hs:107-118) */
-      const float4 n = d.vf[b0 + e], lo = d.vf[b0 + d.emin[b0 + e]], hi = d.vf[b0 + d.emax[b0 + e]];
-      d.ef[b0 + e] = make_float2(__fmaf_rn(lo.x, n.z, lo.y * n.w), __fmaf_rn(hi.x, n.z, hi.y * n.w));
-    }
-    d.box[4 * g + 0] = bx0;
-    d.box[4 * g + 1] = bx1;
-    d.box[4 * g + 2] = by0;
-    d.box[4 * g + 3] = by1;
-    d.boxk[4 * g + 0] = okey(bx0);
-    d.boxk[4 * g + 1] = okey(bx1);
-    d.boxk[4 * g + 2] = okey(by0);
-    d.boxk[4 * g + 3] = okey(by1);
-    uint8_t f = 0;
-    if (d.iml[g] == 0.0 && d.imr[g] == 0.0) f |= kFlagStatic;
-    if (nan_bits(bx0) || nan_bits(bx1) || nan_bits(by0) || nan_bits(by1)) f |= kFlagBoxNaN;
-    d.flags[g] = f;
+    __syncthreads();
   }
 }
 
@@ -1865,8 +1890,8 @@ __global__ void __launch_bounds__(kNpThreads) k_narrowphase(Dev d) {
       queue[atomicAdd(&n_hulls, 1)] = q;
     }
     __syncthreads();
-    /* the first warps get the last, partly filled round: which those are turns with the block, as a block's warps sit on
-     * fixed sub-partitions */
+    /* the first warps get the last, partly filled round; which those are turns
+     * with the block, as a block's warps sit on fixed sub-partitions */
     const int at = (tid + 32 * (int)blockIdx.x) & (kNpThreads - 1);
     for (int t = at; t < n_hulls; t += kNpThreads) {
       const Entry q = queue[t];
