@@ -1125,7 +1125,8 @@ void oracle_sincos(const double* x, double* s, double* c, int64_t n) {
 /* The two phases of shapes_sincos separately (tests of the function itself):
  * mode 0 the accurate phase alone; mode 1 the fast phase's unrounded
  * double-double results (s hi, s lo, c hi, c lo in out4, ok[k] = 0 where it
- * declines); mode 2 the host libm's sin and cos. */
+ * declines); mode 2 the host libm's sin and cos; mode 3 the GPU's fixed-point
+ * fast phase (rounded; ok[k] = 0 where it declines). */
 void oracle_sincos_phase(int32_t mode, const double* x, double* out4, uint8_t* ok, int64_t n) {
   for (int64_t k = 0; k < n; ++k) {
     double* o = out4 + 4 * k;
@@ -1135,6 +1136,9 @@ void oracle_sincos_phase(int32_t mode, const double* x, double* out4, uint8_t* o
       ok[k] = 1;
     } else if (mode == 1) {
       ok[k] = (uint8_t)shapes_sincos_fast(x[k], o);
+    } else if (mode == 3) {
+      ok[k] = (uint8_t)shapes_sincos_fixed(x[k], &o[0], &o[2]);
+      o[1] = o[3] = 0.0;
     } else {
       o[0] = std::sin(x[k]);
       o[2] = std::cos(x[k]);

@@ -14,7 +14,9 @@ Constants:
   - sin(i pi/512), i = 0..256, each as an unevaluated sum hi + lo of two
     doubles (hi = RN(v), lo = RN(v - hi));
   - 1/n!, n = 0..33, in unsigned fixed point with 127 fractional bits (the
-    Taylor coefficients of the accurate phase), rounded to nearest.
+    Taylor coefficients of the accurate phase), rounded to nearest;
+  - for the fixed-point fast phase, 512/pi with 120 and pi/4 with 128
+    fractional bits, truncated, and sin(i pi/512), i = 0..255, with 128.
 The header is committed; tests/test_sincos.py regenerates it in memory and
 checks that the committed file matches.
 """
@@ -156,6 +158,21 @@ def generate() -> str:
         q = ((1 << 128) // fact + 1) >> 1  # round(2^127 / n!)
         assert q < (1 << 128)
         w(f"  0x{q >> 64:016x}ull, 0x{q & ((1 << 64) - 1):016x}ull, \\")
+    w("}")
+    # fixed-point fast phase
+    low = (1 << 64) - 1
+    k512 = (512 << (PREC + 120)) // pi_f
+    pi4 = pi_f >> (PREC - 126)  # pi 2^126 = (pi/4) 2^128
+    w("/* 512/pi * 2^120 and pi/4 * 2^128, truncated: high and low 64-bit words */")
+    w(f"#define SHAPES_512_OVER_PI_Q120_HI 0x{k512 >> 64:016x}ull")
+    w(f"#define SHAPES_512_OVER_PI_Q120_LO 0x{k512 & low:016x}ull")
+    w(f"#define SHAPES_PIO4_Q128_HI 0x{pi4 >> 64:016x}ull")
+    w(f"#define SHAPES_PIO4_Q128_LO 0x{pi4 & low:016x}ull")
+    w("/* sin(i pi/512) * 2^128, i = 0..255: high and low 64-bit words */")
+    w("#define SHAPES_SIN_TABLE_Q128 { \\")
+    for i in range(256):
+        v = sin_fixed(i, 512, pi_t, tb) >> (tb - 128) if i else 0
+        w(f"  0x{v >> 64:016x}ull, 0x{v & low:016x}ull, \\")
     w("}")
     w("")
     w("#endif /* SHAPES_SINCOS_TABLES_H */")

@@ -25,6 +25,13 @@
  *     double-double hi + lo with relative error below 2^-67 (checked on 10^8
  *     arguments against the accurate phase); if hi + lo -/+ 2^-65 |hi| round
  *     to the same double, that double is the correctly rounded result.
+ *   - The GPU's fast phase is the same in 128-bit fixed point (GB300 takes 64
+ *     to 76 cycles for an FP64 warp instruction and sub-partition; the double-
+ *     double phase is about 105 of them, this is integer work): r as a fraction
+ *     of the step from M times 512/pi in 120 fractional bits, the same table and
+ *     series, and a rounding test on the distance from the rounding boundary.
+ *     It declines where that distance is below its error bound (2^-76 absolute,
+ *     2^-70 relative next to a multiple of pi/2) and where r nearly cancelled.
  *   - Accurate phase (the test failed, |x| >= 2^16, or r nearly cancelled):
  *     128-bit fixed-point arithmetic on the integer pipe.  Payne & Hanek's
  *     reduction multiplies the 53-bit significand by a 320-bit window of 2/pi
@@ -68,17 +75,18 @@ typedef struct {
 static const double shapes_sin_tab_h[514] = SHAPES_SIN_TABLE;
 static const uint64_t shapes_two_over_pi_h[20] = SHAPES_TWO_OVER_PI_WORDS;
 static const uint64_t shapes_inv_fact_h[68] = SHAPES_INV_FACT_Q127;
+static const uint64_t shapes_sin_q128_h[512] = SHAPES_SIN_TABLE_Q128;
 #if defined(__CUDACC__)
-static __device__ const double shapes_sin_tab_d[514] = SHAPES_SIN_TABLE;
+static __device__ const uint64_t shapes_sin_q128_d[512] = SHAPES_SIN_TABLE_Q128;
 static __device__ const uint64_t shapes_two_over_pi_d[20] = SHAPES_TWO_OVER_PI_WORDS;
 static __constant__ uint64_t shapes_inv_fact_d[68] = SHAPES_INV_FACT_Q127;
 #endif
 
-SHAPES_HD double shapes_sc_tab(int k) {
+SHAPES_HD shapes_u128 shapes_sc_sin_q128(int i) {
 #if defined(__CUDA_ARCH__)
-  return __ldg(&shapes_sin_tab_d[k]);
+  return ((shapes_u128)__ldg(&shapes_sin_q128_d[2 * i]) << 64) | __ldg(&shapes_sin_q128_d[2 * i + 1]);
 #else
-  return shapes_sin_tab_h[k];
+  return ((shapes_u128)shapes_sin_q128_h[2 * i] << 64) | shapes_sin_q128_h[2 * i + 1];
 #endif
 }
 SHAPES_HD uint64_t shapes_sc_2opi(int k) {
@@ -275,10 +283,12 @@ SHAPES_HD void shapes_sincos_accurate(double x, double* s_out, double* c_out) {
   *c_out = r.c;
 }
 
-/* Fast phase for 2^-27 <= |x| < 2^16: sin x ~ sh + sl and cos x ~ ch + cl
- * (each pair renormalised, relative error below 2^-67).  Returns 0 when the
- * reduced argument nearly cancelled (the accurate phase must be used). */
-SHAPES_HD int shapes_sincos_fast2(double x, double& sh, double& sl, double& ch, double& cl) {
+#if !defined(__CUDA_ARCH__)
+static inline double shapes_sc_tab(int k) { return shapes_sin_tab_h[k]; }
+/* The host's fast phase for 2^-27 <= |x| < 2^16: sin x ~ sh + sl and cos x ~
+ * ch + cl (each pair renormalised, relative error below 2^-67).  Returns 0 when
+ * the reduced argument nearly cancelled (the accurate phase must be used). */
+static inline int shapes_sincos_fast2(double x, double& sh, double& sl, double& ch, double& cl) {
   const double ax = fabs(x);
   const double N = rint(ax * SHAPES_512_OVER_PI);
   /* Cody-Waite: r = ax - N (P1 + P2 + P3 + P4) = rh + rl */
@@ -345,14 +355,127 @@ SHAPES_HD int shapes_sincos_fast2(double x, double& sh, double& sl, double& ch, 
   return 1;
 }
 
-SHAPES_HD int shapes_sincos_fast(double x, double out[4]) {
+static inline int shapes_sincos_fast(double x, double out[4]) {
   return shapes_sincos_fast2(x, out[0], out[1], out[2], out[3]);
 }
 
 /* 1 when every value within 2^-65 |hi| of hi + lo rounds to hi + lo's nearest double. */
-SHAPES_HD int shapes_sc_decided(double hi, double lo) {
+static inline int shapes_sc_decided(double hi, double lo) {
   const double e = fabs(hi) * 0x1p-65;
   return hi + (lo + e) == hi + (lo - e);
+}
+#endif
+
+SHAPES_HD uint64_t shapes_sc_hi(shapes_u128 v) { return (uint64_t)(v >> 64); }
+SHAPES_HD uint64_t shapes_sc_lo(shapes_u128 v) { return (uint64_t)v; }
+SHAPES_HD shapes_u128 shapes_sc_pack(uint64_t hi, uint64_t lo) { return ((shapes_u128)hi << 64) | lo; }
+SHAPES_HD uint64_t shapes_sc_mulhi64(uint64_t a, uint64_t b) {
+#if defined(__CUDA_ARCH__)
+  return __umul64hi(a, b);
+#else
+  return (uint64_t)(((shapes_u128)a * b) >> 64);
+#endif
+}
+/* a * b / 2^128, less than 3 below the exact product's integer part. */
+SHAPES_HD shapes_u128 shapes_sc_mulhi_near(shapes_u128 a, shapes_u128 b) {
+  const uint64_t a1 = shapes_sc_hi(a), b1 = shapes_sc_hi(b);
+  return shapes_sc_pack(shapes_sc_mulhi64(a1, b1), a1 * b1) + shapes_sc_mulhi64(a1, shapes_sc_lo(b)) +
+         shapes_sc_mulhi64(shapes_sc_lo(a), b1);
+}
+/* (hi, mid, lo) >> sh, sh in [0, 63]: the middle and low words of the result. */
+SHAPES_HD uint64_t shapes_sc_funnel(uint64_t hi, uint64_t lo, int sh) { return (lo >> sh) | ((hi << 1) << (63 - sh)); }
+
+/* v / 2^128 (v not 0) rounded to the nearest double; *decided is cleared when
+ * v is within `err` / 2^64 units in the last place of a rounding boundary (err
+ * is given for a v of 128 significant bits and grows with its leading zeros). */
+SHAPES_HD uint64_t shapes_sc_round_q128(shapes_u128 v, uint64_t err_rel, uint64_t err_abs, int* decided) {
+  uint64_t hi = shapes_sc_hi(v), lo = shapes_sc_lo(v);
+  int lz = 0;
+  if (hi == 0) {
+    hi = lo;
+    lo = 0;
+    lz = 64;
+  }
+  const int n = shapes_sc_clz64(hi);
+  hi = (hi << n) | ((lo >> 1) >> (63 - n));
+  lo <<= n;
+  lz += n;
+  const uint64_t rem = (hi << 53) | (lo >> 11); /* below the last place, in 2^-64 of it */
+  const uint64_t dist = rem >> 63 ? rem - 0x8000000000000000ull : 0x8000000000000000ull - rem;
+  if (lz > 40 || dist <= err_rel + (err_abs << lz)) *decided = 0;
+  return ((uint64_t)(1021 - lz) << 52) + (hi >> 11) + (rem >> 63);
+}
+
+/* The GPU's fast phase for 2^-27 <= |x| < 2^16, in fixed point (compiled for the
+ * host too, where the tests check it against the accurate phase).  Returns 0
+ * when it cannot tell how a result rounds.
+ * With |x| = M 2^E, t = |x| 512/pi = N + f, |f| <= 1/2, r = f pi/512 and
+ * R = 2^8 |r| (128 fractional bits; error below 2^-102 from the truncated
+ * 512/pi).  With Z = R^2 (64 fractional bits),
+ *   cos r = 1 - 2^-17 B,  B = Z - 2^-16 Z^2/12 + 2^-32 Z^3/360,
+ *   sin r = r (1 - 2^-16 D),  D = Z/6 - 2^-16 Z^2/120 + 2^-32 Z^3/5040
+ * (next terms below 2^-82 and r 2^-85; each bracket is within 2^-60).  Then
+ * sin(a + r) and cos(a + r) from the table: within 2^-77, and for a = 0 the sine
+ * within 2^-77 of itself and 2^-108. */
+SHAPES_HD int shapes_sincos_fixed(double x, double* s_out, double* c_out) {
+  const uint64_t bits = shapes_sc_bits(x);
+  const uint64_t M = (bits & ((1ull << 52) - 1)) | (1ull << 52);
+  const int E = (int)((bits >> 52) & 0x7ff) - 1075; /* -79 .. -37 */
+  /* M K 2^(E - 120): the binary point is 128 above bit sh */
+  uint64_t p0 = M * SHAPES_512_OVER_PI_Q120_LO;
+  const uint64_t carry = shapes_sc_mulhi64(M, SHAPES_512_OVER_PI_Q120_LO);
+  uint64_t p1 = M * SHAPES_512_OVER_PI_Q120_HI, p2 = shapes_sc_mulhi64(M, SHAPES_512_OVER_PI_Q120_HI);
+  p1 += carry;
+  p2 += p1 < carry;
+  int sh = -8 - E; /* 29 .. 71 */
+  if (sh >= 64) {
+    p0 = p1;
+    p1 = p2;
+    p2 = 0;
+    sh -= 64;
+  }
+  shapes_u128 F = shapes_sc_pack(shapes_sc_funnel(p2, p1, sh), shapes_sc_funnel(p1, p0, sh));
+  uint32_t N = (uint32_t)(p2 >> sh);
+  const int below = (int)(shapes_sc_hi(F) >> 63); /* the nearer multiple is the next one */
+  if (below) {
+    N += 1;
+    F = (shapes_u128)0 - F;
+  }
+  const shapes_u128 R = shapes_sc_mulhi_near(F << 1, shapes_sc_pack(SHAPES_PIO4_Q128_HI, SHAPES_PIO4_Q128_LO));
+  const uint64_t Rh = shapes_sc_hi(R);
+  if (N != 0 && Rh < (1ull << 42)) return 0; /* |r| < 2^-30 (or f = 1/2 exactly) */
+  const int q = (int)(N >> 8) & 3, i = (int)N & 255;
+  const uint64_t Z = shapes_sc_mulhi64(Rh, Rh), Z2 = shapes_sc_mulhi64(Z, Z), Z3 = shapes_sc_mulhi64(Z2, Z);
+  const uint64_t B = Z - (shapes_sc_mulhi64(Z2, 0x1555555555555555ull) >> 16) +
+                     (shapes_sc_mulhi64(Z3, 0x00b60b60b60b60b6ull) >> 32);
+  const uint64_t D = shapes_sc_mulhi64(Z, 0x2aaaaaaaaaaaaaaaull) -
+                     (shapes_sc_mulhi64(Z2, 0x0222222222222222ull) >> 16) +
+                     (shapes_sc_mulhi64(Z3, 0x000d00d00d00d00dull) >> 32);
+  const shapes_u128 T = shapes_sc_pack(shapes_sc_mulhi64(Rh, D), Rh * D) + shapes_sc_mulhi64(shapes_sc_lo(R), D);
+  const shapes_u128 sr = (R >> 8) - (T >> 24);
+  shapes_u128 S, C;
+  if (i == 0) {
+    S = sr;
+    C = (shapes_u128)0 - ((shapes_u128)B << 47);
+  } else {
+    const shapes_u128 sa = shapes_sc_sin_q128(i), ca = shapes_sc_sin_q128(256 - i);
+    const shapes_u128 cs = shapes_sc_mulhi_near(ca, sr), ss = shapes_sc_mulhi_near(sa, sr);
+    S = sa - ((shapes_u128)shapes_sc_mulhi64(shapes_sc_hi(sa), B) << 47);
+    C = ca - ((shapes_u128)shapes_sc_mulhi64(shapes_sc_hi(ca), B) << 47);
+    S = below ? S - cs : S + cs;
+    C = below ? C + ss : C - ss;
+  }
+  int decided = 1;
+  /* 2^-76 in units in the last place of 1 is 2^41 / 2^64; 2^-70 relative at most 2^47, 2^-104 is 2^13 */
+  uint64_t sb = shapes_sc_round_q128(S, i ? 0 : 1ull << 47, i ? 1ull << 41 : 1ull << 13, &decided);
+  uint64_t cb = shapes_sc_round_q128(C, 0, 1ull << 41, &decided);
+  const uint64_t minus = 1ull << 63;
+  if (i == 0 && below) sb |= minus;
+  /* quadrant: (s, c), (c, -s), (-s, -c), (-c, s) */
+  const uint64_t s1 = q & 1 ? cb : sb, c1 = q & 1 ? sb : cb;
+  *s_out = shapes_sc_from_bits(s1 ^ (q & 2 ? minus : 0) ^ (bits & minus));
+  *c_out = shapes_sc_from_bits(c1 ^ (q == 1 || q == 2 ? minus : 0));
+  return decided;
 }
 
 SHAPES_HD void shapes_sincos(double x, double* s_out, double* c_out) {
@@ -374,12 +497,16 @@ SHAPES_HD void shapes_sincos(double x, double* s_out, double* c_out) {
     *c_out = 1.0;
     return;
   }
+#if defined(__CUDA_ARCH__)
+  if (shapes_sincos_fixed(x, s_out, c_out)) return;
+#else
   double sh, sl, ch, cl;
   if (shapes_sincos_fast2(x, sh, sl, ch, cl) && shapes_sc_decided(sh, sl) && shapes_sc_decided(ch, cl)) {
     *s_out = sh + sl;
     *c_out = ch + cl;
     return;
   }
+#endif
   const shapes_sc_pair r = shapes_sincos_accurate_v(x);
   *s_out = r.s;
   *c_out = r.c;
