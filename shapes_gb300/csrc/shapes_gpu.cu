@@ -117,6 +117,7 @@ struct shapes_batch {
   int32_t pair_cap = 0, contact_cap = 0;
   int64_t item_cap = 0;
   int32_t* row_cnt = nullptr;
+  int32_t* row_hits = nullptr;
   int32_t* row_off = nullptr;
   /* grid broadphase */
   int32_t grid_min_bodies = 64;
@@ -158,6 +159,7 @@ struct shapes_batch {
   int32_t* ext_chunk_off = nullptr;
   double* ext_part_sum = nullptr;
   int32_t* ext_part_cnt = nullptr;
+  int32_t* ext_done = nullptr;
   int32_t n_ext_chunks = 0;
   /* sweep and prune for the small bodies of large grid worlds (incremental pairs off) */
   int32_t sap_min_bodies = 0; /* 0: off */
@@ -176,6 +178,21 @@ struct shapes_batch {
     const int64_t scan_n =
         std::max<int64_t>(std::max<int64_t>(std::max<int64_t>(N, contact_cap), n_buckets), n_sap_buckets) + 1;
     return (int32_t)((scan_n + shapes::kScanTile - 1) / shapes::kScanTile) + 1;
+  }
+
+  void free_scan() {
+    dfree(scan_state.tile);
+    dfree(scan_state.ctl);
+    scan_state = {nullptr, nullptr, 0};
+  }
+  void alloc_scan() {
+    free_scan();
+    tile_cap = scan_tiles_needed();
+    scan_state.tile = dalloc<unsigned long long>(tile_cap, "cudaMalloc scan");
+    scan_state.ctl = dalloc<uint32_t>(3, "cudaMalloc scan");
+    scan_state.tiles = tile_cap;
+    ck(cudaMemsetAsync(scan_state.tile, 0, sizeof(unsigned long long) * tile_cap, stream), "memset");
+    ck(cudaMemsetAsync(scan_state.ctl, 0, 3 * sizeof(uint32_t), stream), "memset");
   }
 
   void free_sap() {
@@ -217,13 +234,10 @@ struct shapes_batch {
     sap_cursor = dalloc<int32_t>(std::max<int32_t>(N, 1), "cudaMalloc sweep");
     sap_end = dalloc<int32_t>(W, "cudaMalloc sweep");
     sap_range = dalloc<uint64_t>(2 * (size_t)W, "cudaMalloc sweep");
+    ck(cudaMemsetAsync(sap_cnt, 0, sizeof(int32_t) * ((size_t)nb + 1), stream), "memset");
     ck(cudaMemcpy(world_sap, flag.data(), W, cudaMemcpyHostToDevice), "upload sweep");
     ck(cudaMemcpy(sap_base, base.data(), sizeof(int32_t) * W, cudaMemcpyHostToDevice), "upload sweep");
-    if (tile_sums && tile_cap < scan_tiles_needed()) { /* the sweep buckets' scan is the longest */
-      dfree(tile_sums);
-      tile_cap = scan_tiles_needed();
-      tile_sums = dalloc<int32_t>(tile_cap, "cudaMalloc scan");
-    }
+    if (scan_state.tile && tile_cap < scan_tiles_needed()) alloc_scan(); /* the sweep buckets' scan is the longest */
   }
   int32_t* np_cls = nullptr; /* [2 * kNpClasses + 1] */
   int32_t* world_pair_off = nullptr;
@@ -299,7 +313,7 @@ struct shapes_batch {
   int sm_count = 0;
   std::vector<int32_t> world_order; /* packing order of the worlds; empty = by body count */
   /* scans */
-  int32_t* tile_sums = nullptr;
+  shapes::ScanState scan_state{nullptr, nullptr, 0};
   int32_t tile_cap = 0;
   unsigned long long* counters = nullptr;
   double* world_residual = nullptr;
@@ -457,6 +471,7 @@ struct shapes_batch {
     d.ext_chunk_off = ext_chunk_off;
     d.ext_part_sum = ext_part_sum;
     d.ext_part_cnt = ext_part_cnt;
+    d.ext_done = ext_done;
     d.n_ext_chunks = n_ext_chunks;
     if (any_sap) {
       d.world_sap = world_sap;
@@ -520,6 +535,7 @@ struct shapes_batch {
       d.nbr_cap = nbr_cap;
     }
     d.row_cnt = row_cnt;
+    d.row_hits = row_hits;
     d.row_off = row_off;
     d.pair_a = pair_a;
     d.pair_b = pair_b;
@@ -596,7 +612,7 @@ struct shapes_batch {
     dfree(sched_info); dfree(sched_list); dfree(sched_arr); dfree(gdesc);
     sched_info = nullptr;
     sched_list = sched_arr = nullptr;
-    dfree(tile_sums);
+    free_scan();
     dfree(snap_key); dfree(snap_lam);
     free_row_buffers();
     dfree(lw_refs); dfree(lw_rank); dfree(lw_hrank); dfree(lw_hitflag);
@@ -615,7 +631,6 @@ struct shapes_batch {
     c_val = nullptr;
     con = nullptr;
     gdesc = nullptr;
-    tile_sums = nullptr;
     snap_key = nullptr;
     snap_lam = nullptr;
   }
@@ -661,8 +676,7 @@ struct shapes_batch {
     sched_list = dalloc<int32_t>(2 * (size_t)contact_cap, "cudaMalloc constraints");
     sched_arr = dalloc<int32_t>(contact_cap, "cudaMalloc constraints");
     gdesc = dalloc<int4>(item_cap + W + 1, "cudaMalloc items");
-    tile_cap = scan_tiles_needed();
-    tile_sums = dalloc<int32_t>(tile_cap, "cudaMalloc scan");
+    alloc_scan();
     if (!large_worlds.empty()) {
       lw_refs = dalloc<int32_t>(2 * (size_t)contact_cap, "cudaMalloc large world");
       lw_rank = dalloc<int32_t>(2 * (size_t)contact_cap, "cudaMalloc large world");
@@ -868,7 +882,7 @@ struct shapes_batch {
     shapes::LW w = lw_view(k);
     const int cap = contact_cap;
     const bool ordered = !(cfg.flags & SHAPES_FLAG_COLOURED);
-    stage(3, ordered ? 11 : 7, [&]() {
+    stage(3, ordered ? 7 : 5, [&]() {
       shapes::k_lw_setup<<<grid_for(w.nb + 1, 256), 256, 0, stream>>>(d, w);
       shapes::k_lw_count<<<grid_for(cap, 256), 256, 0, stream>>>(d, w, cfg.iterations);
       scan_raw(w.bcnt, w.nb, nullptr, w.bstart);
@@ -970,9 +984,10 @@ struct shapes_batch {
     ck(cudaMemcpy(grid_T, T.data(), sizeof(int32_t) * W, cudaMemcpyHostToDevice), "upload grid");
     ck(cudaMemcpy(grid_base, base.data(), sizeof(int32_t) * W, cudaMemcpyHostToDevice), "upload grid");
     ck(cudaMemset(row_mode, 0, N), "memset");
+    ck(cudaMemsetAsync(bucket_cnt, 0, sizeof(int32_t) * ((size_t)n_buckets + 1), stream), "memset");
     {
       /* chunks of at most 4096 bodies, never crossing a world (empty worlds have none) */
-      dfree(ext_chunk); dfree(ext_chunk_off); dfree(ext_part_sum); dfree(ext_part_cnt);
+      dfree(ext_chunk); dfree(ext_chunk_off); dfree(ext_part_sum); dfree(ext_part_cnt); dfree(ext_done);
       std::vector<int32_t> ranges, choff(W + 1, 0);
       for (int w = 0; w < W; ++w) {
         choff[w] = (int32_t)(ranges.size() / 2);
@@ -987,6 +1002,8 @@ struct shapes_batch {
       ext_chunk_off = dalloc<int32_t>((size_t)W + 1, "cudaMalloc grid");
       ext_part_sum = dalloc<double>(std::max<int32_t>(n_ext_chunks, 1), "cudaMalloc grid");
       ext_part_cnt = dalloc<int32_t>(std::max<int32_t>(n_ext_chunks, 1), "cudaMalloc grid");
+      ext_done = dalloc<int32_t>(W, "cudaMalloc grid");
+      ck(cudaMemsetAsync(ext_done, 0, sizeof(int32_t) * W, stream), "memset");
       if (n_ext_chunks)
         ck(cudaMemcpy(ext_chunk, ranges.data(), sizeof(int32_t) * ranges.size(), cudaMemcpyHostToDevice),
            "upload grid");
@@ -996,15 +1013,17 @@ struct shapes_batch {
     setup_sap();
   }
 
-  void scan(const int32_t* in, int n_cap, const unsigned long long* n_dev, int32_t* out) {
-    stage(6, 3, [&]() { scan_raw(in, n_cap, n_dev, out); });
+  /* One exclusive scan; clear, total and overflow as in k_scan. */
+  void scan_raw(int32_t* in, int n_cap, const unsigned long long* n_dev, int32_t* out, bool clear = false,
+                unsigned long long* total = nullptr, int32_t total_cap = 0, unsigned overflow_bit = 0) {
+    const int tiles = n_cap / shapes::kScanTile + 1;
+    shapes::k_scan<<<std::min(tiles, 2 * kSMs), shapes::kScanThreads, 0, stream>>>(
+        in, n_cap, n_dev, scan_state, out, clear ? 1 : 0, total, total_cap, counters + shapes::kCntOverflow,
+        overflow_bit, counters + shapes::kCntSolveErr);
   }
-
-  void scan_raw(const int32_t* in, int n_cap, const unsigned long long* n_dev, int32_t* out) {
-    const int tiles = (n_cap + 1 + shapes::kScanTile - 1) / shapes::kScanTile;
-    shapes::k_scan_tiles<<<tiles, shapes::kScanThreads, 0, stream>>>(in, n_cap, n_dev, tile_sums);
-    shapes::k_scan_tile_sums<<<1, 1024, 0, stream>>>(tile_sums, tiles);
-    shapes::k_scan_apply<<<tiles, shapes::kScanThreads, 0, stream>>>(in, n_cap, n_dev, tile_sums, out);
+  template <class... A>
+  void scan(A... a) {
+    stage(6, 1, [&]() { scan_raw(a...); });
   }
 
   void pose(int advance, double dt) {
@@ -1028,69 +1047,74 @@ struct shapes_batch {
       d.judge_res = judge_res;
       d.judge_depth = judge_depth;
     }
-    /* pairs/contacts and the group allocator are per step; hits, items and
-     * levels add up over the call */
-    ck(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * 2, stream), "memset");
-    ck(cudaMemsetAsync(counters + shapes::kCntGroupAlloc, 0, sizeof(unsigned long long), stream), "memset");
-    ck(cudaMemsetAsync(counters + shapes::kCntListAlloc, 0, sizeof(unsigned long long), stream), "memset");
+    ck(cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * shapes::kCntPerStep, stream), "memset");
     const bool inc = any_grid && d.nbr != nullptr;
     const bool sap = any_sap && !inc;
+    auto by_team = [&](auto launch) {
+      if (shapes::row_teams(N)) launch(std::integral_constant<int, shapes::kRowTeam>{});
+      else launch(std::integral_constant<int, shapes::kRowPair>{});
+    };
     if (!sap) d.world_sap = nullptr;
+    /* the bucket counts are zero between steps: their scan leaves them so */
     if (inc) {
-      stage(0, 7, [&]() {
-        ck(cudaMemsetAsync(bucket_cnt, 0, sizeof(int32_t) * ((size_t)n_buckets + 1), stream), "memset");
-        if (n_ext_chunks) shapes::k_extent_parts<<<n_ext_chunks, 256, 0, stream>>>(d, 1);
-        shapes::k_inc_stats<<<grid_for(W, 128), 128, 0, stream>>>(d);
+      stage(0, 3, [&]() {
+        if (n_ext_chunks) shapes::k_grid_stats<<<n_ext_chunks, 256, 0, stream>>>(d, 1);
         shapes::k_inc_mark<<<grid_for(N, 256), 256, 0, stream>>>(d);
-        shapes::k_inc_decide<<<grid_for(W, 128), 128, 0, stream>>>(d);
-        shapes::k_inc_remove<<<grid_for(N, 128), 128, 0, stream>>>(d);
-        shapes::k_inc_refat<<<grid_for(N, 256), 256, 0, stream>>>(d);
+        shapes::k_inc_update<<<grid_for(N, 128), 128, 0, stream>>>(d);
       });
-      scan(bucket_cnt, n_buckets, nullptr, bucket_off);
+      scan(bucket_cnt, n_buckets, nullptr, bucket_off, true);
       stage(0, 2, [&]() {
         shapes::k_inc_scatter<<<grid_for(N, 256), 256, 0, stream>>>(d);
-        shapes::k_inc_query<<<grid_for(N, 128), 128, 0, stream>>>(d);
+        by_team([&](auto team) {
+          constexpr int kTeam = decltype(team)::value;
+          shapes::k_inc_query<kTeam><<<grid_for((long long)N * kTeam, shapes::kRowThreads), shapes::kRowThreads, 0,
+                                       stream>>>(d);
+        });
       });
     } else if (any_grid) {
-      stage(0, 4, [&]() {
-        ck(cudaMemsetAsync(bucket_cnt, 0, sizeof(int32_t) * ((size_t)n_buckets + 1), stream), "memset");
-        if (n_ext_chunks) shapes::k_extent_parts<<<n_ext_chunks, 256, 0, stream>>>(d, 0);
-        shapes::k_grid_stats<<<grid_for(W, 128), 128, 0, stream>>>(d);
+      stage(0, 2, [&]() {
+        if (n_ext_chunks) shapes::k_grid_stats<<<n_ext_chunks, 256, 0, stream>>>(d, 0);
         shapes::k_grid_bin<<<grid_for(N, 256), 256, 0, stream>>>(d);
       });
-      scan(bucket_cnt, n_buckets, nullptr, bucket_off);
+      scan(bucket_cnt, n_buckets, nullptr, bucket_off, true);
       stage(0, 1, [&]() { shapes::k_grid_scatter<<<grid_for(N, 256), 256, 0, stream>>>(d); });
       if (sap) {
-        stage(0, 2, [&]() {
-          ck(cudaMemsetAsync(sap_cnt, 0, sizeof(int32_t) * ((size_t)n_sap_buckets + 1), stream), "memset");
-          shapes::k_sap_count<<<grid_for(N, 256), 256, 0, stream>>>(d);
-        });
-        scan(sap_cnt, n_sap_buckets, nullptr, sap_off);
+        stage(0, 1, [&]() { shapes::k_sap_count<<<grid_for(N, 256), 256, 0, stream>>>(d); });
+        scan(sap_cnt, n_sap_buckets, nullptr, sap_off, true);
         stage(0, 2, [&]() {
           shapes::k_sap_scatter<<<grid_for(N, 256), 256, 0, stream>>>(d);
           shapes::k_sap_ends<<<grid_for(W, 128), 128, 0, stream>>>(d);
         });
       }
     }
-    stage(0, any_grid ? (sap ? 3 : 2) : 1, [&]() {
-      shapes::k_broadphase<true><<<grid_for((long long)N * 32, 256), 256, 0, stream>>>(d);
-      if (inc)
-        shapes::k_inc_rows<true><<<grid_for(N, 128), 128, 0, stream>>>(d);
-      else if (any_grid)
-        shapes::k_grid_rows<true><<<grid_for(N, 128), 128, 0, stream>>>(d);
+    stage(0, sap ? 2 : 1, [&]() {
+      if (any_grid)
+        by_team([&](auto team) {
+          constexpr int kTeam = decltype(team)::value;
+          const int blocks = grid_for((long long)N * kTeam, shapes::kRowThreads);
+          if (inc)
+            shapes::k_count_rows<true, kTeam><<<blocks, shapes::kRowThreads, 0, stream>>>(d);
+          else
+            shapes::k_count_rows<false, kTeam><<<blocks, shapes::kRowThreads, 0, stream>>>(d);
+        });
+      else
+        shapes::k_count_brute<<<grid_for((long long)N * 32, 256), 256, 0, stream>>>(d);
       if (sap) shapes::k_sap_rows<true><<<grid_for(N, 128), 128, 0, stream>>>(d);
     });
-    scan(row_cnt, N, nullptr, row_off);
-    stage(0, any_grid ? (sap ? 4 : 3) : 1, [&]() {
-      shapes::k_broadphase<false><<<grid_for((long long)N * 32, 256), 256, 0, stream>>>(d);
+    scan(row_cnt, N, nullptr, row_off, false, counters + shapes::kCntPairs, pair_cap, 1u);
+    stage(0, sap ? 3 : 1, [&]() {
+      const int blocks = grid_for(N, shapes::kRowThreads);
       if (inc)
-        shapes::k_inc_rows<false><<<grid_for(N, 128), 128, 0, stream>>>(d);
+        shapes::k_write_rows<true, true><<<blocks, shapes::kRowThreads, 0, stream>>>(d);
       else if (any_grid)
-        shapes::k_grid_rows<false><<<grid_for(N, 128), 128, 0, stream>>>(d);
-      if (sap) shapes::k_sap_rows<false><<<grid_for(N, 128), 128, 0, stream>>>(d);
-      if (any_grid) shapes::k_grid_sort_rows<<<grid_for(N, 128), 128, 0, stream>>>(d);
+        shapes::k_write_rows<true, false><<<blocks, shapes::kRowThreads, 0, stream>>>(d);
+      else
+        shapes::k_write_rows<false, false><<<blocks, shapes::kRowThreads, 0, stream>>>(d);
+      if (sap) {
+        shapes::k_sap_rows<false><<<grid_for(N, 128), 128, 0, stream>>>(d);
+        shapes::k_sap_sort_rows<<<grid_for(N, 128), 128, 0, stream>>>(d);
+      }
     });
-    stage(6, 1, [&]() { shapes::k_world_pair_offsets<<<grid_for(W + 1, 128), 128, 0, stream>>>(d); });
     stage(1, np_lanes > 1 ? 4 : 1, [&]() {
       if (np_lanes <= 1) {
         shapes::k_narrowphase<<<grid_for(pair_cap, shapes::kNpThreads), shapes::kNpThreads, 0, stream>>>(d);
@@ -1108,8 +1132,8 @@ struct shapes_batch {
         default: shapes::k_narrowphase_lanes<32><<<grid_for(32LL * pair_cap, 128), 128, 0, stream>>>(d); break;
       }
     });
-    scan(slot_cnt, pair_cap, counters + shapes::kCntPairs, slot_off);
-    stage(6, 1, [&]() { shapes::k_world_contact_offsets<<<grid_for(W + 1, 128), 128, 0, stream>>>(d); });
+    scan(slot_cnt, pair_cap, counters + shapes::kCntPairs, slot_off, false, counters + shapes::kCntContacts, contact_cap,
+         2u);
     stage(2, 2, [&]() {
       shapes::k_contact_slots<<<grid_for(2LL * pair_cap, 256), 256, 0, stream>>>(d);
       shapes::k_build<<<grid_for(contact_cap, 128), 128, 0, stream>>>(d, cfg.baumgarte / cfg.dt, cfg.slop,
@@ -1117,7 +1141,7 @@ struct shapes_batch {
     });
     if (!solve) return;
     if (learn || collect) {
-      stage(7, 4 + (learn ? 2 : 0), [&]() {
+      stage(7, 2 + (learn ? 2 : 0), [&]() {
         scan_raw(miss_flag, contact_cap, counters + shapes::kCntContacts, miss_off);
         shapes::k_learned_features<<<grid_for(contact_cap, 128), 128, 0, stream>>>(d, cfg.external, cfg.accel_x,
                                                                                   cfg.accel_y, cfg.dt);
@@ -1278,7 +1302,7 @@ struct shapes_batch {
       return SHAPES_E_TIMEOUT;
     }
     if (agg[shapes::kCntSolveErr]) {
-      g_last_error = "group solver: a bounded wait gave up";
+      g_last_error = "group solver or scan: a bounded wait gave up";
       return SHAPES_E_TIMEOUT;
     }
     if (!agg[shapes::kCntOverflow] && solve && !large_worlds.empty()) {
@@ -1372,7 +1396,7 @@ struct shapes_batch {
     }
     dfree(wx); dfree(wy); dfree(nx); dfree(ny); dfree(box); dfree(boxk); dfree(flags); dfree(body_changed);
     dfree(vf); dfree(ef);
-    dfree(row_cnt); dfree(row_off); dfree(world_pair_off); dfree(sched_body); dfree(sched_cur); dfree(world_levels);
+    dfree(row_cnt); dfree(row_hits); dfree(row_off); dfree(world_pair_off); dfree(sched_body); dfree(sched_cur); dfree(world_levels);
     for (int k = 0; k < 6; ++k) dfree(snap_body[k]);
     dfree(active);
     active = nullptr;
@@ -1405,6 +1429,7 @@ struct shapes_batch {
     flags = dalloc<uint8_t>(N, "cudaMalloc");
     body_changed = dalloc<uint8_t>(N, "cudaMalloc");
     row_cnt = dalloc<int32_t>(N, "cudaMalloc");
+    row_hits = dalloc<int32_t>(shapes::kRowHits * (size_t)N, "cudaMalloc");
     row_off = dalloc<int32_t>((size_t)N + 1, "cudaMalloc");
     world_pair_off = dalloc<int32_t>(n_worlds + 1, "cudaMalloc");
     if (!cwo[0])
@@ -1496,10 +1521,10 @@ struct shapes_batch {
     }
     dfree(wx); dfree(wy); dfree(nx); dfree(ny); dfree(box); dfree(boxk); dfree(flags); dfree(body_changed);
     dfree(vf); dfree(ef);
-    dfree(row_cnt); dfree(row_off); dfree(world_pair_off);
+    dfree(row_cnt); dfree(row_hits); dfree(row_off); dfree(world_pair_off);
     dfree(grid_T); dfree(grid_base); dfree(grid_inv_s); dfree(grid_lim); dfree(bucket_cnt); dfree(bucket_off);
     dfree(grid_ids); dfree(cell_x); dfree(cell_y); dfree(row_mode); dfree(large_cnt); dfree(large_ids);
-    dfree(ext_chunk); dfree(ext_chunk_off); dfree(ext_part_sum); dfree(ext_part_cnt);
+    dfree(ext_chunk); dfree(ext_chunk_off); dfree(ext_part_sum); dfree(ext_part_cnt); dfree(ext_done);
     free_sap();
     free_incremental();
     dfree(radius);
@@ -3053,8 +3078,8 @@ constexpr int kNaTiles = (kNaMaxPairs + 1 + shapes::kScanTile - 1) / shapes::kSc
 /* Byte offsets of the scratch arrays, each 256-byte aligned. */
 struct NaPlan {
   size_t world_body_off, body_world, lx, ly, emin, emax, wx, wy, nx, ny, vf, ef, box, boxk, flags, row_mode, row_cnt,
-      row_off, pair_a, pair_b, slot_cnt, slot_off, slot_feat, slot_val, world_pair_off, cwo, c_key, c_ga, c_gb,
-      c_flip, c_hit, c_val, tile_sums, counters, total;
+      row_hits, row_off, pair_a, pair_b, slot_cnt, slot_off, slot_feat, slot_val, world_pair_off, cwo, c_key, c_ga, c_gb,
+      c_flip, c_hit, c_val, tiles, scan_ctl, counters, total;
 };
 
 constexpr size_t na_take(size_t& o, size_t bytes) {
@@ -3083,6 +3108,7 @@ constexpr NaPlan na_plan() {
   p.flags = na_take(o, kNaMaxBodies);
   p.row_mode = na_take(o, kNaMaxBodies);
   p.row_cnt = na_take(o, kNaMaxBodies * sizeof(int32_t));
+  p.row_hits = na_take(o, shapes::kRowHits * kNaMaxBodies * sizeof(int32_t));
   p.row_off = na_take(o, (kNaMaxBodies + 1) * sizeof(int32_t));
   p.pair_a = na_take(o, kNaMaxPairs * sizeof(int32_t));
   p.pair_b = na_take(o, kNaMaxPairs * sizeof(int32_t));
@@ -3098,8 +3124,9 @@ constexpr NaPlan na_plan() {
   p.c_flip = na_take(o, kNaMaxContacts);
   p.c_hit = na_take(o, kNaMaxContacts);
   p.c_val = na_take(o, 5 * (size_t)kNaMaxContacts * sizeof(double));
-  p.tile_sums = na_take(o, kNaTiles * sizeof(int32_t));
-  p.counters = na_take(o, 8 * sizeof(unsigned long long));
+  p.tiles = na_take(o, kNaTiles * sizeof(unsigned long long));
+  p.scan_ctl = na_take(o, 3 * sizeof(uint32_t));
+  p.counters = na_take(o, shapes::kCntSlots * sizeof(unsigned long long));
   p.total = o;
   return p;
 }
@@ -3270,6 +3297,7 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   d.flags = base + kNaPlan.flags;
   d.row_mode = base + kNaPlan.row_mode;
   d.row_cnt = reinterpret_cast<int32_t*>(base + kNaPlan.row_cnt);
+  d.row_hits = reinterpret_cast<int32_t*>(base + kNaPlan.row_hits);
   d.row_off = reinterpret_cast<int32_t*>(base + kNaPlan.row_off);
   d.pair_a = reinterpret_cast<int32_t*>(base + kNaPlan.pair_a);
   d.pair_b = reinterpret_cast<int32_t*>(base + kNaPlan.pair_b);
@@ -3286,16 +3314,18 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   d.c_hit = base + kNaPlan.c_hit;
   d.c_val = reinterpret_cast<double*>(base + kNaPlan.c_val);
   d.counters = reinterpret_cast<unsigned long long*>(base + kNaPlan.counters);
-  int32_t* tile_sums = reinterpret_cast<int32_t*>(base + kNaPlan.tile_sums);
-  auto scan = [&](const int32_t* in, int n_cap, const unsigned long long* n_dev, int32_t* out) {
-    const int tiles = (n_cap + 1 + shapes::kScanTile - 1) / shapes::kScanTile;
-    shapes::k_scan_tiles<<<tiles, shapes::kScanThreads, 0, st>>>(in, n_cap, n_dev, tile_sums);
-    shapes::k_scan_tile_sums<<<1, 1024, 0, st>>>(tile_sums, tiles);
-    shapes::k_scan_apply<<<tiles, shapes::kScanThreads, 0, st>>>(in, n_cap, n_dev, tile_sums, out);
+  /* the scan's words are zero when the library is loaded and as the last scan left them after that */
+  const shapes::ScanState scan_state{reinterpret_cast<unsigned long long*>(base + kNaPlan.tiles),
+                                     reinterpret_cast<uint32_t*>(base + kNaPlan.scan_ctl), kNaTiles};
+  auto scan = [&](int32_t* in, int n_cap, const unsigned long long* n_dev, int32_t* out, unsigned long long* total,
+                  int cap, unsigned bit) {
+    shapes::k_scan<<<n_cap / shapes::kScanTile + 1, shapes::kScanThreads, 0, st>>>(
+        in, n_cap, n_dev, scan_state, out, 0, total, cap, d.counters + shapes::kCntOverflow, bit,
+        d.counters + shapes::kCntSolveErr);
   };
   /* counters start at zero; the set-up kernel validates the vertex offsets */
-  cudaError_t e = cudaMemsetAsync(d.counters, 0, 8 * sizeof(unsigned long long), st);
-  unsigned long long cnt[8] = {0};
+  cudaError_t e = cudaMemsetAsync(d.counters, 0, shapes::kCntSlots * sizeof(unsigned long long), st);
+  unsigned long long cnt[shapes::kCntSlots] = {0};
   if (e == cudaSuccess) {
     k_noalloc_setup<<<grid_for(std::max(n_bodies, n_verts), 256), 256, 0, st>>>(
         n_bodies, n_verts, vert_offsets, local_verts_xy, pos_x, pos_y, rot, inv_mass_lin, inv_mass_rot, base);
@@ -3324,13 +3354,12 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   }
   shapes::k_init_extents<<<grid_for(n_verts, 128), 128, 0, st>>>(d);
   launch_pose(st, n_bodies, d, 0.0, 0);
-  shapes::k_broadphase<true><<<grid_for((long long)n_bodies * 32, 256), 256, 0, st>>>(d);
-  scan(d.row_cnt, n_bodies, nullptr, d.row_off);
-  shapes::k_broadphase<false><<<grid_for((long long)n_bodies * 32, 256), 256, 0, st>>>(d);
-  shapes::k_world_pair_offsets<<<1, 32, 0, st>>>(d);
+  shapes::k_count_brute<<<grid_for((long long)n_bodies * 32, 256), 256, 0, st>>>(d);
+  scan(d.row_cnt, n_bodies, nullptr, d.row_off, d.counters + shapes::kCntPairs, d.pair_cap, 1u);
+  shapes::k_write_rows<false, false><<<grid_for(n_bodies, shapes::kRowThreads), shapes::kRowThreads, 0, st>>>(d);
   shapes::k_narrowphase<<<grid_for(kNaMaxPairs, shapes::kNpThreads), shapes::kNpThreads, 0, st>>>(d);
-  scan(d.slot_cnt, kNaMaxPairs, d.counters + shapes::kCntPairs, d.slot_off);
-  shapes::k_world_contact_offsets<<<1, 32, 0, st>>>(d);
+  scan(d.slot_cnt, kNaMaxPairs, d.counters + shapes::kCntPairs, d.slot_off, d.counters + shapes::kCntContacts,
+       d.contact_cap, 2u);
   shapes::k_build<<<grid_for(2LL * kNaMaxPairs, 128), 128, 0, st>>>(d, 0.0, 0.0, 0, 0);
   e = cudaMemcpyAsync(cnt, d.counters, sizeof(cnt), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -3338,6 +3367,10 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   if (e != cudaSuccess) {
     g_last_error = std::string("shapes_collide_noalloc: ") + cudaGetErrorString(e);
     return SHAPES_E_CUDA;
+  }
+  if (cnt[shapes::kCntSolveErr]) {
+    g_last_error = "shapes_collide_noalloc: a scan's bounded wait gave up";
+    return SHAPES_E_TIMEOUT;
   }
   *n_pairs = (int64_t)cnt[shapes::kCntPairs];
   *n_contacts = (int64_t)cnt[shapes::kCntContacts];

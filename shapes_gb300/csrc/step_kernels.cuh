@@ -112,6 +112,7 @@ struct Dev {
   double* inc_margin;    /* [W] fat-box margin */
   int32_t nbr_cap;
   int32_t* row_cnt; /* [N] mirrored per-row pair counts */
+  int32_t* row_hits; /* [kRowHits * N] the pairs of rows with few, descending j */
   int32_t* row_off; /* [N+1] scanned */
   int32_t* pair_a;  /* [pair_cap] global body index, the larger */
   int32_t* pair_b;  /* [pair_cap] */
@@ -123,6 +124,7 @@ struct Dev {
   const int32_t* ext_chunk_off; /* [n_worlds + 1] each world's chunks */
   double* ext_part_sum;         /* [n_ext_chunks] chunk sums of box extents */
   int32_t* ext_part_cnt;        /* [n_ext_chunks] chunk counts */
+  int32_t* ext_done;            /* [W] chunks of the world summed so far this step */
   int32_t n_ext_chunks;
   const uint8_t* world_sap; /* [n_worlds] 1: the world's small bodies pair by sweep and prune (null: none) */
   const int32_t* sap_base;  /* [n_worlds] first of the world's kSapBuckets buckets */
@@ -178,19 +180,21 @@ struct Dev {
 };
 
 enum {
+  /* reset every step, the others every call */
   kCntPairs = 0,
   kCntContacts = 1,
-  kCntHits = 2,
-  kCntItems = 3,
-  kCntLevels = 4,
-  kCntOverflow = 5,
-  kCntBadInput = 6,
-  kCntGroupAlloc = 7, /* bump allocator of the per-group regions (reset every step) */
-  kCntPredicted = 8,  /* contacts started from the network (summed over the call) */
-  kCntReverted = 9,   /* worlds the judge switched back to the plain start */
-  kCntMlpErr = 10,    /* set when a tensor-core wait of the network gave up */
-  kCntListAlloc = 11, /* bump allocator of the lists kept in global memory (reset every step) */
-  kCntSolveErr = 12,  /* set when a wait between a solver group's warps gave up */
+  kCntGroupAlloc = 2, /* bump allocator of the groups' runs of updates kept in global memory */
+  kCntListAlloc = 3,  /* bump allocator of the lists kept in global memory */
+  kCntPerStep = 4,
+  kCntHits = 4,
+  kCntItems = 5,
+  kCntLevels = 6,
+  kCntOverflow = 7,
+  kCntBadInput = 8,
+  kCntPredicted = 9, /* contacts started from the network (summed over the call) */
+  kCntReverted = 10, /* worlds the judge switched back to the plain start */
+  kCntMlpErr = 11,   /* set when a tensor-core wait of the network gave up */
+  kCntSolveErr = 12, /* set when a wait between a solver group's warps or a scan's blocks gave up */
   kCntSlots = 16,
 };
 
@@ -555,10 +559,10 @@ __global__ void __launch_bounds__(kPoseThreads) k_integrate_pose(Dev d, double d
 
 /* culledKeys (Aabb.hs:168-183): not both static, and boundsOverlap
  * (Aabb.hs:69-72) on x and y, i.e. not (c > b || d < a) with (a,b) = box i,
- * (c,d) = box j. */
-__device__ __forceinline__ bool pair_overlaps(const Dev& d, int gi, int gj, uint8_t fi,
-                                              const uint64_t ki[4]) {
-  const uint8_t fj = d.flags[gj];
+ * (c,d) = box j.  The flags and the box of j are loaded together by the
+ * callers: one trip to L2 instead of two. */
+__device__ __forceinline__ bool keys_overlap(const Dev& d, int gi, int gj, uint8_t fi, uint8_t fj,
+                                             const uint64_t ki[4], ulonglong2 kj01, ulonglong2 kj23) {
   if ((fi | fj) & kFlagInactive) return false;
   if ((fi & fj & kFlagStatic)) return false;
   if ((fi | fj) & kFlagBoxNaN) {
@@ -566,54 +570,92 @@ __device__ __forceinline__ bool pair_overlaps(const Dev& d, int gi, int gj, uint
     const double* b = d.box + 4 * gj;
     return !(b[0] > a[1] || b[1] < a[0]) && !(b[2] > a[3] || b[3] < a[2]);
   }
-  const ulonglong2 kj01 = *reinterpret_cast<const ulonglong2*>(d.boxk + 4 * gj);
-  const ulonglong2 kj23 = *reinterpret_cast<const ulonglong2*>(d.boxk + 4 * gj + 2);
   return !(kj01.x > ki[1] || kj01.y < ki[0]) && !(kj23.x > ki[3] || kj23.y < ki[2]);
 }
 
-/* One warp per row i (the larger index of a pair): lanes test j = i-1, i-2, ...
- * 32 at a time, so ballot order is the reference's descending j order.
- * COUNT: writes the row's pair count at its mirrored position
- * q = off + (n_w - 1 - i), so that an exclusive scan over q lays rows out in
- * descending i within each world.  !COUNT: writes the pairs at row_off[q]. */
+__device__ __forceinline__ bool pair_overlaps(const Dev& d, int gi, int gj, uint8_t fi,
+                                              const uint64_t ki[4]) {
+  const uint8_t fj = d.flags[gj];
+  const ulonglong2 kj01 = *reinterpret_cast<const ulonglong2*>(d.boxk + 4 * gj);
+  const ulonglong2 kj23 = *reinterpret_cast<const ulonglong2*>(d.boxk + 4 * gj + 2);
+  return keys_overlap(d, gi, gj, fi, fj, ki, kj01, kj23);
+}
+
+constexpr int kRowHits = 8;        /* pairs of a row that the counting pass keeps */
+constexpr int kRowSorted = 256;    /* pairs of a row that a warp sorts in shared memory */
+constexpr int kRowThreads = 256;
+
+/* Lanes per grid row.  While all of the batch's rows run at once with eight
+ * lanes each (2048 threads an SM), the chain of loads of one lane is what takes
+ * the time, and eight are the fastest; above that two are, because each lane of a
+ * row repeats the row's own loads.  The incremental broadphase with 8, 4, 2 and 1
+ * lanes, us: 9,075 bodies 64, 70, 82, 104; 32,771: 65, 63, 74, 97; 65,539: 89,
+ * 83, 88, 118; 262,144: 198, 178, 171, 196; 505,800: 279, 245, 203, 196. */
+constexpr int kRowTeam = 8, kRowPair = 2;
+inline bool row_teams(long long n) { return n * kRowTeam <= 152 * 2048; }
+
+/* Row i (the larger index of a pair, body g) by brute force, a warp together:
+ * lanes test j = i-1, i-2, ... 64 at a time (two loads in flight per lane),
+ * so ballot order is the reference's descending j order.  COUNT: writes the
+ * row's pair count at its mirrored position q = off + (n_w - 1 - i), so that an
+ * exclusive scan over q lays rows out in descending i within each world, and
+ * keeps the first kRowHits pairs.  !COUNT: writes the pairs at row_off[q]. */
 template <bool COUNT>
-__global__ void k_broadphase(Dev d) {
+__device__ __forceinline__ void brute_row(const Dev& d, int g) {
+  constexpr int kU = 2;
   const int lane = threadIdx.x & 31;
-  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int nw_total = (gridDim.x * blockDim.x) >> 5;
-  for (int g = wid; g < d.n_bodies; g += nw_total) {
-    if (d.row_mode[g]) continue; /* this row comes from the grid */
-    const int wld = d.body_world[g];
-    const int off = d.world_body_off[wld];
-    const int n = d.world_body_off[wld + 1] - off;
-    const int i = g - off;
-    const int q = off + (n - 1 - i);
-    const uint8_t fi = d.flags[g];
-    uint64_t ki[4];
-    ki[0] = d.boxk[4 * g + 0];
-    ki[1] = d.boxk[4 * g + 1];
-    ki[2] = d.boxk[4 * g + 2];
-    ki[3] = d.boxk[4 * g + 3];
-    int count = 0;
-    const int base_out = COUNT ? 0 : d.row_off[q];
-    for (int base = 0; base < i; base += 32) {
-      const int jl = i - 1 - base - lane;
+  const int wld = d.body_world[g];
+  const int off = d.world_body_off[wld];
+  const int n = d.world_body_off[wld + 1] - off;
+  const int i = g - off;
+  const int q = off + (n - 1 - i);
+  const uint8_t fi = d.flags[g];
+  uint64_t ki[4];
+  ki[0] = d.boxk[4 * g + 0];
+  ki[1] = d.boxk[4 * g + 1];
+  ki[2] = d.boxk[4 * g + 2];
+  ki[3] = d.boxk[4 * g + 3];
+  int count = 0;
+  const int base_out = COUNT ? 0 : d.row_off[q];
+  for (int base = 0; base < i; base += 32 * kU) {
+    uint8_t fj[kU];
+    ulonglong2 k01[kU], k23[kU];
+    const int j0 = i - 1 - base - lane;
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      if (j0 - 32 * u < 0) continue;
+      const int gj = off + j0 - 32 * u;
+      fj[u] = d.flags[gj];
+      k01[u] = *reinterpret_cast<const ulonglong2*>(d.boxk + 4 * gj);
+      k23[u] = *reinterpret_cast<const ulonglong2*>(d.boxk + 4 * gj + 2);
+    }
+#pragma unroll
+    for (int u = 0; u < kU; ++u) {
+      const int jl = j0 - 32 * u;
       bool hit = false;
-      if (jl >= 0) hit = pair_overlaps(d, g, off + jl, fi, ki);
+      if (jl >= 0) hit = keys_overlap(d, g, off + jl, fi, fj[u], ki, k01[u], k23[u]);
       const unsigned m = __ballot_sync(0xffffffffu, hit);
-      if (!COUNT && hit) {
-        const int pos = base_out + count + __popc(m & ((1u << lane) - 1u));
-        if (pos < d.pair_cap) {
-          d.pair_a[pos] = g;
-          d.pair_b[pos] = off + jl;
+      if (hit) {
+        const int at = count + __popc(m & ((1u << lane) - 1u));
+        if (COUNT) {
+          if (at < kRowHits) d.row_hits[kRowHits * (size_t)g + at] = off + jl;
+        } else if (base_out + at < d.pair_cap) {
+          d.pair_a[base_out + at] = g;
+          d.pair_b[base_out + at] = off + jl;
         }
       }
       count += __popc(m);
     }
-    if (COUNT && lane == 0) d.row_cnt[q] = count;
   }
+  if (COUNT && lane == 0) d.row_cnt[q] = count;
 }
 
+/* Counts the rows of a batch without a grid world: a warp per row. */
+__global__ void k_count_brute(Dev d) {
+  const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int nw_total = (gridDim.x * blockDim.x) >> 5;
+  for (int g = wid; g < d.n_bodies; g += nw_total) brute_row<true>(d, g);
+}
 
 /* Grid broadphase for larger worlds.  It finds exactly the pairs the
  * brute-force rows find, faster: the cell size s is twice the mean AABB extent
@@ -644,22 +686,44 @@ __device__ __forceinline__ uint32_t cell_bucket(int cx, int cy, int T) {
   return (spread16((uint32_t)cx) | (spread16((uint32_t)cy) << 1)) & (uint32_t)(T - 1);
 }
 
-/* One CTA per world: mean of max(width, height) over finite boxes -> 1/s. */
-/* Mean box extent of each grid world, which sets its cell size (2x the mean).
- * The cell size only decides how fast the grid finds the pairs, never which
- * pairs it finds (any positive size gives the pairs of culledKeys), so the sum
- * may be split: one block per chunk of at most 4096 bodies of one world
- * (k_extent_parts), then one thread per world adds its chunks in order
- * (deterministic; a world of one chunk sums exactly as one block would).  A
- * single large world thus spreads over the GPU instead of one SM. */
-__global__ void k_extent_parts(Dev d, int inc) {
+/* Twice the mean extent over a world's chunks, added in chunk order. */
+__device__ __forceinline__ double world_cell_size(const Dev& d, int wld) {
+  double t = 0.0;
+  int c = 0;
+  for (int k = d.ext_chunk_off[wld]; k < d.ext_chunk_off[wld + 1]; ++k) {
+    t += __ldcg(d.ext_part_sum + k);
+    c += __ldcg(d.ext_part_cnt + k);
+  }
+  return c > 0 ? 2.0 * t / c : 0.0;
+}
+
+/* Mean box extent of each grid world, which sets its cell size (2x the mean),
+ * its reciprocal, the size limit of a grid body and the fat-box margin.  The
+ * cell size only decides how fast the grid finds the pairs, never which pairs
+ * it finds (any positive size gives the pairs of culledKeys), so the sum may be
+ * split: one block per chunk of at most 4096 bodies of one world, and the last
+ * block of a world to finish adds its chunks in order (deterministic; a world
+ * of one chunk sums exactly as one block would).  A single large world thus
+ * spreads over the GPU instead of one SM.  With incremental pairs only a world
+ * that rebuilds needs a cell size.  Every world's large list and moved count
+ * start empty here. */
+__global__ void k_grid_stats(Dev d, int inc) {
   __shared__ double s_sum[32];
   __shared__ int s_cnt[32];
   const int k = blockIdx.x;
   if (k >= d.n_ext_chunks) return;
   const int b0 = d.ext_chunk[2 * k], b1 = d.ext_chunk[2 * k + 1];
   const int wld = d.body_world[b0];
-  if (d.grid_T[wld] == 0 || (inc && d.inc_state[wld] != 0)) return;
+  if (d.grid_T[wld] == 0) return;
+  if (threadIdx.x == 0 && k == d.ext_chunk_off[wld]) {
+    d.large_cnt[wld] = 0;
+    if (inc) d.inc_moved[wld] = 0;
+    if (d.world_sap && d.world_sap[wld]) { /* the small bodies' range of lower x, gathered by k_grid_bin */
+      d.sap_range[2 * wld] = ~0ull;
+      d.sap_range[2 * wld + 1] = 0ull;
+    }
+  }
+  if (inc && d.inc_state[wld] != 0) return;
   double sum = 0.0;
   int cnt = 0;
   for (int g = b0 + threadIdx.x; g < b1; g += blockDim.x) {
@@ -680,43 +744,25 @@ __global__ void k_extent_parts(Dev d, int inc) {
     s_cnt[threadIdx.x >> 5] = cnt;
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = 0.0;
-    int c = 0;
-    for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
-      t += s_sum[q];
-      c += s_cnt[q];
-    }
-    d.ext_part_sum[k] = t;
-    d.ext_part_cnt[k] = c;
-  }
-}
-
-/* Twice the mean extent over a world's chunks, added in chunk order. */
-__device__ __forceinline__ double world_cell_size(const Dev& d, int wld) {
+  if (threadIdx.x != 0) return;
   double t = 0.0;
   int c = 0;
-  for (int k = d.ext_chunk_off[wld]; k < d.ext_chunk_off[wld + 1]; ++k) {
-    t += d.ext_part_sum[k];
-    c += d.ext_part_cnt[k];
+  for (int q = 0; q < (int)(blockDim.x >> 5); ++q) {
+    t += s_sum[q];
+    c += s_cnt[q];
   }
-  return c > 0 ? 2.0 * t / c : 0.0;
-}
-
-/* One thread per world: cell size, its reciprocal and the size limit of a
- * grid body. */
-__global__ void k_grid_stats(Dev d) {
-  const int wld = blockIdx.x * blockDim.x + threadIdx.x;
-  if (wld >= d.n_worlds || d.grid_T[wld] == 0) return;
-  const double s = world_cell_size(d, wld);
-  const double inv = (s > 0.0 && small_mag(s) && small_mag(1.0 / s)) ? 1.0 / s : 0.0;
+  __stcg(d.ext_part_sum + k, t);
+  __stcg(d.ext_part_cnt + k, c);
+  __threadfence();
+  const int chunks = d.ext_chunk_off[wld + 1] - d.ext_chunk_off[wld];
+  if (atomicAdd(d.ext_done + wld, 1) + 1 < chunks) return;
+  d.ext_done[wld] = 0; /* for the next step */
+  __threadfence();
+  const double sz = world_cell_size(d, wld);
+  const double inv = (sz > 0.0 && small_mag(sz) && small_mag(1.0 / sz)) ? 1.0 / sz : 0.0;
   d.grid_inv_s[wld] = inv;
   d.grid_lim[wld] = inv > 0.0 ? (1.0 - 0x1p-20) / inv : 0.0;
-  d.large_cnt[wld] = 0;
-  if (d.world_sap && d.world_sap[wld]) { /* the small bodies' range of lower x, gathered by k_grid_bin */
-    d.sap_range[2 * wld] = ~0ull;
-    d.sap_range[2 * wld + 1] = 0ull;
-  }
+  if (inc) d.inc_margin[wld] = inv > 0.0 ? 0.03125 / inv : 0.0;
 }
 
 /* One thread per body: grid bodies get a cell and a bucket count, the rest go
@@ -771,65 +817,6 @@ __global__ void k_grid_scatter(Dev d) {
     const int b = d.grid_base[wld] + cell_bucket(d.cell_x[g], d.cell_y[g], d.grid_T[wld]);
     const int pos = atomicAdd(&d.bucket_off[b], 1);
     d.grid_ids[pos] = g;
-  }
-}
-
-/* One thread per grid row i: pairs (i, j), j < i, with the 3x3 cells' bodies
- * and with the world's large bodies.  COUNT writes the row count; otherwise
- * the row is written unordered at its offset.  Buckets are read between the
- * starts (the ends of the previous bucket) and the ends left by the scatter. */
-template <bool COUNT>
-__global__ void k_grid_rows(Dev d) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
-    if (!d.row_mode[g]) continue;
-    const int wld = d.body_world[g];
-    const int off = d.world_body_off[wld];
-    const int n = d.world_body_off[wld + 1] - off;
-    const int q = off + (n - 1 - (g - off));
-    const int T = d.grid_T[wld], base = d.grid_base[wld];
-    const int cx = d.cell_x[g], cy = d.cell_y[g];
-    const uint8_t fi = d.flags[g];
-    uint64_t ki[4];
-    ki[0] = d.boxk[4 * g + 0];
-    ki[1] = d.boxk[4 * g + 1];
-    ki[2] = d.boxk[4 * g + 2];
-    ki[3] = d.boxk[4 * g + 3];
-    int count = 0;
-    const int out = COUNT ? 0 : d.row_off[q];
-    const bool sap = d.world_sap && d.world_sap[wld]; /* the sweep adds the small-body pairs */
-    for (int dy = sap ? 2 : -1; dy <= 1; ++dy) {
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int ncx = cx + dx, ncy = cy + dy;
-        const int b = base + cell_bucket(ncx, ncy, T);
-        const int k0 = b > 0 ? d.bucket_off[b - 1] : 0, k1 = d.bucket_off[b];
-        for (int k = k0; k < k1; ++k) {
-          const int j = d.grid_ids[k];
-          if (j >= g || d.cell_x[j] != ncx || d.cell_y[j] != ncy) continue;
-          if (pair_overlaps(d, g, j, fi, ki)) {
-            if (!COUNT && out + count < d.pair_cap) {
-              d.pair_a[out + count] = g;
-              d.pair_b[out + count] = j;
-            }
-            ++count;
-          }
-        }
-      }
-    }
-    const int nl = d.large_cnt[wld];
-    for (int k = 0; k < nl; ++k) {
-      const int j = d.large_ids[off + k];
-      if (j < g && pair_overlaps(d, g, j, fi, ki)) {
-        if (!COUNT && out + count < d.pair_cap) {
-          d.pair_a[out + count] = g;
-          d.pair_b[out + count] = j;
-        }
-        ++count;
-      }
-    }
-    if (COUNT) {
-      d.row_cnt[q] = count;
-      if (sap) d.sap_cursor[q] = count; /* the sweep's pairs follow the large ones */
-    }
   }
 }
 
@@ -930,11 +917,13 @@ __global__ void k_sap_rows(Dev d) {
   }
 }
 
-/* Sorts each grid row's j descending (rows hold a handful of pairs). */
-__global__ void k_grid_sort_rows(Dev d) {
+/* Sorts each grid row's j descending once the sweep has added its pairs (a
+ * handful per row). */
+__global__ void k_sap_sort_rows(Dev d) {
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
     if (!d.row_mode[g]) continue;
     const int wld = d.body_world[g];
+    if (!d.world_sap[wld]) continue;
     const int off = d.world_body_off[wld];
     const int n = d.world_body_off[wld + 1] - off;
     const int q = off + (n - 1 - (g - off));
@@ -1004,26 +993,6 @@ __device__ __forceinline__ bool fat_box(const Dev& d, int g, int wld, double fb[
   return true;
 }
 
-/* One CTA per grid world: in a world that rebuilds, the cell size from the
- * mean extent (as k_grid_stats) and the margin s/32; every world clears its
- * large list and moved count. */
-__global__ void k_inc_stats(Dev d) {
-  const int wld = blockIdx.x * blockDim.x + threadIdx.x;
-  if (wld >= d.n_worlds || d.grid_T[wld] == 0) return;
-  if (d.inc_state[wld] != 0) {
-    d.large_cnt[wld] = 0;
-    d.inc_moved[wld] = 0;
-    return;
-  }
-  const double sz = world_cell_size(d, wld);
-  const double inv = (sz > 0.0 && small_mag(sz) && small_mag(1.0 / sz)) ? 1.0 / sz : 0.0;
-  d.grid_inv_s[wld] = inv;
-  d.grid_lim[wld] = inv > 0.0 ? (1.0 - 0x1p-20) / inv : 0.0;
-  d.inc_margin[wld] = inv > 0.0 ? 0.03125 / inv : 0.0;
-  d.large_cnt[wld] = 0;
-  d.inc_moved[wld] = 0;
-}
-
 /* One thread per body of a grid world: moved or not, and the large list. */
 __global__ void k_inc_mark(Dev d) {
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
@@ -1060,64 +1029,46 @@ __global__ void k_inc_mark(Dev d) {
   }
 }
 
-/* One thread per world: this frame's mode (inc_rebuild) and the next
- * frame's state (inc_state). */
-__global__ void k_inc_decide(Dev d) {
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w < d.n_worlds; w += gridDim.x * blockDim.x) {
-    if (d.grid_T[w] == 0) continue;
-    const int n = d.world_body_off[w + 1] - d.world_body_off[w];
-    const int st = d.inc_state[w], moved = d.inc_moved[w];
-    int mode;
-    if (st == kIncStateNew) {
-      mode = kIncBuild;
-    } else if (st == kIncStateList) {
-      mode = 4 * moved > n ? kIncFull : kIncList;
-    } else { /* FULL: back through BUILD after 4 quiet-enough frames */
-      const int quiet = 8 * moved < n ? d.inc_frames[w] + 1 : 0;
-      d.inc_frames[w] = quiet;
-      mode = quiet >= 4 ? kIncBuild : kIncFull;
-    }
-    if (mode == kIncFull && st != kIncStateFull) d.inc_frames[w] = 0;
-    d.inc_rebuild[w] = mode;
-    d.inc_state[w] = mode == kIncFull ? kIncStateFull : kIncStateList;
-  }
+/* A world's mode this frame, from what its state was before the frame and how
+ * many of its bodies moved (k_inc_mark): read by k_inc_update, which writes it
+ * to inc_rebuild; the state follows in k_inc_scatter. */
+__device__ __forceinline__ int inc_mode(const Dev& d, int w) {
+  const int n = d.world_body_off[w + 1] - d.world_body_off[w];
+  const int st = d.inc_state[w], moved = d.inc_moved[w];
+  if (st == kIncStateNew) return kIncBuild;
+  if (st == kIncStateList) return 4 * moved > n ? kIncFull : kIncList;
+  /* FULL: back through BUILD after 4 quiet-enough frames */
+  return 8 * moved < n && d.inc_frames[w] + 1 >= 4 ? kIncBuild : kIncFull;
 }
 
-/* One thread per moved body that was in the adjacency: its entry in each
- * unmoved neighbour's list becomes -1 (every entry is removed by the thread
- * of the body it names, so the stores never collide). */
-__global__ void k_inc_remove(Dev d) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
-    const int wld = d.body_world[g];
-    if (d.grid_T[wld] == 0 || d.inc_rebuild[wld] != kIncList) continue;
-    const uint8_t mg = d.moved[g];
-    if (!(mg & kMovedBit) || !(mg & kMovedWasGrid)) continue;
-    const int32_t* lst = d.nbr + (size_t)g * d.nbr_cap;
-    const int n = min(d.nbr_cnt[g], d.nbr_cap);
-    for (int k = 0; k < n; ++k) {
-      const int j = lst[k];
-      if (j < 0 || (d.moved[j] & kMovedBit)) continue;
-      int32_t* lj = d.nbr + (size_t)j * d.nbr_cap;
-      const int nj = min(d.nbr_cnt[j], d.nbr_cap);
-      for (int t = 0; t < nj; ++t)
-        if (lj[t] == g) {
-          lj[t] = -1;
-          break;
-        }
-    }
-  }
-}
-
-/* One thread per body: a moved body's grid membership (its fat box and cell
- * were written by k_inc_mark; a staying body keeps the ones it has, which
- * still contain its box); counts grid bodies into the buckets of worlds that
- * search this frame. */
-__global__ void k_inc_refat(Dev d) {
+/* One thread per body.  A moved body that was in the adjacency of a LIST world:
+ * its entry in each unmoved neighbour's list becomes -1 (every entry is removed
+ * by the thread of the body it names, so the stores never collide).  Then a
+ * moved body's grid membership (its fat box and cell were written by k_inc_mark;
+ * a staying body keeps the ones it has, which still contain its box), and the
+ * grid bodies of worlds that search this frame are counted into the buckets. */
+__global__ void k_inc_update(Dev d) {
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
     const int wld = d.body_world[g];
     if (d.grid_T[wld] == 0) continue;
-    const int mode = d.inc_rebuild[wld];
+    const int mode = inc_mode(d, wld);
+    if (g == d.world_body_off[wld]) d.inc_rebuild[wld] = mode;
     const uint8_t mg = d.moved[g];
+    if (mode == kIncList && (mg & kMovedBit) && (mg & kMovedWasGrid)) {
+      const int32_t* lst = d.nbr + (size_t)g * d.nbr_cap;
+      const int n = min(d.nbr_cnt[g], d.nbr_cap);
+      for (int k = 0; k < n; ++k) {
+        const int j = lst[k];
+        if (j < 0 || (d.moved[j] & kMovedBit)) continue;
+        int32_t* lj = d.nbr + (size_t)j * d.nbr_cap;
+        const int nj = min(d.nbr_cnt[j], d.nbr_cap);
+        for (int t = 0; t < nj; ++t)
+          if (lj[t] == g) {
+            lj[t] = -1;
+            break;
+          }
+      }
+    }
     const bool now = (mg & kMovedNowGrid) != 0;
     if (mg & kMovedBit) d.row_mode[g] = now ? 1 : 0;
     if (mode == kIncBuild) d.nbr_cnt[g] = 0;
@@ -1126,10 +1077,22 @@ __global__ void k_inc_refat(Dev d) {
   }
 }
 
+/* Places the grid bodies of worlds that search; and each world's state for the
+ * next frame. */
 __global__ void k_inc_scatter(Dev d) {
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
     const int wld = d.body_world[g];
-    if (d.grid_T[wld] == 0 || !d.row_mode[g] || !(d.inc_rebuild[wld] != kIncList || d.inc_moved[wld] > 0)) continue;
+    if (d.grid_T[wld] == 0) continue;
+    const int mode = d.inc_rebuild[wld];
+    if (g == d.world_body_off[wld]) {
+      const int n = d.world_body_off[wld + 1] - g;
+      if (d.inc_state[wld] == kIncStateFull)
+        d.inc_frames[wld] = 8 * d.inc_moved[wld] < n ? d.inc_frames[wld] + 1 : 0;
+      else if (mode == kIncFull)
+        d.inc_frames[wld] = 0;
+      d.inc_state[wld] = mode == kIncFull ? kIncStateFull : kIncStateList;
+    }
+    if (!d.row_mode[g] || !(mode != kIncList || d.inc_moved[wld] > 0)) continue;
     const int b = d.grid_base[wld] + cell_bucket(d.cell_x[g], d.cell_y[g], d.grid_T[wld]);
     const int pos = atomicAdd(&d.bucket_off[b], 1);
     d.grid_ids[pos] = g;
@@ -1140,11 +1103,24 @@ __device__ __forceinline__ bool fat_overlap(const uint64_t* a, const uint64_t* b
   return !(b[0] > a[1] || b[1] < a[0]) && !(b[2] > a[3] || b[3] < a[2]);
 }
 
-/* One thread per re-inserted grid body: its new list from the 3x3 cells of
- * the fat-box grid; in an incremental frame it is also appended to each
- * unmoved neighbour's list. */
-__global__ void k_inc_query(Dev d) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
+/* The lanes of this thread's team of TEAM neighbours in a warp. */
+template <int TEAM>
+__device__ __forceinline__ unsigned team_mask() {
+  return TEAM == 32 ? 0xffffffffu : ((1u << (TEAM & 31)) - 1u) << (threadIdx.x & 31 & ~(TEAM - 1));
+}
+
+/* TEAM lanes per re-inserted grid body: its new list from the 3x3 cells of
+ * the fat-box grid, a cell per lane; in an incremental frame it is also appended
+ * to each unmoved neighbour's list.  (The order within a list is arbitrary: the
+ * rows are sorted.)  A thread walking all nine cells took 40 us on 75 worlds of
+ * 121 bodies; the chain of its loads, not their number, is what takes the time. */
+template <int TEAM>
+__global__ void __launch_bounds__(kRowThreads) k_inc_query(Dev d) {
+  __shared__ int s_cnt[kRowThreads / TEAM];
+  const int lane = threadIdx.x % TEAM, team = threadIdx.x / TEAM;
+  const unsigned mates = team_mask<TEAM>();
+  for (int g = blockIdx.x * (kRowThreads / TEAM) + team; g < d.n_bodies;
+       g += gridDim.x * (kRowThreads / TEAM)) {
     const int wld = d.body_world[g];
     if (d.grid_T[wld] == 0 || !d.row_mode[g]) continue;
     const int mode = d.inc_rebuild[wld];
@@ -1155,119 +1131,198 @@ __global__ void k_inc_query(Dev d) {
     uint64_t fg[4];
     for (int k = 0; k < 4; ++k) fg[k] = d.fatk[4 * g + k];
     int32_t* lst = d.nbr + (size_t)g * d.nbr_cap;
-    int cnt = 0;
+    if (lane == 0) s_cnt[team] = 0;
+    __syncwarp(mates);
     bool over = false;
-    for (int dy = -1; dy <= 1; ++dy) {
-      for (int dx = -1; dx <= 1; ++dx) {
-        const int ncx = cx + dx, ncy = cy + dy;
-        const int b = base + cell_bucket(ncx, ncy, T);
-        const int k0 = b > 0 ? d.bucket_off[b - 1] : 0, k1 = d.bucket_off[b];
-        for (int k = k0; k < k1; ++k) {
-          const int j = d.grid_ids[k];
-          if (j == g || d.cell_x[j] != ncx || d.cell_y[j] != ncy) continue;
-          if (!fat_overlap(fg, d.fatk + 4 * j)) continue;
-          if (cnt < d.nbr_cap) lst[cnt] = j; else over = true;
-          ++cnt;
-          if (!rebuild && !(d.moved[j] & kMovedBit)) {
-            const int pos = atomicAdd(&d.nbr_cnt[j], 1);
-            if (pos < d.nbr_cap) d.nbr[(size_t)j * d.nbr_cap + pos] = g; else over = true;
-          }
+    for (int c = lane; c < 9; c += TEAM) {
+      const int ncx = cx + c % 3 - 1, ncy = cy + c / 3 - 1;
+      const int b = base + cell_bucket(ncx, ncy, T);
+      const int k0 = b > 0 ? d.bucket_off[b - 1] : 0, k1 = d.bucket_off[b];
+      for (int k = k0; k < k1; ++k) {
+        const int j = d.grid_ids[k];
+        if (j == g || d.cell_x[j] != ncx || d.cell_y[j] != ncy) continue;
+        if (!fat_overlap(fg, d.fatk + 4 * j)) continue;
+        const int cnt = atomicAdd(&s_cnt[team], 1);
+        if (cnt < d.nbr_cap) lst[cnt] = j; else over = true;
+        if (!rebuild && !(d.moved[j] & kMovedBit)) {
+          const int pos = atomicAdd(&d.nbr_cnt[j], 1);
+          if (pos < d.nbr_cap) d.nbr[(size_t)j * d.nbr_cap + pos] = g; else over = true;
         }
       }
     }
-    d.nbr_cnt[g] = cnt;
+    __syncwarp(mates);
+    if (lane == 0) d.nbr_cnt[g] = s_cnt[team];
     if (over) atomicOr(&d.counters[kCntOverflow], 4ull);
   }
 }
 
-/* One thread per grid row i: the entries j < i of its list whose current
- * boxes overlap, then the world's large bodies j < i.  COUNT also compacts
- * the list (drops removed entries). */
-template <bool COUNT>
-__global__ void k_inc_rows(Dev d) {
-  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
-    const int wld = d.body_world[g];
-    if (d.grid_T[wld] == 0 || !d.row_mode[g]) continue;
-    const int off = d.world_body_off[wld];
-    const int n = d.world_body_off[wld + 1] - off;
-    const int q = off + (n - 1 - (g - off));
-    const uint8_t fi = d.flags[g];
-    uint64_t ki[4];
-    ki[0] = d.boxk[4 * g + 0];
-    ki[1] = d.boxk[4 * g + 1];
-    ki[2] = d.boxk[4 * g + 2];
-    ki[3] = d.boxk[4 * g + 3];
-    int count = 0;
-    const int out = COUNT ? 0 : d.row_off[q];
-    if (d.inc_rebuild[wld] == kIncFull) { /* no lists: the 3x3 cells of the fat-box grid */
-      const int T = d.grid_T[wld], base = d.grid_base[wld];
-      const int cx = d.cell_x[g], cy = d.cell_y[g];
-      for (int dy = -1; dy <= 1; ++dy) {
-        for (int dx = -1; dx <= 1; ++dx) {
-          const int ncx = cx + dx, ncy = cy + dy;
-          const int b = base + cell_bucket(ncx, ncy, T);
-          const int k0 = b > 0 ? d.bucket_off[b - 1] : 0, k1 = d.bucket_off[b];
-          for (int k = k0; k < k1; ++k) {
-            const int j = d.grid_ids[k];
-            if (j >= g || d.cell_x[j] != ncx || d.cell_y[j] != ncy) continue;
-            if (pair_overlaps(d, g, j, fi, ki)) {
-              if (!COUNT && out + count < d.pair_cap) {
-                d.pair_a[out + count] = g;
-                d.pair_b[out + count] = j;
-              }
-              ++count;
-            }
-          }
-        }
+/* Calls hit(j) for the partners j < g of grid row g, its candidates dealt over
+ * LANES lanes: with adjacency lists the entries of its list (COMPACT: removed
+ * entries are dropped from it on the way), else the bodies of the 3x3 cells
+ * around it; then the world's large bodies.  A world that is swept finds the
+ * partners among its small bodies elsewhere. */
+template <int LANES, bool INC, bool COMPACT, class Hit>
+__device__ __forceinline__ void grid_partners(const Dev& d, int g, Hit&& hit) {
+  const int lane = threadIdx.x % LANES;
+  const unsigned mates = team_mask<LANES>();
+  const int wld = d.body_world[g];
+  const uint8_t fi = d.flags[g];
+  uint64_t ki[4];
+  ki[0] = d.boxk[4 * g + 0];
+  ki[1] = d.boxk[4 * g + 1];
+  ki[2] = d.boxk[4 * g + 2];
+  ki[3] = d.boxk[4 * g + 3];
+  if (INC && d.inc_rebuild[wld] != kIncFull) {
+    int32_t* lst = d.nbr + (size_t)g * d.nbr_cap;
+    const int listed = d.nbr_cnt[g], nl = min(listed, d.nbr_cap);
+    int kept = 0;
+    for (int k0 = 0; k0 < nl; k0 += LANES) {
+      const int j = k0 + lane < nl ? lst[k0 + lane] : -1;
+      if (COMPACT) {
+        const unsigned m = LANES == 1 ? (j >= 0 ? mates : 0u) : __ballot_sync(mates, j >= 0);
+        const int at = kept + __popc(m & ((1u << (threadIdx.x & 31)) - 1u));
+        if (j >= 0 && at != k0 + lane) lst[at] = j;
+        kept += __popc(m);
       }
-    } else {
-      int32_t* lst = d.nbr + (size_t)g * d.nbr_cap;
-      int nl = min(d.nbr_cnt[g], d.nbr_cap);
-      if (COUNT) {
-        int w = 0;
-        for (int k = 0; k < nl; ++k) {
-          const int j = lst[k];
-          if (j >= 0) lst[w++] = j;
-        }
-        if (d.nbr_cnt[g] <= d.nbr_cap) d.nbr_cnt[g] = w;
-        nl = w;
-      }
-      for (int k = 0; k < nl; ++k) {
-        const int j = lst[k];
-        if (j >= 0 && j < g && pair_overlaps(d, g, j, fi, ki)) {
-          if (!COUNT && out + count < d.pair_cap) {
-            d.pair_a[out + count] = g;
-            d.pair_b[out + count] = j;
-          }
-          ++count;
-        }
+      if (j >= 0 && j < g && pair_overlaps(d, g, j, fi, ki)) hit(j);
+    }
+    if (COMPACT && lane == 0 && listed <= d.nbr_cap) d.nbr_cnt[g] = kept;
+  } else if (INC || !(d.world_sap && d.world_sap[wld])) {
+    const int T = d.grid_T[wld], base = d.grid_base[wld];
+    const int cx = d.cell_x[g], cy = d.cell_y[g];
+    for (int c = lane; c < 9; c += LANES) {
+      const int ncx = cx + c % 3 - 1, ncy = cy + c / 3 - 1;
+      const int b = base + cell_bucket(ncx, ncy, T);
+      const int k0 = b > 0 ? d.bucket_off[b - 1] : 0, k1 = d.bucket_off[b];
+      for (int k = k0; k < k1; ++k) {
+        const int j = d.grid_ids[k];
+        if (j >= g || d.cell_x[j] != ncx || d.cell_y[j] != ncy) continue;
+        if (pair_overlaps(d, g, j, fi, ki)) hit(j);
       }
     }
-    const int nlarge = d.large_cnt[wld];
-    for (int k = 0; k < nlarge; ++k) {
-      const int j = d.large_ids[off + k];
-      if (j < g && pair_overlaps(d, g, j, fi, ki)) {
-        if (!COUNT && out + count < d.pair_cap) {
-          d.pair_a[out + count] = g;
-          d.pair_b[out + count] = j;
-        }
-        ++count;
-      }
-    }
-    if (COUNT) d.row_cnt[q] = count;
+  }
+  const int nlarge = d.large_cnt[wld];
+  const int32_t* large = d.large_ids + d.world_body_off[wld];
+  for (int k = lane; k < nlarge; k += LANES) {
+    const int j = large[k];
+    if (j < g && pair_overlaps(d, g, j, fi, ki)) hit(j);
   }
 }
 
-/* world_pair_off[w] = row_off[world_body_off[w]] (first row of the world in
- * mirrored order); also records the pair total and overflow. */
-__global__ void k_world_pair_offsets(Dev d) {
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w <= d.n_worlds; w += gridDim.x * blockDim.x) {
-    const int p = d.row_off[d.world_body_off[w]];
-    d.world_pair_off[w] = p;
-    if (w == d.n_worlds) {
-      d.counters[kCntPairs] = (unsigned long long)p;
-      if (p > d.pair_cap) d.counters[kCntOverflow] |= 1ull;
+/* Counts the rows of a batch with grid worlds and keeps each row's pairs, in
+ * descending j, where it has at most kRowHits: TEAM lanes per grid row; the
+ * rows of bodies outside the grid (large ones, small worlds) a warp each, dealt
+ * over the block.  A row is a chain of dependent loads, so the latency of one
+ * lane's share counts.  A thread per row, which tested everything once to count
+ * and once more to write, took 53 us for one world of 401 bodies and 135 us for
+ * 4096 worlds of 505,800; counting and writing now take 13 and 100. */
+template <bool INC, int TEAM>
+__global__ void __launch_bounds__(kRowThreads, 5) k_count_rows(Dev d) {
+  constexpr int kTeams = kRowThreads / TEAM;
+  __shared__ int s_cnt[kTeams], s_hits[kTeams][kRowHits + 1], s_brute[kTeams], s_nbrute;
+  const int lane = threadIdx.x % TEAM, team = threadIdx.x / TEAM;
+  const unsigned mates = team_mask<TEAM>();
+  for (int base = blockIdx.x * kTeams; base < d.n_bodies; base += gridDim.x * kTeams) {
+    if (threadIdx.x == 0) s_nbrute = 0;
+    if (lane == 0) s_cnt[team] = 0;
+    __syncthreads();
+    const int g = base + team;
+    if (g < d.n_bodies) {
+      if (d.row_mode[g]) {
+        grid_partners<TEAM, INC, true>(d, g, [&](int j) {
+          const int k = atomicAdd(&s_cnt[team], 1);
+          if (k < kRowHits) s_hits[team][k] = j;
+        });
+        __syncwarp(mates);
+        const int count = s_cnt[team];
+        for (int e = lane; e < count && count <= kRowHits; e += TEAM) {
+          const int j = s_hits[team][e];
+          int rank = 0;
+          for (int k = 0; k < count; ++k) rank += s_hits[team][k] > j;
+          d.row_hits[kRowHits * (size_t)g + rank] = j;
+        }
+        if (lane == 0) {
+          const int wld = d.body_world[g];
+          const int off = d.world_body_off[wld];
+          const int q = off + (d.world_body_off[wld + 1] - 1 - g);
+          d.row_cnt[q] = count;
+          if (!INC && d.world_sap && d.world_sap[wld]) d.sap_cursor[q] = count; /* the sweep's pairs follow */
+        }
+      } else if (lane == 0) {
+        s_brute[atomicAdd(&s_nbrute, 1)] = g;
+      }
     }
+    __syncthreads();
+    for (int k = threadIdx.x >> 5; k < s_nbrute; k += kRowThreads / 32) brute_row<true>(d, s_brute[k]);
+    __syncthreads();
+  }
+}
+
+/* Writes the pairs: a thread per row that kept its pairs; the others a warp
+ * each, tested again (in a grid row sorted in shared memory, or by brute force,
+ * which finds them in order, where there are more than that holds).  In a swept
+ * world a thread writes its row's pairs with large bodies. */
+template <bool GRID, bool INC>
+__global__ void __launch_bounds__(kRowThreads) k_write_rows(Dev d) {
+  constexpr int kWarps = kRowThreads / 32;
+  __shared__ int s_heavy[kRowThreads], s_nheavy, s_cnt[kWarps], s_hits[GRID ? kWarps : 1][kRowSorted];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int base = blockIdx.x * kRowThreads; base < d.n_bodies; base += gridDim.x * kRowThreads) {
+    if (threadIdx.x == 0) s_nheavy = 0;
+    __syncthreads();
+    const int g = base + threadIdx.x;
+    if (g < d.n_bodies) {
+      const int wld = d.body_world[g];
+      const int off = d.world_body_off[wld];
+      const int q = off + (d.world_body_off[wld + 1] - 1 - g);
+      const int out = d.row_off[q], count = d.row_off[q + 1] - out;
+      auto put = [&](int k, int j) {
+        if (out + k < d.pair_cap) {
+          d.pair_a[out + k] = g;
+          d.pair_b[out + k] = j;
+        }
+      };
+      if (GRID && !INC && d.world_sap && d.world_sap[wld] && d.row_mode[g]) {
+        int k = 0;
+        grid_partners<1, false, false>(d, g, [&](int j) { put(k++, j); });
+      } else if (count <= kRowHits) {
+        const int32_t* hits = d.row_hits + kRowHits * (size_t)g;
+        for (int k = 0; k < count; ++k) put(k, hits[k]);
+      } else {
+        s_heavy[atomicAdd(&s_nheavy, 1)] = g;
+      }
+    }
+    __syncthreads();
+    for (int h = warp; h < s_nheavy; h += kWarps) {
+      const int gh = s_heavy[h];
+      const int wld = d.body_world[gh];
+      const int off = d.world_body_off[wld];
+      const int q = off + (d.world_body_off[wld + 1] - 1 - gh);
+      const int out = d.row_off[q], count = d.row_off[q + 1] - out;
+      if (!GRID || !d.row_mode[gh] || count > kRowSorted) {
+        brute_row<false>(d, gh);
+        continue;
+      }
+      if (lane == 0) s_cnt[warp] = 0;
+      __syncwarp();
+      grid_partners<32, INC, false>(d, gh, [&](int j) {
+        const int k = atomicAdd(&s_cnt[warp], 1);
+        if (k < kRowSorted) s_hits[GRID ? warp : 0][k] = j;
+      });
+      __syncwarp();
+      const int found = min(s_cnt[warp], kRowSorted);
+      for (int e = lane; e < found; e += 32) {
+        const int j = s_hits[GRID ? warp : 0][e];
+        int rank = 0;
+        for (int k = 0; k < found; ++k) rank += s_hits[GRID ? warp : 0][k] > j;
+        if (out + rank < d.pair_cap) {
+          d.pair_a[out + rank] = gh;
+          d.pair_b[out + rank] = j;
+        }
+      }
+      __syncwarp();
+    }
+    __syncthreads();
   }
 }
 
@@ -2037,19 +2092,6 @@ __global__ void k_narrowphase_lanes(Dev d) {
 /* A8-A9 constraint build + warm-start lookup                                 */
 /* ------------------------------------------------------------------------ */
 
-/* world_contact_off[w] = slot_off[world_pair_off[w]]; totals + overflow. */
-__global__ void k_world_contact_offsets(Dev d) {
-  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w <= d.n_worlds; w += gridDim.x * blockDim.x) {
-    const int p = min(d.world_pair_off[w], d.pair_cap);
-    const int c = d.slot_off[p];
-    d.world_contact_off[w] = c;
-    if (w == d.n_worlds) {
-      d.counters[kCntContacts] = (unsigned long long)c;
-      if (c > d.contact_cap) d.counters[kCntOverflow] |= 2ull;
-    }
-  }
-}
-
 /* One thread per contact slot.  Compacts the contact, builds its
  * ContactConstraint (NonPenetration.hs:16-56, Friction.hs:18-44,
  * Restitution.hs:21-31, flip handling Utils.hs:175-215 / Constraint.hs:96-98),
@@ -2061,10 +2103,16 @@ __global__ void k_world_contact_offsets(Dev d) {
 /* The slot of every contact, so that k_build's threads take contacts rather
  * than slots: about half the slots of a settled pile are empty (separated
  * pairs, pairs with one contact), and an idle lane still costs its warp's FP64
- * instructions. */
+ * instructions; and the worlds' first pairs (row_off at their first row in
+ * mirrored order) and first contacts. */
 __global__ void k_contact_slots(Dev d) {
   const int P = min((int)d.counters[kCntPairs], d.pair_cap);
   const int C = (int)d.counters[kCntContacts];
+  for (int w = blockIdx.x * blockDim.x + threadIdx.x; w <= d.n_worlds; w += gridDim.x * blockDim.x) {
+    const int p = d.row_off[d.world_body_off[w]];
+    d.world_pair_off[w] = p;
+    d.world_contact_off[w] = d.slot_off[min(p, d.pair_cap)];
+  }
   if (C > d.contact_cap) return;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * P; t += gridDim.x * blockDim.x) {
     const int p = t >> 1, s = t & 1;
@@ -2182,39 +2230,6 @@ __global__ void k_build(Dev d, double beta_dt, double slop, int warm_start, int 
 /* ------------------------------------------------------------------------ */
 /* A9-A10 one update                                                          */
 /* ------------------------------------------------------------------------ */
-
-/* Block-wide exclusive scan of in-place int array a[0..n), returns total. */
-__device__ int block_exclusive_scan(int32_t* a, int n, int32_t* smem /* >= 32 */) {
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int lane = tid & 31, wid = tid >> 5, nwarp = (nt + 31) >> 5;
-  int carry = 0;
-  for (int base = 0; base < n; base += nt) {
-    const int idx = base + tid;
-    const int x = idx < n ? a[idx] : 0;
-    int incl = x;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
-    }
-    if (lane == 31) smem[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-      int ws = lane < nwarp ? smem[lane] : 0;
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, ws, o);
-        if (lane >= o) ws += y;
-      }
-      if (lane < nwarp) smem[lane] = ws; /* inclusive warp sums */
-    }
-    __syncthreads();
-    const int wprefix = wid > 0 ? smem[wid - 1] : 0;
-    const int chunk_total = smem[nwarp - 1];
-    if (idx < n) a[idx] = carry + wprefix + incl - x;
-    carry += chunk_total;
-    __syncthreads();
-  }
-  return carry;
-}
 
 /* J . v as a left fold (Shapes/Linear/Template.hs:108-110) of a stored row. */
 __device__ __forceinline__ double row_dot(const double r[4], const double v[6]) {
@@ -2356,75 +2371,154 @@ __global__ void k_metric_final(Dev d, int wld, const double* part) {
 /* scans                                                                      */
 /* ------------------------------------------------------------------------ */
 
-constexpr int kScanThreads = 256;
+constexpr int kScanThreads = 1024;
 constexpr int kScanPerThread = 8;
 constexpr int kScanTile = kScanThreads * kScanPerThread;
 
-/* Tile sums of in[0..n) (n read from *n_dev when non-null, capped at n_cap). */
-__global__ void k_scan_tiles(const int32_t* in, int n_cap, const unsigned long long* n_dev,
-                             int32_t* tile_sums) {
-  __shared__ int32_t s[32];
-  const int n = n_dev ? (int)min((unsigned long long)n_cap, *n_dev) : n_cap;
-  const int base = blockIdx.x * kScanTile;
-  int sum = 0;
-  for (int k = 0; k < kScanPerThread; ++k) {
-    const int idx = base + k * kScanThreads + threadIdx.x;
-    if (idx < n) sum += in[idx];
-  }
-  for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = sum;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int k = 0; k < kScanThreads / 32; ++k) t += s[k];
-    tile_sums[blockIdx.x] = t;
-  }
-}
+/* What a scan keeps between launches: a word per tile, {value, epoch << 2 |
+ * kind}, and {epoch, tiles taken, tiles done}.  The epoch tells this launch's
+ * words from older ones; the last block to finish raises it and clears the
+ * counts, so that nothing has to be reset before the next scan (the launches
+ * that share a state follow one another on a stream). */
+struct ScanState {
+  unsigned long long* tile; /* zero (kind 0: no word) to begin with */
+  uint32_t* ctl;            /* [3] */
+  int tiles;
+};
+constexpr uint32_t kTileSum = 1, kTilePrefix = 2;
+constexpr long long kScanPollLimit = 1ll << 24;
 
-/* Exclusive scan of the tile sums (one block). */
-__global__ void k_scan_tile_sums(int32_t* tile_sums, int n_tiles) {
-  __shared__ int32_t s[32];
-  block_exclusive_scan(tile_sums, n_tiles, s);
-}
-
-/* out[k] = exclusive prefix of in; out[n] = total. */
-__global__ void k_scan_apply(const int32_t* in, int n_cap, const unsigned long long* n_dev,
-                             const int32_t* tile_sums, int32_t* out) {
-  __shared__ int32_t s_vals[kScanTile];
-  __shared__ int32_t s_scan[32];
+/* out[k] = exclusive prefix of in[0..n), out[n] = total, in one launch (n read
+ * from *n_dev when non-null, capped at n_cap): decoupled look-back (Merrill and
+ * Garland, "Single-pass Parallel Prefix Scan with Decoupled Look-back", 2016).
+ * Tiles are taken in order from a counter, so a block waits only for blocks
+ * that already run; the waits are bounded.  in and out start on 16 bytes.  Tiles
+ * of 8192, so that the chain of prefixes is short: a million elements took 37 us
+ * in tiles of 2048.  clear: in is left zeroed.  total:
+ * gets out[n], and where that exceeds total_cap the overflow counter gets
+ * overflow_bit.  As three launches (tile sums, their scan, the prefixes) a scan
+ * of 50 to 500 thousand elements took 11 to 13 us. */
+__global__ void __launch_bounds__(kScanThreads) k_scan(int32_t* in, int n_cap, const unsigned long long* n_dev,
+                                                       ScanState st, int32_t* out, int clear,
+                                                       unsigned long long* total, int total_cap,
+                                                       unsigned long long* overflow, unsigned overflow_bit,
+                                                       unsigned long long* err) {
+  __shared__ int32_t s_scan[kScanThreads / 32];
+  __shared__ int32_t s_prefix, s_tile;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int n = n_dev ? (int)min((unsigned long long)n_cap, *n_dev) : n_cap;
-  const int base = blockIdx.x * kScanTile;
-  for (int k = threadIdx.x; k < kScanTile; k += kScanThreads) {
-    const int idx = base + k;
-    s_vals[k] = idx < n ? in[idx] : 0;
-  }
-  __syncthreads();
-  /* per-thread serial over a contiguous run, then block scan of run totals */
-  const int r0 = threadIdx.x * kScanPerThread;
-  int run = 0;
-  for (int k = 0; k < kScanPerThread; ++k) run += s_vals[r0 + k];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  int incl = run;
-  for (int o = 1; o < 32; o <<= 1) {
-    const int y = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += y;
-  }
-  if (lane == 31) s_scan[wid] = incl;
-  __syncthreads();
-  if (wid == 0) {
-    int ws = lane < kScanThreads / 32 ? s_scan[lane] : 0;
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, ws, o);
-      if (lane >= o) ws += y;
+  const int tiles = n / kScanTile + 1; /* the last one also holds out[n] */
+  const uint32_t epoch = __ldcg(st.ctl);
+  for (;;) {
+    if (tid == 0) s_tile = (int)atomicAdd(st.ctl + 1, 1u);
+    __syncthreads();
+    const int tile = s_tile;
+    if (tile >= tiles) break;
+    /* per-thread serial over a contiguous run, then block scan of run totals */
+    const int r0 = tile * kScanTile + tid * kScanPerThread;
+    int32_t v[kScanPerThread] = {};
+    if (r0 + kScanPerThread <= n) {
+#pragma unroll
+      for (int k = 0; k < kScanPerThread; k += 4) {
+        const int4 x = *reinterpret_cast<const int4*>(in + r0 + k);
+        v[k] = x.x;
+        v[k + 1] = x.y;
+        v[k + 2] = x.z;
+        v[k + 3] = x.w;
+        if (clear) *reinterpret_cast<int4*>(in + r0 + k) = make_int4(0, 0, 0, 0);
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanPerThread; ++k)
+        if (r0 + k < n) {
+          v[k] = in[r0 + k];
+          if (clear) in[r0 + k] = 0;
+        }
     }
-    if (lane < kScanThreads / 32) s_scan[lane] = ws;
+    int run = 0;
+#pragma unroll
+    for (int k = 0; k < kScanPerThread; ++k) run += v[k];
+    int incl = run;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_scan[wid] = incl;
+    __syncthreads();
+    if (wid == 0) {
+      int ws = s_scan[lane]; /* as many warps as lanes */
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, ws, o);
+        if (lane >= o) ws += y;
+      }
+      const int sum = __shfl_sync(0xffffffffu, ws, 31);
+      s_scan[lane] = ws;
+      auto publish = [&](int value, uint32_t kind) {
+        asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(st.tile + tile),
+                     "l"((unsigned long long)(uint32_t)value | (unsigned long long)(epoch << 2 | kind) << 32)
+                     : "memory");
+      };
+      int prefix = 0;
+      if (tile > 0) {
+        if (lane == 0) publish(sum, kTileSum);
+        long long polls = 0;
+        for (int at = tile - 1;;) { /* 32 tiles before, nearest first */
+          const int q = at - lane;
+          unsigned long long word = (unsigned long long)(epoch << 2 | kTilePrefix) << 32; /* before the first: 0 */
+          if (q >= 0) asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(word) : "l"(st.tile + q) : "memory");
+          const uint32_t tag = (uint32_t)(word >> 32);
+          const bool here = tag >> 2 == epoch && (tag & 3u) != 0;
+          const unsigned known = __ballot_sync(0xffffffffu, here);
+          const unsigned full = __ballot_sync(0xffffffffu, here && (tag & 3u) == kTilePrefix);
+          /* the run of known tiles from the nearest on, up to the first with its whole prefix */
+          const int usable = known == 0xffffffffu ? 32 : __ffs(~known) - 1;
+          const int stop = full ? __ffs(full) - 1 : 32;
+          const bool end = stop < usable;
+          const int take = end ? stop + 1 : usable;
+          prefix += __reduce_add_sync(0xffffffffu, lane < take ? (int)(uint32_t)word : 0);
+          if (end) break;
+          at -= take;
+          if (take == 0 && ++polls > kScanPollLimit) {
+            if (lane == 0 && err) atomicOr(err, 1ull);
+            break;
+          }
+        }
+      }
+      if (lane == 0) {
+        publish(prefix + sum, kTilePrefix);
+        s_prefix = prefix;
+        if (tile == tiles - 1 && total) {
+          *total = (unsigned long long)(uint32_t)(prefix + sum);
+          if (prefix + sum > total_cap) atomicOr(overflow, (unsigned long long)overflow_bit);
+        }
+      }
+    }
+    __syncthreads();
+    int prefix = s_prefix + (wid > 0 ? s_scan[wid - 1] : 0) + incl - run;
+    int32_t o[kScanPerThread];
+#pragma unroll
+    for (int k = 0; k < kScanPerThread; ++k) {
+      o[k] = prefix;
+      prefix += v[k];
+    }
+    if (r0 + kScanPerThread <= n) {
+#pragma unroll
+      for (int k = 0; k < kScanPerThread; k += 4)
+        *reinterpret_cast<int4*>(out + r0 + k) = make_int4(o[k], o[k + 1], o[k + 2], o[k + 3]);
+    } else {
+#pragma unroll
+      for (int k = 0; k < kScanPerThread; ++k)
+        if (r0 + k <= n) out[r0 + k] = o[k];
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  int prefix = tile_sums[blockIdx.x] + (wid > 0 ? s_scan[wid - 1] : 0) + incl - run;
-  for (int k = 0; k < kScanPerThread; ++k) {
-    const int idx = base + r0 + k;
-    if (idx <= n) out[idx] = prefix;
-    prefix += s_vals[r0 + k];
+  if (tid == 0 && atomicAdd(st.ctl + 2, 1u) + 1 == gridDim.x) { /* every block is past its last tile */
+    st.ctl[1] = 0;
+    st.ctl[2] = 0;
+    const uint32_t next = (epoch + 1) & 0x3fffffffu;
+    if (next == 0) /* the words of 2^30 scans ago would be this round's */
+      for (int k = 0; k < st.tiles; ++k) st.tile[k] = 0;
+    st.ctl[0] = next;
   }
 }
 
