@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes
 import os
+import struct
 from pathlib import Path
 
 import numpy as np
@@ -218,7 +219,9 @@ def _ptr(a: np.ndarray, kind):
 def make_bodies(arrays: dict) -> tuple[Bodies, list]:
     """Bodies struct over contiguous float64 arrays; returns (struct, keepalive)."""
     keep = [np.ascontiguousarray(arrays[f], dtype=np.float64) for f in BODY_FIELDS]
-    b = Bodies(*[_ptr(a, _dp) for a in keep])
+    # ten addresses at once: a ctypes pointer object each took half of a small state's copy
+    b = Bodies.from_buffer_copy(struct.pack("10P", *[a.ctypes.data for a in keep]))
+    b.keep = keep
     return b, keep
 
 
