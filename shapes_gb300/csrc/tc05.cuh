@@ -138,6 +138,20 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int k = 0; k < 16; ++k) v[k] = __uint_as_float(r[k]);
 }
 
+/* Transposes four 8 x 8 blocks of bf16, a warp together: lane l names row l % 8
+ * of block l / 8, 16 bytes each, where it is read (src) and where the row of the
+ * transposed block goes (dst). */
+__device__ __forceinline__ void transpose8x8x4(uint32_t src, uint32_t dst) {
+  uint32_t r0, r1, r2, r3;
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(src)
+               : "memory");
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1,%2,%3,%4};" ::"r"(dst), "r"(r0), "r"(r1), "r"(r2),
+               "r"(r3)
+               : "memory");
+}
+
 /* TMEM address of (lane, column) relative to an allocation base. */
 __device__ __forceinline__ uint32_t taddr(uint32_t base, int lane, int col) {
   return base + ((uint32_t)lane << 16) + (uint32_t)col;
