@@ -389,7 +389,7 @@ struct BodyStore {
 
 __device__ __forceinline__ void prefetch_l1(const char* p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 
-/* An update is spread over two or eight lanes.  Of the lanes' rows, the even
+/* An update is spread over two, four or eight lanes.  Of the lanes' rows, the even
  * lanes carry the normal row and the odd lanes the friction row: its fold, its
  * quotient and its accumulated Lagrangian `cached`.  Warm: applySln of the
  * cached Lagrangians (Solvers/Contact.hs:105-113).  Otherwise improveContactSln
@@ -420,7 +420,8 @@ __device__ __forceinline__ double2 update_impulse(bool warm, double dot, double 
  * another level runs. */
 struct LaneConstants {
   double mc, rc, mu, bn0;
-  double c[9]; /* pair: own row, the other row on this lane's body, inverse masses; split: both rows' entry, mass */
+  double c[9]; /* pair: own row, the other row on this lane's body, inverse masses; quad: own row on this lane's body,
+                * inverse masses; split: both rows' entry, mass */
   int32_t no_bounce;
 };
 
@@ -556,19 +557,96 @@ __device__ __forceinline__ void solve_split(const Dev& d, const int4 u, const La
   if (live && t.j < 6 && (u.w & (t.side ? kInfoDynB : kInfoDynA))) bs.set_component(s, t.k, v1);
 }
 
-/* How a level of `count` updates is dealt: `pairs` chunks of sixteen updates,
- * two lanes each, then the rest four to a warp. */
-struct Deal {
-  int pairs, units;
-  __device__ __forceinline__ Deal(int count, int split_limit) {
-    int split = count;
-    pairs = 0;
-    if (count > split_limit) {
-      const int rest = count & 15;
-      split = rest <= 4 ? rest : 0; /* 20 instructions, against 36 */
-      pairs = (count - split + 15) >> 4;
+/* Four lanes to an update, eight updates a warp (all 32 lanes call it, live or
+ * not): lane 2 * side + fric has its row's three entries on its side's body.  The
+ * second side continues the first one's fold; a lane forms the three changes that
+ * its row makes to its side's body, and the two lanes of a side trade: the normal
+ * one moves x and y, the friction one w.  25 FP64 instructions: for levels of
+ * 17 to 32 updates that is one chunk per sub-partition, where two lanes to an
+ * update keep half of them idle for 36 (a step of 901 stacked bodies, 27 updates
+ * a level: 715 -> 671 us), and a remainder of five to eight costs 25 instead of
+ * 36 (4096 worlds of columns 715 -> 672 us). */
+__device__ __forceinline__ void load_quad(const Con* con, LaneConstants& x) {
+  const int fric = threadIdx.x & 1, side = (threadIdx.x >> 1) & 1;
+  const double2 lin = *reinterpret_cast<const double2*>(con->row[fric]);
+  const double2 im = reinterpret_cast<const double2*>(con->im)[side];
+  x.c[0] = lin.x;
+  x.c[1] = lin.y;
+  x.c[2] = con->row[fric][2 + side];
+  x.c[3] = im.x;
+  x.c[4] = im.y;
+  load_common(con, fric, x);
+}
+
+template <bool SM>
+__device__ __forceinline__ void solve_quad(const Dev& d, const int4 u, const LaneConstants& k, bool live,
+                                           const BodyStore<SM>& bs) {
+  const unsigned kAll = 0xffffffffu;
+  const int fric = threadIdx.x & 1, side = (threadIdx.x >> 1) & 1;
+  const int s = side ? u.z : u.y;
+  const bool warm = ((uint32_t)u.x & kWarmBit) != 0;
+  double x, y, w;
+  bs.load(s, x, y, w);
+  const unsigned slow = __ballot_sync(kAll, !((k.no_bounce != 0) & small_mag(x) & small_mag(y) & small_mag(w)));
+  double bias = fric ? 0.0 : k.bn0;
+  if (slow) { /* some update of the warp has a restitution term */
+    double v[6];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      v[3 * q] = __shfl_sync(kAll, x, 2 * q, 4);
+      v[3 * q + 1] = __shfl_sync(kAll, y, 2 * q, 4);
+      v[3 * q + 2] = __shfl_sync(kAll, w, 2 * q, 4);
     }
-    units = pairs + ((split + 3) >> 2);
+    const Con* con = con_of(d, u);
+    if (!fric && ((slow >> (threadIdx.x & 28)) & 0xfu)) bias = con->bn + bounce_term(con, v);
+  }
+  const double jx = side ? k.c[0] : flip_sign(k.c[0]), jy = side ? k.c[1] : flip_sign(k.c[1]), ja = k.c[2];
+  const double px = jx * x, py = jy * y, pw = ja * w;
+  const double first = (px + py) + pw; /* of the first side */
+  const double dot = ((__shfl_sync(kAll, first, fric, 4) + px) + py) + pw; /* of the second */
+  double now;
+  const double2 l = update_impulse(warm, __shfl_sync(kAll, dot, 2 + fric, 4), bias, k.mc, k.rc, k.mu,
+                                   bs.lagrangian(u, fric), &now);
+  if (live & !warm & (side == 0)) bs.set_lagrangian(u, fric, now);
+  const double mine = fric ? l.y : l.x;
+  const double dx = (jx * mine) * k.c[3], dy = (jy * mine) * k.c[3], dw = (ja * mine) * k.c[4];
+  const double got = __shfl_xor_sync(kAll, fric ? dx : dw, 1), got_y = __shfl_xor_sync(kAll, dy, 1);
+  double a = fric ? w : x;
+  a = a + (fric ? got : dx);
+  a = a + (fric ? dw : got);
+  y = y + dy;
+  y = y + got_y;
+  if (live && (u.w & (side ? kInfoDynB : kInfoDynA))) {
+    bs.set_component(s, fric ? 2 : 0, a);
+    if (!fric) bs.set_component(s, 1, y);
+  }
+}
+
+/* How a level of `count` updates is dealt: first `pairs` chunks of sixteen
+ * updates with two lanes each, then `quads` of eight with four, then the rest
+ * four to a warp with eight (36, 25 and 20 FP64 instructions a chunk). */
+struct Deal {
+  int pairs, quads, units;
+  __device__ __forceinline__ Deal(int count, int split_limit) {
+    int split = 0;
+    pairs = quads = 0;
+    if (count <= split_limit) {
+      split = count;
+    } else if (count <= 2 * split_limit) { /* as many chunks as the line above has */
+      quads = (count + 7) >> 3;
+    } else {
+      const int rest = count & 15;
+      if (rest <= 4) split = rest;
+      else if (rest <= 8) quads = 1;
+      pairs = (count - split - (quads ? rest : 0) + 15) >> 4;
+    }
+    units = pairs + quads + ((split + 3) >> 2);
+  }
+  /* unit t's update of this lane, counted from the level's begin */
+  __device__ __forceinline__ int at(int t, int lane) const {
+    if (t < pairs) return 16 * t + (lane >> 1);
+    if (t < pairs + quads) return 16 * pairs + 8 * (t - pairs) + (lane >> 2);
+    return 16 * pairs + 8 * quads + 4 * (t - pairs - quads) + (lane >> 3);
   }
 };
 
@@ -588,13 +666,13 @@ __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, c
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   /* this lane's update of unit t of the level [begin, end) */
   auto update_of = [&](const Deal& deal, int t, int begin, int end, bool* live) {
-    const int i =
-        t < deal.pairs ? begin + 16 * t + (lane >> 1) : begin + 16 * deal.pairs + 4 * (t - deal.pairs) + (lane >> 3);
+    const int i = begin + deal.at(t, lane);
     *live = i < end;
     return ls.get(min(i, end - 1));
   };
   auto load = [&](const Deal& deal, int t, const int4 u, LaneConstants& k) {
     if (t < deal.pairs) load_pair(d, u, k);
+    else if (t < deal.pairs + deal.quads) load_quad(con_of(d, u), k);
     else load_split(con_of(d, u), k);
   };
   int begin = 0;
@@ -627,6 +705,7 @@ __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, c
         load(deal, t, u, k);
       }
       if (t < deal.pairs) solve_pair(d, u, k, live, bs);
+      else if (t < deal.pairs + deal.quads) solve_quad(d, u, k, live, bs);
       else solve_split(d, u, k, live, bs);
     }
     ahead = published > level + 1;
@@ -651,9 +730,9 @@ __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, c
  * beside light ones instead of beside the next heaviest.
  *
  * split_limit: levels of at most this many updates run eight lanes to an
- * update: sixteen for a group alone on its SM (four warps of 20 instructions
- * on four sub-partitions, against one of 36), four where several groups share
- * the SM and the pipe's total work counts (20 against 36). */
+ * update, of at most twice as many four: sixteen for a group alone on its SM (so
+ * that a level is one chunk on each of the four sub-partitions), four where
+ * several groups share the SM and the pipe's total work counts. */
 template <int P>
 __global__ void __launch_bounds__(32 * (P + 1), P == 8 ? 1 : (P == 4 ? 4 : 6))
     k_frontier(Dev d, int iterations, int warm_start, int external, double ax, double ay, double dt, int n_groups,

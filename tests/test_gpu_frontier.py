@@ -62,3 +62,19 @@ def test_one_world_outside_shared_memory(built):
     got, st = _run(sc, 12, lambda b: None)
     assert st["contacts"] > 3000
     _check(sc, got, 12, [0])
+
+
+@pytest.mark.parametrize("count", [3, 4, 5, 8, 9, 16, 17, 20, 24, 25, 31, 32, 33, 36, 37, 40, 41, 48, 64, 69, 72])
+@pytest.mark.parametrize("warps", [4, 8])
+def test_levels_of_every_width(built, count, warps):
+    """Levels of exactly `count` updates: pairs of boxes that touch nothing else, one contact pair each, dealt
+    eight, four and two lanes to an update."""
+    b = scenes.SceneBuilder()
+    box = scenes.rectangle_vertices(1.0, 1.0)
+    for k in range(count):
+        b.add(box, (8.0 * k, 0.0), rot=0.0)
+        b.add(box, (8.0 * k + 0.02 * (k % 7), 0.995), rot=0.001 * (1 + k % 5))
+    sc = b.build(dt=1.0 / 60.0, baumgarte=0.01, slop=0.02, accel=(0.0, -9.8), iterations=6, steps=4)
+    got, st = _run(sc, 4, lambda h: h.set_group_warps(warps))
+    assert st["contacts"] >= count
+    _check(sc, got, 4, [0])
