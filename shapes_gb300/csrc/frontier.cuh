@@ -34,8 +34,9 @@
  * sub-partition (76 with all four busy), whatever lanes are active, and a
  * dependent instruction can follow at once: the cost of a level is the number
  * of FP64 warp instructions its slowest warp issues.  On one lane an update is
- * 65 of them for 32 updates; on two lanes (solve_pair) 36 for sixteen, about the
- * same pipe time at half the latency; on eight (solve_split) 20 for four.
+ * 65 of them for 32 updates; on two lanes (solve_pair) 34 for sixteen, about the
+ * same pipe time at half the latency; on four (solve_quad) 24 for eight; on eight
+ * (solve_split) 20 for four.
  */
 #pragma once
 #include "step_kernels.cuh"
@@ -46,6 +47,7 @@ constexpr int kMaxGroupWorlds = 32;
 constexpr int kEndRing = 64;              /* published level ends in flight */
 constexpr uint32_t kSlotBits = 14;        /* shared-memory groups hold fewer than 2^14 bodies */
 constexpr uint32_t kSlotMask = (1u << kSlotBits) - 1u;
+constexpr int kMoves = 2;                 /* cursors a lane of the scheduling warp moves together */
 constexpr int kFrontierPollLimit = 1 << 24; /* polls of a wait between a group's warps before giving up */
 
 /* Entries of the ring that hands frontiers to the solver: a power of two, at
@@ -168,37 +170,58 @@ __device__ __forceinline__ int32_t ld_acquire_cta(const volatile int32_t* shared
   return v;
 }
 
+__device__ __forceinline__ void st_release_cta(volatile int32_t* shared, int32_t v) {
+  const uint32_t at = (uint32_t)__cvta_generic_to_shared(const_cast<int32_t*>(shared));
+  asm volatile("st.release.cta.shared.s32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
+}
+
 __device__ __forceinline__ void solver_barrier(int threads) {
   asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
-/* Moves the cursor of slot s from (pass, pos) on to its next update, skipping
- * contacts without a cache entry in the warm-start pass.  Returns that update's
- * contact with the pass in *pass when its other body already waits there (or
- * is static) so that it joins the frontier, -1 when it does not, -2 when the
- * body has no update left. */
+/* A body's cursor on the move from (pass, pos) on to its next update, skipping
+ * contacts without a cache entry in the warm-start pass.  In steps, so that a lane
+ * can move several cursors with their loads in flight together. */
 template <class Lists>
-__device__ __forceinline__ int frontier_advance(Lists& ls, int s, int* pass, int pos, int iterations) {
-  const int nb = ls.bn[s], r0 = ls.r0[s], n = nb + (int)ls.r1[s] - r0, b0 = ls.b0[s];
-  if (n == 0) return -2;
-  int p = *pass, q;
+struct Advance {
+  int s, p, pos, n, nb, r0, b0, q;
   uint32_t fl;
-  for (;;) {
+  bool on; /* a cursor to move, until it runs past the last pass */
+  __device__ __forceinline__ void load(const Lists& ls) {
+    nb = ls.bn[s];
+    r0 = ls.r0[s];
+    n = nb + (int)ls.r1[s] - r0;
+    b0 = ls.b0[s];
+  }
+  __device__ __forceinline__ void next() { /* a position past the list is the first of the next pass */
     if (pos >= n) {
       pos = 0;
       ++p;
     }
-    if (p > iterations) return -2;
-    q = pos < nb ? (int)ls.list[b0 + pos] : r0 + pos - nb;
-    fl = ls.flags(q);
-    if (p > 0 || (fl & kInfoHit)) break;
-    ++pos;
   }
-  ls.cur[s] = ls.pack(p, pos);
-  *pass = p;
-  const bool both = (fl & kInfoDynA) && (fl & kInfoDynB);
-  return both && !ls.arrive(q) ? -1 : q;
-}
+  __device__ __forceinline__ void contact(const Lists& ls) {
+    q = pos < nb ? (int)ls.list[b0 + pos] : r0 + pos - nb;
+  }
+  __device__ __forceinline__ void skip(const Lists& ls, int iterations) { /* warm-start pass only */
+    while (p == 0 && !(fl & kInfoHit)) {
+      ++pos;
+      next();
+      if (p > iterations) {
+        on = false;
+        return;
+      }
+      contact(ls);
+      fl = ls.flags(q);
+    }
+  }
+  /* That update's contact when its other body already waits there (or is
+   * static) so that it joins the frontier, else -1. */
+  __device__ __forceinline__ int arrive(Lists& ls) {
+    ls.cur[s] = ls.pack(p, pos);
+    const bool both = (fl & kInfoDynA) && (fl & kInfoDynB);
+    return both && !ls.arrive(q) ? -1 : q;
+  }
+};
 
 /* Builds the group's lists and the first frontier (all the CTA's threads).
  * SM: slots and contacts numbered within the group. */
@@ -272,9 +295,19 @@ __device__ __forceinline__ void frontier_build(const Dev& d, Lists& ls, Frontier
   k = 0;
   for (int t = threadIdx.x; t < NB; t += nt) {
     const int s = slot(t);
-    int p = p0;
-    const int q = frontier_advance(ls, s, &p, 0, iterations);
-    if (q >= 0) ls.put(atomicAdd(&ctl.n0, 1), q, p == 0);
+    Advance<Lists> a;
+    a.s = s;
+    a.p = p0;
+    a.pos = 0;
+    a.load(ls);
+    if (a.n == 0 || p0 > iterations) continue;
+    a.on = true;
+    a.contact(ls);
+    a.fl = ls.flags(a.q);
+    a.skip(ls, iterations);
+    if (!a.on) continue;
+    const int q = a.arrive(ls);
+    if (q >= 0) ls.put(atomicAdd(&ctl.n0, 1), q, a.p == 0);
   }
 }
 
@@ -292,8 +325,10 @@ __device__ __forceinline__ bool frontier_wait(FrontierCtl& ctl, F&& ready) {
 }
 
 /* The scheduling warp: level after level, the frontier that the previous
- * one's updates open.  Lanes take (update, side) pairs.  It waits when the
- * ring of level ends or of updates is full. */
+ * one's updates open.  Lanes take (update, side) pairs, two each: a cursor's move
+ * is a chain of six shared-memory accesses, and a level of 17 to 32 updates took
+ * two of them in turn.  It waits when the ring of level ends or of updates is
+ * full. */
 template <class Lists>
 __device__ __forceinline__ void frontier_schedule(const Dev& d, Lists& ls, FrontierCtl& ctl, int bodies,
                                                   int iterations) {
@@ -303,10 +338,8 @@ __device__ __forceinline__ void frontier_schedule(const Dev& d, Lists& ls, Front
   while (end > begin) {
     __syncwarp();
     if (lane == 0) {
-      __threadfence_block();
       ctl.ends[level % kEndRing] = end;
-      __threadfence_block();
-      ctl.published = level + 1;
+      st_release_cta(&ctl.published, level + 1);
     }
     const int need = level + 3 - kEndRing; /* levels solved before the next level's end may overwrite a slot */
     const bool room = ctl.done >= need && ls.space(end, ctl.solved) >= bodies;
@@ -316,25 +349,50 @@ __device__ __forceinline__ void frontier_schedule(const Dev& d, Lists& ls, Front
       if (!__all_sync(0xffffffffu, ok)) break;
     }
     int pos = end;
-    for (int base = begin; base < end; base += 16) {
-      const int i = base + (lane >> 1);
-      int q = -1, p = 0;
-      if (i < end) {
-        const int4 u = ls.get(i);
-        const int s = (lane & 1) ? u.z : u.y;
-        if (u.w & ((lane & 1) ? kInfoDynB : kInfoDynA)) {
-          const uint32_t cu = ls.cur[s];
-          p = ls.pass_of(cu);
-          q = frontier_advance(ls, s, &p, ls.pos_of(cu) + 1, iterations);
-          if (q == -2) { /* the body's last update: its world has at least this many levels */
-            const int c = (int)((uint32_t)u.x & ~kWarmBit);
-            atomicMax(&d.world_levels[d.body_world[d.c_ga[c]]], level + 1);
-          }
-        }
+    for (int base = begin; base < end; base += 16 * kMoves) {
+      Advance<Lists> a[kMoves];
+      int4 u[kMoves];
+#pragma unroll
+      for (int k = 0; k < kMoves; ++k) {
+        const int i = base + 16 * k + (lane >> 1);
+        u[k] = ls.get(min(i, end - 1));
+        a[k].s = (lane & 1) ? u[k].z : u[k].y;
+        a[k].on = i < end && (u[k].w & ((lane & 1) ? kInfoDynB : kInfoDynA));
       }
-      const unsigned m = __ballot_sync(0xffffffffu, q >= 0);
-      if (q >= 0) ls.put(pos + __popc(m & below), q, p == 0);
-      pos += __popc(m);
+#pragma unroll
+      for (int k = 0; k < kMoves; ++k) {
+        const uint32_t cu = ls.cur[a[k].s];
+        a[k].load(ls);
+        a[k].p = ls.pass_of(cu);
+        a[k].pos = ls.pos_of(cu) + 1;
+        a[k].next();
+      }
+      bool last[kMoves];
+#pragma unroll
+      for (int k = 0; k < kMoves; ++k) {
+        last[k] = a[k].on && a[k].p > iterations;
+        a[k].on = a[k].on && a[k].p <= iterations;
+        a[k].q = 0;
+        if (a[k].on) a[k].contact(ls);
+      }
+#pragma unroll
+      for (int k = 0; k < kMoves; ++k) a[k].fl = ls.flags(a[k].q);
+#pragma unroll
+      for (int k = 0; k < kMoves; ++k) {
+        if (a[k].on && a[k].p == 0) {
+          a[k].skip(ls, iterations);
+          last[k] = !a[k].on;
+        }
+        int q = -1;
+        if (a[k].on) q = a[k].arrive(ls);
+        if (last[k]) { /* the body's last update: its world has at least this many levels */
+          const int c = (int)((uint32_t)u[k].x & ~kWarmBit);
+          atomicMax(&d.world_levels[d.body_world[d.c_ga[c]]], level + 1);
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, q >= 0);
+        if (q >= 0) ls.put(pos + __popc(m & below), q, a[k].p == 0);
+        pos += __popc(m);
+      }
     }
     begin = end;
     end = pos;
@@ -420,7 +478,7 @@ __device__ __forceinline__ double2 update_impulse(bool warm, double dot, double 
  * another level runs. */
 struct LaneConstants {
   double mc, rc, mu, bn0;
-  double c[9]; /* pair: own row, the other row on this lane's body, inverse masses; quad: own row on this lane's body,
+  double c[7]; /* pair: own row, the other row's arm on this lane's body, inverse masses; quad: own row on this lane's body,
                 * inverse masses; split: both rows' entry, mass */
   int32_t no_bounce;
 };
@@ -441,24 +499,24 @@ __device__ __forceinline__ void load_pair(const Dev& d, const int4 u, LaneConsta
   const int fric = threadIdx.x & 1;
   const Con* con = con_of(d, u);
   const double2* own = reinterpret_cast<const double2*>(con->row[fric]);
-  const double2 r0 = own[0], r1 = own[1], q0 = *reinterpret_cast<const double2*>(con->row[1 - fric]);
+  const double2 r0 = own[0], r1 = own[1];
   const double2 im = reinterpret_cast<const double2*>(con->im)[fric];
   x.c[0] = r0.x;
   x.c[1] = r0.y;
   x.c[2] = r1.x;
   x.c[3] = r1.y;
-  x.c[4] = q0.x;
-  x.c[5] = q0.y;
-  x.c[6] = con->row[1 - fric][2 + fric];
-  x.c[7] = im.x;
-  x.c[8] = im.y;
+  x.c[4] = con->row[1 - fric][2 + fric];
+  x.c[5] = im.x;
+  x.c[6] = im.y;
   load_common(con, fric, x);
 }
 
 /* Two lanes to an update, sixteen updates a warp: each lane folds its row from
  * all six velocity components, then moves one body (the even lane a, the odd
- * lane b).  36 FP64 instructions for sixteen updates; one lane to an update
- * took 65 for 32, the same pipe time for twice the latency. */
+ * lane b).  A row's linear products are the same for both bodies but for their
+ * sign: its own lane forms them and the two trade.  34 FP64 instructions for
+ * sixteen updates; one lane to an update took 65 for 32, the same pipe time for
+ * twice the latency. */
 template <class Store>
 __device__ __forceinline__ void solve_pair(const Dev& d, const int4 u, const LaneConstants& k, bool live,
                                            const Store& bs) {
@@ -466,25 +524,29 @@ __device__ __forceinline__ void solve_pair(const Dev& d, const int4 u, const Lan
   double v[6];
   bs.load(u.y, v[0], v[1], v[2]);
   bs.load(u.z, v[3], v[4], v[5]);
+  const double cached = bs.lagrangian(u, fric);
+  const double dot = row_dot(k.c, v);
+  const bool bounce = !((k.no_bounce != 0) & small_velocities(v));
   double bias = fric ? 0.0 : k.bn0;
-  if (!(k.no_bounce && small_velocities(v)) && !fric) bias = con_of(d, u)->bn + bounce_term(con_of(d, u), v);
+  if (__any_sync(0xffffffffu, bounce)) { /* some update of the warp has a restitution term */
+    if (bounce && !fric) bias = con_of(d, u)->bn + bounce_term(con_of(d, u), v);
+  }
   const bool warm = ((uint32_t)u.x & kWarmBit) != 0;
   double now;
-  const double2 l = update_impulse(warm, row_dot(k.c, v), bias, k.mc, k.rc, k.mu, bs.lagrangian(u, fric), &now);
+  const double2 l = update_impulse(warm, dot, bias, k.mc, k.rc, k.mu, cached, &now);
   if (live & !warm) bs.set_lagrangian(u, fric, now);
-  /* this lane's body: its row and the other row on it */
-  const double sx = fric ? k.c[0] : flip_sign(k.c[0]), sy = fric ? k.c[1] : flip_sign(k.c[1]);
-  const double sa = fric ? k.c[3] : k.c[2];
-  const double tx = fric ? k.c[4] : flip_sign(k.c[4]), ty = fric ? k.c[5] : flip_sign(k.c[5]);
-  const double nx = fric ? tx : sx, ny = fric ? ty : sy, na = fric ? k.c[6] : sa;
-  const double fx = fric ? sx : tx, fy = fric ? sy : ty, fa = fric ? sa : k.c[6];
+  const double mine = fric ? l.y : l.x;
+  const double px = k.c[0] * mine, py = k.c[1] * mine; /* on b; the negative on a */
+  const double qx = __shfl_xor_sync(0xffffffffu, px, 1), qy = __shfl_xor_sync(0xffffffffu, py, 1);
+  const double nx = fric ? qx : flip_sign(px), ny = fric ? qy : flip_sign(py), na = fric ? k.c[4] : k.c[2];
+  const double fx = fric ? px : flip_sign(qx), fy = fric ? py : flip_sign(qy), fa = fric ? k.c[3] : k.c[4];
   double x = fric ? v[3] : v[0], y = fric ? v[4] : v[1], w = fric ? v[5] : v[2];
-  x = x + (nx * l.x) * k.c[7];
-  y = y + (ny * l.x) * k.c[7];
-  w = w + (na * l.x) * k.c[8];
-  x = x + (fx * l.y) * k.c[7];
-  y = y + (fy * l.y) * k.c[7];
-  w = w + (fa * l.y) * k.c[8];
+  x = x + nx * k.c[5];
+  y = y + ny * k.c[5];
+  w = w + (na * l.x) * k.c[6];
+  x = x + fx * k.c[5];
+  y = y + fy * k.c[5];
+  w = w + (fa * l.y) * k.c[6];
   if (live && (u.w & (fric ? kInfoDynB : kInfoDynA))) bs.store(fric ? u.z : u.y, x, y, w);
 }
 
@@ -521,14 +583,6 @@ __device__ __forceinline__ double split_update(const Con* con, const LaneConstan
   const SplitLane t;
   const bool flip = t.side == 0 && t.k < 2;
   const double jn = flip ? flip_sign(x.c[0]) : x.c[0], jf = flip ? flip_sign(x.c[1]) : x.c[1], m = x.c[2];
-  const unsigned slow = __ballot_sync(kAll, !((x.no_bounce != 0) & small_mag(v0)));
-  double bias = t.fric ? 0.0 : x.bn0;
-  if (slow) { /* some update of the warp has a restitution term */
-    double v[6];
-#pragma unroll
-    for (int q = 0; q < 6; ++q) v[q] = __shfl_sync(kAll, v0, q, 8);
-    if (!t.fric && ((slow >> (threadIdx.x & 24)) & 0xffu)) bias = con->bn + bounce_term(con, v);
-  }
   const double pn = jn * v0, pf = jf * v0;
   /* pairs of lanes trade: an even lane 2 i ends with the normal row's products 2 i and 2 i + 1, its neighbour with the
    * friction row's */
@@ -540,6 +594,14 @@ __device__ __forceinline__ double split_update(const Con* con, const LaneConstan
   dot = dot + __shfl_sync(kAll, hi, 2 + t.fric, 8);
   dot = dot + __shfl_sync(kAll, lo, 4 + t.fric, 8);
   dot = dot + __shfl_sync(kAll, hi, 4 + t.fric, 8);
+  const unsigned slow = __ballot_sync(kAll, !((x.no_bounce != 0) & small_mag(v0)));
+  double bias = t.fric ? 0.0 : x.bn0;
+  if (slow) { /* some update of the warp has a restitution term */
+    double v[6];
+#pragma unroll
+    for (int q = 0; q < 6; ++q) v[q] = __shfl_sync(kAll, v0, q, 8);
+    if (!t.fric && ((slow >> (threadIdx.x & 24)) & 0xffu)) bias = con->bn + bounce_term(con, v);
+  }
   const double2 l = update_impulse(warm, dot, bias, x.mc, x.rc, x.mu, cached, now);
   const double v1 = v0 + (jn * l.x) * m;
   return v1 + (jf * l.y) * m;
@@ -561,11 +623,13 @@ __device__ __forceinline__ void solve_split(const Dev& d, const int4 u, const La
  * not): lane 2 * side + fric has its row's three entries on its side's body.  The
  * second side continues the first one's fold; a lane forms the three changes that
  * its row makes to its side's body, and the two lanes of a side trade: the normal
- * one moves x and y, the friction one w.  25 FP64 instructions: for levels of
+ * one moves x and y, the friction one w.  24 FP64 instructions: for levels of
  * 17 to 32 updates that is one chunk per sub-partition, where two lanes to an
- * update keep half of them idle for 36 (a step of 901 stacked bodies, 27 updates
- * a level: 715 -> 671 us), and a remainder of five to eight costs 25 instead of
- * 36 (4096 worlds of columns 715 -> 672 us). */
+ * update keep half of them idle for 34 (a step of 901 stacked bodies, 27 updates
+ * a level: 715 -> 671 us), and a remainder of five to eight costs 24 instead of
+ * 34 (4096 worlds of columns 715 -> 672 us).  In all three forms the fold comes
+ * before the test for a restitution term: a branch ahead of it would keep the
+ * other instructions out of the FP64 ones' shadow. */
 __device__ __forceinline__ void load_quad(const Con* con, LaneConstants& x) {
   const int fric = threadIdx.x & 1, side = (threadIdx.x >> 1) & 1;
   const double2 lin = *reinterpret_cast<const double2*>(con->row[fric]);
@@ -587,6 +651,12 @@ __device__ __forceinline__ void solve_quad(const Dev& d, const int4 u, const Lan
   const bool warm = ((uint32_t)u.x & kWarmBit) != 0;
   double x, y, w;
   bs.load(s, x, y, w);
+  const double cached = bs.lagrangian(u, fric);
+  const double jx = side ? k.c[0] : flip_sign(k.c[0]), jy = side ? k.c[1] : flip_sign(k.c[1]), ja = k.c[2];
+  const double px = jx * x, py = jy * y, pw = ja * w;
+  const double first = (px + py) + pw; /* of the first side */
+  double dot = ((__shfl_sync(kAll, first, fric, 4) + px) + py) + pw; /* of the second */
+  dot = __shfl_sync(kAll, dot, 2 + fric, 4);
   const unsigned slow = __ballot_sync(kAll, !((k.no_bounce != 0) & small_mag(x) & small_mag(y) & small_mag(w)));
   double bias = fric ? 0.0 : k.bn0;
   if (slow) { /* some update of the warp has a restitution term */
@@ -600,16 +670,14 @@ __device__ __forceinline__ void solve_quad(const Dev& d, const int4 u, const Lan
     const Con* con = con_of(d, u);
     if (!fric && ((slow >> (threadIdx.x & 28)) & 0xfu)) bias = con->bn + bounce_term(con, v);
   }
-  const double jx = side ? k.c[0] : flip_sign(k.c[0]), jy = side ? k.c[1] : flip_sign(k.c[1]), ja = k.c[2];
-  const double px = jx * x, py = jy * y, pw = ja * w;
-  const double first = (px + py) + pw; /* of the first side */
-  const double dot = ((__shfl_sync(kAll, first, fric, 4) + px) + py) + pw; /* of the second */
   double now;
-  const double2 l = update_impulse(warm, __shfl_sync(kAll, dot, 2 + fric, 4), bias, k.mc, k.rc, k.mu,
-                                   bs.lagrangian(u, fric), &now);
+  const double2 l = update_impulse(warm, dot, bias, k.mc, k.rc, k.mu, cached, &now);
   if (live & !warm & (side == 0)) bs.set_lagrangian(u, fric, now);
   const double mine = fric ? l.y : l.x;
-  const double dx = (jx * mine) * k.c[3], dy = (jy * mine) * k.c[3], dw = (ja * mine) * k.c[4];
+  /* the row's linear products, the same for both sides but for their sign: x by the second side, y by the first */
+  const double half = (side ? k.c[0] : k.c[1]) * mine, traded = __shfl_xor_sync(kAll, half, 2);
+  const double dx = (side ? half : flip_sign(traded)) * k.c[3], dy = (side ? traded : flip_sign(half)) * k.c[3];
+  const double dw = (ja * mine) * k.c[4];
   const double got = __shfl_xor_sync(kAll, fric ? dx : dw, 1), got_y = __shfl_xor_sync(kAll, dy, 1);
   double a = fric ? w : x;
   a = a + (fric ? got : dx);
@@ -624,7 +692,7 @@ __device__ __forceinline__ void solve_quad(const Dev& d, const int4 u, const Lan
 
 /* How a level of `count` updates is dealt: first `pairs` chunks of sixteen
  * updates with two lanes each, then `quads` of eight with four, then the rest
- * four to a warp with eight (36, 25 and 20 FP64 instructions a chunk). */
+ * four to a warp with eight (34, 24 and 20 FP64 instructions a chunk). */
 struct Deal {
   int pairs, quads, units;
   __device__ __forceinline__ Deal(int count, int split_limit) {
@@ -679,14 +747,15 @@ __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, c
   bool ahead = false, live = false;
   int4 u = make_int4(0, 0, 0, 0);
   LaneConstants k;
+  int known = 0; /* levels that this warp has seen published */
   for (int level = 0;; ++level) {
-    if (wib == 0) {
+    if (wib == 0 && known <= level) {
       const bool ok = frontier_wait(
           ctl, [&]() { return ld_acquire_cta(&ctl.published) > level || ld_acquire_cta(&ctl.total) >= 0; });
       if (!__all_sync(0xffffffffu, ok) && lane == 0) ctl.stop = level; /* every warp stops at the same level */
     }
     solver_barrier(32 * P); /* the level before is solved, this one is published */
-    const int published = ctl.published;
+    const int published = ld_acquire_cta(&ctl.published);
     if (ctl.stop <= level || published <= level) break; /* published holds all levels once total is known */
     if (threadIdx.x == 0) {
       ctl.solved = begin;
@@ -708,7 +777,8 @@ __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, c
       else if (t < deal.pairs + deal.quads) solve_quad(d, u, k, live, bs);
       else solve_split(d, u, k, live, bs);
     }
-    ahead = published > level + 1;
+    known = published;
+    ahead = known > level + 1;
     if (ahead) {
       const int end2 = ctl.ends[(level + 1) % kEndRing];
       const Deal deal2(end2 - end, split_limit);
