@@ -807,6 +807,7 @@ template <int P>
 __global__ void __launch_bounds__(32 * (P + 1), P == 8 ? 1 : (P == 4 ? 4 : 6))
     k_frontier(Dev d, int iterations, int warm_start, int external, double ax, double ay, double dt, int n_groups,
                int smem_bytes, int heavy_first, int split_limit) {
+  chained_wait(); /* the next kernel's blocks would hold places through the whole solve, that other streams can use */
   extern __shared__ __align__(16) unsigned char s_dyn[];
   __shared__ FrontierCtl ctl;
   if (d.counters[kCntOverflow]) return; /* buffers incomplete: the host retries */

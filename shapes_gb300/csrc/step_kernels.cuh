@@ -180,12 +180,11 @@ struct Dev {
 };
 
 enum {
-  /* reset every step, the others every call */
+  /* set anew every step (the first two by the scans, the others by k_contact_slots), the others every call */
   kCntPairs = 0,
   kCntContacts = 1,
   kCntGroupAlloc = 2, /* bump allocator of the groups' runs of updates kept in global memory */
   kCntListAlloc = 3,  /* bump allocator of the lists kept in global memory */
-  kCntPerStep = 4,
   kCntHits = 4,
   kCntItems = 5,
   kCntLevels = 6,
@@ -343,6 +342,16 @@ __global__ void k_commit_bodies(Ptr10 p, int n, uint8_t* changed, const unsigned
 /* helpers                                                                    */
 /* ------------------------------------------------------------------------ */
 
+/* First statement of every kernel that launch_chained launches: nothing before it
+ * reads or writes memory.  Waits until the kernels before are complete and their
+ * writes visible (at once in a kernel launched plainly); chained_entry also lets
+ * the next one's blocks take their places as soon as all of this one's have. */
+__device__ __forceinline__ void chained_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void chained_entry() {
+  chained_wait();
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ bool is_nan(double d) { return d != d; }
 
 
@@ -359,6 +368,7 @@ __device__ __forceinline__ uint64_t pack_key(int i, int j, int fa, int fb) {
  * strict min / max vertex along its local unit normal (extentAlong',
  * ConvexHull.hs:81-92).  One thread per edge. */
 __global__ void k_init_extents(Dev d) {
+  chained_entry();
   for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < d.n_verts; v += gridDim.x * blockDim.x) {
     /* find the owning body by binary search over vert_off */
     int lo = 0, hi = d.n_bodies - 1;
@@ -421,6 +431,7 @@ __device__ __forceinline__ void write_box(const Dev& d, int g, double x0, double
 constexpr int kPoseThreads = 128;
 __global__ void __launch_bounds__(kPoseThreads) k_integrate_pose(Dev d, double dt, int advance, int per_block,
                                                                  const uint8_t* only = nullptr) {
+  chained_entry();
   __shared__ double mat[6][kPoseThreads];   /* the matrix's two rows */
   __shared__ int32_t vstart[kPoseThreads + 1];
   __shared__ uint8_t kind[kPoseThreads];    /* a hull to pose: 1, with a NaN translation: 2; else 0 */
@@ -652,6 +663,7 @@ __device__ __forceinline__ void brute_row(const Dev& d, int g) {
 
 /* Counts the rows of a batch without a grid world: a warp per row. */
 __global__ void k_count_brute(Dev d) {
+  chained_entry();
   const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nw_total = (gridDim.x * blockDim.x) >> 5;
   for (int g = wid; g < d.n_bodies; g += nw_total) brute_row<true>(d, g);
@@ -708,6 +720,7 @@ __device__ __forceinline__ double world_cell_size(const Dev& d, int wld) {
  * that rebuilds needs a cell size.  Every world's large list and moved count
  * start empty here. */
 __global__ void k_grid_stats(Dev d, int inc) {
+  chained_entry();
   __shared__ double s_sum[32];
   __shared__ int s_cnt[32];
   const int k = blockIdx.x;
@@ -768,6 +781,7 @@ __global__ void k_grid_stats(Dev d, int inc) {
 /* One thread per body: grid bodies get a cell and a bucket count, the rest go
  * on their world's list of large bodies. */
 __global__ void k_grid_bin(Dev d) {
+  chained_entry();
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
     const int wld = d.body_world[g];
     const int T = d.grid_T[wld];
@@ -810,6 +824,7 @@ __global__ void k_grid_bin(Dev d) {
 
 /* Places grid bodies into their buckets (bucket_off turns from starts into ends). */
 __global__ void k_grid_scatter(Dev d) {
+  chained_entry();
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
     if (!d.row_mode[g]) continue;
     const int wld = d.body_world[g];
@@ -995,6 +1010,7 @@ __device__ __forceinline__ bool fat_box(const Dev& d, int g, int wld, double fb[
 
 /* One thread per body of a grid world: moved or not, and the large list. */
 __global__ void k_inc_mark(Dev d) {
+  chained_entry();
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
     const int wld = d.body_world[g];
     if (d.grid_T[wld] == 0) continue;
@@ -1048,6 +1064,7 @@ __device__ __forceinline__ int inc_mode(const Dev& d, int w) {
  * a staying body keeps the ones it has, which still contain its box), and the
  * grid bodies of worlds that search this frame are counted into the buckets. */
 __global__ void k_inc_update(Dev d) {
+  chained_entry();
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
     const int wld = d.body_world[g];
     if (d.grid_T[wld] == 0) continue;
@@ -1080,6 +1097,7 @@ __global__ void k_inc_update(Dev d) {
 /* Places the grid bodies of worlds that search; and each world's state for the
  * next frame. */
 __global__ void k_inc_scatter(Dev d) {
+  chained_entry();
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < d.n_bodies; g += gridDim.x * blockDim.x) {
     const int wld = d.body_world[g];
     if (d.grid_T[wld] == 0) continue;
@@ -1116,6 +1134,7 @@ __device__ __forceinline__ unsigned team_mask() {
  * 121 bodies; the chain of its loads, not their number, is what takes the time. */
 template <int TEAM>
 __global__ void __launch_bounds__(kRowThreads) k_inc_query(Dev d) {
+  chained_entry();
   __shared__ int s_cnt[kRowThreads / TEAM];
   const int lane = threadIdx.x % TEAM, team = threadIdx.x / TEAM;
   const unsigned mates = team_mask<TEAM>();
@@ -1218,6 +1237,7 @@ __device__ __forceinline__ void grid_partners(const Dev& d, int g, Hit&& hit) {
  * 4096 worlds of 505,800; counting and writing now take 13 and 100. */
 template <bool INC, int TEAM>
 __global__ void __launch_bounds__(kRowThreads, 5) k_count_rows(Dev d) {
+  chained_entry();
   constexpr int kTeams = kRowThreads / TEAM;
   __shared__ int s_cnt[kTeams], s_hits[kTeams][kRowHits + 1], s_brute[kTeams], s_nbrute;
   const int lane = threadIdx.x % TEAM, team = threadIdx.x / TEAM;
@@ -1264,6 +1284,7 @@ __global__ void __launch_bounds__(kRowThreads, 5) k_count_rows(Dev d) {
  * world a thread writes its row's pairs with large bodies. */
 template <bool GRID, bool INC>
 __global__ void __launch_bounds__(kRowThreads) k_write_rows(Dev d) {
+  chained_entry();
   constexpr int kWarps = kRowThreads / 32;
   __shared__ int s_heavy[kRowThreads], s_nheavy, s_cnt[kWarps], s_hits[GRID ? kWarps : 1][kRowSorted];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1904,6 +1925,7 @@ constexpr int kNpThreads = 128;
 constexpr int kNpRounds = 4; /* pairs a thread filters before the block goes on, at most */
 
 __global__ void __launch_bounds__(kNpThreads) k_narrowphase(Dev d) {
+  chained_entry();
   struct Entry {
     AxisSets ab, ba;
     int p;
@@ -2104,10 +2126,12 @@ __global__ void k_narrowphase_lanes(Dev d) {
  * than slots: about half the slots of a settled pile are empty (separated
  * pairs, pairs with one contact), and an idle lane still costs its warp's FP64
  * instructions; and the worlds' first pairs (row_off at their first row in
- * mirrored order) and first contacts. */
+ * mirrored order) and first contacts; and the group solver's allocators. */
 __global__ void k_contact_slots(Dev d) {
+  chained_entry();
   const int P = min((int)d.counters[kCntPairs], d.pair_cap);
   const int C = (int)d.counters[kCntContacts];
+  if (blockIdx.x == 0 && threadIdx.x == 0) d.counters[kCntGroupAlloc] = d.counters[kCntListAlloc] = 0;
   for (int w = blockIdx.x * blockDim.x + threadIdx.x; w <= d.n_worlds; w += gridDim.x * blockDim.x) {
     const int p = d.row_off[d.world_body_off[w]];
     d.world_pair_off[w] = p;
@@ -2121,6 +2145,7 @@ __global__ void k_contact_slots(Dev d) {
 }
 
 __global__ void k_build(Dev d, double beta_dt, double slop, int warm_start, int build_solver) {
+  chained_entry();
   const int P = min((int)d.counters[kCntPairs], d.pair_cap);
   const int C = (int)d.counters[kCntContacts];
   if (C > d.contact_cap) return;
@@ -2403,6 +2428,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(int32_t* in, int n_cap, c
                                                        unsigned long long* total, int total_cap,
                                                        unsigned long long* overflow, unsigned overflow_bit,
                                                        unsigned long long* err) {
+  chained_entry();
   __shared__ int32_t s_scan[kScanThreads / 32];
   __shared__ int32_t s_prefix, s_tile;
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
