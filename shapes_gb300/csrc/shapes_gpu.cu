@@ -152,9 +152,8 @@ struct shapes_batch {
   double* grid_lim = nullptr;
   int32_t* bucket_cnt = nullptr;
   int32_t* bucket_off = nullptr;
-  int32_t* grid_ids = nullptr;
-  int32_t* cell_x = nullptr;
-  int32_t* cell_y = nullptr;
+  int4* grid_ent = nullptr;
+  int2* cell = nullptr;
   uint8_t* row_mode = nullptr;
   int32_t* large_cnt = nullptr;
   int32_t* large_ids = nullptr;
@@ -539,9 +538,8 @@ struct shapes_batch {
     d.grid_lim = grid_lim;
     d.bucket_cnt = bucket_cnt;
     d.bucket_off = bucket_off;
-    d.grid_ids = grid_ids;
-    d.cell_x = cell_x;
-    d.cell_y = cell_y;
+    d.grid_ent = grid_ent;
+    d.cell = cell;
     d.row_mode = row_mode;
     d.large_cnt = large_cnt;
     d.large_ids = large_ids;
@@ -974,7 +972,7 @@ struct shapes_batch {
   /* Worlds with at least grid_min_bodies bodies use the grid broadphase. */
   void setup_grid() {
     dfree(grid_T); dfree(grid_base); dfree(grid_inv_s); dfree(grid_lim); dfree(bucket_cnt); dfree(bucket_off);
-    dfree(grid_ids); dfree(cell_x); dfree(cell_y); dfree(row_mode); dfree(large_cnt); dfree(large_ids);
+    dfree(grid_ent); dfree(cell); dfree(row_mode); dfree(large_cnt); dfree(large_ids);
     std::vector<int32_t> T(W), base(W);
     int64_t nb = 0;
     any_grid = false;
@@ -998,9 +996,8 @@ struct shapes_batch {
     grid_lim = dalloc<double>(W, "cudaMalloc grid");
     bucket_cnt = dalloc<int32_t>((size_t)n_buckets + 1, "cudaMalloc grid");
     bucket_off = dalloc<int32_t>((size_t)n_buckets + 1, "cudaMalloc grid");
-    grid_ids = dalloc<int32_t>(N, "cudaMalloc grid");
-    cell_x = dalloc<int32_t>(N, "cudaMalloc grid");
-    cell_y = dalloc<int32_t>(N, "cudaMalloc grid");
+    grid_ent = dalloc<int4>(N, "cudaMalloc grid");
+    cell = dalloc<int2>(N, "cudaMalloc grid");
     row_mode = dalloc<uint8_t>(N, "cudaMalloc grid");
     large_cnt = dalloc<int32_t>(W, "cudaMalloc grid");
     large_ids = dalloc<int32_t>(N, "cudaMalloc grid");
@@ -1567,7 +1564,7 @@ struct shapes_batch {
     dfree(vf); dfree(ef);
     dfree(row_cnt); dfree(row_hits); dfree(row_off); dfree(world_pair_off);
     dfree(grid_T); dfree(grid_base); dfree(grid_inv_s); dfree(grid_lim); dfree(bucket_cnt); dfree(bucket_off);
-    dfree(grid_ids); dfree(cell_x); dfree(cell_y); dfree(row_mode); dfree(large_cnt); dfree(large_ids);
+    dfree(grid_ent); dfree(cell); dfree(row_mode); dfree(large_cnt); dfree(large_ids);
     dfree(ext_chunk); dfree(ext_chunk_off); dfree(ext_part_sum); dfree(ext_part_cnt); dfree(ext_done);
     free_sap();
     free_incremental();

@@ -93,9 +93,9 @@ struct Dev {
   double* grid_lim;         /* [W] (1 - 2^-20) * cell size: bodies below it in x and y use the grid */
   int32_t* bucket_cnt;      /* [n_buckets + 1] counts, then scanned offsets */
   int32_t* bucket_off;      /* [n_buckets + 1] */
-  int32_t* grid_ids;        /* [N] body ids sorted by bucket */
-  int32_t* cell_x;          /* [N] */
-  int32_t* cell_y;          /* [N] */
+  int4* grid_ent;           /* [N] {body, cell x, cell y, flags} sorted by bucket: all that a searching row needs of
+                             * a candidate in another cell, in one access where id, cells and flags were four */
+  int2* cell;               /* [N] */
   uint8_t* row_mode;        /* [N] 1 = row found through the grid */
   int32_t* large_cnt;       /* [W] bodies of the world off the grid */
   int32_t* large_ids;       /* [N] per-world region at world_body_off[w] */
@@ -584,12 +584,16 @@ __device__ __forceinline__ bool keys_overlap(const Dev& d, int gi, int gj, uint8
   return !(kj01.x > ki[1] || kj01.y < ki[0]) && !(kj23.x > ki[3] || kj23.y < ki[2]);
 }
 
-__device__ __forceinline__ bool pair_overlaps(const Dev& d, int gi, int gj, uint8_t fi,
-                                              const uint64_t ki[4]) {
-  const uint8_t fj = d.flags[gj];
+__device__ __forceinline__ bool box_overlaps(const Dev& d, int gi, int gj, uint8_t fi, uint8_t fj,
+                                             const uint64_t ki[4]) {
   const ulonglong2 kj01 = *reinterpret_cast<const ulonglong2*>(d.boxk + 4 * gj);
   const ulonglong2 kj23 = *reinterpret_cast<const ulonglong2*>(d.boxk + 4 * gj + 2);
   return keys_overlap(d, gi, gj, fi, fj, ki, kj01, kj23);
+}
+
+__device__ __forceinline__ bool pair_overlaps(const Dev& d, int gi, int gj, uint8_t fi,
+                                              const uint64_t ki[4]) {
+  return box_overlaps(d, gi, gj, fi, d.flags[gj], ki);
 }
 
 constexpr int kRowHits = 8;        /* pairs of a row that the counting pass keeps */
@@ -804,8 +808,7 @@ __global__ void k_grid_bin(Dev d) {
       }
       if (small) {
         mode = 1;
-        d.cell_x[g] = cx;
-        d.cell_y[g] = cy;
+        d.cell[g] = make_int2(cx, cy);
         if (d.world_sap && d.world_sap[wld]) {
           const uint64_t k = okey(d.box[4 * g + 0]);
           atomicMin(reinterpret_cast<unsigned long long*>(&d.sap_range[2 * wld]), (unsigned long long)k);
@@ -829,9 +832,9 @@ __global__ void k_grid_scatter(Dev d) {
     if (!d.row_mode[g]) continue;
     const int wld = d.body_world[g];
     if (d.world_sap && d.world_sap[wld]) continue; /* swept, not binned */
-    const int b = d.grid_base[wld] + cell_bucket(d.cell_x[g], d.cell_y[g], d.grid_T[wld]);
-    const int pos = atomicAdd(&d.bucket_off[b], 1);
-    d.grid_ids[pos] = g;
+    const int2 c = d.cell[g];
+    const int pos = atomicAdd(&d.bucket_off[d.grid_base[wld] + cell_bucket(c.x, c.y, d.grid_T[wld])], 1);
+    d.grid_ent[pos] = make_int4(g, c.x, c.y, d.flags[g]);
   }
 }
 
@@ -1030,14 +1033,16 @@ __global__ void k_inc_mark(Dev d) {
       fits = fat_box(d, g, wld, fb, &cx, &cy);
       if (fits) { /* its new fat box (read by nothing before k_inc_scatter) */
         for (int k = 0; k < 4; ++k) d.fatk[4 * g + k] = okey(fb[k]);
-        d.cell_x[g] = cx;
-        d.cell_y[g] = cy;
+        d.cell[g] = make_int2(cx, cy);
       }
     }
     const bool moved = rebuild || (!inside && (was || fits));
     const bool now = inside || fits;
     d.moved[g] = (moved ? kMovedBit : 0) | (was ? kMovedWasGrid : 0) | (now ? kMovedNowGrid : 0);
-    if (moved && !rebuild) atomicAdd(&d.inc_moved[wld], 1);
+    if (moved && !rebuild) { /* one atomic for the warp's bodies of a world: its counter is one address */
+      const unsigned peers = __match_any_sync(__activemask(), wld);
+      if ((int)(threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&d.inc_moved[wld], __popc(peers));
+    }
     if (!now) {
       const int k = atomicAdd(&d.large_cnt[wld], 1);
       d.large_ids[d.world_body_off[wld] + k] = g;
@@ -1089,8 +1094,10 @@ __global__ void k_inc_update(Dev d) {
     const bool now = (mg & kMovedNowGrid) != 0;
     if (mg & kMovedBit) d.row_mode[g] = now ? 1 : 0;
     if (mode == kIncBuild) d.nbr_cnt[g] = 0;
-    if (now && (mode != kIncList || d.inc_moved[wld] > 0))
-      atomicAdd(&d.bucket_cnt[d.grid_base[wld] + cell_bucket(d.cell_x[g], d.cell_y[g], d.grid_T[wld])], 1);
+    if (now && (mode != kIncList || d.inc_moved[wld] > 0)) {
+      const int2 c = d.cell[g];
+      atomicAdd(&d.bucket_cnt[d.grid_base[wld] + cell_bucket(c.x, c.y, d.grid_T[wld])], 1);
+    }
   }
 }
 
@@ -1111,9 +1118,9 @@ __global__ void k_inc_scatter(Dev d) {
       d.inc_state[wld] = mode == kIncFull ? kIncStateFull : kIncStateList;
     }
     if (!d.row_mode[g] || !(mode != kIncList || d.inc_moved[wld] > 0)) continue;
-    const int b = d.grid_base[wld] + cell_bucket(d.cell_x[g], d.cell_y[g], d.grid_T[wld]);
-    const int pos = atomicAdd(&d.bucket_off[b], 1);
-    d.grid_ids[pos] = g;
+    const int2 c = d.cell[g];
+    const int pos = atomicAdd(&d.bucket_off[d.grid_base[wld] + cell_bucket(c.x, c.y, d.grid_T[wld])], 1);
+    d.grid_ent[pos] = make_int4(g, c.x, c.y, d.flags[g]);
   }
 }
 
@@ -1146,7 +1153,7 @@ __global__ void __launch_bounds__(kRowThreads) k_inc_query(Dev d) {
     const bool rebuild = mode == kIncBuild;
     if (mode == kIncFull || (!rebuild && !(d.moved[g] & kMovedBit))) continue;
     const int T = d.grid_T[wld], base = d.grid_base[wld];
-    const int cx = d.cell_x[g], cy = d.cell_y[g];
+    const int2 cell = d.cell[g];
     uint64_t fg[4];
     for (int k = 0; k < 4; ++k) fg[k] = d.fatk[4 * g + k];
     int32_t* lst = d.nbr + (size_t)g * d.nbr_cap;
@@ -1154,12 +1161,13 @@ __global__ void __launch_bounds__(kRowThreads) k_inc_query(Dev d) {
     __syncwarp(mates);
     bool over = false;
     for (int c = lane; c < 9; c += TEAM) {
-      const int ncx = cx + c % 3 - 1, ncy = cy + c / 3 - 1;
+      const int ncx = cell.x + c % 3 - 1, ncy = cell.y + c / 3 - 1;
       const int b = base + cell_bucket(ncx, ncy, T);
       const int k0 = b > 0 ? d.bucket_off[b - 1] : 0, k1 = d.bucket_off[b];
       for (int k = k0; k < k1; ++k) {
-        const int j = d.grid_ids[k];
-        if (j == g || d.cell_x[j] != ncx || d.cell_y[j] != ncy) continue;
+        const int4 e = d.grid_ent[k];
+        const int j = e.x;
+        if (j == g || e.y != ncx || e.z != ncy) continue;
         if (!fat_overlap(fg, d.fatk + 4 * j)) continue;
         const int cnt = atomicAdd(&s_cnt[team], 1);
         if (cnt < d.nbr_cap) lst[cnt] = j; else over = true;
@@ -1208,15 +1216,15 @@ __device__ __forceinline__ void grid_partners(const Dev& d, int g, Hit&& hit) {
     if (COMPACT && lane == 0 && listed <= d.nbr_cap) d.nbr_cnt[g] = kept;
   } else if (INC || !(d.world_sap && d.world_sap[wld])) {
     const int T = d.grid_T[wld], base = d.grid_base[wld];
-    const int cx = d.cell_x[g], cy = d.cell_y[g];
+    const int2 cell = d.cell[g];
     for (int c = lane; c < 9; c += LANES) {
-      const int ncx = cx + c % 3 - 1, ncy = cy + c / 3 - 1;
+      const int ncx = cell.x + c % 3 - 1, ncy = cell.y + c / 3 - 1;
       const int b = base + cell_bucket(ncx, ncy, T);
       const int k0 = b > 0 ? d.bucket_off[b - 1] : 0, k1 = d.bucket_off[b];
       for (int k = k0; k < k1; ++k) {
-        const int j = d.grid_ids[k];
-        if (j >= g || d.cell_x[j] != ncx || d.cell_y[j] != ncy) continue;
-        if (pair_overlaps(d, g, j, fi, ki)) hit(j);
+        const int4 e = d.grid_ent[k];
+        if (e.x >= g || e.y != ncx || e.z != ncy) continue;
+        if (box_overlaps(d, g, e.x, fi, (uint8_t)e.w, ki)) hit(e.x);
       }
     }
   }
