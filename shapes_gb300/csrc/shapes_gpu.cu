@@ -1156,8 +1156,10 @@ struct shapes_batch {
          2u);
     stage(2, 2, [&]() {
       launch_chained(chain(), shapes::k_contact_slots, grid_for(2LL * pair_cap, 256), 256, 0, stream, d);
-      launch_chained(chain(), shapes::k_build, grid_for(contact_cap, 128), 128, 0, stream, d,
-                     cfg.baumgarte / cfg.dt, cfg.slop, cfg.warm_start, solve ? 1 : 0);
+      const bool staged = shapes::build_staged(contact_cap) && chain();
+      launch_chained(chain(), shapes::k_build, grid_for(contact_cap, shapes::kBuildThreads), shapes::kBuildThreads,
+                     staged ? shapes::kBuildThreads * sizeof(shapes::Con) : 0, stream, d, cfg.baumgarte / cfg.dt,
+                     cfg.slop, cfg.warm_start, solve ? 1 : 0, staged ? 1 : 0);
     });
     if (!solve) return;
     if (learn || collect) {
@@ -3449,7 +3451,8 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   launch_chained(true, shapes::k_narrowphase, grid_for(kNaMaxPairs, shapes::kNpThreads), shapes::kNpThreads, 0, st, d);
   scan(d.slot_cnt, kNaMaxPairs, d.counters + shapes::kCntPairs, d.slot_off, d.counters + shapes::kCntContacts,
        d.contact_cap, 2u);
-  launch_chained(true, shapes::k_build, grid_for(2LL * kNaMaxPairs, 128), 128, 0, st, d, 0.0, 0.0, 0, 0);
+  launch_chained(true, shapes::k_build, grid_for(2LL * kNaMaxPairs, shapes::kBuildThreads), shapes::kBuildThreads, 0, st,
+                 d, 0.0, 0.0, 0, 0, 0);
   e = cudaMemcpyAsync(cnt, d.counters, sizeof(cnt), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e == cudaSuccess) e = cudaGetLastError();

@@ -2122,14 +2122,17 @@ __global__ void k_narrowphase_lanes(Dev d) {
 /* A8-A9 constraint build + warm-start lookup                                 */
 /* ------------------------------------------------------------------------ */
 
-/* One thread per contact slot.  Compacts the contact, builds its
- * ContactConstraint (NonPenetration.hs:16-56, Friction.hs:18-44,
- * Restitution.hs:21-31, flip handling Utils.hs:175-215 / Constraint.hs:96-98),
- * the step-invariant solver factors, and looks the key up in the previous
- * cache: descZipVector (Utils/Descending.hs:47-71) over two strictly
- * descending key lists pairs each new key with an equal old key exactly when
- * one exists, which a binary search over the world's old entries finds.
- * `build_solver` = 0 compacts contacts only (collide). */
+constexpr int kBuildThreads = 128;
+
+/* Whether k_build stages its constants in shared memory: a warp's constants lie one
+ * after another, and staged they leave 512 bytes to a store instruction, where a
+ * thread storing its own 224 touches a line for each (521 thousand contacts: 76 us
+ * in place of 110, 165 thousand: 39 in place of 51).  Few contacts gain nothing, and
+ * the group solver's block, which may need all of an SM's shared memory, then cannot
+ * take its place before k_build is done (401 boxes: 12 us a step lost); nor can
+ * those of other handles in flight (eight handles of 30 thousand contacts: 1.3 %). */
+inline bool build_staged(long long contacts) { return contacts >= 65536; }
+
 /* The slot of every contact, so that k_build's threads take contacts rather
  * than slots: about half the slots of a settled pile are empty (separated
  * pairs, pairs with one contact), and an idle lane still costs its warp's FP64
@@ -2152,18 +2155,30 @@ __global__ void k_contact_slots(Dev d) {
   }
 }
 
-__global__ void k_build(Dev d, double beta_dt, double slop, int warm_start, int build_solver) {
+/* One thread per contact (or contact slot, where k_contact_slots did not run).  Compacts the contact, builds its
+ * ContactConstraint (NonPenetration.hs:16-56, Friction.hs:18-44,
+ * Restitution.hs:21-31, flip handling Utils.hs:175-215 / Constraint.hs:96-98),
+ * the step-invariant solver factors, and looks the key up in the previous
+ * cache: descZipVector (Utils/Descending.hs:47-71) over two strictly
+ * descending key lists pairs each new key with an equal old key exactly when
+ * one exists, which a search over the world's old entries finds.
+ * `build_solver` = 0 compacts contacts only (collide). */
+__global__ void __launch_bounds__(kBuildThreads) k_build(Dev d, double beta_dt, double slop, int warm_start,
+                                                         int build_solver, int staged) {
+  extern __shared__ __align__(16) unsigned char s_build[];
+  Con* s_con = reinterpret_cast<Con*>(s_build); /* [kBuildThreads] if staged */
   chained_entry();
+  const int lane = threadIdx.x & 31;
   const int P = min((int)d.counters[kCntPairs], d.pair_cap);
   const int C = (int)d.counters[kCntContacts];
   if (C > d.contact_cap) return;
   const int n = d.c_slot ? C : 2 * P; /* contacts (k_contact_slots ran), else slots */
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  auto one = [&](int i) {
     int t = i, c = i;
     if (d.c_slot) {
       t = d.c_slot[i];
     } else {
-      if ((t & 1) >= d.slot_cnt[t >> 1]) continue;
+      if ((t & 1) >= d.slot_cnt[t >> 1]) return;
       c = d.slot_off[t >> 1] + (t & 1);
     }
     const int p = t >> 1;
@@ -2185,7 +2200,7 @@ __global__ void k_build(Dev d, double beta_dt, double slop, int warm_start, int 
     cv[2] = px;
     cv[3] = py;
     cv[4] = depth;
-    if (!build_solver) continue;
+    if (!build_solver) return;
     /* constraintGen: positions of (a, b) = (i, j); a Flip contact is built
      * with the bodies swapped, then its Jacobian halves are swapped back.  The
      * differences and products that the two rows, the restitution radii and the
@@ -2231,22 +2246,39 @@ __global__ void k_build(Dev d, double beta_dt, double slop, int warm_start, int 
     cc.no_bounce = (small_mag(cc.ra[0]) & small_mag(cc.ra[1]) & small_mag(cc.ra[2]) & small_mag(cc.ra[3]) &
                     below_two(nx) & below_two(ny) & (mag_bits(cc.e) == 0)) ? 1 : 0;
     cc.pad = 0;
-    d.con[c] = cc;
+    if (staged) s_con[threadIdx.x] = cc;
+    else d.con[c] = cc;
     /* warm-start lookup */
     double l0 = 0.0, l1 = 0.0;
     uint8_t hit = 0;
     if (warm_start) {
-      int lo = d.old_cwo[wld], hi = d.old_cwo[wld + 1] - 1;
-      while (lo <= hi) { /* keys strictly descending */
-        const int mid = (lo + hi) >> 1;
-        const uint64_t k = d.old_key[mid];
+      /* keys strictly descending.  From one step to the next a world's contacts hardly change: the search starts at the
+       * contact's place of now and widens from there (a settled world: one access, its neighbours' the same line, in
+       * place of one per bit of the world's contact count, each waiting for the last) */
+      const int first = d.old_cwo[wld], end = d.old_cwo[wld + 1];
+      int lo = first, hi = end - 1, at = min(first + (c - d.world_contact_off[wld]), hi), step = 1;
+      bool below = false, above = false; /* bounded by a key that was read */
+      while (lo <= hi) {
+        const uint64_t k = d.old_key[at];
         if (k == key) {
           hit = 1;
-          l0 = d.old_lam[2 * mid];
-          l1 = d.old_lam[2 * mid + 1];
+          l0 = d.old_lam[2 * at];
+          l1 = d.old_lam[2 * at + 1];
           break;
         }
-        if (k > key) lo = mid + 1; else hi = mid - 1;
+        if (k > key) {
+          lo = at + 1;
+          below = true;
+        } else {
+          hi = at - 1;
+          above = true;
+        }
+        if (below && above) {
+          at = (lo + hi) >> 1;
+        } else {
+          at = below ? min(lo + step - 1, hi) : max(hi - step + 1, lo);
+          step <<= 1;
+        }
       }
     }
     if (d.miss_flag)
@@ -2257,6 +2289,16 @@ __global__ void k_build(Dev d, double beta_dt, double slop, int warm_start, int 
     d.c_hit[c] = info;
     d.lam[2 * c] = l0;
     d.lam[2 * c + 1] = l1;
+  };
+  for (int base = blockIdx.x * blockDim.x + (threadIdx.x & ~31); base < n; base += gridDim.x * blockDim.x) {
+    if (base + lane < n) one(base + lane);
+    if (!build_solver || !staged) continue;
+    __syncwarp();
+    const int4* src = reinterpret_cast<const int4*>(s_con + (threadIdx.x & ~31));
+    int4* dst = reinterpret_cast<int4*>(d.con + base);
+    const int words = min(32, n - base) * (int)(sizeof(Con) / 16);
+    for (int k = lane; k < words; k += 32) dst[k] = src[k];
+    __syncwarp();
   }
 }
 

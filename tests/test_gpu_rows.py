@@ -51,3 +51,24 @@ def test_rows_match_the_oracle(n):
             b.collide()
             compare_collision(b, [ow], f"{n} bodies, incremental {incremental}")
         b.close()
+
+
+@pytest.mark.parametrize("cols,rows", [(6, 5), (160, 130)])
+def test_constants_and_cache_entries(cols, rows):
+    """The contact build with its constants stored directly and staged (capacity from 65,536 contacts on), and
+    the search for last step's entries where every contact stays, moves and goes: steps equal the oracle's."""
+    from tests.parity import assert_bits_equal, config_of
+
+    sc = scenes.single_world_boxes(seed=9, cols=cols, rows=rows)
+    sc["config"]["iterations"] = 2
+    b, ow = batch_from_scene(sc), O.world_from_scene(sc)
+    c = sc["config"]
+    for k in range(3):
+        b.step(config_of(sc), 2)
+        ow.step(c["dt"], c["baumgarte"], c["slop"], c["accel"], c["iterations"], nsteps=2)
+        state = b.get_bodies()
+        for f in state:
+            assert_bits_equal(state[f], ow.bodies()[f], f"step {2 * k + 2} {f}")
+        if k == 1:
+            assert b.stats()["cache_hits"] > 0
+    b.close()
