@@ -55,9 +55,9 @@ METRIC = "body-steps/s at matched residual, plain vs learned warm-start, 1 GB300
 UNIT = "body-steps/s"
 
 # Algorithmic bytes per solver update (one contact in one warm-start or sweep
-# pass): constraint 152 B + cache 16 B + two bodies x (velocity 24 + inverse
-# mass 16 + material 16) read, two velocities 2 x 24 + cache 16 written.
-SOLVER_BYTES_PER_ITEM = (152 + 16 + 2 * (24 + 16 + 16)) + (2 * 24 + 16)
+# pass): constraint with inverse masses and friction 160 B + cache 16 B + two
+# velocities 2 x 24 read, two velocities 2 x 24 + cache 16 written.
+SOLVER_BYTES_PER_ITEM = (160 + 16 + 2 * 24) + (2 * 24 + 16)
 
 WORKLOADS = {
     "learned": "1024 worlds x 256 mixed boxes and 3-8 vertex polygons (sizes U[0.4,1.5], friction U[0.2,0.8]), "
@@ -765,9 +765,9 @@ def run_ours(args, rank, world, local):
         b.close()
 
     # ---- roofline of the dominant stage (profiled pass of the same window) -
-    solver_kernel = "k_schedule_solve" if not tuned or tuned[2] == 1 else f"k_group_solve<{tuned[2]}>"
+    solver_kernel = "k_frontier"
     if args.workload == "container":
-        solver_kernel = "k_lw_color_pass + k_lw_color_seq" if args.coloured else "k_lw_ordered"
+        solver_kernel = "k_lw_coloured" if args.coloured else "k_lw_ordered"
     items = st_prof["solver_items"]
     if items == 0 and st_prof["contacts"] > 0:
         # large-world solvers count no items: the last step's contacts x (sweeps + warm-start pass)
@@ -938,11 +938,11 @@ def run_contacts(args, rank, world, local, scene, stream):
         bytes_per_launch = pairs * NARROWPHASE_BYTES_PER_PAIR + st["contacts"] * 57
         achieved = bytes_per_launch / (avg_ms * 1e-3) / 1e9
         peaks = measured_peaks()
-        roof = {"kernel": "k_narrowphase (+ class sort)", "bound": "hbm", "achieved": achieved,
+        roof = {"kernel": "k_narrowphase", "bound": "hbm", "achieved": achieved,
                 "peak": peaks["hbm_gbs"], "unit": "GB/s", "frac": achieved / peaks["hbm_gbs"],
                 "peak_source": peaks["source"], "traffic": None, "bytes_per_pair": NARROWPHASE_BYTES_PER_PAIR,
                 "pairs_per_launch": pairs, "avg_launch_ms": avg_ms,
-                "note": "FP64-bound: SAT projections are 2 multiplies + 1 add per vertex and edge"}
+                "note": "binary32 decides most axes; FP64 for the rest and the manifolds"}
     cpu = None
     if world == 1 and rank == 0 and not args.no_cpu:
         import multiprocessing
@@ -998,7 +998,7 @@ def stage_bytes(stage, units, vbar):
 
 
 STAGE_KERNELS = {"integrate": "k_integrate_pose", "broadphase": "grid / incremental pair kernels",
-                 "narrowphase": "k_narrowphase (+ class sort)", "build": "k_build", "schedule": "levels",
+                 "narrowphase": "k_narrowphase", "build": "k_build", "schedule": "levels",
                  "scan": "scans", "learned": "k_learned_features + k_mlp_predict"}
 
 
@@ -1015,7 +1015,7 @@ def stage_roofline(prof, units, vbar, solver_kernel, peaks):
         per_launch = by / launches
         achieved = per_launch / (avg_ms * 1e-3) / 1e9
         kernel = solver_kernel if k == "solve" else STAGE_KERNELS.get(k, k)
-        dram = STAGE_DRAM_BYTES_PER_UNIT.get(k if k != "solve" or "group" in solver_kernel else "solve_schedule")
+        dram = STAGE_DRAM_BYTES_PER_UNIT.get(k if k != "solve" or solver_kernel == "k_frontier" else None)
         unit_key = k
         return {"kernel": kernel, "stage": k, "stage_share": ms / sum(v[0] for v in prof.values()),
                 "bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
@@ -1030,32 +1030,32 @@ def stage_roofline(prof, units, vbar, solver_kernel, peaks):
 # Algorithmic bytes of k_integrate_pose per body: velocities, position and
 # angle, inverse masses and the vertex offset read (24 + 24 + 16 + 8); position
 # and angle, box, box keys and flags written (24 + 32 + 32 + 1); per vertex the
-# local point and the two extent indices read (16 + 8), the world point, unit
-# normal and the two self extents written (16 + 16 + 16).
+# local point and the two extent indices read (16 + 8), the world point and unit
+# normal written in binary64 (16 + 16) and, with the self extents, in binary32
+# (16 + 8).
 POSE_BYTES_FIXED = 24 + 24 + 16 + 8 + 24 + 32 + 32 + 1
-POSE_BYTES_PER_VERTEX = 16 + 8 + 16 + 16 + 16
+POSE_BYTES_PER_VERTEX = 16 + 8 + 16 + 16 + 16 + 8
 # broadphase: box keys and flags read per body, one (i, j) pair written.
 BROADPHASE_BYTES_PER_BODY = 32 + 1
 BROADPHASE_BYTES_PER_PAIR = 8
 # k_build per contact: contact key and values (57) + both bodies' positions
 # and inverse masses (2 x 32) + the previous cache entry (32) read; the
-# 152-byte constraint lines + the new cache entry (32) written.
-BUILD_BYTES_PER_CONTACT = 57 + 64 + 32 + 152 + 32
+# 224-byte constraint record + the contact (57) + the new cache entry (32) written.
+BUILD_BYTES_PER_CONTACT = 57 + 64 + 32 + 224 + 57 + 32
 # DRAM bytes per unit measured by ncu (dram__bytes_read.sum + write.sum over
 # the launch's units), for the `traffic` field: the settled mixed scene (128
-# worlds x 256 bodies, step 306: 68,786 pairs, 70,521 contacts, 634,429 solver
+# worlds x 256 bodies, step 201: 65,963 pairs, 64,336 contacts, 576,935 solver
 # updates), profiles/fp64_units_mixed128.md.
 STAGE_DRAM_BYTES_PER_UNIT = {
-    "solve": (30.2, "ncu dram bytes per update of k_group_solve<4, parallel levels> (mixed, 256 worlds) x updates"),
-    "solve_schedule": (30.5, "ncu dram bytes per update of k_schedule_solve (settled mixed, 128 worlds) x updates"),
-    "narrowphase": (123.5, "ncu dram bytes per pair of k_narrowphase (settled mixed, 128 worlds) x pairs"),
-    "build": (147.0, "ncu dram bytes per contact of k_build (settled mixed, 128 worlds) x contacts"),
-    "integrate": (177.0, "ncu dram bytes per body of k_integrate_pose (settled mixed, 128 worlds) x bodies"),
+    "solve": (30.0, "ncu dram bytes per update of k_frontier<4> (settled mixed, 128 worlds) x updates"),
+    "narrowphase": (152.7, "ncu dram bytes per pair of k_narrowphase (settled mixed, 128 worlds) x pairs"),
+    "build": (148.1, "ncu dram bytes per contact of k_build (settled mixed, 128 worlds) x contacts"),
+    "integrate": (176.3, "ncu dram bytes per body of k_integrate_pose (settled mixed, 128 worlds) x bodies"),
 }
 # FP64 lane-operations (ncu DADD + DMUL + DFMA thread instructions, predicated
 # on) per unit of each stage, same capture: per solver update, per pair, per
-# contact, per body.  The broadphase, scans and schedule issue none.
-FP64_OPS_PER_UNIT = {"solve": 68.5, "narrowphase": 264.5, "build": 84.6, "integrate": 328.6}
+# contact, per body.  The scans and schedule issue none, the broadphase next to none.
+FP64_OPS_PER_UNIT = {"solve": 73.9, "narrowphase": 38.5, "build": 55.0, "integrate": 172.4}
 FP64_OPS_SOURCE = ("ncu dadd+dmul+dfma thread-instruction counts per unit of each kernel (settled mixed scene, "
                    "profiles/fp64_units_mixed128.md), times this window's units")
 

@@ -135,9 +135,9 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
 
 /* a * b in binary64, round to nearest even, computed on the integer pipe.
  * Measured on GB300: 4.8e11 of these per second against 5.3e11 hardware
- * products, on a separate pipe, so a kernel bound by FP64 throughput at high
- * occupancy gains by moving part of its products here (a latency-bound
- * dependency chain loses: the sequence is about 30 instructions long).  Fast path: both operands normal with biased exponents in
+ * products, on a separate pipe: independent products split between the two
+ * pipes go almost twice as fast, a dependency chain loses (the sequence is about
+ * 30 instructions long).  No kernel of the step uses it now.  Fast path: both operands normal with biased exponents in
  * [512, 1534] (the product is then normal, or overflows to infinity exactly
  * as IEEE rounding does), or one operand a zero and the other finite (a
  * signed zero).  The 106-bit product of the 53-bit significands comes from
