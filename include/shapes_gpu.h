@@ -251,8 +251,9 @@ int shapes_batch_get_world_metrics(shapes_batch* b, double* residual, double* ma
 
 /* Solver packing.  Worlds are sorted by size and packed into groups, one CTA
  * per group; target_bodies_per_group > 0 closes a group once it holds that many
- * bodies (0 = automatic: four groups per SM, at most 512 bodies each).  threads
- * (a multiple of 32, at most 256; 0 = 32) is kept and reported; the warps of a
+ * bodies (0 = automatic: one group per SM up to 224 bodies to an SM, above that
+ * four groups per SM, each closed at 512 bodies at the latest).  threads (a
+ * multiple of 32, at most 256; 0 = 32) is kept and reported; the warps of a
  * group are shapes_batch_set_group_warps'.  Results do not depend on the
  * packing. */
 int shapes_batch_set_launch(shapes_batch* b, int32_t target_bodies_per_group, int32_t threads);

@@ -736,9 +736,12 @@ struct shapes_batch {
 
   /* Solver groups: worlds sorted by body count (largest first, so the longest
    * dependency chains start first) and packed by the caller's choice of
-   * worlds or bodies per group, else so that four groups fall to each SM but
-   * a group closes at kAutoGroupBodies bodies: small batches get one world a
-   * group, spread over the GPU, large ones groups whose levels fill warps. */
+   * worlds or bodies per group.  Else so that one group falls to each SM, with
+   * eight solver warps, while that is at most kLoneGroupBodies bodies (per step,
+   * ms, against four groups to an SM: 119 bodies to an SM 0.345 / 0.435, 197
+   * 0.326 / 0.364, 215 0.485 / 0.52; 252 0.373 / 0.338, 526 0.686 / 0.662), and
+   * above it four groups that close at kAutoGroupBodies bodies. */
+  static constexpr int kLoneGroupBodies = 224;
   static constexpr int kAutoGroupBodies = 512;
   void make_groups(int iterations) {
     if (stream) ck(cudaStreamSynchronize(stream), "sync"); /* no kernel may still read the old groups */
@@ -760,7 +763,9 @@ struct shapes_batch {
     if (!by_worlds && target <= 0) {
       int64_t total = 0;
       for (int w : order) total += h_world_body_off[w + 1] - h_world_body_off[w];
-      target = (int32_t)std::max<int64_t>(1, std::min<int64_t>(kAutoGroupBodies, total / (4 * num_sms())));
+      const int64_t per_sm = total / num_sms();
+      target = (int32_t)std::max<int64_t>(
+          1, per_sm <= kLoneGroupBodies ? per_sm : std::min<int64_t>(kAutoGroupBodies, per_sm / 4));
     }
     h_group_world_off.assign(1, 0);
     int32_t max_bodies = 0, bodies = 0, in_group = 0;
@@ -870,7 +875,12 @@ struct shapes_batch {
     const int P = !group_warps_auto ? group_warps : (per_sm <= 1 ? 8 : 4);
     const int64_t contacts = (per_sm <= 1 ? 10LL : 5LL) * group_max_bodies / 2;
     const size_t want = shapes::frontier_bytes(group_max_bodies, contacts, true);
-    const int smem = (int)std::min<size_t>(want, kFrontierSmem / std::min(per_sm, 3));
+    /* four groups resident in place of three where their lists fit a quarter of the SM, the Lagrangians then in
+     * global memory: 500 groups of 560 bodies run in one wave in place of two, 1.90 -> 1.64 ms a step */
+    size_t most = kFrontierSmem / std::min(per_sm, 3);
+    if (per_sm >= 4 && shapes::frontier_bytes(group_max_bodies, contacts, false) <= kFrontierSmem / 4)
+      most = kFrontierSmem / 4;
+    const int smem = (int)std::min<size_t>(want, most);
     const int split_limit = per_sm <= 1 ? 16 : 4;
     if (P == 1) launch_frontier<1>(d, cfg, smem, split_limit);
     else if (P == 2) launch_frontier<2>(d, cfg, smem, split_limit);

@@ -78,3 +78,14 @@ def test_levels_of_every_width(built, count, warps):
     got, st = _run(sc, 4, lambda h: h.set_group_warps(warps))
     assert st["contacts"] >= count
     _check(sc, got, 4, [0])
+
+
+@pytest.mark.parametrize("worlds,bodies", [(200, 60), (480, 71), (480, 72), (700, 140)])
+def test_default_packing(built, worlds, bodies):
+    """The default packing on both sides of its rule (one group to an SM up to 224 bodies to an SM), and groups
+    of which four fit an SM only without their Lagrangians."""
+    sc = scenes.batched_mixed(seed=bodies, n_worlds=worlds, n_bodies=bodies)
+    sc["config"]["iterations"] = 3
+    got, st = _run(sc, 80, lambda b: None)
+    assert st["contacts"] > 1000
+    _check(sc, got, 80, [0, worlds // 2, worlds - 1])
