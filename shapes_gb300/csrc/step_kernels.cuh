@@ -2592,7 +2592,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(int32_t* in, int n_cap, c
     st.ctl[1] = 0;
     st.ctl[2] = 0;
     const uint32_t next = (epoch + 1) & 0x3fffffffu;
-    if (next == 0) /* the words of 2^30 scans ago would be this round's */
+    if (next == 0) /* the words of 2^30 scans ago would pass for new ones */
       for (int k = 0; k < st.tiles; ++k) st.tile[k] = 0;
     st.ctl[0] = next;
   }
