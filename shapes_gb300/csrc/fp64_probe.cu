@@ -547,3 +547,50 @@ extern "C" int shapes_probe_lw_ticket_check(int max_p, int max_r, unsigned long 
   *bad = nbad;
   return 0;
 }
+
+/* ---- the step's scan (scan.cuh) ---- */
+#include "scan.cuh"
+
+/* The scan's sum on the host: out[k] = the sum of in[0..k) from the left,
+ * *tree the sum of all of them pairwise. */
+extern "C" int shapes_probe_scan_sum(const int* in, int n, int* out, int* tree) {
+  std::vector<int> level(in, in + n);
+  out[0] = 0;
+  for (int k = 0; k < n; ++k) out[k + 1] = shapes::scan_sum(out[k], in[k]);
+  while (level.size() > 1) {
+    std::vector<int> next;
+    for (size_t k = 0; k < level.size(); k += 2)
+      next.push_back(k + 1 < level.size() ? shapes::scan_sum(level[k], level[k + 1]) : level[k]);
+    level.swap(next);
+  }
+  *tree = n ? level[0] : 0;
+  return 0;
+}
+
+/* One k_scan over in[0..n) of a capacity n_cap: out[0..n], the total and the overflow and error words. */
+extern "C" int shapes_probe_scan(const int* in, int n, int n_cap, int total_cap, int* out, unsigned long long* words3) {
+  if (n < 0 || n > n_cap || n_cap > (1 << 24)) return -1;
+  const int tiles = n_cap / shapes::kScanTile + 1;
+  int32_t *d_in = nullptr, *d_out = nullptr;
+  unsigned long long* d_words = nullptr; /* total, overflow, error, n, then the scan's own */
+  const size_t words = 4 + tiles + 2;
+  cudaError_t e = cudaMalloc(&d_in, sizeof(int32_t) * (n_cap + 1));
+  if (e == cudaSuccess) e = cudaMalloc(&d_out, sizeof(int32_t) * (n_cap + 1));
+  if (e == cudaSuccess) e = cudaMalloc(&d_words, sizeof(unsigned long long) * words);
+  if (e == cudaSuccess) e = cudaMemset(d_words, 0, sizeof(unsigned long long) * words);
+  const unsigned long long count = n;
+  if (e == cudaSuccess) e = cudaMemcpy(d_words + 3, &count, sizeof(count), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d_in, in, sizeof(int32_t) * n, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    const shapes::ScanState st{d_words + 4, reinterpret_cast<uint32_t*>(d_words + 4 + tiles), tiles};
+    shapes::k_scan<<<tiles, shapes::kScanThreads>>>(d_in, n_cap, d_words + 3, st, d_out, 0, d_words, total_cap,
+                                                    d_words + 1, 1u, d_words + 2);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(out, d_out, sizeof(int32_t) * (n + 1), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(words3, d_words, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost);
+  cudaFree(d_in);
+  cudaFree(d_out);
+  cudaFree(d_words);
+  return e == cudaSuccess ? 0 : -5;
+}
