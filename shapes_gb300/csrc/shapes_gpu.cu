@@ -3175,11 +3175,21 @@ constexpr int kNaMaxPairs = SHAPES_NOALLOC_MAX_PAIRS;
 constexpr int kNaMaxContacts = 2 * kNaMaxPairs;
 constexpr int kNaTiles = (kNaMaxPairs + 1 + shapes::kScanTile - 1) / shapes::kScanTile + 1;
 
+/* What a call counts on being zero: its counters and what its scans keep.  One
+ * block, cleared at the start of every call, so that nothing an earlier call
+ * left (calls that overlapped, which is the caller's fault, leave the scans'
+ * words of several launches mixed) reaches a later one. */
+struct NaWords {
+  unsigned long long counters[shapes::kCntSlots];
+  unsigned long long tiles[kNaTiles];
+  uint32_t scan_ctl[3];
+};
+
 /* Byte offsets of the scratch arrays, each 256-byte aligned. */
 struct NaPlan {
   size_t world_body_off, body_world, lx, ly, emin, emax, wx, wy, nx, ny, vf, ef, box, boxk, flags, row_mode, row_cnt,
       row_hits, row_off, pair_a, pair_b, slot_cnt, slot_off, slot_feat, slot_val, world_pair_off, cwo, c_key, c_ga, c_gb,
-      c_flip, c_hit, c_val, tiles, scan_ctl, counters, total;
+      c_flip, c_hit, c_val, words, total;
 };
 
 constexpr size_t na_take(size_t& o, size_t bytes) {
@@ -3224,9 +3234,7 @@ constexpr NaPlan na_plan() {
   p.c_flip = na_take(o, kNaMaxContacts);
   p.c_hit = na_take(o, kNaMaxContacts);
   p.c_val = na_take(o, 5 * (size_t)kNaMaxContacts * sizeof(double));
-  p.tiles = na_take(o, kNaTiles * sizeof(unsigned long long));
-  p.scan_ctl = na_take(o, 3 * sizeof(uint32_t));
-  p.counters = na_take(o, shapes::kCntSlots * sizeof(unsigned long long));
+  p.words = na_take(o, sizeof(NaWords));
   p.total = o;
   return p;
 }
@@ -3262,7 +3270,7 @@ __global__ void k_noalloc_setup(int n, int nv, const int32_t* vert_off, const do
   uint8_t* mode = base + kNaPlan.row_mode;
   double* lx = reinterpret_cast<double*>(base + kNaPlan.lx);
   double* ly = reinterpret_cast<double*>(base + kNaPlan.ly);
-  unsigned long long* cnt = reinterpret_cast<unsigned long long*>(base + kNaPlan.counters);
+  unsigned long long* cnt = reinterpret_cast<NaWords*>(base + kNaPlan.words)->counters;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
   if (t0 == 0) {
     wbo[0] = 0;
@@ -3413,18 +3421,17 @@ extern "C" int shapes_collide_noalloc(int32_t n_bodies, const double* pos_x, con
   d.c_flip = base + kNaPlan.c_flip;
   d.c_hit = base + kNaPlan.c_hit;
   d.c_val = reinterpret_cast<double*>(base + kNaPlan.c_val);
-  d.counters = reinterpret_cast<unsigned long long*>(base + kNaPlan.counters);
-  /* the scan's words are zero when the library is loaded and as the last scan left them after that */
-  const shapes::ScanState scan_state{reinterpret_cast<unsigned long long*>(base + kNaPlan.tiles),
-                                     reinterpret_cast<uint32_t*>(base + kNaPlan.scan_ctl), kNaTiles};
+  NaWords* const words = reinterpret_cast<NaWords*>(base + kNaPlan.words);
+  d.counters = words->counters;
+  const shapes::ScanState scan_state{words->tiles, words->scan_ctl, kNaTiles};
   auto scan = [&](int32_t* in, int n_cap, const unsigned long long* n_dev, int32_t* out, unsigned long long* total,
                   int cap, unsigned bit) {
     launch_chained(true, shapes::k_scan, n_cap / shapes::kScanTile + 1, shapes::kScanThreads, 0, st, in, n_cap, n_dev,
                    scan_state, out, 0, total, cap, d.counters + shapes::kCntOverflow, bit,
                    d.counters + shapes::kCntSolveErr);
   };
-  /* counters start at zero; the set-up kernel validates the vertex offsets */
-  cudaError_t e = cudaMemsetAsync(d.counters, 0, shapes::kCntSlots * sizeof(unsigned long long), st);
+  /* counters and scans start at zero; the set-up kernel validates the vertex offsets */
+  cudaError_t e = cudaMemsetAsync(words, 0, sizeof(NaWords), st);
   unsigned long long cnt[shapes::kCntSlots] = {0};
   if (e == cudaSuccess) {
     k_noalloc_setup<<<grid_for(std::max(n_bodies, n_verts), 256), 256, 0, st>>>(
