@@ -309,11 +309,14 @@ int shapes_batch_autotune(shapes_batch* b, const shapes_config* cfg, int32_t ste
 int shapes_batch_set_stream(shapes_batch* b, void* cuda_stream);
 
 /* CUDA-graph replay of the step (default on): each step is captured once per
- * configuration and buffer layout and replayed with one graph launch; steps
+ * configuration, buffer layout and launch shape (a handle stepped alone, or
+ * beside others) and replayed with one graph launch; steps
  * are launched kernel by kernel while profiling, or when the stream is a
  * legacy default stream or already capturing.  Results are identical either
  * way. */
 int shapes_batch_set_graphs(shapes_batch* b, int32_t enabled);
+/* How many steps were captured since the handle was made. */
+int shapes_batch_get_graph_captures(shapes_batch* b, int64_t* captures);
 
 /* Incremental grid pairs (on by default).  Worlds on the grid broadphase
  * keep, per body, a fat box (its AABB grown by 1/32 of the world's cell size)

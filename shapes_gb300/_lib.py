@@ -168,6 +168,7 @@ SIGNATURES = [
     ("shapes_mlp_train", ctypes.c_int, [ctypes.c_void_p, _fp, _fp, ctypes.c_int64, ctypes.POINTER(TrainConfig),
                                         _fp]),
     ("shapes_batch_set_graphs", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32]),
+    ("shapes_batch_get_graph_captures", ctypes.c_int, [ctypes.c_void_p, _lp]),
     ("shapes_batch_set_incremental", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32]),
     ("shapes_batch_delete_body", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, ctypes.c_int32]),
     ("shapes_batch_append_body", ctypes.c_int, [ctypes.c_void_p, ctypes.c_int32, _dp, ctypes.c_int32, _dp, _ip]),
@@ -496,6 +497,12 @@ class Batch:
     def set_graphs(self, enabled: bool) -> None:
         """CUDA-graph replay of the step (default on)."""
         check(lib().shapes_batch_set_graphs(self._h, int(bool(enabled))), "shapes_batch_set_graphs")
+
+    def graph_captures(self) -> int:
+        """Steps captured since the handle was made."""
+        v = ctypes.c_int64()
+        check(lib().shapes_batch_get_graph_captures(self._h, ctypes.byref(v)), "shapes_batch_get_graph_captures")
+        return v.value
 
     def set_incremental(self, enabled: bool) -> None:
         """Incremental grid pairs (fat boxes, default on); the pairs are identical either way."""

@@ -377,27 +377,46 @@ struct shapes_batch {
 
   shapes_stats stats{};
 
-  /* CUDA graphs: one captured step per write buffer, replayed while the
-   * configuration and every buffer the step touches stay the same.  Anything
-   * that reallocates a buffer, regroups the solver or changes which kernels a
-   * step launches bumps graph_epoch. */
+  /* What the number of handles that share the GPU decides about a step's
+   * launches (solve_shape); the rest of them follows from the configuration and
+   * from what bumps graph_epoch. */
+  struct SolveShape {
+    bool chained;
+    int warps, smem, split_limit;
+    bool operator==(const SolveShape& o) const {
+      return chained == o.chained && warps == o.warps && smem == o.smem && split_limit == o.split_limit;
+    }
+  };
+
+  /* CUDA graphs: captured steps, replayed while the configuration and every
+   * buffer the step touches stay the same.  Anything that reallocates a buffer,
+   * regroups the solver or changes which kernels a step launches bumps
+   * graph_epoch.  Per write buffer the kStepGraphs used last are kept, one for
+   * each configuration and shape, so that a handle stepped now alone, now beside
+   * others captures once for each: five shapes can occur (alone; beside others
+   * with one, two, three or more groups to an SM). */
+  static constexpr int kStepGraphs = 6;
   bool graphs_enabled = true;
   uint64_t graph_epoch = 1;
   struct StepGraph {
     cudaGraphExec_t exec = nullptr;
-    uint64_t epoch = 0;
+    uint64_t epoch = 0, used = 0;
     shapes_config cfg{};
+    SolveShape shape{};
   };
-  StepGraph graph[2];
+  StepGraph graph[2][kStepGraphs];
+  uint64_t graph_clock = 0;
   int64_t graph_captures = 0;
 
   void invalidate_graphs() { ++graph_epoch; }
 
+  void drop_graph(StepGraph& g) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    g.exec = nullptr;
+  }
   void drop_graphs() {
-    for (auto& g : graph) {
-      if (g.exec) cudaGraphExecDestroy(g.exec);
-      g.exec = nullptr;
-    }
+    for (auto& of_buffer : graph)
+      for (auto& g : of_buffer) drop_graph(g);
   }
 
   /* One solver step writing buffer wb: replayed from its graph, captured on
@@ -412,10 +431,17 @@ struct shapes_batch {
       enqueue_step(cfg, true, wb);
       return;
     }
-    StepGraph& g = graph[wb];
-    if (!g.exec || g.epoch != graph_epoch || std::memcmp(&g.cfg, &cfg, sizeof cfg) != 0) {
-      if (g.exec) cudaGraphExecDestroy(g.exec);
-      g.exec = nullptr;
+    const SolveShape shape = solve_shape();
+    StepGraph* hit = nullptr;
+    StepGraph* oldest = &graph[wb][0];
+    for (auto& g : graph[wb]) {
+      if (g.exec && g.epoch != graph_epoch) drop_graph(g);
+      if (g.exec && g.shape == shape && std::memcmp(&g.cfg, &cfg, sizeof cfg) == 0) hit = &g;
+      if (oldest->exec && (!g.exec || g.used < oldest->used)) oldest = &g;
+    }
+    StepGraph& g = hit ? *hit : *oldest;
+    if (!hit) {
+      drop_graph(g);
       cudaGraph_t gr = nullptr;
       ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
       try {
@@ -431,8 +457,10 @@ struct shapes_batch {
       ck(e, "cudaGraphInstantiate");
       g.epoch = graph_epoch;
       g.cfg = cfg;
+      g.shape = shape;
       ++graph_captures;
     }
+    g.used = ++graph_clock;
     ck(cudaGraphLaunch(g.exec, stream), "cudaGraphLaunch");
   }
 
@@ -861,18 +889,12 @@ struct shapes_batch {
    * Groups that have an SM to themselves take eight warps, of which four
    * prepare a narrow level while four solve one; groups that share one take
    * four. */
-  template <int P>
-  void launch_frontier(const Dev& d, const shapes_config& cfg, int smem, int split_limit) {
-    const int G = num_groups();
-    ck(cudaFuncSetAttribute(shapes::k_frontier<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFrontierSmem),
-       "cudaFuncSetAttribute");
-    launch_chained(chain(), shapes::k_frontier<P>, G, 32 * (P + 1), smem, stream, d, cfg.iterations, cfg.warm_start,
-                   cfg.external, cfg.accel_x, cfg.accel_y, cfg.dt, G, smem, spread_heavy ? num_sms() : 0, split_limit);
-  }
   static constexpr int kFrontierSmem = 220 * 1024;
-  void launch_groups(const Dev& d, const shapes_config& cfg) {
-    const int per_sm = (int)(((int64_t)num_groups() * handles_in_flight + num_sms() - 1) / num_sms());
-    const int P = !group_warps_auto ? group_warps : (per_sm <= 1 ? 8 : 4);
+  SolveShape solve_shape() {
+    const int per_sm = std::max(1, (int)(((int64_t)num_groups() * handles_in_flight + num_sms() - 1) / num_sms()));
+    SolveShape s{};
+    s.chained = chain();
+    s.warps = !group_warps_auto ? group_warps : (per_sm <= 1 ? 8 : 4);
     const int64_t contacts = (per_sm <= 1 ? 10LL : 5LL) * group_max_bodies / 2;
     const size_t want = shapes::frontier_bytes(group_max_bodies, contacts, true);
     /* four groups resident in place of three where their lists fit a quarter of the SM, the Lagrangians then in
@@ -880,12 +902,25 @@ struct shapes_batch {
     size_t most = kFrontierSmem / std::min(per_sm, 3);
     if (per_sm >= 4 && shapes::frontier_bytes(group_max_bodies, contacts, false) <= kFrontierSmem / 4)
       most = kFrontierSmem / 4;
-    const int smem = (int)std::min<size_t>(want, most);
-    const int split_limit = per_sm <= 1 ? 16 : 4;
-    if (P == 1) launch_frontier<1>(d, cfg, smem, split_limit);
-    else if (P == 2) launch_frontier<2>(d, cfg, smem, split_limit);
-    else if (P == 4) launch_frontier<4>(d, cfg, smem, split_limit);
-    else launch_frontier<8>(d, cfg, smem, split_limit);
+    s.smem = (int)std::min<size_t>(want, most);
+    s.split_limit = per_sm <= 1 ? 16 : 4;
+    return s;
+  }
+  template <int P>
+  void launch_frontier(const Dev& d, const shapes_config& cfg, const SolveShape& s) {
+    const int G = num_groups();
+    ck(cudaFuncSetAttribute(shapes::k_frontier<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kFrontierSmem),
+       "cudaFuncSetAttribute");
+    launch_chained(s.chained, shapes::k_frontier<P>, G, 32 * (P + 1), s.smem, stream, d, cfg.iterations, cfg.warm_start,
+                   cfg.external, cfg.accel_x, cfg.accel_y, cfg.dt, G, s.smem, spread_heavy ? num_sms() : 0,
+                   s.split_limit);
+  }
+  void launch_groups(const Dev& d, const shapes_config& cfg) {
+    const SolveShape s = solve_shape();
+    if (s.warps == 1) launch_frontier<1>(d, cfg, s);
+    else if (s.warps == 2) launch_frontier<2>(d, cfg, s);
+    else if (s.warps == 4) launch_frontier<4>(d, cfg, s);
+    else launch_frontier<8>(d, cfg, s);
   }
 
   /* Solve one large world: ranks of every contact on its bodies, then the
@@ -1305,10 +1340,7 @@ struct shapes_batch {
   }
 
   void prepare(const shapes_config& cfg, bool solve, int handles = 1) {
-    if (handles != handles_in_flight) { /* the launch shape of the group solve follows it */
-      handles_in_flight = handles;
-      invalidate_graphs();
-    }
+    handles_in_flight = handles; /* the launch shape follows it, and with that the graph of a step */
     ensure_items(solve ? cfg.iterations : 0);
     /* (re)build the solver groups before any device view of this call is
      * taken: make_groups reallocates the group arrays */
@@ -2836,6 +2868,12 @@ int shapes_batch_set_graphs(shapes_batch* b, int32_t enabled) {
     b->invalidate_graphs();
     return SHAPES_OK;
   });
+}
+
+int shapes_batch_get_graph_captures(shapes_batch* b, int64_t* captures) {
+  if (!b || !captures) return SHAPES_E_INVALID_ARG;
+  *captures = b->graph_captures;
+  return SHAPES_OK;
 }
 
 int shapes_batch_set_mlp(shapes_batch* b, const shapes_mlp* m) {
