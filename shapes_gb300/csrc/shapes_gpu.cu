@@ -2023,6 +2023,23 @@ static bool copy_finite(double* dst, const double* src, int n) {
   return !bad;
 }
 
+/* Makes a device current while it lives. */
+class OnDevice {
+ public:
+  explicit OnDevice(int device) {
+    ck(cudaGetDevice(&before_), "cudaGetDevice");
+    if (before_ != device) ck(cudaSetDevice(device), "cudaSetDevice");
+  }
+  OnDevice(const OnDevice&) = delete;
+  ~OnDevice() {
+    int now = before_;
+    if (cudaGetDevice(&now) == cudaSuccess && now != before_) cudaSetDevice(before_);
+  }
+
+ private:
+  int before_ = 0;
+};
+
 static dim3 copy10_grid(int n, int fields = 10) {
   const int64_t per_block = 256 * shapes::kCopy10PerThread;
   return dim3((unsigned)std::max<int64_t>(1, std::min<int64_t>((n + per_block - 1) / per_block, 1024)),
@@ -2108,6 +2125,7 @@ int shapes_batch_get_bodies(shapes_batch* b, shapes_bodies* out) {
       shapes::k_copy10<<<copy10_grid(b->N), 256, 0, b->stream>>>(p, b->N, nullptr);
       ck(cudaGetLastError(), "launch");
     } else if (b->N > 0 && b->N <= shapes_batch::kStageBodies && pageable10(bp)) {
+      const OnDevice on_device(b->device); /* a kernel, unlike a copy, needs its stream's device to be the current one */
       b->pinned_block();
       shapes::Ptr10 p{};
       for (int k = 0; k < 10; ++k) {
