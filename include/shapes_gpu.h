@@ -277,11 +277,12 @@ int shapes_batch_get_parallel_levels(shapes_batch* b, int32_t* enabled);
 int shapes_batch_set_spread_heavy(shapes_batch* b, int32_t enabled);
 int shapes_batch_get_spread_heavy(shapes_batch* b, int32_t* enabled);
 /* The packing in use (any pointer may be NULL); worlds_per_group is 0 when
- * groups are packed by body count (shapes_batch_get_group_target). */
+ * groups are packed by body count (shapes_batch_get_group_target), or
+ * automatically. */
 int shapes_batch_get_launch(shapes_batch* b, int32_t* worlds_per_group, int32_t* threads, int32_t* group_warps);
 /* The body count at which groups close (shapes_batch_set_launch; the
- * autotuner tries such packings for batches of uneven world sizes), 0 when
- * they are packed by world count. */
+ * autotuner tries such packings too), 0 when they are packed by world count or,
+ * with worlds_per_group 0 as well, automatically. */
 int shapes_batch_get_group_target(shapes_batch* b, int32_t* target_bodies);
 /* The order in which worlds are packed into groups: a permutation of
  * 0..n_worlds-1 (NULL = by body count, largest first, the default).  The
@@ -293,10 +294,14 @@ int shapes_batch_get_world_order(shapes_batch* b, int32_t* order);
 int shapes_batch_get_world_levels(shapes_batch* b, int32_t* levels);
 
 /* Autotuner for the solver packing: from the current state, times
- * `steps_per_trial` steps for each candidate (worlds per group x warps per
- * group, each in size and in level order) after one untimed
+ * `steps_per_trial` steps for each candidate (the packing that is set; the
+ * automatic one, as the body count and warps it comes to on this GPU; worlds per
+ * group x warps per group, each in size and in level order; body counts for
+ * uneven worlds) after one untimed
  * step, restores the state exactly after every trial, and keeps the fastest (read it back with
- * shapes_batch_get_launch).  The world state and cache are left exactly as they were; results
+ * shapes_batch_get_launch and shapes_batch_get_group_target).  The trials time
+ * the handle by itself, whatever others it is stepped beside later.
+ * The world state and cache are left exactly as they were; results
  * never depend on the packing.  Tune on a state that has contacts (e.g. after
  * the scene settles).  chosen_* may be NULL.  Allocates temporary device
  * memory for the saved state. */

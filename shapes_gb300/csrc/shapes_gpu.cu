@@ -807,6 +807,16 @@ struct shapes_batch {
    * above it four groups that close at kAutoGroupBodies bodies. */
   static constexpr int kLoneGroupBodies = 224;
   static constexpr int kAutoGroupBodies = 512;
+  int32_t auto_group_target() {
+    int64_t total = 0;
+    for (int w = 0; w < W; ++w) {
+      const int32_t n = h_world_body_off[w + 1] - h_world_body_off[w];
+      if (n < large_world_bodies) total += n;
+    }
+    const int64_t per_sm = total / num_sms();
+    return (int32_t)std::max<int64_t>(
+        1, per_sm <= kLoneGroupBodies ? per_sm : std::min<int64_t>(kAutoGroupBodies, per_sm / 4));
+  }
   void make_groups(int iterations) {
     if (stream) ck(cudaStreamSynchronize(stream), "sync"); /* no kernel may still read the old groups */
     invalidate_graphs();
@@ -824,13 +834,7 @@ struct shapes_batch {
     const bool by_worlds = worlds_per_group_override > 0;
     const int per_group = by_worlds ? std::min(shapes::kMaxGroupWorlds, worlds_per_group_override) : 0;
     int32_t target = by_worlds ? 0 : target_group_bodies;
-    if (!by_worlds && target <= 0) {
-      int64_t total = 0;
-      for (int w : order) total += h_world_body_off[w + 1] - h_world_body_off[w];
-      const int64_t per_sm = total / num_sms();
-      target = (int32_t)std::max<int64_t>(
-          1, per_sm <= kLoneGroupBodies ? per_sm : std::min<int64_t>(kAutoGroupBodies, per_sm / 4));
-    }
+    if (!by_worlds && target <= 0) target = auto_group_target();
     h_group_world_off.assign(1, 0);
     int32_t max_bodies = 0, bodies = 0, in_group = 0;
     for (int k = 0; k < n_small; ++k) {
@@ -2467,6 +2471,7 @@ int shapes_batch_autotune(shapes_batch* b, const shapes_config* cfg, int32_t ste
     void* scwo = keep(b->cwo[cache_buf0], sizeof(int32_t) * (W + 1));
     const int32_t wpg0 = b->worlds_per_group_override, thr0 = b->solve_threads, tgt0 = b->target_group_bodies;
     const int32_t gw0 = b->group_warps;
+    const bool auto0 = b->group_warps_auto, spread0 = b->spread_heavy;
     const std::vector<int32_t> order0 = b->world_order;
     const bool prof0 = b->profiling;
     b->profiling = false;
@@ -2499,8 +2504,19 @@ int shapes_batch_autotune(shapes_batch* b, const shapes_config* cfg, int32_t ste
     /* (worlds per group, warps per group, level order, heavy groups spread,
      * target bodies per group: when non-zero, groups close at that many bodies
      * instead of at a world count, so the largest worlds of a ragged batch get
-     * groups of their own) */
+     * groups of their own); ahead of them the packing that was set, kCurrent,
+     * and the automatic one, spelled out so that it can be read back and given
+     * to another handle */
+    constexpr int kCurrent = -1;
     std::vector<std::array<int, 5>> cands;
+    const bool was_auto = b->worlds_per_group_override <= 0 && b->target_group_bodies <= 0;
+    if (!was_auto || !b->group_warps_auto || b->spread_heavy || !order0.empty()) cands.push_back({kCurrent, 0, 0, 0, 0});
+    {
+      b->worlds_per_group_override = b->target_group_bodies = 0;
+      b->group_warps_auto = true;
+      b->make_groups(cfg->iterations);
+      cands.push_back({1, b->solve_shape().warps, 0, 0, b->auto_group_target()});
+    }
     auto add = [&](int wpg, int gw, int lo, int spread = 0, int target = 0) {
       const std::array<int, 5> c{wpg, gw, lo, spread, target};
       if (wpg >= 1 && wpg <= shapes::kMaxGroupWorlds && std::find(cands.begin(), cands.end(), c) == cands.end())
@@ -2526,9 +2542,18 @@ int shapes_batch_autotune(shapes_batch* b, const shapes_config* cfg, int32_t ste
     ck(cudaEventCreate(&e0), "event");
     ck(cudaEventCreate(&e1), "event");
     float best = 1e30f;
-    const bool auto0 = b->group_warps_auto, spread0 = b->spread_heavy;
-    std::array<int, 5> best_c{wpg0, gw0, -1, spread0 ? 1 : 0, tgt0};
+    std::array<int, 5> best_c{kCurrent, 0, 0, 0, 0};
     auto apply = [&](const std::array<int, 5>& c) {
+      if (c[0] == kCurrent) {
+        b->worlds_per_group_override = wpg0;
+        b->target_group_bodies = tgt0;
+        b->solve_threads = thr0;
+        b->group_warps = gw0;
+        b->group_warps_auto = auto0;
+        b->spread_heavy = spread0;
+        b->world_order = order0;
+        return;
+      }
       b->worlds_per_group_override = c[4] ? 0 : c[0];
       b->target_group_bodies = c[4];
       b->solve_threads = 32 * c[1];
@@ -2561,17 +2586,7 @@ int shapes_batch_autotune(shapes_batch* b, const shapes_config* cfg, int32_t ste
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     restore_state();
-    if (rc == SHAPES_OK && best_c[2] >= 0) {
-      apply(best_c);
-    } else {
-      b->worlds_per_group_override = wpg0;
-      b->target_group_bodies = tgt0;
-      b->solve_threads = thr0;
-      b->group_warps = gw0;
-      b->group_warps_auto = auto0;
-      b->spread_heavy = spread0;
-      b->world_order = order0;
-    }
+    apply(rc == SHAPES_OK ? best_c : std::array<int, 5>{kCurrent, 0, 0, 0, 0});
     b->invalidate_graphs();
     b->make_groups(cfg->iterations);
     ck(cudaStreamSynchronize(b->stream), "sync");
