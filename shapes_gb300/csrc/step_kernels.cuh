@@ -2121,8 +2121,15 @@ constexpr int kBuildThreads = 128;
  * in place of 110, 165 thousand: 39 in place of 51).  Few contacts gain nothing, and
  * the group solver's block, which may need all of an SM's shared memory, then cannot
  * take its place before k_build is done (401 boxes: 12 us a step lost); nor can
- * those of other handles in flight (eight handles of 30 thousand contacts: 1.3 %). */
-inline bool build_staged(long long contacts) { return contacts >= 65536; }
+ * those of other handles in flight (eight handles of 30 thousand contacts: 1.3 %).
+ * The line is drawn in the contacts that the buffers hold, because a captured step
+ * is launched before its contacts are counted: a new handle has room for 16 a body,
+ * so it lies at 4,096 bodies.  Whole steps of one handle, us, plain and staged, by
+ * the contacts they had: 2 to 50 thousand (17 handles of 2,048 to 34,018 bodies)
+ * within 1.1 % of each other either way; 35 thousand in 512 ragged columns 469 and
+ * 404, 76 thousand 566 and 474, 100 thousand 589 and 503, 200 thousand 685 and 677;
+ * 62 thousand in 512 worlds of 64 bodies, two sweeps, 209 and 219. */
+inline bool build_staged(long long contact_cap) { return contact_cap >= 65536; }
 
 /* The slot of every contact, so that k_build's threads take contacts rather
  * than slots: about half the slots of a settled pile are empty (separated
