@@ -353,11 +353,16 @@ int shapes_batch_set_sweep_prune(shapes_batch* b, int32_t min_bodies);
  * exactly, including which axis wins among equal or NaN depths). */
 int shapes_batch_set_narrowphase_lanes(shapes_batch* b, int32_t lanes);
 
-/* The order-preserving solve of large worlds waits for each update's
- * predecessors by polling completion counts; a lane that polls one dependency
- * more than `polls` times (default 2^22, restored by 0) makes the step return
+/* Solves wait on the device: the order-preserving solve of large worlds for each
+ * update's predecessors, the coloured one at the barriers between its colours, a
+ * group of small worlds for the dependency levels that one of its warps finds.
+ * A wait of more than `polls` polls (default, restored by 0: 2^22 in large
+ * worlds, 2^24 in groups) makes the step return
  * SHAPES_E_TIMEOUT, with the state of the steps that ran partly solved.  The
- * next run starts with the flag clear.  No counterpart in the reference. */
+ * next run starts with the flag clear.  The scans of a step, of
+ * shapes_batch_collide and of shapes_collide_noalloc wait too (for the sums of
+ * the blocks before them, at most 2^24 polls), as does the learned start's
+ * network; the limit does not change those.  No counterpart in the reference. */
 int shapes_batch_set_wait_limit(shapes_batch* b, int64_t polls);
 
 /* Per-stage device timing.  While enabled, CUDA events on the handle's stream

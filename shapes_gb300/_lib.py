@@ -515,8 +515,8 @@ class Batch:
         check(lib().shapes_batch_set_sweep_prune(self._h, int(min_bodies)), "shapes_batch_set_sweep_prune")
 
     def set_wait_limit(self, polls: int) -> None:
-        """Polls of one dependency before the large-world ordered solve gives up with
-        SHAPES_E_TIMEOUT (0 restores the default, 2**22)."""
+        """Polls of one wait before a solve gives up with SHAPES_E_TIMEOUT (0 restores
+        the defaults, 2**22 in large worlds and 2**24 in groups of small ones)."""
         check(lib().shapes_batch_set_wait_limit(self._h, int(polls)), "shapes_batch_set_wait_limit")
 
     def set_narrowphase_lanes(self, lanes: int) -> None:

@@ -312,10 +312,10 @@ __device__ __forceinline__ void frontier_build(const Dev& d, Lists& ls, Frontier
 }
 
 /* Waits until `ready` (a volatile read of the control block) holds; false when
- * the group gave up. */
+ * the group gave up, after poll_limit polls here or elsewhere. */
 template <class F>
-__device__ __forceinline__ bool frontier_wait(FrontierCtl& ctl, F&& ready) {
-  for (int n = 0; n < kFrontierPollLimit; ++n) {
+__device__ __forceinline__ bool frontier_wait(FrontierCtl& ctl, int poll_limit, F&& ready) {
+  for (int n = 0; n < poll_limit; ++n) {
     if (ready()) return true;
     if (ctl.err) return false;
     if (n > 64) __nanosleep(40);
@@ -331,7 +331,7 @@ __device__ __forceinline__ bool frontier_wait(FrontierCtl& ctl, F&& ready) {
  * full. */
 template <class Lists>
 __device__ __forceinline__ void frontier_schedule(const Dev& d, Lists& ls, FrontierCtl& ctl, int bodies,
-                                                  int iterations) {
+                                                  int iterations, int poll_limit) {
   const int lane = threadIdx.x & 31;
   const unsigned below = (1u << lane) - 1u;
   int begin = 0, end = ctl.n0, level = 0;
@@ -345,7 +345,7 @@ __device__ __forceinline__ void frontier_schedule(const Dev& d, Lists& ls, Front
     const bool room = ctl.done >= need && ls.space(end, ctl.solved) >= bodies;
     if (!__all_sync(0xffffffffu, room)) {
       const bool ok =
-          frontier_wait(ctl, [&]() { return ctl.done >= need && ls.space(end, ctl.solved) >= bodies; });
+          frontier_wait(ctl, poll_limit, [&]() { return ctl.done >= need && ls.space(end, ctl.solved) >= bodies; });
       if (!__all_sync(0xffffffffu, ok)) break;
     }
     int pos = end;
@@ -728,7 +728,7 @@ struct Deal {
  * else to L1. */
 template <int P, bool SM, class Lists>
 __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, const Lists& ls,
-                                               const BodyStore<SM>& bs, int split_limit) {
+                                               const BodyStore<SM>& bs, int split_limit, int poll_limit) {
   constexpr bool kStage = P == 8;
   constexpr int kTurn = P > 1 ? P / 2 : 1;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -751,7 +751,7 @@ __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, c
   for (int level = 0;; ++level) {
     if (wib == 0 && known <= level) {
       const bool ok = frontier_wait(
-          ctl, [&]() { return ld_acquire_cta(&ctl.published) > level || ld_acquire_cta(&ctl.total) >= 0; });
+          ctl, poll_limit, [&]() { return ld_acquire_cta(&ctl.published) > level || ld_acquire_cta(&ctl.total) >= 0; });
       if (!__all_sync(0xffffffffu, ok) && lane == 0) ctl.stop = level; /* every warp stops at the same level */
     }
     solver_barrier(32 * P); /* the level before is solved, this one is published */
@@ -806,7 +806,7 @@ __device__ __forceinline__ void frontier_solve(const Dev& d, FrontierCtl& ctl, c
 template <int P>
 __global__ void __launch_bounds__(32 * (P + 1), P == 8 ? 1 : (P == 4 ? 4 : 6))
     k_frontier(Dev d, int iterations, int warm_start, int external, double ax, double ay, double dt, int n_groups,
-               int smem_bytes, int heavy_first, int split_limit) {
+               int smem_bytes, int heavy_first, int split_limit, int poll_limit) {
   chained_wait(); /* the next kernel's blocks would hold places through the whole solve, that other streams can use */
   extern __shared__ __align__(16) unsigned char s_dyn[];
   __shared__ FrontierCtl ctl;
@@ -921,13 +921,13 @@ __global__ void __launch_bounds__(32 * (P + 1), P == 8 ? 1 : (P == 4 ? 4 : 6))
       atomicAdd(&d.counters[kCntHits], h);
       atomicAdd(&d.counters[kCntItems], h + (unsigned long long)iterations * NC);
     }
-    if (fits) frontier_schedule(d, ls, ctl, NB, iterations);
-    else frontier_schedule(d, lg, ctl, NB, iterations);
+    if (fits) frontier_schedule(d, ls, ctl, NB, iterations, poll_limit);
+    else frontier_schedule(d, lg, ctl, NB, iterations, poll_limit);
     if (d.phase_clock && tid == 32 * P) d.phase_clock[8 * grp + 2] = clock64();
     return;
   }
-  if (fits) frontier_solve<P>(d, ctl, ls, BodyStore<true>{&d, vel, lam, lam_local}, split_limit);
-  else frontier_solve<P>(d, ctl, lg, BodyStore<false>{&d, nullptr, lam, false}, split_limit);
+  if (fits) frontier_solve<P>(d, ctl, ls, BodyStore<true>{&d, vel, lam, lam_local}, split_limit, poll_limit);
+  else frontier_solve<P>(d, ctl, lg, BodyStore<false>{&d, nullptr, lam, false}, split_limit, poll_limit);
   if (ctl.err && tid == 0) atomicOr(&d.counters[kCntSolveErr], 1ull);
   {
     int k = 0;

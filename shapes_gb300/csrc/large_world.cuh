@@ -268,7 +268,7 @@ __global__ void k_lw_end(Dev d, LW w) {
  * velocities and fences between them; 3.07 ms so.  Rows in flight (rows an SM:
  * time): 4: 8.1 ms, 16: 3.83, 32: 3.32, 64: 3.07, 64 in one block: 3.29. */
 constexpr int kOrderedThreads = 256;
-constexpr long long kPollLimit = 1ll << 22; /* polls of one dependency before giving up */
+constexpr long long kPollLimit = 1ll << 22; /* polls of one dependency, or at one barrier, before giving up */
 constexpr int kOrderedBlocksPerSM = 2;
 
 __global__ void __launch_bounds__(kOrderedThreads) k_lw_ordered(Dev d, LW w, int iterations, int warm_start,
@@ -392,19 +392,20 @@ __device__ __forceinline__ uint32_t lw_prio(int k) {
 }
 
 /* A barrier over all blocks of a cooperative launch, counting up on *arrived.
- * False when it gave up (it never does while every block runs). */
-__device__ __forceinline__ bool grid_barrier(unsigned long long* arrived, unsigned long long& target) {
+ * False when it gave up (with the default limit it never does while every block runs). */
+__device__ __forceinline__ bool grid_barrier(unsigned long long* arrived, unsigned long long& target,
+                                             int poll_limit) {
   __syncthreads();
   target += gridDim.x;
   bool ok = true;
   if (threadIdx.x == 0) {
     __threadfence();
     asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(arrived) : "memory");
-    for (long long n = 0;;) {
+    for (int n = 0;;) {
       unsigned long long now;
       asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(arrived) : "memory");
       if (now >= target) break;
-      if (++n > kPollLimit) {
+      if (++n > poll_limit) {
         ok = false;
         break;
       }
@@ -497,13 +498,14 @@ constexpr int kColourThreads = 512;
 constexpr int kColourBlocksPerSM = 1;
 
 __global__ void __launch_bounds__(kColourThreads, kColourBlocksPerSM)
-    k_lw_coloured(Dev d, LW w, int iterations, int warm_start, int external, double ax, double ay, double dt) {
+    k_lw_coloured(Dev d, LW w, int iterations, int warm_start, int external, double ax, double ay, double dt,
+                  int poll_limit) {
   if (d.counters[kCntOverflow]) return;
   lw_range(w);
   const int stride = gridDim.x * blockDim.x, t0 = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long target = 0;
   auto barrier = [&]() {
-    const bool ok = grid_barrier(&w.ctl[0], target);
+    const bool ok = grid_barrier(&w.ctl[0], target, poll_limit);
     if (!ok && threadIdx.x == 0) atomicExch(&w.ctl[1], 1ull);
     return ok;
   };
@@ -527,7 +529,7 @@ __global__ void __launch_bounds__(kColourThreads, kColourBlocksPerSM)
       coloured[i] = k >= w.nc;
       if (!coloured[i]) search[i].begin(d, w, k);
     }
-    long long idle = 0;
+    int idle = 0;
     for (bool left = true; left;) {
       left = false;
       bool any = false;
@@ -553,7 +555,7 @@ __global__ void __launch_bounds__(kColourThreads, kColourBlocksPerSM)
         }
       }
       idle = any ? 0 : idle + 1;
-      if (idle > kPollLimit) {
+      if (idle > poll_limit) {
         atomicExch(&w.ctl[1], 1ull);
         break;
       }

@@ -222,7 +222,10 @@ struct shapes_batch {
   /* sweep and prune for the small bodies of large grid worlds (incremental pairs off) */
   int32_t sap_min_bodies = 0; /* 0: off */
   int32_t np_lanes = 1;       /* lanes per pair in the narrowphase (1: k_narrowphase) */
-  long long lw_poll_limit = shapes::kPollLimit; /* ordered large-world solve: polls of one dependency */
+  long long poll_limit = 0; /* polls of a wait in a solve before it gives up; 0: each kernel's own limit */
+  int poll_limit_or(long long own) const {
+    return (int)std::min<long long>(poll_limit > 0 ? poll_limit : own, INT32_MAX);
+  }
   bool any_sap = false;
   int32_t n_sap_buckets = 0;
   uint8_t* world_sap = nullptr;
@@ -953,7 +956,7 @@ struct shapes_batch {
        "cudaFuncSetAttribute");
     launch_chained(s.chained, shapes::k_frontier<P>, G, 32 * (P + 1), s.smem, stream, d, cfg.iterations, cfg.warm_start,
                    cfg.external, cfg.accel_x, cfg.accel_y, cfg.dt, G, s.smem, spread_heavy ? num_sms() : 0,
-                   s.split_limit);
+                   s.split_limit, poll_limit_or(shapes::kFrontierPollLimit));
   }
   void launch_groups(const Dev& d, const shapes_config& cfg) {
     const SolveShape s = solve_shape();
@@ -1004,7 +1007,7 @@ struct shapes_batch {
         shapes::k_lw_begin<<<grid_for(2LL * cap, 256), 256, 0, stream>>>(d, w, cfg.external, cfg.accel_x, cfg.accel_y,
                                                                          cfg.dt);
         shapes::k_lw_ordered<<<kSMs * shapes::kOrderedBlocksPerSM, shapes::kOrderedThreads, 0, stream>>>(
-            d, w, cfg.iterations, cfg.warm_start, lw_poll_limit);
+            d, w, cfg.iterations, cfg.warm_start, poll_limit > 0 ? poll_limit : shapes::kPollLimit);
         shapes::k_lw_end<<<grid_for(2LL * cap, 256), 256, 0, stream>>>(d, w);
         return;
       }
@@ -1018,7 +1021,7 @@ struct shapes_batch {
       lc.attrs = at;
       lc.numAttrs = 1;
       ck(cudaLaunchKernelEx(&lc, shapes::k_lw_coloured, d, w, cfg.iterations, cfg.warm_start, cfg.external, cfg.accel_x,
-                            cfg.accel_y, cfg.dt),
+                            cfg.accel_y, cfg.dt, poll_limit_or(shapes::kPollLimit)),
          "k_lw_coloured");
     });
   }
@@ -3091,7 +3094,7 @@ int shapes_batch_set_wait_limit(shapes_batch* b, int64_t polls) {
   if (!b || polls < 0) return SHAPES_E_INVALID_ARG;
   return guarded([&]() -> int {
     ck(cudaStreamSynchronize(b->stream), "sync");
-    b->lw_poll_limit = polls ? (long long)polls : shapes::kPollLimit;
+    b->poll_limit = (long long)polls;
     b->invalidate_graphs();
     return SHAPES_OK;
   });
