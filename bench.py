@@ -315,7 +315,7 @@ def run_reference(args, rank, world):
 
 INCREMENTAL_PAIRS = True  # --no-incremental turns the fat-box pair lists off
 SWEEP_PRUNE = 0  # --sweep-prune N: grid worlds of N bodies or more pair by sweep and prune (incremental off)
-NP_DESC = {1: "SAT one thread per pair (pairs ordered by vertex counts)", 32: "SAT one warp per pair, shuffle-reduced "
+NP_DESC = {1: "SAT one thread per pair behind a binary32 filter", 32: "SAT one warp per pair, shuffle-reduced "
            "axis search"}
 NP_DESC.update({k: f"SAT {k} lanes per pair, shuffle-reduced axis search" for k in (2, 4, 8, 16)})
 NP_LANES = 1  # --np-lanes L: lanes per pair in the narrowphase (1 = a thread per pair, 32 = a warp per pair)

@@ -137,7 +137,8 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
  * Measured on GB300: 4.8e11 of these per second against 5.3e11 hardware
  * products, on a separate pipe: independent products split between the two
  * pipes go almost twice as fast, a dependency chain loses (the sequence is about
- * 30 instructions long).  No kernel of the step uses it now.  Fast path: both operands normal with biased exponents in
+ * 30 instructions long).  The pose takes one product of each vertex coordinate from
+ * it, and the narrowphase's full axis search one of each projection.  Fast path: both operands normal with biased exponents in
  * [512, 1534] (the product is then normal, or overflows to infinity exactly
  * as IEEE rounding does), or one operand a zero and the other finite (a
  * signed zero).  The 106-bit product of the 53-bit significands comes from

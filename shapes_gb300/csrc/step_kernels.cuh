@@ -2314,18 +2314,6 @@ __device__ __forceinline__ double row_dot(const double r[4], const double v[6]) 
   return s + r[3] * v[5];
 }
 
-/* applyLagrangian2 (Constraint.hs:197-204): v += (J * lambda) * invMass; the
- * two bodies' linear products differ only in sign and are computed once. */
-__device__ __forceinline__ void row_apply(const double r[4], double l, double v[6], const double im[4]) {
-  const double px = r[0] * l, py = r[1] * l;
-  v[0] = v[0] + (-px) * im[0];
-  v[1] = v[1] + (-py) * im[0];
-  v[2] = v[2] + (r[2] * l) * im[1];
-  v[3] = v[3] + px * im[2];
-  v[4] = v[4] + py * im[2];
-  v[5] = v[5] + (r[3] * l) * im[3];
-}
-
 /* The restitution term (bounceB, Restitution.hs:34-51): min 0 (e * (closing
  * velocity . n)), closing velocity ((-va + (-wa) z x ra) + vb) + wb z x rb. */
 __device__ __forceinline__ double bounce_term(const Con* con, const double v[6]) {
